@@ -200,63 +200,6 @@ extern "C" int add_rmsnorm(float* resid, const void* delta, int delta_dtype, con
 #undef NORM_CASE
 }
 
-// ----------------------------------------------------------------------------- float32 GEMM
-// y[M, N] = x[M, K] * w[N, K]^T, plain FFMA.  Each output element is one accumulator
-// running over k = 0..K-1 in order, so its value does not depend on M or on the tile
-// it falls in.  No tensor cores, no TF32.
-#define GB 64
-#define GK 16
-__global__ void __launch_bounds__(256) gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w,
-                                                       float* __restrict__ y, int M, int N, int K) {
-    __shared__ float xs[GK][GB + 4];
-    __shared__ float ws[GK][GB + 4];
-    pdl_launch_dependents();
-    pdl_wait();
-    int m0 = blockIdx.y * GB, n0 = blockIdx.x * GB;
-    int tx = threadIdx.x % 16, ty = threadIdx.x / 16;  // 16 x 16 threads, 4 x 4 outputs each
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += GK) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            int idx = threadIdx.x + i * 256;  // 0..1023 over a 64 x 16 tile
-            int r = idx / GK, c = idx % GK;
-            int gm = m0 + r, gn = n0 + r, gk = k0 + c;
-            xs[c][r] = (gm < M && gk < K) ? x[(size_t)gm * K + gk] : 0.f;
-            ws[c][r] = (gn < N && gk < K) ? w[(size_t)gn * K + gk] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GK; ++kk) {
-            float a[4], b[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = xs[kk][ty * 4 + i];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = ws[kk][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        int gm = m0 + ty * 4 + i;
-        if (gm >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            int gn = n0 + tx * 4 + j;
-            if (gn < N) y[(size_t)gm * N + gn] = acc[i][j];
-        }
-    }
-}
-
-extern "C" int gemm_f32(const float* x, const float* w, float* y, int M, int N, int K, cudaStream_t stream) {
-    if (M <= 0 || N <= 0) return 0;
-    dim3 grid((N + GB - 1) / GB, (M + GB - 1) / GB);
-    return (int)launch_kernel(gemm_f32_kernel, grid, 256, 0, stream, x, w, y, M, N, K);
-}
-
 // ----------------------------------------------------------------------------- rotation + cache write
 // One row of the fused projection per token: [q (nq heads) | k (nkv heads) | v (nkv heads)].
 // Rotates q in place and writes rotated k and plain v to the token's slot of its page.

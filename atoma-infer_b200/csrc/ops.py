@@ -24,7 +24,7 @@ MAX_GROUPS = 8
 STATUS_WORDS = 8
 SKINNY_MAX_ROWS = 16  # bfloat16 linears with at most this many rows stream the weights
 
-CORE_SOURCES = ["kernels/core.cu", "kernels/layer_ops.cu", "kernels/linear_bf16.cu", "kernels/linear_stream.cu", "kernels/sampling.cu"]
+CORE_SOURCES = ["kernels/core.cu", "kernels/gemm_f32.cu", "kernels/layer_ops.cu", "kernels/linear_bf16.cu", "kernels/linear_stream.cu", "kernels/sampling.cu"]
 ATTENTION_SOURCES = ["kernels/attention_bf16.cu"]
 GEMM_SOURCES = ["kernels/gemm_tcgen05.cu"]
 ATTENTION_TC_SOURCES = ["kernels/attention_tcgen05.cu"]

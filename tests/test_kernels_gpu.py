@@ -111,6 +111,26 @@ def test_float32_gemm_is_true_float32_and_row_independent(rts):
     assert torch.equal(one[0], y[11])  # a row's bits do not depend on its neighbours
 
 
+@pytest.mark.parametrize("M,N,Kd", [(1, 1, 1), (17, 130, 33), (65, 129, 100), (129, 260, 24), (33, 2056, 120), (128, 128, 16), (130, 132, 2048)])
+def test_float32_gemm_gives_the_same_bits_with_every_tile(rts, M, N, Kd):
+    """Every tile size, at row, column and k counts that fill tiles and leave remainders, with rows that start on 16 bytes and
+    not: one accumulator over k in order, so the bits are those of any other tile."""
+    rt = rts["float32"]
+    g = torch.Generator().manual_seed(M + N + Kd)
+    x, w = torch.randn(M, Kd, generator=g), torch.randn(N, Kd, generator=g)
+    want = x.double() @ w.double().T
+    ys = []
+    try:
+        for tile in (1, 2, 3, 4, 5, 0):
+            rt.ops.lib.gemm_f32_set_tile(tile)
+            ys.append(rt.ops.linear(x.to(rt.device), w.to(rt.device)))
+    finally:
+        rt.ops.lib.gemm_f32_set_tile(0)
+    # at most Kd roundings of partial sums of Kd products of unit variance: a random walk, far below sqrt(Kd) * Kd * 2^-24
+    assert (ys[0].double().cpu() - want).abs().max() < 2 ** -24 * Kd * math.sqrt(Kd) + 1e-6
+    assert all(torch.equal(y, ys[0]) for y in ys[1:])
+
+
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16, 17, 40])
 @pytest.mark.parametrize("N,Kd", [(48, 64), (3000, 2048), (1001, 200)])
 def test_bfloat16_linear_all_row_counts(rts, M, N, Kd):
