@@ -5,6 +5,7 @@
 //  * the norm per head behind both, with a weight per channel of every head, a gate, and (for the memory) the division by
 //    max(|n . q|, exp(-m)) + 1e-6.
 // Projections are stored as float32 or bfloat16; gates, states, norms and everything between are float32.
+#include "chunk_scan.cuh"
 #include "matrix_scan.cuh"
 
 int g_use_pdl = 1;
@@ -49,16 +50,43 @@ extern "C" int memory_scan(const void* q, long long q_stride, const void* k, lon
     return run_matrix_scan<SCAN_MEMORY>(a, stream);
 }
 
+// The same for bfloat16 prompts as matrix products over chunks of CHUNK tokens (chunk_scan.cuh); log_a float32 [T, heads], the logs of
+// the gates' decays.  memory_chunk_scan_takes: whether these sizes and addresses are served.
+extern "C" size_t memory_chunk_scan_scratch_floats(int heads, int N, int P, int max_chunks) {
+    return chunk_scratch_floats<CHUNK_MEMORY>(heads, N, P, max_chunks);
+}
+
+extern "C" int memory_chunk_scan_takes(const void* q, long long q_stride, const void* k, long long k_stride, const void* v,
+                                       long long v_stride, const float* o, int N, int P) {
+    return chunk_scan_takes(q, k, v, q_stride, k_stride, v_stride, o, N, P);
+}
+
+extern "C" int memory_chunk_scan(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
+                                 const float* gates, const float* log_a, float q_scale, float* state, float* n_state,
+                                 long long slot_stride, float* o, float* nq, const int* meta, const int* cu_tokens, const int* slots,
+                                 int S, int heads, int N, int P, int max_chunks, float* scratch, cudaStream_t stream) {
+    ChunkArgs a = {};
+    a.q = (const __nv_bfloat16*)q, a.k = (const __nv_bfloat16*)k, a.v = (const __nv_bfloat16*)v;
+    a.q_stride = q_stride, a.k_stride = k_stride, a.v_stride = v_stride;
+    a.share = 1;
+    a.gates = gates, a.log_a = log_a, a.q_scale = q_scale;
+    a.state = state, a.n_state = n_state, a.slot_stride = slot_stride, a.o = o, a.nq = nq;
+    a.meta = meta, a.cu_tokens = cu_tokens, a.slots = slots;
+    a.S = S, a.heads = heads, a.N = N, a.P = P, a.max_chunks = max_chunks, a.scratch = scratch;
+    return chunk_scan<CHUNK_MEMORY>(a, stream);
+}
+
 // ----------------------------------------------------------------------------- exponential gates
 // logits float32 [T, 2 * heads], the input gates' first; bias float32 [2 * heads].  Per head: i = cap * tanh((x_i + b_i) / cap),
 // f = log sigmoid(cap * tanh((x_f + b_f) / cap)); m_t = max(f_t + m_(t-1), i_t) from the request's kept m (0 at its start);
-// gates[t, h] = (exp(f_t + m_(t-1) - m_t), exp(i_t - m_t)); floor[t, h] = exp(-m_t); the last m goes back to the slot.
+// gates[t, h] = (exp(f_t + m_(t-1) - m_t), exp(i_t - m_t)); floor[t, h] = exp(-m_t); the last m goes back to the slot.  With `log_a`
+// the first gate's log is left there too (float32 [T, heads]).
 // One block per (head, entry).  A token maps m to max(m + F, I) with F = f, I = i; such maps compose to (F1 + F2,
 // max(I1 + F2, I2)), so a block's tokens are taken as an inclusive scan over lanes, then over warps in order.
 __global__ void __launch_bounds__(256)
 memory_gates_kernel(const float* __restrict__ logits, const float* __restrict__ bias, float cap, float* __restrict__ m_state,
-                    long long slot_stride, float* __restrict__ gates, float* __restrict__ floor_out, const int* __restrict__ meta,
-                    const int* __restrict__ cu_tokens, const int* __restrict__ slots, int heads) {
+                    long long slot_stride, float* __restrict__ gates, float* __restrict__ floor_out, float* __restrict__ log_a,
+                    const int* __restrict__ meta, const int* __restrict__ cu_tokens, const int* __restrict__ slots, int heads) {
     __shared__ float wf[8], wi[8], s_m;
     const int h = blockIdx.x, e = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
     pdl_launch_dependents();
@@ -97,6 +125,7 @@ memory_gates_kernel(const float* __restrict__ logits, const float* __restrict__ 
         if (in) {
             float2* dst = reinterpret_cast<float2*>(gates) + (size_t)t * heads + h;
             *dst = make_float2(expf(f + m_prev - m_t), expf(i - m_t));
+            if (log_a) log_a[(size_t)t * heads + h] = f + m_prev - m_t;
             floor_out[(size_t)t * heads + h] = expf(-m_t);
         }
         if (t == end - 1 || (in && threadIdx.x == blockDim.x - 1)) s_m = m_t;
@@ -107,12 +136,12 @@ memory_gates_kernel(const float* __restrict__ logits, const float* __restrict__ 
 }
 
 extern "C" int memory_gates(const float* logits, const float* bias, float cap, float* m_state, long long slot_stride, float* gates,
-                            float* floor_out, const int* meta, const int* cu_tokens, const int* slots, int S, int heads, int longest,
+                            float* floor_out, float* log_a, const int* meta, const int* cu_tokens, const int* slots, int S, int heads, int longest,
                             cudaStream_t stream) {
     if (S <= 0) return 0;
     if (cap <= 0.f) return (int)cudaErrorInvalidValue;
     return (int)launch_kernel(memory_gates_kernel, dim3(heads, S), longest > 32 ? 256 : 32, 0, stream, logits, bias, cap, m_state,
-                              slot_stride, gates, floor_out, meta, cu_tokens, slots, heads);
+                              slot_stride, gates, floor_out, log_a, meta, cu_tokens, slots, heads);
 }
 
 // ----------------------------------------------------------------------------- norm per head, a weight per channel, gate

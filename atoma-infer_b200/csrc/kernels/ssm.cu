@@ -2,7 +2,7 @@
 // front of the recurrence, the recurrence itself (sequential over a request's tokens, or cut into chunks of time that
 // run side by side), and the gated norm in equal parts behind it.  Storage is float32 or bfloat16; the recurrence,
 // its step sizes and decays, the gate and the norm are float32 always.
-#include "common.cuh"
+#include "chunk_scan.cuh"
 
 // ----------------------------------------------------------------------------- causal convolution, bias, activation
 // y[t, c] = act(bias[c] + sum_j w[j, c] * u[t - taps + 1 + j, c]) over the rows of each request, zeros before its
@@ -431,6 +431,36 @@ extern "C" int ssm_scan(const void* xbc, int dtype, int xbc_stride, const void* 
     if (err) return err;
     return dtype == DT_F32 ? SCAN_PASS(float, 3, max_chunks) : SCAN_PASS(__nv_bfloat16, 3, max_chunks);
 #undef SCAN_PASS
+}
+
+// The same for bfloat16 prompts as matrix products over chunks of CHUNK tokens (chunk_scan.cuh).  ssm_chunk_scan_takes: whether these
+// sizes and addresses are served.
+extern "C" size_t ssm_chunk_scan_scratch_floats(int heads, int P, int N, int max_chunks) {
+    return chunk_scratch_floats<CHUNK_SSM>(heads, N, P, max_chunks);
+}
+
+extern "C" int ssm_chunk_scan_takes(const void* xbc, int xbc_stride, const float* y, int heads, int P, int N, int groups) {
+    const __nv_bfloat16 *x = (const __nv_bfloat16*)xbc, *B = x + (size_t)heads * P, *C = B + (size_t)groups * N;
+    return chunk_scan_takes(C, B, x, xbc_stride, xbc_stride, xbc_stride, y, N, P);
+}
+
+extern "C" int ssm_chunk_scan(const void* xbc, int xbc_stride, const void* dt, long long dt_stride, const float* dt_bias,
+                              const float* a_log, const float* d_skip, float* state, long long slot_stride, float* y, const int* meta,
+                              const int* cu_tokens, const int* slots, int S, int heads, int P, int N, int groups, int max_chunks,
+                              float* scratch, cudaStream_t stream) {
+    if (heads <= 0 || groups <= 0 || heads % groups) return (int)cudaErrorInvalidValue;
+    ChunkArgs a = {};
+    a.v = (const __nv_bfloat16*)xbc;
+    a.k = a.v + (size_t)heads * P;
+    a.q = a.k + (size_t)groups * N;
+    a.q_stride = a.k_stride = a.v_stride = xbc_stride;
+    a.share = heads / groups;
+    a.dt = (const __nv_bfloat16*)dt, a.dt_stride = dt_stride, a.dt_bias = dt_bias, a.a_log = a_log, a.d_skip = d_skip;
+    a.q_scale = 1.f;
+    a.state = state, a.slot_stride = slot_stride, a.o = y;
+    a.meta = meta, a.cu_tokens = cu_tokens, a.slots = slots;
+    a.S = S, a.heads = heads, a.N = N, a.P = P, a.max_chunks = max_chunks, a.scratch = scratch;
+    return chunk_scan<CHUNK_SSM>(a, stream);
 }
 
 // ----------------------------------------------------------------------------- gate, then the norm in equal parts

@@ -640,6 +640,7 @@ class CudaOps:
         if lib is None:
             lib = self._mixer_lib = build.load_library("mixers", MIXER_SOURCES, cuda=True)
             lib.ssm_scan_scratch_floats.restype = ctypes.c_size_t
+            lib.ssm_chunk_scan_scratch_floats.restype = ctypes.c_size_t
             lib.kernels_set_pdl(int(self.pdl))
         return lib
 
@@ -712,6 +713,21 @@ class CudaOps:
     SCAN_CHUNK = 64        # tokens of a chunk when a long portion's recurrence is cut into chunks that run side by side
     SCAN_CHUNK_FROM = 128  # ... which happens from this many tokens of the step's longest entry on
 
+    MATRIX_SCAN_CHUNK = 128
+    matrix_scan = True  # (a test lever)
+
+    def _matrix_scan_chunks(self, ctx) -> int:
+        """bfloat16 prompts whose state decays by one number per head and token run the recurrence as matrix products over
+        chunks of 128 tokens (kernels/chunk_scan.cuh) where the other kernel would cut it into chunks of time too: from
+        SCAN_CHUNK_FROM tokens of the step's longest entry on.  Measured there, one prompt, 64 heads of 128 x 64: 200 tokens 25
+        against 90 us, 2,048 tokens 108 against 471.  Shorter ones stay in order: they need no scratch memory, which a
+        step of many short entries would otherwise ask for (40 tokens: 19 against 28 us).  Above 256 chunks the other kernel's
+        scratch stops growing and this one's would not.  Returns at least as many chunks as all entries have together, or 0."""
+        longest = ctx.max_tokens_per_entry
+        if not self.matrix_scan or not self.SCAN_CHUNK_FROM <= longest <= 256 * self.MATRIX_SCAN_CHUNK:
+            return 0
+        return ctx.T // self.MATRIX_SCAN_CHUNK + ctx.S
+
     def ssm_scan(self, xbc, dt, dt_bias, a_log, d_skip, state, ctx, y, *, heads: int, head_dim: int, nstate: int, groups: int):
         """The state-space recurrence of every entry's tokens: rows of ``xbc`` are [x | B | C], ``dt`` a slice of wider
         rows (softplus(dt + dt_bias) is taken here), ``state`` float32 [slots, heads, nstate, head_dim] (read and
@@ -720,6 +736,14 @@ class CudaOps:
             raise KernelError("a recurrence state is float32 [slots, heads, rows, columns] with contiguous slots")
         dp, ds = self._rows(dt, "ssm_scan")
         lib = self._mixers()
+        chunks = self._matrix_scan_chunks(ctx) if xbc.dtype == torch.bfloat16 else 0
+        if chunks and lib.ssm_chunk_scan_takes(_p(xbc), xbc.stride(0), _p(y), heads, head_dim, nstate, groups):
+            scratch = torch.empty(lib.ssm_chunk_scan_scratch_floats(heads, head_dim, nstate, chunks), dtype=torch.float32, device=y.device)
+            self._check(lib.ssm_chunk_scan(_p(xbc), xbc.stride(0), dp, ds, _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
+                                           ctypes.c_longlong(state.stride(0)), _p(y), _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots),
+                                           ctx.S, heads, head_dim, nstate, groups, chunks, _p(scratch), self._stream()), "ssm_chunk_scan")
+            self.launches += 2
+            return
         longest = ctx.max_tokens_per_entry
         chunk = self.SCAN_CHUNK if longest >= self.SCAN_CHUNK_FROM else 0
         while chunk and longest // chunk > 256:
@@ -1156,6 +1180,7 @@ class CudaOps:
             lib = self._matrix_recurrent_lib = build.load_library("matrix_recurrent", MATRIX_RECURRENT_SOURCES, cuda=True)
             lib.bonus_scan_scratch_floats.restype = ctypes.c_size_t
             lib.memory_scan_scratch_floats.restype = ctypes.c_size_t
+            lib.memory_chunk_scan_scratch_floats.restype = ctypes.c_size_t
             lib.kernels_set_pdl(int(self.pdl))
         return lib
 
@@ -1201,9 +1226,20 @@ class CudaOps:
             raise KernelError("memory_scan: two gates per head")
         (qp, qs), (kp, ks), (vp, vs) = (self._rows(t, "memory_scan") for t in (q, k, v))
         gates = torch.empty((ctx.T, heads, 2), dtype=torch.float32, device=o.device)
-        self._check(lib.memory_gates(_p(logits), _p(bias), ctypes.c_float(cap), _p(m_state), slot_stride, _p(gates), _p(floor),
+        chunked = bool(q.dtype == torch.bfloat16 and self._matrix_scan_chunks(ctx)
+                       and lib.memory_chunk_scan_takes(qp, qs, kp, ks, vp, vs, _p(o), dim, vdim))
+        log_a = torch.empty((ctx.T, heads), dtype=torch.float32, device=o.device) if chunked else None
+        self._check(lib.memory_gates(_p(logits), _p(bias), ctypes.c_float(cap), _p(m_state), slot_stride, _p(gates), _p(floor), _p(log_a),
                                      _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, heads, ctx.max_tokens_per_entry,
                                      self._stream()), "memory_gates")
+        if chunked:
+            chunks = self._matrix_scan_chunks(ctx)
+            scratch = torch.empty(lib.memory_chunk_scan_scratch_floats(heads, dim, vdim, chunks), dtype=torch.float32, device=o.device)
+            self._check(lib.memory_chunk_scan(qp, qs, kp, ks, vp, vs, _p(gates), _p(log_a), ctypes.c_float(q_scale), _p(state), _p(n_state),
+                                              slot_stride, _p(o), _p(nq), _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, heads,
+                                              dim, vdim, chunks, _p(scratch), self._stream()), "memory_chunk_scan")
+            self.launches += 2
+            return
         chunk, chunks = self._scan_chunks(ctx)
         scratch = (torch.empty(lib.memory_scan_scratch_floats(ctx.S, heads, dim, vdim, chunks), dtype=torch.float32, device=o.device)
                    if chunk else None)

@@ -1,0 +1,136 @@
+"""The scans that run as matrix products over chunks of 128 tokens, at the sizes where that can go wrong: rows of state that fill a
+tile partly, columns that leave a part of a block of 64, chunks of 1, 16, 17, 127 and 128 tokens, entries with one chunk beside
+entries with several, slots that start on any float.  Against a float64 restatement."""
+import pytest
+import torch
+
+import kernel_utils as K
+
+pytestmark = pytest.mark.gpu
+LENGTHS = [(128,), (129, 1, 16), (127, 17, 256, 300, 2)]
+# Sums of a few hundred float32 terms of mixed sign, each good to 2^-24, beside states of the same size: a few 1e-6 of the
+# largest value (the bound for the scan in order is 2e-5).
+TOL = 1e-5
+
+
+@pytest.fixture(scope="module")
+def rt():
+    from atoma_infer_b200.engine.runtime import make_runtime
+
+    return make_runtime("bfloat16", "cuda:0")
+
+
+def context(rt, lengths):
+    ctx, _ = K.make_context(rt, [(3, n) for n in lengths], 16, [[1] * (-(-(n + 3) // 16)) for n in lengths])
+    ctx.state_slots.copy_(torch.tensor([len(lengths) - 1 - k for k in range(len(lengths))], dtype=torch.int32))  # not the order of the entries
+    return ctx
+
+
+def scan(q, k, v, log_a, b, S):
+    """q, k [T, H, N], v [T, H, P], log_a and b [T, H], S [H, N, P], all float64: the outputs and the last state."""
+    out = torch.empty_like(v)
+    for t in range(q.shape[0]):
+        S = torch.exp(log_a[t])[:, None, None] * S + (b[t][:, None] * k[t])[:, :, None] * v[t][:, None, :]
+        out[t] = torch.einsum("hnp,hn->hp", S, q[t])
+    return out, S
+
+
+def err(got, want):
+    return ((got.double().cpu() - want).abs().max() / want.abs().max()).item()
+
+
+def both(rt, run):
+    """``run()`` on the chunked kernels (three launches) and on the one that goes token by token."""
+    got = []
+    for flag in (True, False):
+        rt.ops.matrix_scan = flag
+        try:
+            got.append(run())
+        finally:
+            rt.ops.matrix_scan = type(rt.ops).matrix_scan
+    rt.ops.check_status()
+    return got
+
+
+@pytest.mark.parametrize("lengths", LENGTHS)
+@pytest.mark.parametrize("heads,P,N,G", [(2, 64, 128, 1), (4, 8, 8, 2), (2, 72, 40, 2), (3, 136, 64, 3), (2, 128, 120, 1)])
+def test_state_space_in_matrix_chunks(rt, lengths, heads, P, N, G):
+    g = torch.Generator().manual_seed(heads * P + N + len(lengths))
+    T, inner = sum(lengths), heads * P
+    xbc = (torch.randn(T, inner + 2 * G * N, generator=g) * 0.7).bfloat16()
+    dt = torch.randn(T, heads + 8, generator=g).bfloat16()
+    dt_bias, a_log, d = torch.randn(heads, generator=g) - 2, torch.randn(heads, generator=g), torch.randn(heads, generator=g)
+    S0 = torch.randn(len(lengths), heads * N * P + 5, generator=g) * 0.5  # an odd slot stride
+    want_y, want_s, at = [], {}, 0
+    for e, n in enumerate(lengths):
+        x = xbc[at:at + n].double()
+        step = torch.nn.functional.softplus(dt[at:at + n, :heads].double() + dt_bias.double(), threshold=50)
+        xs = x[:, :inner].view(n, heads, P)
+        B, C = (x[:, inner + i * G * N:inner + (i + 1) * G * N].view(n, G, N).repeat_interleave(heads // G, 1) for i in (0, 1))
+        slot = len(lengths) - 1 - e
+        o, S = scan(C, B, xs, -torch.exp(a_log.double()) * step, step, S0[slot, 3:3 + heads * N * P].view(heads, N, P).double())
+        want_y.append((o + d.double()[:, None] * xs).reshape(n, inner))
+        want_s[slot] = S
+        at += n
+    want_y, want_s = torch.cat(want_y), torch.stack([want_s[k] for k in range(len(lengths))])
+    ctx, dev = context(rt, lengths), lambda t: t.to(rt.device)
+
+    def run():
+        state, y = dev(S0.clone()), torch.full((T, inner), float("nan"), device=rt.device)
+        mats = state[:, 3:3 + heads * N * P].view(len(lengths), heads, N, P)
+        rt.ops.ssm_scan(dev(xbc), dev(dt)[:, :heads], dev(dt_bias), dev(a_log), dev(d), mats, ctx, y, heads=heads, head_dim=P, nstate=N, groups=G)
+        assert torch.equal(state[:, :3].cpu(), S0[:, :3]) and torch.equal(state[:, -2:].cpu(), S0[:, -2:])
+        return err(y, want_y), err(mats, want_s)
+
+    new, old = both(rt, run)
+    assert max(new) < TOL, (new, old)
+
+
+@pytest.mark.parametrize("lengths", LENGTHS)
+@pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 256), (3, 8, 72), (2, 64, 64), (1, 104, 8)])
+def test_matrix_memory_in_matrix_chunks(rt, lengths, heads, dim, vdim):
+    g = torch.Generator().manual_seed(heads * dim + vdim + len(lengths))
+    T, cap, nk, nv = sum(lengths), 9.0, heads * dim, heads * vdim
+    rows = torch.randn(T, 2 * nk + nv + 8, generator=g).bfloat16()
+    logits = torch.randn(T, 2 * heads, generator=g) * 3
+    bias = torch.cat([torch.randn(heads, generator=g), 3 + torch.randn(heads, generator=g)])
+    up = lambda n: -(-n // 4) * 4  # noqa: E731
+    a, b = up(nk * vdim), up(nk)
+    S0 = torch.randn(len(lengths), a + b + up(heads) + 4, generator=g) * 0.5
+    want, wo, wn, at = {}, [], [], 0
+    for e, n in enumerate(lengths):
+        x, z = rows[at:at + n].double(), logits[at:at + n].double() + bias.double()
+        slot = len(lengths) - 1 - e
+        i_g = cap * torch.tanh(z[:, :heads] / cap)
+        f_g = -torch.nn.functional.softplus(-cap * torch.tanh(z[:, heads:] / cap))
+        m, log_a, w = S0[slot, a + b:a + b + heads].double(), [], []
+        for t in range(n):
+            new = torch.maximum(f_g[t] + m, i_g[t])
+            log_a.append(f_g[t] + m - new)
+            w.append(torch.exp(i_g[t] - new))
+            m = new
+        log_a, w = torch.stack(log_a), torch.stack(w)
+        q, k, v = x[:, :nk].view(n, heads, dim) * dim ** -0.5, x[:, nk:2 * nk].view(n, heads, dim), x[:, 2 * nk:2 * nk + nv].view(n, heads, vdim)
+        full = torch.cat([v, torch.ones(n, heads, 1, dtype=torch.float64)], -1)  # n is the state of a column of ones
+        start = torch.cat([S0[slot, :nk * vdim].view(heads, dim, vdim), S0[slot, a:a + nk].view(heads, dim, 1)], -1).double()
+        o, S = scan(q, k, full, log_a, w, start)
+        wo.append(o[..., :vdim].reshape(n, nv))
+        wn.append(o[..., vdim])
+        want[slot] = (S[..., :vdim], S[..., vdim], m)
+        at += n
+    wo, wn = torch.cat(wo), torch.cat(wn)
+    ws = [torch.stack([want[k][j] for k in range(len(lengths))]) for j in range(3)]
+    ctx, dev = context(rt, lengths), lambda t: t.to(rt.device)
+
+    def run():
+        st = dev(S0.clone())
+        state, n_state, m_state = st[:, :nk * vdim].view(-1, heads, dim, vdim), st[:, a:a + nk].view(-1, heads, dim), st[:, a + b:a + b + heads]
+        o = torch.full((T, nv), float("nan"), device=rt.device)
+        nq, floor = torch.full((T, heads), float("nan"), device=rt.device), torch.full((T, heads), float("nan"), device=rt.device)
+        r = dev(rows)
+        rt.ops.memory_scan(r[:, :nk], r[:, nk:2 * nk], r[:, 2 * nk:2 * nk + nv], dev(logits), dev(bias), cap, dim ** -0.5, state, n_state, m_state,
+                           ctx, o, nq, floor, heads=heads, dim=dim, vdim=vdim)
+        return err(o, wo), err(nq, wn), err(state, ws[0]), err(n_state, ws[1]), err(m_state, ws[2])
+
+    new, old = both(rt, run)
+    assert max(new) < TOL, (new, old)
