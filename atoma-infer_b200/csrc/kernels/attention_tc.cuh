@@ -1,4 +1,4 @@
-// What the tcgen05 attention kernels share (-DHEAD_DIM=64 or 128): bounded mbarrier waits, TMA, tensor memory, MMA
+// What the tcgen05 attention kernels share (-DHEAD_DIM=64, 128 or 256): bounded mbarrier waits, TMA, tensor memory, MMA
 // instructions and their descriptors, the tensor map of a layer's cache.
 #pragma once
 #include <cuda.h>
@@ -8,7 +8,7 @@
 #ifndef HEAD_DIM
 #define HEAD_DIM 64
 #endif
-static_assert(HEAD_DIM == 64 || HEAD_DIM == 128, "the tcgen05 attention kernels are built for head sizes 64 and 128");
+static_assert(HEAD_DIM == 64 || HEAD_DIM == 128 || HEAD_DIM == 256, "the tcgen05 attention kernels are built for head sizes 64, 128 and 256");
 
 namespace {
 

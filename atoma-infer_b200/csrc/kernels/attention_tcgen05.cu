@@ -1,4 +1,4 @@
-// Prefill attention on the 5th-generation tensor cores (-DHEAD_DIM=64 or 128).
+// Prefill attention on the 5th-generation tensor cores (-DHEAD_DIM=64 or 128; 256 where keys and values are the same vectors).
 //
 // One block = 128 query rows ((token, query head of the group) pairs of one key/value head) of one
 // request, walking that request's keys 128 at a time through the block table.  The block's warps
@@ -21,6 +21,11 @@
 // head size 64; the softmax warps then take registers that the other two warps give up.
 // A portion of a prompt that starts inside a cached context attends to all of it.
 //
+// Head size 256 serves attention whose cache holds the same vector on the key and the value plane (latent attention): a tile of
+// 128 such vectors is 64 KB, so Q and two stages of ONE plane fill a multiprocessor's shared memory, and separate values
+// would not fit.  A stage is both products' B operand, K-major for the scores and MN-major for P V, and is free when P V is
+// done.  Measured, 16 heads of 256 over one, window 1,024, learned sinks, a prompt of 4,096 tokens: @@.
+//
 // The reference's prefill kernel is FlashAttention-2 for sm80 (csrc/kernels/flash_fwd_kernel.h:56-500,
 // mma.sync m16n8k16, cp.async), which also cannot see a cached prefix (models/src/flash_attention.rs:384-410).
 //
@@ -40,6 +45,7 @@ constexpr int BKV = 128;           // keys per tile
 // key loop: P V of every tile is added to it by the tensor core itself.
 constexpr uint32_t S_COL = 0, P_COL = 128, O_COL = 192;
 constexpr uint32_t TMEM_COLS = D == 64 ? 256 : 512;
+constexpr bool ONE_PLANE = D == 256;  // keys and values are the same vectors: only the key plane is read
 // The exponentials of a row use one base until the row's maximum has grown by more than this (in powers of two):
 // only then are O and the row's sum scaled down.  P then stays below 2^8, far inside the range of bfloat16.
 constexpr float RESCALE_STEP = 8.f;
@@ -69,7 +75,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
     constexpr int STAGE = HALVES * HALF_BYTES;  // one K or V tile: 128 rows of the head
     unsigned char* q_s = smem;
     unsigned char* k_s = q_s + STAGE;       // two stages
-    unsigned char* v_s = k_s + 2 * STAGE;   // two stages
+    unsigned char* v_s = ONE_PLANE ? k_s : k_s + 2 * STAGE;   // two stages
     uint64_t* bars = reinterpret_cast<uint64_t*>(v_s + 2 * STAGE);
     // k_full, v_full [2]: a K / V stage filled by TMA.  s_done, pv_done [2, by tile parity]: the scores / the P V
     // product of a tile complete (tensor core); they also free the tile's K / V stage.  s_free: every softmax warp has
@@ -170,16 +176,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
             };
             int last_k[2] = {-1, -1}, last_v[2] = {-1, -1};  // the last tile whose copy was started into a stage
             for (int t = 0; t < 2 && t < ntiles; ++t) { issue_loads(t, 0, k_s + t * STAGE, &k_full[t]); last_k[t] = t; }
-            for (int t = 0; !STATS && t < 2 && t < ntiles; ++t) { issue_loads(t, 1, v_s + t * STAGE, &v_full[t]); last_v[t] = t; }
+            for (int t = 0; !STATS && !ONE_PLANE && t < 2 && t < ntiles; ++t) { issue_loads(t, 1, v_s + t * STAGE, &v_full[t]); last_v[t] = t; }
             bool ok = true;
             for (int t = 0; t + 2 < ntiles; ++t) {
                 const int b = t & 1;
                 const uint32_t par = (uint32_t)(t >> 1) & 1u;
-                ok = mbar_wait(&s_done[b], par, status, abort_flag);  // the scores of tile t are done: its K stage is free
+                // the scores of tile t are done: its K stage is free (with one plane: its P V is)
+                ok = mbar_wait(ONE_PLANE && !STATS ? &pv_done[b] : &s_done[b], par, status, abort_flag);
                 if (!ok) break;
                 issue_loads(t + 2, 0, k_s + b * STAGE, &k_full[b]);
                 last_k[b] = t + 2;
-                if constexpr (STATS) continue;
+                if constexpr (STATS || ONE_PLANE) continue;
                 ok = mbar_wait(&pv_done[b], par, status, abort_flag);  // P V of tile t is done: its V stage is free
                 if (!ok) break;
                 issue_loads(t + 2, 1, v_s + b * STAGE, &v_full[b]);
@@ -225,7 +232,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
                 if constexpr (STATS) continue;
                 ok = mbar_wait(p_ready, (uint32_t)t & 1u, status, abort_flag);  // P(t) is in tensor memory, O is scaled
                 if (!ok) break;
-                ok = mbar_wait(&v_full[b], par, status, abort_flag);
+                if constexpr (!ONE_PLANE) ok = mbar_wait(&v_full[b], par, status, abort_flag);  // (one plane: it was there for the scores)
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll
@@ -270,7 +277,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(s_free);
-            const bool need_mask = window > 0 || k0 + BKV - 1 > p_first || k0 < kbeg || nt < TPT || k0 < chunk_last;  // same for the whole block
+            const bool need_mask = (window > 0 && k0 <= p_last - window) || k0 + BKV - 1 > p_first || k0 < kbeg || nt < TPT || k0 < chunk_last;  // same for the whole block
             if (need_mask) {
 #pragma unroll
                 for (int i = 0; i < 64; ++i) {
@@ -345,7 +352,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
             // ---- V rows that no page delivered, or that lie beyond the last key, must be zero (0 * NaN would
             // poison P V): the last tile, a tile that starts before the window, a block table with holes
             if (k0 + BKV > kend || k0 < kbeg || any_bad) {
-                if (!mbar_wait(&v_full[b], par, status, abort_flag)) ok = false;
+                if (!ONE_PLANE && !mbar_wait(&v_full[b], par, status, abort_flag)) ok = false;
                 if (half == 0) {
                     int key = k0 + row, pidx = key / ps - page_lo;
                     bool have = key < kend && pidx < page_cnt && bt_s[pidx] > 0;
@@ -402,7 +409,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
 
 // ----------------------------------------------------------------------------- host side
 namespace {
-constexpr size_t TC_SMEM_FIXED = (size_t)(5 * HALVES) * HALF_BYTES + 12 * 8 + 16 + 4 * BQ * 4 + 1024;  // Q, 2 K, 2 V; barriers; slots; alignment
+constexpr size_t TC_SMEM_FIXED = (size_t)((ONE_PLANE ? 3 : 5) * HALVES) * HALF_BYTES + 12 * 8 + 16 + 4 * BQ * 4 + 1024;  // Q, 2 K, 2 V; barriers; slots; alignment
+// Pages of the block table that a block can meet.
+int table_slice(int max_context, int page_size, int tpt, int window, int chunk) {
+    int span = window > 0 ? min(max_context, window + tpt + 2 * BKV) : max_context;
+    if (chunk > 0) span = min(span, chunk + tpt + 2 * BKV);
+    return span / page_size + 2 + BKV / page_size;
+}
 }  // namespace
 
 extern "C" int attn_tc_head_dim() { return D; }
@@ -411,6 +424,11 @@ extern "C" int attn_tc_head_dim() { return D; }
 extern "C" int attn_prefill_tc_supports(int page_size, int nq, int nkv) {
     bool ps_ok = page_size >= 8 && page_size <= 128 && (page_size & (page_size - 1)) == 0;
     return ps_ok && nq % nkv == 0 && nq / nkv <= 16;
+}
+
+// Whether a step whose longest request has max_context tokens fits shared memory with the block table's slice.
+extern "C" int attn_prefill_tc_fits(int page_size, int nq, int nkv, int window, int chunk, int max_context) {
+    return TC_SMEM_FIXED + (size_t)table_slice(max_context, page_size, BQ / (nq / nkv), window, chunk) * sizeof(int) <= 227 * 1024;
 }
 
 // sink_values (one float per query head, or null): the sink's score per head instead of 0.
@@ -441,9 +459,7 @@ extern "C" int attn_prefill_tc_scores(const void* q, int q_stride, const void* c
     if (!cache_map(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;
     CacheLayout L{nkv, page_size, D};
     const int tpt = BQ / (nq / nkv);
-    int span = window > 0 ? min(max_context, window + tpt + 2 * BKV) : max_context;
-    if (chunk > 0) span = min(span, chunk + tpt + 2 * BKV);
-    int bt_cap = span / page_size + 2 + BKV / page_size;
+    const int bt_cap = table_slice(max_context, page_size, tpt, window, chunk);
     size_t smem = TC_SMEM_FIXED + (size_t)bt_cap * sizeof(int);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
     const bool cs = chunk > 0 || sink || softcap > 0.f || slopes != nullptr;
@@ -477,8 +493,7 @@ extern "C" int attn_prefill_tc_stats(const void* q, int q_stride, const void* ca
     if (!cache_map(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;
     CacheLayout L{nkv, page_size, D};
     const int tpt = BQ / (nq / nkv);
-    const int span = chunk > 0 ? min(max_context, chunk + tpt + 2 * BKV) : max_context;
-    const int bt_cap = span / page_size + 2 + BKV / page_size;
+    const int bt_cap = table_slice(max_context, page_size, tpt, 0, chunk);
     const size_t smem = TC_SMEM_FIXED + (size_t)bt_cap * sizeof(int);
     if (smem > 227 * 1024) return (int)cudaErrorInvalidValue;
     static size_t configured = 0;

@@ -41,6 +41,7 @@ MATRIX_RECURRENT_SOURCES = ["kernels/matrix_recurrent.cu"]
 # several residual streams side by side, attention as the difference of two maps
 STREAMS_SOURCES = ["kernels/stream_mix.cu", "kernels/differential.cu"]
 ATTENTION_TC_HEAD_DIMS = (64, 128)  # head sizes of the tcgen05 prefill attention
+ATTENTION_TC_ONE_PLANE_DIMS = (256,)  # ... and those where keys and values must be the same vectors
 ATTENTION_HEAD_DIMS = tuple(range(16, 257, 16))  # every head size the kernels take; the build check builds them all, a model only its own
 
 
@@ -98,6 +99,7 @@ class CudaOps:
         # ATOMA_INFER_PDL: "0" off, "1" every kernel, "linear" without the norm, default "linear+norm".
         mode = os.environ.get("ATOMA_INFER_PDL", "linear+norm")
         self.pdl = {"0": 0, "1": 1, "linear": 2, "linear+norm": 6}.get(mode, 6)
+        self.one_plane_attention = True  # attention takes the hint that keys and values are the same vectors
         self.fused_rope = True  # the decode attention rotates q and k and writes the new key and value itself
         self.masked_fast_attention = True  # chunk masks and sinks on the tensor-core attention kernels (False: on the plain one; a test lever)
         self.scored_fast_attention = True  # likewise score caps, distance slopes and windows that keep the first tokens
@@ -464,7 +466,7 @@ class CudaOps:
 
     def attention(self, q, q_stride: int, cache_layer, ctx, group: int, out, nq: int, nkv: int, d: int,
                   page_size: int, num_pages: int, window: int, scale: float, rope=None, chunk: int = 0, sink: bool = False,
-                  keep_first: int = 0, softcap: float = 0.0, slopes=None):
+                  keep_first: int = 0, softcap: float = 0.0, slopes=None, one_plane: bool = False):
         """Attention of the step's queries over what their requests have cached (the step's own
         keys included).  bfloat16 with a head size in steps of 16 up to 256 runs the tensor-core
         kernels (one library per head size, built at first use); anything else, and all of
@@ -475,7 +477,8 @@ class CudaOps:
         has one more term in its denominator, a key of score 0 without a value.  ``keep_first`` (beside a window): the
         first so many keys of a request stay visible behind the window.  ``softcap`` > 0: a score s becomes softcap *
         tanh(s / softcap).  ``slopes`` (float32, one per query head): slopes[h] * (query position - key position) is
-        taken off the score."""
+        taken off the score.  ``one_plane``: the cache holds the same vectors as keys and as values (both planes are written all
+        the same); a kernel may then read one plane only."""
         T, S = ctx.T, ctx.S
         if slopes is not None and (slopes.dtype != torch.float32 or slopes.numel() != nq or not slopes.is_contiguous()):
             raise KernelError("distance slopes are one contiguous float32 number per query head")
@@ -536,9 +539,9 @@ class CudaOps:
                                                    window, int(chunk), int(bool(sink)), _p(sinks), ctypes.c_float(scale), splits,
                                                    int(cluster), ctx.max_context, *extra, _p(self.status), self._stream()),
                             "attn_decode")
-            elif not keep_first and self._prefill_tc(d, page_size, nq, nkv) is not None:
+            elif not keep_first and self._prefill_tc(d, page_size, nq, nkv, one_plane, (window, int(chunk), ctx.max_context)) is not None:
                 # (a window that keeps first keys is the mma.sync kernel's: its kept keys are tiles of their own)
-                tc = self._prefill_tc(d, page_size, nq, nkv)
+                tc = self._prefill_tc(d, page_size, nq, nkv, one_plane, (window, int(chunk), ctx.max_context))
                 self._check(tc.attn_prefill_tc_scores(_p(q), q_stride, _p(cache_layer), _p(ctx.meta), group, _p(ctx.cu_tokens),
                                                       _p(ctx.context_lens), _p(out), S, ctx.max_tokens_per_entry, nq, nkv,
                                                       page_size, num_pages, window, int(chunk), int(bool(sink)), _p(sinks),
@@ -1343,9 +1346,12 @@ class CudaOps:
             blocks = self._flat_blocks[key] = int(lib.attn_decode_flat_blocks(S))
         return blocks if blocks and 2 * S * nkv >= blocks else 0
 
-    def _prefill_tc(self, d: int, page_size: int, nq: int, nkv: int):
-        """The tcgen05 prefill attention library for this geometry, or None (then the mma.sync kernel runs)."""
-        if d not in ATTENTION_TC_HEAD_DIMS or not self.tc_attention:
+    def _prefill_tc(self, d: int, page_size: int, nq: int, nkv: int, one_plane: bool = False, reach=None):
+        """The tcgen05 prefill attention library for this geometry, or None (then the mma.sync kernel runs).  ``reach`` =
+        (window, chunk, longest context): head sizes that fill the shared memory leave room for the block table of about
+        130,000 visible keys at 16 a page; beyond that they stay on the mma.sync kernel."""
+        wide = d in ATTENTION_TC_ONE_PLANE_DIMS and one_plane and reach is not None
+        if not self.tc_attention or not (wide or d in ATTENTION_TC_HEAD_DIMS):
             return None
         lib = self._attn_tc_libs.get(d)
         if lib is None:
@@ -1353,7 +1359,9 @@ class CudaOps:
             if lib.attn_tc_head_dim() != d:
                 raise KernelError(f"tcgen05 attention library was built for head size {lib.attn_tc_head_dim()}, wanted {d}")
             self._attn_tc_libs[d] = lib
-        return lib if lib.attn_prefill_tc_supports(page_size, nq, nkv) else None
+        if not lib.attn_prefill_tc_supports(page_size, nq, nkv) or wide and not lib.attn_prefill_tc_fits(page_size, nq, nkv, *reach):
+            return None
+        return lib
 
     def _attention_library(self, d: int):
         lib = self._attn_libs.get(d)

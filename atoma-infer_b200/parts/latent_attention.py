@@ -126,7 +126,8 @@ class LatentAttention(Mixer):
                         **({"halves": True} if self.halves else {}))
         out = torch.empty((T, H * D), dtype=x.dtype, device=x.device)
         ops.attention(q_full, H * D, cache.pages, ctx, cache.group, out, H, 1, D, cache.page_size, cache.num_pages,
-                      int(self.window or 0), self.scale, sink=self.sink_values if self.sink else False)
+                      int(self.window or 0), self.scale, sink=self.sink_values if self.sink else False,
+                      **({"one_plane": True} if getattr(ops, "one_plane_attention", False) else {}))
         o = torch.empty((T, H, self.v_head_dim), dtype=x.dtype, device=x.device)
         gate = a[:, self.first + self.latent:self.first + self.latent + self.gate_rows] if self.gate else None
         if gate is not None and not self.head_gate:

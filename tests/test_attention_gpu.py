@@ -296,3 +296,43 @@ def test_decode_page_loads_by_tma(rts):
         assert worst(got, want) < 3e-2
     finally:
         lib.attn_set_decode_tma(0)
+
+
+@pytest.mark.parametrize("nq,page", [(16, 16), (5, 8), (1, 128), (12, 64)])
+@pytest.mark.parametrize("window,sink", [(0, False), (200, True), (130, False)])
+def test_prefill_over_one_plane_of_wide_heads(rts, nq, page, window, sink):
+    """Heads of 256 whose keys are their values, on the tcgen05 kernel that reads one plane: portions behind cached contexts, key
+    tiles that end inside a page, windows that start inside a tile, group sizes that do not divide 128, learned sinks; the value
+    plane holds NaN, so a kernel that read it would show.  Against the plain sums and the mma.sync kernel over both planes."""
+    rt, d = rts["bfloat16"], 256
+    g = torch.Generator().manual_seed(nq + page + window)
+    entries = [(0, 70), (37, 429), (130, 2), (250, 262), (0, 1)]
+    lengths = [c + n for c, n in entries]
+    tables, num_pages = K.scrambled_tables(lengths, page, nq)
+    ks = [torch.randn(n, 1, d, generator=g).bfloat16() for n in lengths]
+    q = torch.randn(sum(n for _, n in entries), nq * d, generator=g).bfloat16()
+    sinks = (torch.randn(nq, generator=g) * 2).to(rt.device) if sink else False
+    scale = 1 / math.sqrt(d)
+    both = torch.full((num_pages, 2, 1, page, d), float("nan"), dtype=rt.dtype, device=rt.device)
+    K.fill_cache(both, tables, ks, ks, page)
+    one = both.clone()
+    one[:, 1] = float("nan")
+    ctx, _ = K.make_context(rt, entries, page, tables)
+    outs = []
+    for cache, kw in ((one, {"one_plane": True}), (both, {})):
+        out = torch.full((ctx.T, nq * d), float("nan"), dtype=rt.dtype, device=rt.device)
+        rt.ops.attention(q.to(rt.device), nq * d, cache, ctx, 0, out, nq, 1, d, page, num_pages, window, scale, sink=sinks, **kw)
+        outs.append(out.float().cpu())
+    rt.ops.check_status()
+    row = 0
+    for (c, n), k in zip(entries, ks):
+        kk = k[:, 0].double()
+        s = torch.einsum("ihd,jd->hij", q[row:row + n].double().view(n, nq, d), kk) * scale
+        i, j = c + torch.arange(n)[:, None], torch.arange(c + n)[None]
+        s = s.masked_fill((j > i) | ((i - j >= window) if window else torch.zeros_like(j > i)), -math.inf)
+        if sink:
+            s = torch.cat([s, sinks.double().cpu()[:, None, None].expand(nq, n, 1)], -1)
+        want = torch.einsum("hij,jd->ihd", torch.softmax(s, -1)[..., :c + n], kk).reshape(n, nq * d)
+        assert (outs[0][row:row + n] - want).abs().max() < 2e-2  # values are O(1); bfloat16 P and outputs
+        assert (outs[1][row:row + n] - want).abs().max() < 2e-2
+        row += n
