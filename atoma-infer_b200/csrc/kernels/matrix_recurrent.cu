@@ -155,13 +155,13 @@ head_weight_norm_gate_kernel(const float* __restrict__ o, const float* __restric
                              T* __restrict__ out, const int* __restrict__ meta, int heads, int P, int vec4, int LPH) {
     pdl_launch_dependents();
     pdl_wait();
-    const int t = blockIdx.x, lane = threadIdx.x % LPH, h = blockIdx.y * (blockDim.x / LPH) + threadIdx.x / LPH;
-    if (t >= meta[META_NUM_TOKENS]) return;
-    const bool live = h < heads;  // (lanes without a head still take part in their warp's sums)
-    const size_t at = ((size_t)t * heads + (live ? h : 0)) * P;
+    // (token, head) pairs one behind the other; lanes without one still take part in their warp's sums
+    const int lane = threadIdx.x % LPH, item = blockIdx.x * (blockDim.x / LPH) + threadIdx.x / LPH, t = item / heads, h = item % heads;
+    const bool live = t < meta[META_NUM_TOKENS];
+    const size_t at = live ? (size_t)item * P : 0;
     const float* row = o + at;
-    const T* gate = g + (size_t)t * g_stride + (size_t)(live ? h : 0) * P;
-    const float* wr = w + (size_t)(live ? h : 0) * P;
+    const T* gate = g + (live ? (size_t)t * g_stride + (size_t)h * P : 0);
+    const float* wr = w + (live ? (size_t)h * P : 0);
     float c = 1.f;
     if (nq && live) c = 1.f / (fmaxf(fabsf(nq[(size_t)t * heads + h]), floor_in[(size_t)t * heads + h]) + 1e-6f);
     auto group_sum = [&](float v) {
@@ -169,6 +169,35 @@ head_weight_norm_gate_kernel(const float* __restrict__ o, const float* __restric
         return v;
     };
     float ss = 0.f;
+    if (vec4 && P <= LPH * 16) {  // at most four loads a lane, which stay in registers
+        float v[4][4], gv[4][4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = (lane + LPH * k) * 4;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[k][j] = gv[k][j] = 0.f;
+            if (live && i < P) load4(row + i, v[k]), load4(gate + i, gv[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { v[k][j] *= c; ss = fmaf(v[k][j], v[k][j], ss); }
+        const float inv = rsqrtf(group_sum(ss) / (float)P + eps);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = (lane + LPH * k) * 4;
+            if (!live || i >= P) continue;
+            float wv[4];
+            load4(wr + i, wv);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float s = sigmoid_as<T>(gv[k][j]);
+                wv[j] = v[k][j] * inv * wv[j] * (kind == 1 ? gv[k][j] * s : s);
+            }
+            store4(out + at + i, wv);
+        }
+        return;
+    }
     if (vec4) {
         const int step = LPH * 4;
         for (int i = lane * 4; i < P; i += step) {
@@ -211,7 +240,7 @@ extern "C" int head_weight_norm_gate(const float* o, const float* nq, const floa
     int LPH = 1;
     while (LPH < 32 && LPH * (vec4 ? 4 : 1) < P) LPH *= 2;
     const int threads = heads * LPH > 128 ? 256 : 128;
-    const dim3 grid(T, (heads + threads / LPH - 1) / (threads / LPH));
+    const int grid = (T * heads + threads / LPH - 1) / (threads / LPH);
     if (dtype == DT_F32)
         return (int)launch_kernel(head_weight_norm_gate_kernel<float>, grid, threads, 0, stream, o, nq, floor_in, (const float*)g, g_stride, w, eps,
                                   kind, (float*)out, meta, heads, P, vec4, LPH);

@@ -5,77 +5,124 @@
 #include "common.cuh"
 
 // ----------------------------------------------------------------------------- router
-// One block per token: logits z_e = w_router[e] . h (float32, a warp per expert, lanes over k, summed in the fixed
-// order of warp_sum); scores softmax(z); the `top` largest scores, ties to the lower index; weights = those scores
-// divided by their sum (+ 1e-20).
-template <typename T>
-__global__ void __launch_bounds__(256)
+// Logits of TOK tokens: z[q * stride + e] = w[e] . x_q (float32; a warp takes EXP experts at a time, its lanes run over k, summed in
+// the fixed order of warp_sum, so a logit's sum depends on H alone).  Bound by the shared reads of x and w through the
+// first-level cache: a row of w is read once for TOK tokens, a row of x once for EXP experts.
+template <typename T, int TOK, int EXP>
+__device__ __forceinline__ void route_logits(const T* __restrict__ x, const float* __restrict__ w, int H, int E, int tokens, float* z, int stride) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const bool vec = H % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+    for (int e0 = warp * EXP; e0 < E; e0 += nwarps * EXP) {
+        float acc[TOK][EXP];
+        if (vec) {  // four columns a lane and step
+            float part[TOK][EXP][4] = {};
+#pragma unroll 4
+            for (int k = lane * 4; k < H; k += 128) {
+                float wv[EXP][4];
+#pragma unroll
+                for (int j = 0; j < EXP; ++j) load4(w + (size_t)min(e0 + j, E - 1) * H + k, wv[j]);
+#pragma unroll
+                for (int q = 0; q < TOK; ++q) {
+                    float xv[4];
+                    load4(x + (size_t)(q < tokens ? q : 0) * H + k, xv);
+#pragma unroll
+                    for (int j = 0; j < EXP; ++j)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) part[q][j][i] = fmaf(xv[i], wv[j][i], part[q][j][i]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < TOK; ++q)
+#pragma unroll
+                for (int j = 0; j < EXP; ++j) acc[q][j] = (part[q][j][0] + part[q][j][1]) + (part[q][j][2] + part[q][j][3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < TOK; ++q)
+#pragma unroll
+                for (int j = 0; j < EXP; ++j) {
+                    acc[q][j] = 0.f;
+                    const T* row = x + (size_t)(q < tokens ? q : 0) * H;
+                    const float* we = w + (size_t)min(e0 + j, E - 1) * H;
+                    for (int k = lane; k < H; k += 32) acc[q][j] = fmaf(to_float(row[k]), we[k], acc[q][j]);
+                }
+        }
+#pragma unroll
+        for (int q = 0; q < TOK; ++q)
+#pragma unroll
+            for (int j = 0; j < EXP; ++j) {
+                const float v = warp_sum(acc[q][j]);
+                if (lane == 0 && q < tokens && e0 + j < E) z[q * stride + e0 + j] = v;
+            }
+    }
+}
+
+// The largest of n values in shared memory, ties to the lower index (n: no value is a number); the winner is struck out.  Warp-wide.
+__device__ __forceinline__ int take_best(float* v, int n, float* value = nullptr) {
+    const int lane = threadIdx.x & 31;
+    float bv = -INFINITY;
+    int best = n;
+    for (int i = lane; i < n; i += 32)
+        if (v[i] > bv) { bv = v[i]; best = i; }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, best, o);
+        if (ov > bv || (ov == bv && oi < best)) { bv = ov; best = oi; }
+    }
+    __syncwarp();
+    if (best < n && lane == 0) v[best] = -INFINITY;
+    __syncwarp();
+    if (value) *value = bv;
+    return best;
+}
+
+// Logits (+ bias); scores softmax(z); the `top` largest scores, ties to the lower index; weights = those scores divided by their
+// sum (+ 1e-20).  over_chosen: the largest logits choose and the weights are the softmax over the chosen logits alone.
+// A block takes TOK tokens and a warp a token chooses.  Measured, 2,048 tokens of 2,048, 16 experts: a block a token with one
+// choosing thread 40 us, four tokens a block 27 (waiting for x and w; they are 8 MB and 128 KB).
+template <typename T, int TOK, int EXP>
+__global__ void __launch_bounds__(256, 2)
 moe_route_kernel(const T* __restrict__ h, const float* __restrict__ w, int* __restrict__ ids, float* __restrict__ wts,
                  const int* __restrict__ meta, int H, int E, int top, const float* __restrict__ bias, int over_chosen) {
-    extern __shared__ float z[];  // E logits, then E scores that selection consumes
+    extern __shared__ float sh[];  // per token: E logits, then scores that selection consumes
     pdl_wait();
     pdl_launch_dependents();
-    const int t = blockIdx.x;
-    if (t >= meta[META_NUM_TOKENS]) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const T* x = h + (size_t)t * H;
-    const bool vec = H % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-    for (int e = warp; e < E; e += nwarps) {
-        const float* we = w + (size_t)e * H;
-        float acc = 0.f;
-        if (vec) {  // four columns a lane and step; the order of a logit's sum depends on H alone
-            float part[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int k = lane * 4; k < H; k += 128) {
-                float xv[4], wv[4];
-                load4(x + k, xv);
-                load4(we + k, wv);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) part[i] = fmaf(xv[i], wv[i], part[i]);
-            }
-            acc = (part[0] + part[1]) + (part[2] + part[3]);
-        } else {
-            for (int k = lane; k < H; k += 32) acc = fmaf(to_float(x[k]), we[k], acc);
-        }
-        acc = warp_sum(acc);
-        if (lane == 0) z[e] = acc + (bias ? bias[e] : 0.f);
-    }
+    const int t0 = blockIdx.x * TOK, tokens = min(TOK, meta[META_NUM_TOKENS] - t0);
+    if (tokens <= 0) return;
+    route_logits<T, TOK, EXP>(h + (size_t)t0 * H, w, H, E, tokens, sh, E);
     __syncthreads();
-    if (threadIdx.x != 0) return;
-    float* s = z + E;
-    if (over_chosen) {
-        // the largest logits choose (ties to the lower index); the weights are the softmax over the chosen logits alone
-        float first = 0.f, sum = 0.f;
-        for (int k = 0; k < top; ++k) {
-            int best = 0;
-            float bv = -INFINITY;
-            for (int e = 0; e < E; ++e)
-                if (z[e] > bv) { bv = z[e]; best = e; }
-            if (k == 0) first = bv;
-            const float w_k = expf(bv - first);
-            ids[(size_t)t * top + k] = best;
-            wts[(size_t)t * top + k] = w_k;
-            sum += w_k;
-            z[best] = -INFINITY;
-        }
-        for (int k = 0; k < top; ++k) wts[(size_t)t * top + k] = wts[(size_t)t * top + k] / sum;
-        return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp >= tokens) return;
+    float* z = sh + warp * E;
+    int* id = ids + (size_t)(t0 + warp) * top;
+    float* wt = wts + (size_t)(t0 + warp) * top;
+    float mx = -INFINITY;
+    for (int e = lane; e < E; e += 32) {
+        if (bias) z[e] += bias[e];
+        mx = fmaxf(mx, z[e]);
     }
-    float mx = -INFINITY, sum = 0.f;
-    for (int e = 0; e < E; ++e) mx = fmaxf(mx, z[e]);
-    for (int e = 0; e < E; ++e) { s[e] = expf(z[e] - mx); sum += s[e]; }
-    for (int e = 0; e < E; ++e) s[e] = s[e] / sum;
+    mx = warp_max(mx);
+    __syncwarp();
     float chosen = 0.f;
-    for (int k = 0; k < top; ++k) {
-        int best = 0;
-        float bv = -1.f;
-        for (int e = 0; e < E; ++e)
-            if (s[e] > bv) { bv = s[e]; best = e; }
-        ids[(size_t)t * top + k] = best;
-        wts[(size_t)t * top + k] = bv;
-        chosen += bv;
-        s[best] = -2.f;
+    if (!over_chosen) {
+        float sum = 0.f;
+        for (int e = lane; e < E; e += 32) sum += z[e] = expf(z[e] - mx);
+        sum = warp_sum(sum);
+        for (int e = lane; e < E; e += 32) z[e] = z[e] / sum;
+        __syncwarp();
     }
-    for (int k = 0; k < top; ++k) wts[(size_t)t * top + k] = wts[(size_t)t * top + k] / (chosen + 1e-20f);
+    for (int k = 0; k < top; ++k) {
+        float v;
+        int best = take_best(z, E, &v);
+        if (best >= E) best = 0;  // (scores that are no numbers: any expert)
+        if (over_chosen) v = expf(v - mx);  // (the largest logit is the first choice)
+        chosen += v;
+        if (lane == 0) id[k] = best, wt[k] = v;
+    }
+    if (lane == 0) {
+        if (!over_chosen) chosen += 1e-20f;
+        for (int k = 0; k < top; ++k) wt[k] = wt[k] / chosen;
+    }
 }
 
 extern "C" int moe_route_biased(const void* h, int dtype, const float* w, const float* bias, int over_chosen, int* ids, float* wts,
@@ -91,13 +138,20 @@ extern "C" int moe_route(const void* h, int dtype, const float* w, int* ids, flo
 extern "C" int moe_route_biased(const void* h, int dtype, const float* w, const float* bias, int over_chosen, int* ids, float* wts,
                                 const int* meta, int T, int H, int E, int top, cudaStream_t stream) {
     if (T <= 0) return 0;
-    const size_t smem = (size_t)2 * E * sizeof(float);
-    if (smem > 48 * 1024 || top > E) return (int)cudaErrorInvalidValue;
-    if (dtype == DT_F32)
-        return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, moe_route_kernel<float>, T, 256, smem, stream, (const float*)h, w, ids, wts,
-                                      meta, H, E, top, bias, over_chosen);
-    return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, moe_route_kernel<__nv_bfloat16>, T, 256, smem, stream,
-                                  (const __nv_bfloat16*)h, w, ids, wts, meta, H, E, top, bias, over_chosen);
+    if ((size_t)2 * E * sizeof(float) > 48 * 1024 || top > E) return (int)cudaErrorInvalidValue;
+    // few tokens: a block each, so that a step of few tokens fills more multiprocessors
+    const int tok = T > 64 && (size_t)4 * E * sizeof(float) <= 48 * 1024 ? 4 : 1, blocks = (T + tok - 1) / tok;
+    const size_t smem = (size_t)tok * E * sizeof(float);
+#define ROUTE_CASE(TT, TOK, EXP)                                                                                           \
+    return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, moe_route_kernel<TT, TOK, EXP>, blocks, 256, smem, stream, (const TT*)h, w, ids, wts, \
+                                  meta, H, E, top, bias, over_chosen)
+    if (dtype == DT_F32) {
+        if (tok == 4) ROUTE_CASE(float, 4, 2);
+        ROUTE_CASE(float, 1, 1);
+    }
+    if (tok == 4) ROUTE_CASE(__nv_bfloat16, 4, 2);
+    ROUTE_CASE(__nv_bfloat16, 1, 1);
+#undef ROUTE_CASE
 }
 
 // Sigmoid scores, a correction that only the choice sees, choice within the best groups.  Per token: s_e = sigmoid(w_router[e] .
@@ -116,69 +170,18 @@ moe_route_sigmoid_kernel(const T* __restrict__ h, const float* __restrict__ w, c
     pdl_launch_dependents();
     const int t0 = blockIdx.x * TOK, tokens = min(TOK, meta[META_NUM_TOKENS] - t0);
     if (tokens <= 0) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int stride = 2 * E + (groups > 1 ? 2 * groups : 0);
-    const T* x = h + (size_t)t0 * H;
-    const bool vec = H % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-    for (int e = warp; e < E; e += nwarps) {
-        const float* we = w + (size_t)e * H;
-        float acc[TOK];
-        if (vec) {  // four columns a lane and step; the order of a logit's sum depends on H alone
-            float part[TOK][4];
-#pragma unroll
-            for (int q = 0; q < TOK; ++q) part[q][0] = part[q][1] = part[q][2] = part[q][3] = 0.f;
-#pragma unroll 4
-            for (int k = lane * 4; k < H; k += 128) {
-                float wv[4];
-                load4(we + k, wv);
-#pragma unroll
-                for (int q = 0; q < TOK; ++q) {
-                    float xv[4];
-                    load4(x + (size_t)(q < tokens ? q : 0) * H + k, xv);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) part[q][i] = fmaf(xv[i], wv[i], part[q][i]);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < TOK; ++q) acc[q] = (part[q][0] + part[q][1]) + (part[q][2] + part[q][3]);
-        } else {
-#pragma unroll
-            for (int q = 0; q < TOK; ++q) {
-                acc[q] = 0.f;
-                for (int k = lane; k < H; k += 32) acc[q] = fmaf(to_float(x[(size_t)(q < tokens ? q : 0) * H + k]), we[k], acc[q]);
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < TOK; ++q) {
-            const float z = warp_sum(acc[q]);
-            if (lane == 0 && q < tokens) {
-                const float s = 1.f / (1.f + expf(-z));
-                sh[q * stride + e] = s;
-                sh[q * stride + E + e] = s + correction[e];
-            }
-        }
-    }
+    route_logits<T, TOK, TOK == 1 ? 1 : 2>(h + (size_t)t0 * H, w, H, E, tokens, sh, stride);
     __syncthreads();
     if (warp >= tokens) return;
     const int t = t0 + warp;
     float *z = sh + warp * stride, *c = z + E, *gs = c + E;
-    // the largest of n values in shared memory, ties to the lower index; the winner is struck out
-    auto take_best = [&](float* v, int n) {
-        float bv = -INFINITY;
-        int best = n;
-        for (int i = lane; i < n; i += 32)
-            if (v[i] > bv) { bv = v[i]; best = i; }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, best, o);
-            if (ov > bv || (ov == bv && oi < best)) { bv = ov; best = oi; }
-        }
-        __syncwarp();
-        if (best < n && lane == 0) v[best] = -INFINITY;
-        __syncwarp();
-        return best;
-    };
+    for (int e = lane; e < E; e += 32) {
+        z[e] = 1.f / (1.f + expf(-z[e]));
+        c[e] = z[e] + correction[e];
+    }
+    __syncwarp();
     if (groups > 1) {
         const int per = E / groups;
         int* kept = reinterpret_cast<int*>(gs + groups);
@@ -233,54 +236,78 @@ extern "C" int moe_route_sigmoid(const void* h, int dtype, const float* w, const
 
 // ----------------------------------------------------------------------------- pairs sorted by expert
 // One block.  offsets[e] .. offsets[e + 1] is expert e's stretch of `order`, which lists its pairs (token * top + choice)
-// in ascending order.  A warp takes the experts e = warp, warp + warps, ...: it walks all pairs 32 at a time and
-// places the matching ones by a ballot, once to count and once to write.
+// in ascending order.  Every warp takes a stretch of the pairs, 32 at a time: pairs of one expert find one another by a match
+// across the warp, once to count (base[warp][expert]) and, after the counts have become places, once to write.
 // `place` (optional): place[pair] = where the pair stands in `order`.
+// Bound by the chain of loads and matches of one block: 4,096 pairs of 16 experts 7.5 us (each expert's warp walking all pairs
+// twice: 38 us).
 __global__ void __launch_bounds__(1024)
 moe_sort_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ place,
                 const int* __restrict__ meta, int top, int E) {
-    extern __shared__ int counts[];  // E + 1
+    extern __shared__ int base[];  // [warps][E]
     pdl_launch_dependents();
     pdl_wait();
-    const int n = meta[META_NUM_TOKENS] * top;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (int e = warp; e < E; e += nwarps) {
-        int c = 0;
-        for (int i0 = 0; i0 < n; i0 += 32) {
-            const int i = i0 + lane;
-            c += __popc(__ballot_sync(0xffffffffu, i < n && ids[i] == e));
-        }
-        if (lane == 0) counts[e] = c;
-    }
+    const int n = meta[META_NUM_TOKENS] * top, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int share = ((n + nwarps - 1) / nwarps + 31) / 32 * 32, from = min(n, warp * share), to = min(n, from + share);
+    for (int i = threadIdx.x; i < nwarps * E; i += blockDim.x) base[i] = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int at = 0;
-        for (int e = 0; e < E; ++e) { const int c = counts[e]; counts[e] = at; offsets[e] = at; at += c; }
-        counts[E] = at;
-        offsets[E] = at;
-    }
-    __syncthreads();
-    for (int e = warp; e < E; e += nwarps) {
-        int at = counts[e];
-        for (int i0 = 0; i0 < n; i0 += 32) {
-            const int i = i0 + lane;
-            const bool mine = i < n && ids[i] == e;
-            const unsigned m = __ballot_sync(0xffffffffu, mine);
-            if (mine) {
-                const int to = at + __popc(m & ((1u << lane) - 1u));
-                order[to] = i;
-                if (place) place[i] = to;
+    int* own = base + warp * E;
+    auto walk = [&](auto&& visit) {
+        for (int i0 = from; i0 < to; i0 += 128) {
+            int id[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) id[u] = i0 + u * 32 + lane < to ? ids[i0 + u * 32 + lane] : -1;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const unsigned same = __match_any_sync(0xffffffffu, id[u]);
+                if (id[u] >= 0) visit(i0 + u * 32 + lane, id[u], __popc(same & ((1u << lane) - 1u)));
+                __syncwarp();
+                if (id[u] >= 0 && lane == __ffs(same) - 1) own[id[u]] += __popc(same);
+                __syncwarp();
             }
-            at += __popc(m);
         }
+    };
+    walk([](int, int, int) {});
+    __syncthreads();
+    if (warp == 0) {
+        int before = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane;
+            int total = 0;
+            if (e < E)
+                for (int w = 0; w < nwarps; ++w) total += base[w * E + e];
+            int upto = total;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int below = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= d) upto += below;
+            }
+            if (e < E) {
+                int at = before + upto - total;
+                offsets[e] = at;
+                for (int w = 0; w < nwarps; ++w) {
+                    const int c = base[w * E + e];
+                    base[w * E + e] = at;
+                    at += c;
+                }
+            }
+            before += __shfl_sync(0xffffffffu, upto, 31);
+        }
+        if (lane == 0) offsets[E] = before;
     }
+    __syncthreads();
+    walk([&](int i, int e, int rank) {
+        const int at = own[e] + rank;
+        order[at] = i;
+        if (place) place[i] = at;
+    });
 }
 
 extern "C" int moe_sort(const int* ids, int* offsets, int* order, int* place, const int* meta, int top, int E,
                         cudaStream_t stream) {
-    const size_t smem = (size_t)(E + 1) * sizeof(int);
-    if (smem > 48 * 1024) return (int)cudaErrorInvalidValue;
-    return (int)launch_kernel(moe_sort_kernel, 1, 1024, smem, stream, ids, offsets, order, place, meta, top, E);
+    if (E < 1 || (size_t)(E + 1) * sizeof(int) > 48 * 1024) return (int)cudaErrorInvalidValue;
+    const int most = 48 * 1024 / 4 / E, warps = most < 32 ? most : 32;  // as many warps as have counts in shared memory
+    return (int)launch_kernel(moe_sort_kernel, 1, warps * 32, (size_t)warps * E * sizeof(int), stream, ids, offsets, order, place, meta, top, E);
 }
 
 // ----------------------------------------------------------------------------- grouped products
@@ -400,11 +427,30 @@ extern "C" int moe_grouped_ff(const void* x, const void* w_gate_up, void* act, c
 template <typename TY, typename T>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, const float* __restrict__ wts,
-                   const T* __restrict__ shared, T* __restrict__ out, const int* __restrict__ meta, int top, int H) {
+                   const T* __restrict__ shared, T* __restrict__ out, const int* __restrict__ meta, int top, int H, int vec4) {
     pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x;
     if (t >= meta[META_NUM_TOKENS]) return;
+    if (vec4) {  // the same, four neighbouring values a thread
+        for (int i = threadIdx.x * 4; i < H; i += blockDim.x * 4) {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
+            for (int k = 0; k < top; ++k) {
+                const size_t row = place ? (size_t)place[(size_t)t * top + k] : (size_t)t * top + k;
+                const float weight = wts[(size_t)t * top + k];
+                load4(y + row * H + i, v);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[j] = fmaf(weight, v[j], acc[j]);
+            }
+            if (shared) {
+                load4(shared + (size_t)t * H + i, v);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[j] += v[j];
+            }
+            store4(out + (size_t)t * H + i, acc);
+        }
+        return;
+    }
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
         float acc = 0.f;
         for (int k = 0; k < top; ++k) {
@@ -420,15 +466,16 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, cons
 extern "C" int moe_combine(const void* y, int y_dtype, const int* place, const float* wts, const void* shared, void* out,
                            int dtype, const int* meta, int T, int top, int H, cudaStream_t stream) {
     if (T <= 0) return 0;
+    const int vec4 = H % 4 == 0 && (((uintptr_t)y | (uintptr_t)shared | (uintptr_t)out) & 15) == 0;  // (8 bytes would do for bfloat16)
     const int threads = H >= 1024 ? 256 : 128;
     if (dtype == DT_F32)
         return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, moe_combine_kernel<float, float>, T, threads, 0, stream, (const float*)y,
-                                      place, wts, (const float*)shared, (float*)out, meta, top, H);
+                                      place, wts, (const float*)shared, (float*)out, meta, top, H, vec4);
     if (y_dtype == DT_F32)
         return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, moe_combine_kernel<float, __nv_bfloat16>, T, threads, 0, stream,
-                                      (const float*)y, place, wts, (const __nv_bfloat16*)shared, (__nv_bfloat16*)out, meta, top, H);
+                                      (const float*)y, place, wts, (const __nv_bfloat16*)shared, (__nv_bfloat16*)out, meta, top, H, vec4);
     return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, moe_combine_kernel<__nv_bfloat16, __nv_bfloat16>, T, threads, 0, stream,
-                                  (const __nv_bfloat16*)y, place, wts, (const __nv_bfloat16*)shared, (__nv_bfloat16*)out, meta, top, H);
+                                  (const __nv_bfloat16*)y, place, wts, (const __nv_bfloat16*)shared, (__nv_bfloat16*)out, meta, top, H, vec4);
 }
 
 // ----------------------------------------------------------------------------- few pairs: a pair at a time

@@ -63,9 +63,59 @@ head_norm_gate_kernel(const float* __restrict__ o, const T* __restrict__ g, long
     for (int i = lane; i < P; i += 32) dst[i] = from_float<T>(row[i] * inv * w[i] * silu_f(to_float(gate[i])));
 }
 
+// The same with at most 128 K values a head, four consecutive ones a lane and 16-byte accesses, all loads ahead of the sum.
+template <typename T, int K>
+__global__ void __launch_bounds__(256)
+head_norm_gate_vec_kernel(const float* __restrict__ o, const T* __restrict__ g, long long g_stride, const float* __restrict__ w,
+                          float eps, T* __restrict__ out, const int* __restrict__ meta, int heads, int P) {
+    pdl_launch_dependents();
+    pdl_wait();
+    const int lane = threadIdx.x & 31, item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), t = item / heads, h = item % heads;
+    if (t >= meta[META_NUM_TOKENS]) return;
+    const float* row = o + (size_t)item * P;
+    const T* gate = g + (size_t)t * g_stride + (size_t)h * P;
+    float v[K][4], gv[K][4], ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = (lane + 32 * k) * 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[k][j] = gv[k][j] = 0.f;
+        if (i < P) load4(row + i, v[k]), load4(gate + i, gv[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) ss = fmaf(v[k][j], v[k][j], ss);
+    const float inv = rsqrtf(warp_sum(ss) / (float)P + eps);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = (lane + 32 * k) * 4;
+        if (i >= P) continue;
+        float wv[4];
+        load4(w + i, wv);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wv[j] = v[k][j] * inv * wv[j] * silu_as<T>(gv[k][j]);
+        store4(out + (size_t)item * P + i, wv);
+    }
+}
+
+template <typename T>
+static int launch_head_norm_vec(const float* o, const T* g, long long g_stride, const float* w, float eps, T* out, const int* meta, int rows,
+                                int heads, int P, cudaStream_t stream) {
+    const int blocks = (rows * heads + 7) / 8;
+    if (P <= 128) return (int)launch_kernel(head_norm_gate_vec_kernel<T, 1>, blocks, 256, 0, stream, o, g, g_stride, w, eps, out, meta, heads, P);
+    if (P <= 256) return (int)launch_kernel(head_norm_gate_vec_kernel<T, 2>, blocks, 256, 0, stream, o, g, g_stride, w, eps, out, meta, heads, P);
+    return (int)launch_kernel(head_norm_gate_vec_kernel<T, 4>, blocks, 256, 0, stream, o, g, g_stride, w, eps, out, meta, heads, P);
+}
+
 extern "C" int head_norm_gate(const float* o, const void* g, int dtype, long long g_stride, const float* w, float eps, void* out,
                               const int* meta, int T, int heads, int P, cudaStream_t stream) {
     if (T <= 0) return 0;
+    const int esz = dtype == DT_F32 ? 4 : 2;
+    if ((long)T * heads >= 8 * 148 && P % 4 == 0 && P <= 512 && g_stride % 4 == 0 && (((uintptr_t)o | (uintptr_t)w) & 15) == 0 && ((uintptr_t)g | (uintptr_t)out) % (4 * esz) == 0) {
+        if (dtype == DT_F32) return launch_head_norm_vec(o, (const float*)g, g_stride, w, eps, (float*)out, meta, T, heads, P, stream);
+        return launch_head_norm_vec(o, (const __nv_bfloat16*)g, g_stride, w, eps, (__nv_bfloat16*)out, meta, T, heads, P, stream);
+    }
     const dim3 grid(T, (heads + 3) / 4);
     if (dtype == DT_F32)
         return (int)launch_kernel(head_norm_gate_kernel<float>, grid, 128, 0, stream, o, (const float*)g, g_stride, w, eps,

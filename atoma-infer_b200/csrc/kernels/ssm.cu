@@ -105,6 +105,89 @@ causal_conv_act_vec_kernel(const T* __restrict__ u, long long u_stride, const fl
     }
 }
 
+// The same for steps with prompt tokens: a thread takes V channels of CONV_TOKENS tokens, so weights, bias and all rows but the
+// first TAPS - 1 are loaded once (each token for itself read every row TAPS times and TAPS rows of float32 weights for one row of
+// results).  All of a thread's rows are in flight before the first is used.  Bound by memory: 2,048 tokens of 6,144 channels 25.6 us
+// against 35.5, of 4,096 18.5 against 25 (50 MB: 7.7 at the copy bandwidth; it still spends most of its issue slots on the activation).
+#define CONV_TOKENS 8
+template <typename T, int V, int TAPS>
+__global__ void __launch_bounds__(128)
+causal_conv_tile_kernel(const T* __restrict__ u, long long u_stride, const float* __restrict__ w, const float* __restrict__ bias,
+                        const float* __restrict__ state, long long slot_stride, T* __restrict__ y, const int* __restrict__ meta,
+                        const int* __restrict__ positions, const int* __restrict__ token_entry, const int* __restrict__ cu_tokens,
+                        const int* __restrict__ slots, int C, int act) {
+    constexpr int R = TAPS - 1;
+    struct alignas(V * sizeof(T)) Row { T x[V]; };
+    const int t0 = blockIdx.x * CONV_TOKENS, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
+    const int n = min(CONV_TOKENS, meta[META_NUM_TOKENS] - t0);
+    const bool live = n > 0 && c < C;
+    float wv[TAPS][V], bv[V];
+    if (live) {  // weights and bias depend on no earlier kernel: fetched before the wait
+#pragma unroll
+        for (int i = 0; i < V; i += 4) {
+            float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (bias) b = *reinterpret_cast<const float4*>(bias + c + i);
+            bv[i] = b.x, bv[i + 1] = b.y, bv[i + 2] = b.z, bv[i + 3] = b.w;
+#pragma unroll
+            for (int j = 0; j < TAPS; ++j) {
+                const float4 x = *reinterpret_cast<const float4*>(w + (size_t)j * C + c + i);
+                wv[j][i] = x.x, wv[j][i + 1] = x.y, wv[j][i + 2] = x.z, wv[j][i + 3] = x.w;
+            }
+        }
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    if (!live) return;
+    Row rows[CONV_TOKENS + R];  // tokens t0 - R ..: those ahead of t0 may belong to another entry, and are then not used
+#pragma unroll
+    for (int i = 0; i < CONV_TOKENS + R; ++i) {
+        const int t = t0 - R + i;
+        if (t >= 0 && t < t0 + n) rows[i] = *reinterpret_cast<const Row*>(u + (size_t)t * u_stride + c);
+    }
+#pragma unroll
+    for (int tt = 0; tt < CONV_TOKENS; ++tt) {
+        if (tt >= n) break;
+        const int t = t0 + tt, e = token_entry[t], p = positions[t], first = cu_tokens[e];
+        float acc[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i) acc[i] = bv[i];
+#pragma unroll
+        for (int j = 0; j < TAPS; ++j) {  // oldest tap first: a fixed order
+            const int back = R - j, src = p - back;
+            float v[V];
+            if (t - back >= first) {
+#pragma unroll
+                for (int i = 0; i < V; ++i) v[i] = to_float(rows[tt + j].x[i]);
+            } else if (src >= 0) {
+                const float* ring = state + (size_t)slots[e] * slot_stride + (size_t)(src % R) * C + c;
+#pragma unroll
+                for (int i = 0; i < V; ++i) v[i] = ring[i];
+            } else {
+                continue;
+            }
+#pragma unroll
+            for (int i = 0; i < V; ++i) acc[i] = fmaf(wv[j][i], v[i], acc[i]);
+        }
+        Row out;
+#pragma unroll
+        for (int i = 0; i < V; ++i) out.x[i] = from_float<T>(act == 1 ? silu_as<T>(acc[i]) : acc[i]);
+        *reinterpret_cast<Row*>(y + (size_t)t * C + c) = out;
+    }
+}
+
+template <typename T, int V>
+static int launch_conv_tile(const T* u, long long u_stride, const float* w, const float* bias, const float* state, long long slot_stride, T* y,
+                            const int* meta, const int* positions, const int* token_entry, const int* cu_tokens, const int* slots, int rows,
+                            int C, int taps, int act, cudaStream_t stream) {
+    const dim3 grid((rows + CONV_TOKENS - 1) / CONV_TOKENS, (C / V + 127) / 128);
+#define CONV_CASE(K)                                                                                                       \
+    case K: return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, causal_conv_tile_kernel<T, V, K>, grid, 128, 0, stream, u, u_stride, w, bias, \
+                                          state, slot_stride, y, meta, positions, token_entry, cu_tokens, slots, C, act);
+    switch (taps) { CONV_CASE(2) CONV_CASE(3) CONV_CASE(4) }
+#undef CONV_CASE
+    return (int)cudaErrorInvalidValue;
+}
+
 extern "C" int causal_conv_act(const void* u, int dtype, long long u_stride, const float* w, const float* bias,
                                float* state, long long slot_stride, void* y, const int* meta, const int* positions,
                                const int* token_entry, const int* cu_tokens, const int* slots, int T, int C, int taps,
@@ -114,6 +197,14 @@ extern "C" int causal_conv_act(const void* u, int dtype, long long u_stride, con
     const int V = dtype == DT_F32 ? 4 : 8;
     if (C % V == 0 && u_stride % V == 0 && slot_stride % 4 == 0 &&
         (((uintptr_t)u | (uintptr_t)w | (uintptr_t)bias | (uintptr_t)state | (uintptr_t)y) & 15) == 0) {
+        // two to four taps, unless the ring is updated on the way (one token an entry)
+        if (!save_own && taps >= 2 && taps <= 4) {
+            if (dtype == DT_F32)
+                return launch_conv_tile<float, 4>((const float*)u, u_stride, w, bias, state, slot_stride, (float*)y, meta, positions, token_entry,
+                                                  cu_tokens, slots, T, C, taps, act, stream);
+            return launch_conv_tile<__nv_bfloat16, 4>((const __nv_bfloat16*)u, u_stride, w, bias, state, slot_stride, (__nv_bfloat16*)y, meta,
+                                                      positions, token_entry, cu_tokens, slots, T, C, taps, act, stream);
+        }
         dim3 grid(T, (C / V + 127) / 128);
         if (dtype == DT_F32)
             return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, causal_conv_act_vec_kernel<float, 4>, grid, 128, 0, stream,
@@ -142,32 +233,31 @@ extern "C" int causal_conv_act_saves(const void* u, int dtype, long long u_strid
            (((uintptr_t)u | (uintptr_t)w | (uintptr_t)bias | (uintptr_t)state | (uintptr_t)y) & 15) == 0;
 }
 
-// The last R rows of u of every entry go to its ring.
+// The last R rows of u of every entry go to its ring.  A block an entry and row back from its end.
 template <typename T>
 __global__ void __launch_bounds__(256)
 causal_conv_save_kernel(const T* __restrict__ u, long long u_stride, float* __restrict__ state, long long slot_stride,
-                        const int* __restrict__ meta, const int* __restrict__ positions, const int* __restrict__ token_entry,
-                        const int* __restrict__ cu_tokens, const int* __restrict__ slots, int C, int R) {
+                        const int* __restrict__ meta, const int* __restrict__ positions, const int* __restrict__ cu_tokens,
+                        const int* __restrict__ slots, int C, int R) {
     pdl_launch_dependents();
     pdl_wait();
-    const int t = blockIdx.x;
-    if (t >= meta[META_NUM_TOKENS]) return;
-    const int e = token_entry[t];
-    if (t < cu_tokens[e + 1] - R) return;
-    float* st = state + (size_t)slots[e] * slot_stride + (size_t)(positions[t] % R) * C;
-    for (int c = threadIdx.x; c < C; c += blockDim.x) st[c] = to_float(u[(size_t)t * u_stride + c]);
+    const int e = blockIdx.y, c = blockIdx.z * blockDim.x + threadIdx.x;
+    if (e >= meta[META_NUM_ENTRIES] || c >= C) return;
+    const int t = cu_tokens[e + 1] - 1 - (int)blockIdx.x;
+    if (t < cu_tokens[e]) return;
+    state[(size_t)slots[e] * slot_stride + (size_t)(positions[t] % R) * C + c] = to_float(u[(size_t)t * u_stride + c]);
 }
 
 extern "C" int causal_conv_save(const void* u, int dtype, long long u_stride, float* state, long long slot_stride,
-                                const int* meta, const int* positions, const int* token_entry, const int* cu_tokens,
-                                const int* slots, int T, int C, int taps, cudaStream_t stream) {
-    if (T <= 0 || taps <= 1) return 0;
-    const int threads = C >= 1024 ? 256 : 128;
+                                const int* meta, const int* positions, const int* cu_tokens, const int* slots, int T, int S, int C,
+                                int taps, cudaStream_t stream) {
+    if (T <= 0 || S <= 0 || taps <= 1) return 0;
+    const dim3 grid(taps - 1, S, (C + 255) / 256);
     if (dtype == DT_F32)
-        return (int)launch_kernel(causal_conv_save_kernel<float>, T, threads, 0, stream, (const float*)u, u_stride, state,
-                                  slot_stride, meta, positions, token_entry, cu_tokens, slots, C, taps - 1);
-    return (int)launch_kernel(causal_conv_save_kernel<__nv_bfloat16>, T, threads, 0, stream, (const __nv_bfloat16*)u, u_stride,
-                              state, slot_stride, meta, positions, token_entry, cu_tokens, slots, C, taps - 1);
+        return (int)launch_kernel(causal_conv_save_kernel<float>, grid, 256, 0, stream, (const float*)u, u_stride, state,
+                                  slot_stride, meta, positions, cu_tokens, slots, C, taps - 1);
+    return (int)launch_kernel(causal_conv_save_kernel<__nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)u, u_stride,
+                              state, slot_stride, meta, positions, cu_tokens, slots, C, taps - 1);
 }
 
 // ----------------------------------------------------------------------------- the recurrence
@@ -546,6 +636,61 @@ gated_group_norm_kernel(const float* __restrict__ y, const T* __restrict__ z, lo
     }
 }
 
+// The same, a warp a (token, part) of at most 128 K values: four consecutive values a lane and 16-byte accesses, no barrier.
+// Bound by memory; a block a part spent its time in its three barriers: 2,048 rows of 4,096 in 8 parts 77 us, here 30 (67 MB:
+// 10.3 at the copy bandwidth; behind the scan, whose results and scratch fill the L2, it also waits for their way out: 19 alone).
+template <typename T, int K>
+__global__ void __launch_bounds__(256)
+gated_group_norm_warp_kernel(const float* __restrict__ y, const T* __restrict__ z, long long z_stride, const float* __restrict__ w,
+                             float eps, T* __restrict__ out, const int* __restrict__ meta, int n, int parts) {
+    const int lane = threadIdx.x & 31, item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int t = item / parts, len = n / parts, at = item % parts * len;
+    pdl_wait();
+    pdl_launch_dependents();
+    if (t >= meta[META_NUM_TOKENS]) return;
+    const float* yr = y + (size_t)t * n + at;
+    const T* zr = z + (size_t)t * z_stride + at;
+    float yv[K][4], zv[K][4], ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = (lane + 32 * k) * 4;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) yv[k][j] = zv[k][j] = 0.f;
+        if (i < len) load4(yr + i, yv[k]), load4(zr + i, zv[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            yv[k][j] *= silu_as<T>(zv[k][j]);
+            ss = fmaf(yv[k][j], yv[k][j], ss);
+        }
+    const float inv = rsqrtf(warp_sum(ss) / (float)len + eps);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = (lane + 32 * k) * 4;
+        if (i >= len) continue;
+        float wv[4];
+        load4(w + at + i, wv);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wv[j] = yv[k][j] * inv * wv[j];
+        store4(out + (size_t)t * n + at + i, wv);
+    }
+}
+
+template <typename T>
+static int launch_group_norm_warp(const float* y, const T* z, long long z_stride, const float* w, float eps, T* out, const int* meta, int rows,
+                                  int n, int parts, cudaStream_t stream) {
+    const int len = n / parts, blocks = (rows * parts + 7) / 8;
+#define NORM_CASE(K)                                                                                                       \
+    return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, gated_group_norm_warp_kernel<T, K>, blocks, 256, 0, stream, y, z, z_stride, w, \
+                                  eps, out, meta, n, parts)
+    if (len <= 256) NORM_CASE(2);
+    if (len <= 512) NORM_CASE(4);
+    NORM_CASE(8);
+#undef NORM_CASE
+}
+
 extern "C" int gated_group_norm(const float* y, const void* z, int dtype, long long z_stride, const float* w, float eps,
                                 void* out, const int* meta, int T, int n, int parts, cudaStream_t stream) {
     if (T <= 0) return 0;
@@ -553,6 +698,12 @@ extern "C" int gated_group_norm(const float* y, const void* z, int dtype, long l
     const int len = n / parts, threads = len >= 1024 ? 256 : 128;
     // four values per access: parts and rows start on multiples of four elements and the buffers on 16 bytes
     const int vec4 = len % 4 == 0 && z_stride % 4 == 0 && (((uintptr_t)y | (uintptr_t)z | (uintptr_t)w | (uintptr_t)out) & 15) == 0;
+    // enough parts for a block of eight a multiprocessor; with fewer a block a part is the faster one (4 rows: 28.7 against 29.7 us
+    // for a whole state-space layer)
+    if (vec4 && len <= 1024 && (long)T * parts >= 8 * 148) {
+        if (dtype == DT_F32) return launch_group_norm_warp(y, (const float*)z, z_stride, w, eps, (float*)out, meta, T, n, parts, stream);
+        return launch_group_norm_warp(y, (const __nv_bfloat16*)z, z_stride, w, eps, (__nv_bfloat16*)out, meta, T, n, parts, stream);
+    }
     if (dtype == DT_F32)
         return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, gated_group_norm_kernel<float>, dim3(T, parts), threads, 0, stream, y,
                                       (const float*)z, z_stride, w, eps, (float*)out, meta, n, parts, vec4);

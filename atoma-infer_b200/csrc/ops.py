@@ -709,9 +709,8 @@ class CudaOps:
         if taps > 1:
             up, us = self._rows(u, "causal_conv_save")
             self._check(self._mixers().causal_conv_save(up, _code(u), us, _p(state), self._slot_stride(state), _p(ctx.meta),
-                                                        _p(ctx.positions), _p(ctx.token_entry), _p(ctx.cu_tokens),
-                                                        _p(ctx.state_slots), ctx.T, u.shape[1], taps, self._stream()),
-                        "causal_conv_save")
+                                                        _p(ctx.positions), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.T, ctx.S,
+                                                        u.shape[1], taps, self._stream()), "causal_conv_save")
 
     SCAN_CHUNK = 64        # tokens of a chunk when a long portion's recurrence is cut into chunks that run side by side
     SCAN_CHUNK_FROM = 128  # ... which happens from this many tokens of the step's longest entry on
