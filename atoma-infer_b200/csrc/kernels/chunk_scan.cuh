@@ -123,7 +123,8 @@ __device__ __forceinline__ void chunk_logs(ChunkLogs& L, const ChunkArgs& A, int
 }
 // exp(c_t - c_s) for c_t <= c_s
 __device__ __forceinline__ float decay_between(float hi_t, float lo_t, float hi_s, float lo_s) {
-    return expf(fminf((hi_t - hi_s) + (lo_t - lo_s), 0.f));
+    const float d = (hi_t - hi_s) + (lo_t - lo_s);
+    return expf(d > 0.f ? 0.f : d);  // (what is no number stays none)
 }
 
 // Rows t0 .. t0 + nt of `src` (n of `ROW / 2` values wanted, zeros behind them and behind the rows) into a tile.
@@ -138,17 +139,18 @@ __device__ __forceinline__ void stage_rows(char* tile, const __nv_bfloat16* src,
     }
 }
 
-// Which chunk the step's `index`-th one is: its entry, its first token and its tokens, and whether it is the entry's only one.
+// Which chunk (of LEN tokens) the step's `index`-th one is: its entry, its first token and its tokens, and whether it is the entry's only one.
 // Every warp finds out by itself: a lane an entry, chunks counted up over the lanes.
 struct ChunkPlace {
     int e, t0, nt, only;
 };
-__device__ __forceinline__ bool chunk_of(const ChunkArgs& A, int index, ChunkPlace& p) {
-    const int entries = A.meta[META_NUM_ENTRIES], lane = threadIdx.x & 31;
+template <int LEN>
+__device__ __forceinline__ bool chunk_of(const int* __restrict__ meta, const int* __restrict__ cu_tokens, int index, ChunkPlace& p) {
+    const int entries = meta[META_NUM_ENTRIES], lane = threadIdx.x & 31;
     int before = 0;
     for (int e0 = 0; e0 < entries; e0 += 32) {
-        const int e = e0 + lane, first = e < entries ? A.cu_tokens[e] : 0, count = e < entries ? A.cu_tokens[e + 1] - first : 0;
-        const int own = (count + CHUNK - 1) / CHUNK;
+        const int e = e0 + lane, first = e < entries ? cu_tokens[e] : 0, count = e < entries ? cu_tokens[e + 1] - first : 0;
+        const int own = (count + LEN - 1) / LEN;
         int upto = own;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -159,8 +161,8 @@ __device__ __forceinline__ bool chunk_of(const ChunkArgs& A, int index, ChunkPla
         if (hit) {
             const int from = __ffs(hit) - 1, c = index - before - __shfl_sync(0xffffffffu, upto - own, from);
             p.e = e0 + from;
-            p.t0 = __shfl_sync(0xffffffffu, first, from) + c * CHUNK;
-            p.nt = min(__shfl_sync(0xffffffffu, count, from) - c * CHUNK, CHUNK);
+            p.t0 = __shfl_sync(0xffffffffu, first, from) + c * LEN;
+            p.nt = min(__shfl_sync(0xffffffffu, count, from) - c * LEN, LEN);
             p.only = __shfl_sync(0xffffffffu, own, from) == 1;
             return true;
         }
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(256, 2) chunk_states_kernel(const ChunkArgs A,
     pdl_launch_dependents();
     pdl_wait();
     ChunkPlace at;
-    if (!chunk_of(A, c, at)) return;
+    if (!chunk_of<CHUNK>(A.meta, A.cu_tokens, c, at)) return;
     const int t0 = at.t0, nt = at.nt;
     const int rows = (nt + 15) / 16 * 16;
     stage_rows<KROW>(ks, A.k + (size_t)(h / A.share) * A.N, A.k_stride, t0, nt, rows, A.N);
@@ -279,7 +281,7 @@ __global__ void __launch_bounds__(256, 2) chunk_states_kernel(const ChunkArgs A,
 
 // ----------------------------------------------------------------------------- the chunks' start states
 // In place: share -> S_in of the chunk, S_out = decay * S_in + share; the last one goes to the slot.  A thread walks four neighbouring
-// elements over the chunks, four chunks loaded ahead (one element a thread: four times the blocks, each a chain of dependent
+// elements over the chunks, four to eight chunks loaded ahead (one element a thread: four times the blocks, each a chain of dependent
 // loads before its first useful one: 42 against 35 us for 96 heads of 128 x 64 and three prompts of 17 chunks together).
 template <int KIND>
 __global__ void __launch_bounds__(256) chunk_chain_kernel(const ChunkArgs A) {
@@ -300,11 +302,15 @@ __global__ void __launch_bounds__(256) chunk_chain_kernel(const ChunkArgs A) {
     float* at = A.scratch + ((size_t)before * A.heads + h) * CS + i;
     const float* dec = A.decay + (size_t)before * A.heads + h;
     const size_t step = (size_t)A.heads * CS;
-    for (int c0 = 0; c0 < chunks; c0 += 4) {
-        float own[4][4], d[4];
+    float own[4][4], d[4], own_next[4][4], d_next[4];
+    auto fetch = [&](int c0, float (&x)[4][4], float (&f)[4]) {
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-            if (c0 + u < chunks) load4(at + (c0 + u) * step, own[u]), d[u] = dec[(size_t)(c0 + u) * A.heads];
+            if (c0 + u < chunks) load4(at + (c0 + u) * step, x[u]), f[u] = dec[(size_t)(c0 + u) * A.heads];
+    };
+    fetch(0, own, d);
+    for (int c0 = 0; c0 < chunks; c0 += 4) {
+        fetch(c0 + 4, own_next, d_next);  // ahead of the stores
 #pragma unroll
         for (int u = 0; u < 4; ++u)
             if (c0 + u < chunks) {
@@ -312,6 +318,12 @@ __global__ void __launch_bounds__(256) chunk_chain_kernel(const ChunkArgs A) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) s[j] = fmaf(d[u], s[j], own[u][j]);
             }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            d[u] = d_next[u];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) own[u][j] = own_next[u][j];
+        }
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) slot[j] = s[j];
@@ -332,7 +344,7 @@ __global__ void __launch_bounds__(256, 2) chunk_outputs_kernel(const ChunkArgs A
     pdl_launch_dependents();
     pdl_wait();
     ChunkPlace at;
-    if (!chunk_of(A, c, at)) return;
+    if (!chunk_of<CHUNK>(A.meta, A.cu_tokens, c, at)) return;
     const int t0 = at.t0, nt = at.nt;
     const int rows = (nt + 15) / 16 * 16;
     stage_rows<KROW>(qs, A.q + (size_t)(h / A.share) * A.N, A.q_stride, t0, nt, rows, A.N);

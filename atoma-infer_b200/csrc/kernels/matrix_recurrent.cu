@@ -7,6 +7,7 @@
 // Projections are stored as float32 or bfloat16; gates, states, norms and everything between are float32.
 #include "chunk_scan.cuh"
 #include "matrix_scan.cuh"
+#include "row_scan.cuh"
 
 int g_use_pdl = 1;
 extern "C" void kernels_set_pdl(int mode) { g_use_pdl = mode; }
@@ -29,6 +30,26 @@ extern "C" int bonus_scan(const void* r, long long r_stride, const void* k, long
     const ScanArgs a = {r, k, v, r_stride, k_stride, v_stride, dtype, z, z_bias, z_stride, 1.f, 1.f, state, slot_stride, o, meta,
                         cu_tokens, slots, S, heads, N, P, chunk_len, max_chunks, scratch, 0, ex};
     return run_matrix_scan<SCAN_BONUS>(a, stream);
+}
+
+// The same for bfloat16 prompts as matrix products over chunks of RCHUNK tokens (row_scan.cuh; head floats and rounds as gla_row_scan).
+extern "C" size_t bonus_row_scan_head_floats(const void* r, long long r_stride, const void* k, long long k_stride, const void* v, long long v_stride,
+                                             const float* o, int N, int P, int max_chunks) {
+    return chunk_scan_takes(r, k, v, r_stride, k_stride, v_stride, o, N, P) && max_chunks <= 65535 ? row_scan_head_floats(N, P, max_chunks) : 0;
+}
+
+extern "C" int bonus_row_scan(const void* r, long long r_stride, const void* k, long long k_stride, const void* v, long long v_stride,
+                              const float* z, long long z_stride, const float* z_bias, const float* bonus, float* state,
+                              long long slot_stride, float* o, const int* meta, const int* cu_tokens, const int* slots, int S, int heads,
+                              int N, int P, int max_chunks, float* scratch, size_t scratch_floats, cudaStream_t stream) {
+    RowScanArgs a = {};
+    a.q = (const __nv_bfloat16*)r, a.k = (const __nv_bfloat16*)k, a.v = (const __nv_bfloat16*)v;
+    a.q_stride = r_stride, a.k_stride = k_stride, a.v_stride = v_stride;
+    a.z = z, a.z_stride = z_stride, a.z_bias = z_bias, a.bonus = bonus, a.inv_tau = a.q_scale = 1.f;
+    a.state = state, a.slot_stride = slot_stride, a.o = o;
+    a.meta = meta, a.cu_tokens = cu_tokens, a.slots = slots;
+    a.S = S, a.heads = heads, a.N = N, a.P = P, a.max_chunks = max_chunks;
+    return row_scan<ROW_BONUS>(a, scratch, scratch_floats, stream);
 }
 
 extern "C" size_t memory_scan_scratch_floats(int S, int heads, int N, int P, int max_chunks) {

@@ -9,6 +9,7 @@
 // amount to, a small kernel chains the chunks' start states in order, pass 3 runs every chunk again from its start
 // state and writes the outputs, the last chunk the slot.  Every sum runs in an order that depends on the sizes only.
 #include "matrix_scan.cuh"
+#include "row_scan.cuh"
 
 int g_use_pdl = 1;
 extern "C" void kernels_set_pdl(int mode) { g_use_pdl = mode; }
@@ -40,6 +41,29 @@ extern "C" int gla_scan(const void* q, long long q_stride, const void* k, long l
                         int S, int heads, int N, int P, int chunk_len, int max_chunks, float* scratch, cudaStream_t stream) {
     return gla_scan_mode(q, q_stride, k, k_stride, v, v_stride, dtype, z, z_stride, z_bias, tau, q_scale, state, slot_stride, o, meta,
                          cu_tokens, slots, S, heads, N, P, chunk_len, max_chunks, scratch, 0, stream);
+}
+
+// The same for bfloat16 prompts with decay logits, as matrix products over chunks of RCHUNK tokens (row_scan.cuh).  max_chunks: at least
+// the chunks of all entries together.  gla_row_scan_head_floats: scratch of one head, 0 where the sizes or addresses are not served;
+// with scratch for fewer than all heads they run in rounds.
+extern "C" size_t gla_row_scan_head_floats(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
+                                           const float* o, int N, int P, int max_chunks) {
+    return chunk_scan_takes(q, k, v, q_stride, k_stride, v_stride, o, N, P) && max_chunks <= 65535 ? row_scan_head_floats(N, P, max_chunks) : 0;
+}
+
+extern "C" int gla_row_scan(const void* q, long long q_stride, const void* k, long long k_stride, const void* v, long long v_stride,
+                            const float* z, long long z_stride, const float* z_bias, float tau, float q_scale, float* state,
+                            long long slot_stride, float* o, const int* meta, const int* cu_tokens, const int* slots, int S, int heads,
+                            int N, int P, int max_chunks, float* scratch, size_t scratch_floats, cudaStream_t stream) {
+    if (S > 0 && (!z || tau <= 0.f)) return (int)cudaErrorInvalidValue;
+    RowScanArgs a = {};
+    a.q = (const __nv_bfloat16*)q, a.k = (const __nv_bfloat16*)k, a.v = (const __nv_bfloat16*)v;
+    a.q_stride = q_stride, a.k_stride = k_stride, a.v_stride = v_stride;
+    a.z = z, a.z_stride = z_stride, a.z_bias = z_bias, a.inv_tau = 1.f / tau, a.q_scale = q_scale;
+    a.state = state, a.slot_stride = slot_stride, a.o = o;
+    a.meta = meta, a.cu_tokens = cu_tokens, a.slots = slots;
+    a.S = S, a.heads = heads, a.N = N, a.P = P, a.max_chunks = max_chunks;
+    return row_scan<ROW_DECAY>(a, scratch, scratch_floats, stream);
 }
 
 // ----------------------------------------------------------------------------- norm per head, shared weight, gate

@@ -897,6 +897,7 @@ class CudaOps:
         if lib is None:
             lib = self._recurrent_lib = build.load_library("recurrent", RECURRENT_SOURCES, cuda=True)
             lib.gla_scan_scratch_floats.restype = ctypes.c_size_t
+            lib.gla_row_scan_head_floats.restype = ctypes.c_size_t
             lib.selective_scan_scratch_floats.restype = ctypes.c_size_t
             lib.kernels_set_pdl(int(self.pdl))
         return lib
@@ -909,6 +910,26 @@ class CudaOps:
         while chunk and longest // chunk > 256:
             chunk *= 2
         return chunk, (-(-longest // chunk) if chunk else 1)
+
+    ROW_SCAN_CHUNK = 64           # tokens of a chunk of kernels/row_scan.cuh
+    ROW_SCAN_SCRATCH = 24 << 20   # floats of scratch (96 MB) that are taken even where the other kernel would take fewer
+
+    def _row_scan(self, lib, name: str, rows, q, ctx, o, heads: int, dim: int, vdim: int, chunk: int, chunks: int):
+        """bfloat16 prompts whose state decays by a number per row run as matrix products over chunks of 64 tokens
+        (kernels/row_scan.cuh) where the other kernel would cut them into chunks of time.  Its scratch holds the chunks' operands
+        beside their states, about twice the other's; where that is more than the other kernel would take and more than
+        ROW_SCAN_SCRATCH, the heads run in rounds, and where not one head fits, the other kernel runs.  Returns (at least the
+        chunks of all entries together, scratch), or None."""
+        if not chunk or not self.matrix_scan or q.dtype != torch.bfloat16:
+            return None
+        most = ctx.T // self.ROW_SCAN_CHUNK + ctx.S
+        head = getattr(lib, name + "_row_scan_head_floats")(*rows, _p(o), dim, vdim, most)
+        room = max(getattr(lib, name + "_scan_scratch_floats")(ctx.S, heads, dim, vdim, chunks), self.ROW_SCAN_SCRATCH)
+        at_once = min(heads, room // head) if head else 0
+        if not at_once:
+            return None
+        self.launches += 4 * -(-heads // at_once) - 1
+        return most, torch.empty(at_once * head, dtype=torch.float32, device=o.device)
 
     @staticmethod
     def _slot_state(state, shape, what: str):
@@ -938,6 +959,13 @@ class CudaOps:
             zp, zs = self._rows(z, "gla_scan")
         mode = (1 if head_decay is not None else 0) | (2 if silu else 0)
         chunk, chunks = self._scan_chunks(ctx)
+        rows = self._row_scan(lib, "gla", (qp, qs, kp, ks, vp, vs), q, ctx, o, heads, dim, vdim, chunk, chunks) if not mode else None
+        if rows is not None:
+            chunks, scratch = rows
+            self._check(lib.gla_row_scan(qp, qs, kp, ks, vp, vs, zp, zs, _p(z_bias), ctypes.c_float(tau), ctypes.c_float(q_scale), _p(state),
+                                         slot_stride, _p(o), _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, heads, dim, vdim,
+                                         chunks, _p(scratch), ctypes.c_size_t(scratch.numel()), self._stream()), "gla_row_scan")
+            return
         scratch = (torch.empty(lib.gla_scan_scratch_floats(ctx.S, heads, dim, vdim, chunks), dtype=torch.float32, device=o.device)
                    if chunk else None)
         self._check(lib.gla_scan_mode(qp, qs, kp, ks, vp, vs, _code(q), zp, zs, _p(z_bias), ctypes.c_float(tau), ctypes.c_float(q_scale),
@@ -1181,6 +1209,7 @@ class CudaOps:
         if lib is None:
             lib = self._matrix_recurrent_lib = build.load_library("matrix_recurrent", MATRIX_RECURRENT_SOURCES, cuda=True)
             lib.bonus_scan_scratch_floats.restype = ctypes.c_size_t
+            lib.bonus_row_scan_head_floats.restype = ctypes.c_size_t
             lib.memory_scan_scratch_floats.restype = ctypes.c_size_t
             lib.memory_chunk_scan_scratch_floats.restype = ctypes.c_size_t
             lib.kernels_set_pdl(int(self.pdl))
@@ -1199,6 +1228,13 @@ class CudaOps:
             raise KernelError("bonus_scan: bonus and the logits' bias are one number per head and key channel")
         (rp, rs), (kp, ks), (vp, vs), (zp, zs) = (self._rows(t, "bonus_scan") for t in (r, k, v, z))
         chunk, chunks = self._scan_chunks(ctx)
+        rows = self._row_scan(lib, "bonus", (rp, rs, kp, ks, vp, vs), r, ctx, o, heads, dim, vdim, chunk, chunks)
+        if rows is not None:
+            chunks, scratch = rows
+            self._check(lib.bonus_row_scan(rp, rs, kp, ks, vp, vs, zp, zs, _p(z_bias), _p(bonus), _p(state), slot_stride, _p(o), _p(ctx.meta),
+                                           _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, heads, dim, vdim, chunks, _p(scratch),
+                                           ctypes.c_size_t(scratch.numel()), self._stream()), "bonus_row_scan")
+            return
         scratch = (torch.empty(lib.bonus_scan_scratch_floats(ctx.S, heads, dim, vdim, chunks), dtype=torch.float32, device=o.device)
                    if chunk else None)
         self._check(lib.bonus_scan(rp, rs, kp, ks, vp, vs, _code(r), zp, zs, _p(z_bias), _p(bonus), _p(state), slot_stride, _p(o),

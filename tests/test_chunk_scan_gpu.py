@@ -1,6 +1,8 @@
 """The scans that run as matrix products over chunks of 128 tokens, at the sizes where that can go wrong: rows of state that fill a
 tile partly, columns that leave a part of a block of 64, chunks of 1, 16, 17, 127 and 128 tokens, entries with one chunk beside
 entries with several, slots that start on any float.  Against a float64 restatement."""
+import ctypes
+
 import pytest
 import torch
 
@@ -27,10 +29,11 @@ def context(rt, lengths):
 
 
 def scan(q, k, v, log_a, b, S):
-    """q, k [T, H, N], v [T, H, P], log_a and b [T, H], S [H, N, P], all float64: the outputs and the last state."""
+    """q, k [T, H, N], v [T, H, P], log_a [T, H] or per row [T, H, N], b [T, H], S [H, N, P], all float64: the outputs and the last
+    state."""
     out = torch.empty_like(v)
     for t in range(q.shape[0]):
-        S = torch.exp(log_a[t])[:, None, None] * S + (b[t][:, None] * k[t])[:, :, None] * v[t][:, None, :]
+        S = torch.exp(log_a[t]).view(q.shape[1], -1, 1) * S + (b[t][:, None] * k[t])[:, :, None] * v[t][:, None, :]
         out[t] = torch.einsum("hnp,hn->hp", S, q[t])
     return out, S
 
@@ -133,4 +136,64 @@ def test_matrix_memory_in_matrix_chunks(rt, lengths, heads, dim, vdim):
         return err(o, wo), err(nq, wn), err(state, ws[0]), err(n_state, ws[1]), err(m_state, ws[2])
 
     new, old = both(rt, run)
+    assert max(new) < TOL, (new, old)
+
+
+@pytest.mark.parametrize("lengths", [(128,), (129, 1, 16), (127, 17, 64, 300, 2)])
+@pytest.mark.parametrize("heads,dim,vdim", [(3, 128, 256), (2, 8, 72), (2, 64, 64), (1, 104, 8), (2, 40, 16)])
+@pytest.mark.parametrize("kind", ["decay", "bonus"])
+@pytest.mark.parametrize("rounds", [False, True])
+def test_a_decay_per_row_in_matrix_chunks(rt, lengths, heads, dim, vdim, kind, rounds):
+    """Sub-blocks of 16 tokens and triangles of 8 inside chunks of 64; strong decays (rows that forget within a token, whose logs sum
+    to thousands within a chunk) beside weak ones; all heads at once, and in rounds of one where scratch is short."""
+    g = torch.Generator().manual_seed(heads * dim + vdim + len(lengths))
+    T, nk, nv, tau = sum(lengths), heads * dim, heads * vdim, 2.0
+    rows = torch.randn(T, 2 * nk + nv + 8, generator=g).bfloat16()
+    z, bias, u = torch.randn(T, nk, generator=g) * 2, torch.randn(nk, generator=g), torch.randn(nk, generator=g)
+    z[:, 1::7] += 6 if kind == "bonus" else -60  # decays of nearly zero
+    z[:, 2::7] -= 9 if kind == "bonus" else -9   # and of nearly one
+    S0 = torch.randn(len(lengths), nk * vdim + 5, generator=g) * 0.5
+    want, wo, at = {}, [], 0
+    for e, n in enumerate(lengths):
+        x, x_z = rows[at:at + n].double(), (z[at:at + n].double() + bias.double()).view(n, heads, dim)
+        slot = len(lengths) - 1 - e
+        q, k, v = x[:, :nk].view(n, heads, dim), x[:, nk:2 * nk].view(n, heads, dim), x[:, 2 * nk:2 * nk + nv].view(n, heads, vdim)
+        log_a = -torch.exp(x_z) if kind == "bonus" else -torch.nn.functional.softplus(-x_z, threshold=50) / tau
+        S = S0[slot, 3:3 + nk * vdim].view(heads, dim, vdim).double()
+        if kind == "decay":
+            o, S = scan(q * dim ** -0.5, k, v, log_a, torch.ones(n, heads, dtype=torch.float64), S)
+        else:
+            o = torch.empty_like(v)
+            for t in range(n):
+                kv = k[t][:, :, None] * v[t][:, None, :]
+                o[t] = torch.einsum("hnp,hn->hp", S + u.double().view(heads, dim, 1) * kv, q[t])
+                S = torch.exp(log_a[t])[:, :, None] * S + kv
+        wo.append(o.reshape(n, nv))
+        want[slot] = S
+        at += n
+    wo, ws = torch.cat(wo), torch.stack([want[k] for k in range(len(lengths))])
+    ctx, dev = context(rt, lengths), lambda t: t.to(rt.device)
+
+    def run():
+        st, o, r = dev(S0.clone()), torch.full((T, nv), float("nan"), device=rt.device), dev(rows)
+        state = st[:, 3:3 + nk * vdim].view(len(lengths), heads, dim, vdim)
+        parts = r[:, :nk], r[:, nk:2 * nk], r[:, 2 * nk:2 * nk + nv]
+        if kind == "decay":
+            rt.ops.gla_scan(*parts, dev(z), dev(bias), tau, dim ** -0.5, state, ctx, o, heads=heads, dim=dim, vdim=vdim)
+        else:
+            rt.ops.bonus_scan(*parts, dev(z), dev(bias), dev(u), state, ctx, o, heads=heads, dim=dim, vdim=vdim)
+        assert torch.equal(st[:, :3].cpu(), S0[:, :3]) and torch.equal(st[:, -2:].cpu(), S0[:, -2:])
+        return err(o, wo), err(state, ws)
+
+    if rounds:
+        lib = rt.ops._recurrent() if kind == "decay" else rt.ops._matrix_recurrent()
+        x = torch.empty(16, device=rt.device, dtype=torch.bfloat16)
+        p, stride = ctypes.c_void_p(x.data_ptr()), ctypes.c_longlong(8)
+        head = getattr(lib, ("gla" if kind == "decay" else "bonus") + "_row_scan_head_floats")(p, stride, p, stride, p, stride, p, dim, vdim,
+                                                                                               ctx.T // 64 + ctx.S)
+        rt.ops.ROW_SCAN_SCRATCH = head + 100  # at least one head's; the other kernel's scratch may make it more
+    try:
+        new, old = both(rt, run)
+    finally:
+        rt.ops.ROW_SCAN_SCRATCH = type(rt.ops).ROW_SCAN_SCRATCH
     assert max(new) < TOL, (new, old)
