@@ -3,9 +3,9 @@
 // One block = 128 query rows ((token, query head of the group) pairs of one key/value head) of one
 // request, walking that request's keys 128 at a time through the block table.  The block's warps
 // have three jobs and talk through mbarriers only (no block-wide barrier inside the key loop):
-//   * a copy warp: K and V pages travel by TMA (one box per page, 128-byte swizzle) straight from
-//     the paged cache into two-stage shared-memory rings; the page ids come from the block table
-//     in shared memory;
+//   * two copy warps, one for K and one for V: pages travel by TMA (one box per page, 128-byte swizzle)
+//     straight from the paged cache into two-stage shared-memory rings; the page ids come from the
+//     block table in shared memory;
 //   * an MMA warp (one elected thread): S = Q K^T is one tcgen05.mma chain (M = 128, N = 128,
 //     K = head size) into tensor memory; O += P V is a second chain whose A operand P is read from
 //     tensor memory and whose B operand V is read MN-major from shared memory (no transpose copy); O
@@ -17,7 +17,10 @@
 //     grows by less than 2^8 the old base stays, so O (in tensor memory) and the row sum are scaled
 //     down only now and then, by the softmax threads, between two P V products.
 // So the tensor core computes the next tile's scores while the exponentials of the current tile run,
-// and the copies run two tiles ahead.  Two blocks fit a multiprocessor for
+// and the copies run two tiles ahead.  (A K stage is free long before a V stage: one warp that waited for both in turn
+// started K so late that every tile's scores waited some 2,000 clocks for it.  A box a page and 64-column half
+// instead of one a page kept the copy engine, which starts a box in about a hundred clocks, busy for longer than a
+// tile takes.  32 heads of 128 over 8, 4,096 tokens: 247 -> 217 us; over 4, 16,384 tokens: 3,111 -> 2,579 us.)  Two blocks fit a multiprocessor for
 // head size 64; the softmax warps then take registers that the other two warps give up.
 // A portion of a prompt that starts inside a cached context attends to all of it.
 //
@@ -46,13 +49,14 @@ constexpr int BKV = 128;           // keys per tile
 // key loop: P V of every tile is added to it by the tensor core itself.
 constexpr uint32_t S_COL = 0, P_COL = 128, O_COL = 192;
 constexpr uint32_t TMEM_COLS = D == 64 ? 256 : 512;
+constexpr int GROUP_BYTES = HALVES * 1024;  // from one group of 8 rows of K or V to the next, all halves of a row in between
 constexpr bool ONE_PLANE = D == 256;  // keys and values are the same vectors: only the key plane is read
 // The exponentials of a row use one base until the row's maximum has grown by more than this (in powers of two):
 // only then are O and the row's sum scaled down.  P then stays below 2^8, far inside the range of bfloat16.
 constexpr float RESCALE_STEP = 8.f;
 constexpr int SOFTMAX_THREADS = 256, SOFTMAX_WARPS = 8;
-constexpr int COPY_WARP = 8, MMA_WARP = 9;
-constexpr int TC_THREADS = 384;  // three warpgroups: two of softmax warps, one with the copy and the MMA warp
+constexpr int COPY_WARP = 8, MMA_WARP = 9, COPY_V_WARP = 10;
+constexpr int TC_THREADS = 384;  // three warpgroups: two of softmax warps, one with the copy warps and the MMA warp
 
 }  // namespace
 
@@ -156,51 +160,42 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
 
     if (warp >= SOFTMAX_WARPS) {
         if (D == 64) regs_release<32>();
-        if (warp == COPY_WARP) {
+        if (warp == COPY_WARP || (warp == COPY_V_WARP && !STATS && !ONE_PLANE)) {
             // ------------------------------------------------------------------ copies, two tiles ahead
-            // The K (kv = 0) or V (kv = 1) rows of tile t: one box of `ps` rows per page, per 64-column half.
-            // Lane 0 announces the bytes, then lane i starts the boxes of page i (starting a copy costs
+            // The K (kv = 0) or V (kv = 1) rows of tile t: one box per page.
+            // Lane 0 announces the bytes, then lane i starts the box of page i (starting a copy costs
             // about a hundred cycles; eight pages started by one thread would take eight times as long).
-            auto issue_loads = [&](int t, int kv, unsigned char* dst, uint64_t* bar) {
+            const int kv = warp == COPY_V_WARP;
+            unsigned char* ring = kv ? v_s : k_s;
+            uint64_t* full = kv ? v_full : k_full;
+            // a K stage is free when the scores of its tile are done (with one plane: when its P V is), a V stage when its P V is
+            uint64_t* empty = !STATS && (ONE_PLANE || kv) ? pv_done : s_done;
+            auto start = [&](int t) {
                 const int k0 = k_first + t * BKV;
                 const int pg = lane, pidx = k0 / ps + pg - page_lo;
                 const bool mine = pg < BKV / ps && pidx < page_cnt && bt_s[pidx] > 0;
                 const uint32_t pages = __popc(__ballot_sync(0xffffffffu, mine));
+                uint64_t* bar = &full[t & 1];
                 if (lane == 0) mbar_expect_tx(bar, pages * (uint32_t)ps * 128u * HALVES);
                 __syncwarp();
                 if (mine) {
                     int r = ((bt_s[pidx] * 2 + kv) * L.num_kv_heads + kvh) * ps;  // row of the page's first slot in the cache as a matrix
-#pragma unroll
-                    for (int h = 0; h < HALVES; ++h)
-                        tma_load_2d(dst + h * HALF_BYTES + pg * ps * 128, &map_kv, h * 64, r, bar);
+                    tma_load_4d(ring + (t & 1) * STAGE + pg * ps * 128 * HALVES, &map_kv, 0, 0, 0, r / 8, bar);
                 }
             };
-            int last_k[2] = {-1, -1}, last_v[2] = {-1, -1};  // the last tile whose copy was started into a stage
-            for (int t = 0; t < 2 && t < ntiles; ++t) { issue_loads(t, 0, k_s + t * STAGE, &k_full[t]); last_k[t] = t; }
-            for (int t = 0; !STATS && !ONE_PLANE && t < 2 && t < ntiles; ++t) { issue_loads(t, 1, v_s + t * STAGE, &v_full[t]); last_v[t] = t; }
-            bool ok = true;
+            int last[2] = {-1, -1};  // the last tile whose copy was started into a stage
+            for (int t = 0; t < 2 && t < ntiles; ++t) { start(t); last[t] = t; }
             for (int t = 0; t + 2 < ntiles; ++t) {
                 const int b = t & 1;
-                const uint32_t par = (uint32_t)(t >> 1) & 1u;
-                // the scores of tile t are done: its K stage is free (with one plane: its P V is)
-                ok = mbar_wait(ONE_PLANE && !STATS ? &pv_done[b] : &s_done[b], par, status, abort_flag);
-                if (!ok) break;
-                issue_loads(t + 2, 0, k_s + b * STAGE, &k_full[b]);
-                last_k[b] = t + 2;
-                if constexpr (STATS || ONE_PLANE) continue;
-                ok = mbar_wait(&pv_done[b], par, status, abort_flag);  // P V of tile t is done: its V stage is free
-                if (!ok) break;
-                issue_loads(t + 2, 1, v_s + b * STAGE, &v_full[b]);
-                last_v[b] = t + 2;
+                if (!mbar_wait(&empty[b], (uint32_t)(t >> 1) & 1u, status, abort_flag)) break;
+                start(t + 2);
+                last[b] = t + 2;
             }
             if (*abort_flag && lane == 0) {
                 // somebody gave up on a barrier: let the copies in flight land (bounded) before the block leaves
-                for (int b = 0; b < 2; ++b) {
-                    if (last_k[b] >= 0)
-                        for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try_wait(&k_full[b], (uint32_t)(last_k[b] >> 1) & 1u); ++i) {}
-                    if (last_v[b] >= 0)
-                        for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try_wait(&v_full[b], (uint32_t)(last_v[b] >> 1) & 1u); ++i) {}
-                }
+                for (int b = 0; b < 2; ++b)
+                    if (last[b] >= 0)
+                        for (uint32_t i = 0; i < WAIT_LIMIT && !mbar_try_wait(&full[b], (uint32_t)(last[b] >> 1) & 1u); ++i) {}
             }
         } else if (warp == MMA_WARP && lane == 0) {
             // ------------------------------------------------------------------ the tensor core's instruction stream
@@ -212,11 +207,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
                 if (!ok) return;
                 tc_fence_after();
 #pragma unroll
-                for (int kd = 0; kd < D / 16; ++kd) {
-                    uint32_t off = (kd / 4) * HALF_BYTES + (kd % 4) * 32;
-                    umma_bf16(tmem_base + S_COL, make_desc(smem_u32(q_s) + off, 0),
-                              make_desc(smem_u32(k_s) + b * STAGE + off, 0), idesc_s, kd > 0);
-                }
+                for (int kd = 0; kd < D / 16; ++kd)
+                    umma_bf16(tmem_base + S_COL, make_desc(smem_u32(q_s) + (kd / 4) * HALF_BYTES + (kd % 4) * 32, 0),
+                              make_desc(smem_u32(k_s) + b * STAGE + (kd / 4) * 1024 + (kd % 4) * 32, 0, GROUP_BYTES), idesc_s, kd > 0);
                 umma_commit(&s_done[b]);
             };
             issue_scores(0);
@@ -238,7 +231,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
                 tc_fence_after();
 #pragma unroll
                 for (int ks = 0; ks < BKV / 16; ++ks) {
-                    uint64_t bd = make_desc(smem_u32(v_s) + b * STAGE + ks * 16 * 128, HALF_BYTES);
+                    uint64_t bd = make_desc(smem_u32(v_s) + b * STAGE + ks * 2 * GROUP_BYTES, 1024, GROUP_BYTES);
                     umma_bf16_a_tmem(tmem_base + O_COL, tmem_base + P_COL + ks * 8, bd, idesc_o, (t > 0 || ks > 0) ? 1u : 0u);
                 }
                 umma_commit(&pv_done[b]);
@@ -360,7 +353,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
                     if (!have) {
 #pragma unroll
                         for (int c = 0; c < D / 8; ++c)
-                            *reinterpret_cast<uint4*>(v_s + b * STAGE + (c / 8) * HALF_BYTES + swz(row, c % 8)) = make_uint4(0u, 0u, 0u, 0u);
+                            *reinterpret_cast<uint4*>(v_s + b * STAGE + (row / 8) * GROUP_BYTES + (c / 8) * 1024 + swz(row % 8, c % 8)) = make_uint4(0u, 0u, 0u, 0u);
                         fence_async_smem();
                     }
                 }
@@ -421,7 +414,7 @@ int table_slice(int max_context, int page_size, int tpt, int window, int chunk) 
 
 extern "C" int attn_tc_head_dim() { return D; }
 
-// Page sizes this kernel takes: one TMA box per page, boxes that tile a 128-key tile and start on a swizzle atom.
+// Page sizes this kernel takes: one TMA box per page, boxes that tile a 128-key tile and hold whole groups of 8 rows.
 extern "C" int attn_prefill_tc_supports(int page_size, int nq, int nkv) {
     bool ps_ok = page_size >= 8 && page_size <= 128 && (page_size & (page_size - 1)) == 0;
     return ps_ok && nq % nkv == 0 && nq / nkv <= 16;
@@ -457,7 +450,7 @@ extern "C" int attn_prefill_tc_scores(const void* q, int q_stride, const void* c
     if (S <= 0 || max_q_len <= 0) return 0;
     if (!attn_prefill_tc_supports(page_size, nq, nkv)) return (int)cudaErrorInvalidValue;
     CUtensorMap map;
-    if (!cache_map(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;
+    if (!cache_map_groups(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;
     CacheLayout L{nkv, page_size, D};
     const int tpt = BQ / (nq / nkv);
     const int bt_cap = table_slice(max_context, page_size, tpt, window, chunk);
@@ -491,7 +484,7 @@ extern "C" int attn_prefill_tc_stats(const void* q, int q_stride, const void* ca
     if (S <= 0 || max_q_len <= 0) return 0;
     if (!attn_prefill_tc_supports(page_size, nq, nkv) || scale <= 0.f) return (int)cudaErrorInvalidValue;
     CUtensorMap map;
-    if (!cache_map(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;
+    if (!cache_map_groups(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;
     CacheLayout L{nkv, page_size, D};
     const int tpt = BQ / (nq / nkv);
     const int bt_cap = table_slice(max_context, page_size, tpt, 0, chunk);
