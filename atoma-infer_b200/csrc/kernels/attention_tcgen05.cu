@@ -55,8 +55,8 @@ constexpr bool ONE_PLANE = D == 256;  // keys and values are the same vectors: o
 // only then are O and the row's sum scaled down.  P then stays below 2^8, far inside the range of bfloat16.
 constexpr float RESCALE_STEP = 8.f;
 constexpr int SOFTMAX_THREADS = 256, SOFTMAX_WARPS = 8;
-constexpr int COPY_WARP = 8, MMA_WARP = 9, COPY_V_WARP = 10;
-constexpr int TC_THREADS = 384;  // three warpgroups: two of softmax warps, one with the copy warps and the MMA warp
+constexpr int COPY_WARP = 8, MMA_WARP = 9, COPY_V_WARP = 10, MMA_PV_WARP = 11;
+constexpr int TC_THREADS = 384;  // three warpgroups: two of softmax warps, one with the copy and the MMA warps
 
 }  // namespace
 
@@ -199,7 +199,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
             }
         } else if (warp == MMA_WARP && lane == 0) {
             // ------------------------------------------------------------------ the tensor core's instruction stream
-            constexpr uint32_t idesc_s = make_idesc(BQ, BKV, false), idesc_o = make_idesc(BQ, D, true);
+            constexpr uint32_t idesc_s = make_idesc(BQ, BKV, false);
             bool ok = true;
             auto issue_scores = [&](int t) {  // S(t) = Q K(t)^T
                 const int b = t & 1;
@@ -212,22 +212,17 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
                               make_desc(smem_u32(k_s) + b * STAGE + (kd / 4) * 1024 + (kd % 4) * 32, 0, GROUP_BYTES), idesc_s, kd > 0);
                 umma_commit(&s_done[b]);
             };
-            issue_scores(0);
             for (int t = 0; t < ntiles && ok; ++t) {
+                // the softmax warps hold the scores of the tile before in registers: this tile's may take their place
+                if (t > 0) ok = mbar_wait(s_free, (uint32_t)(t - 1) & 1u, status, abort_flag);
+                if (ok) issue_scores(t);
+            }
+        } else if (warp == MMA_PV_WARP && lane == 0 && !STATS) {
+            constexpr uint32_t idesc_o = make_idesc(BQ, D, true);
+            for (int t = 0; t < ntiles; ++t) {
                 const int b = t & 1;
-                const uint32_t par = (uint32_t)(t >> 1) & 1u;
-                if (t + 1 < ntiles) {
-                    // the softmax warps hold the scores of tile t in registers: the next tile's may take their place
-                    ok = mbar_wait(s_free, (uint32_t)t & 1u, status, abort_flag);
-                    if (!ok) break;
-                    issue_scores(t + 1);
-                    if (!ok) break;
-                }
-                if constexpr (STATS) continue;
-                ok = mbar_wait(p_ready, (uint32_t)t & 1u, status, abort_flag);  // P(t) is in tensor memory, O is scaled
-                if (!ok) break;
-                if constexpr (!ONE_PLANE) ok = mbar_wait(&v_full[b], par, status, abort_flag);  // (one plane: it was there for the scores)
-                if (!ok) break;
+                if (!mbar_wait(p_ready, (uint32_t)t & 1u, status, abort_flag)) break;  // P(t) is in tensor memory, O is scaled
+                if (!ONE_PLANE && !mbar_wait(&v_full[b], (uint32_t)(t >> 1) & 1u, status, abort_flag)) break;  // (one plane: it was there for the scores)
                 tc_fence_after();
 #pragma unroll
                 for (int ks = 0; ks < BKV / 16; ++ks) {
