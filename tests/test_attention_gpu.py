@@ -235,6 +235,22 @@ def test_head_sizes_beyond_the_kernels_are_refused(rts):
         run_attention(rts["bfloat16"], [(0, 4)], 1, 1, 528, 16)
 
 
+@pytest.mark.parametrize("blocks", [1, 7, 61, 444])
+@pytest.mark.parametrize("d,nq,nkv,page,window", [(64, 8, 2, 16, None), (128, 4, 2, 16, 90), (96, 3, 1, 8, None)])
+def test_decode_flat_deals_out_requests_of_any_length(rts, d, nq, nkv, page, window, blocks):
+    """Requests of one key beside long ones: runs of a block that hold only what a pair counts beside its tiles, pairs cut inside
+    and right behind that, and as many blocks as that some hold nothing."""
+    entries = [(n, 1) for n in (0, 1, 0, 31, 32, 1500, 5, 63, 700, 0, 2, 447)]
+    ops = rts["bfloat16"].ops
+    ops._decode_flat_blocks = lambda *a: blocks
+    try:
+        got, want = run_attention(rts["bfloat16"], entries, nq, nkv, d, page, window=window, seed=blocks)
+    finally:
+        del ops._decode_flat_blocks
+    assert worst(got, want) < 2e-2
+    assert int(ops._counters.abs().sum()) == 0  # the kernel leaves them as it found them
+
+
 @pytest.mark.parametrize("flat", [0, 3, 100])  # 0: fixed splits; else the large-batch kernel with that many blocks
 @pytest.mark.parametrize("d,rot,nq,nkv,page,splits", [(64, 64, 32, 8, 16, 3), (64, 64, 3, 1, 8, 1), (128, 64, 8, 2, 16, 2),
                                                        (16, 16, 4, 2, 4, 4)])
