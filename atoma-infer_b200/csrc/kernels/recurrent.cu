@@ -154,9 +154,16 @@ extern "C" int head_norm_gate(const float* o, const void* g, int dtype, long lon
 // state [slots][inner][N]; out [T, inner] = (sum_n S[c, n] C_n + D_c u_c) * silu(zg_c).
 // One block per (channel block, entry[, chunk]).  Thread (c, r) keeps NPT states n = r * NPT .. of channel c, as pairs of
 // neighbouring states that one two-wide instruction updates.  y is the even states' sum plus the odd states', each in
-// ascending order, then the R threads' sums by halving.  B and C of 16 tokens are staged in shared memory; the channel's
-// own u, step size and gate input of those tokens go straight into the thread's registers.
+// ascending order, then the R threads' sums by halving.  B and C of SEL_TT tokens are staged in shared memory; the channel's
+// own u, step size and gate input of those tokens go straight into the thread's registers.  Pass 1 leaves the
+// step sizes for pass 3, so an entry's last chunk runs it too.
+// Bound by the special-function pipe (an ex2 per state, token and pass: 60 of the us below) and the issue slots beside it:
+// tiles of 8 tokens (128 registers, four blocks a multiprocessor; tiles of 16 took 236, two blocks) and then the softplus
+// once instead of in both passes and bfloat16 gates by the reciprocal instruction took the scan of 2,048 tokens of 4,096
+// channels x 16 states from 175 over 156 to 147 us, of 8,192 channels from 324 over 292 to 272, and 200 tokens of 4,096
+// from 53 over 49 to 44.  Loading the next tile ahead (4 to 8 tokens, B and C of 64 at a time) gave 147 to 163 us.
 #define LOG2E_F 1.4426950408889634f
+#define SEL_TT 8
 
 // 2^x for x <= 0 by one approximate PTX instruction (a result below the smallest normal number is zero, which a decay of
 // that size is for every state that float32 holds).
@@ -166,19 +173,20 @@ __device__ __forceinline__ float ex2_nonpositive(float x) {
     return y;
 }
 
-template <typename T, int NPT, bool WRITE_Y>
-__global__ void __launch_bounds__(256)
+template <typename T, int NPT, int PASS>
+__global__ void __launch_bounds__(128, NPT <= 16 ? 4 : 1)
 selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* __restrict__ dt_raw,
                       const float* __restrict__ dt_bias, const T* __restrict__ bc, long long bc_stride,
                       const T* __restrict__ zg, long long z_stride, const float* __restrict__ a_log,
                       const float* __restrict__ d_skip, float* __restrict__ state, long long slot_stride, T* __restrict__ out,
                       const int* __restrict__ meta, const int* __restrict__ cu_tokens, const int* __restrict__ slots,
-                      int inner, int N, int R, int CPB, int pass, int chunk_len, int max_chunks, float* __restrict__ scratch,
-                      float* __restrict__ dt_sums) {
+                      int inner, int N, int R, int CPB, int chunk_len, int max_chunks, float* __restrict__ scratch,
+                      float* __restrict__ dt_sums, float* __restrict__ steps) {
+    constexpr bool WRITE_Y = PASS != 1;
     extern __shared__ __align__(16) float sm[];
     const int SL = R > 1 ? NPT + 4 : NPT, NL = R * NPT, NP = R * SL;
-    float* Bs = sm;                      // [REC_TT][NP]
-    float* Cs = Bs + REC_TT * NP;        // [REC_TT][NP]
+    float* Bs = sm;                      // [SEL_TT][NP]
+    float* Cs = Bs + SEL_TT * NP;        // [SEL_TT][NP]
     const int e = blockIdx.y, ch = blockIdx.z;
     const int tid = threadIdx.x, cl = tid / R, r = tid % R, c = blockIdx.x * CPB + cl;
     const bool real = cl < CPB && c < inner;
@@ -195,13 +203,13 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
     pdl_wait();
     if (e >= meta[META_NUM_ENTRIES]) return;
     const int first = cu_tokens[e], count = cu_tokens[e + 1] - first;
-    const int nchunks = pass == 0 ? 1 : (count + chunk_len - 1) / chunk_len;
-    if (ch >= nchunks || (pass == 1 && ch == nchunks - 1)) return;
-    const int t0 = first + (pass == 0 ? 0 : ch * chunk_len), t1 = pass == 0 ? first + count : min(first + count, t0 + chunk_len);
+    const int nchunks = PASS == 0 ? 1 : (count + chunk_len - 1) / chunk_len;
+    if (ch >= nchunks) return;
+    const int t0 = first + (PASS == 0 ? 0 : ch * chunk_len), t1 = PASS == 0 ? first + count : min(first + count, t0 + chunk_len);
     const size_t HS = (size_t)inner * N;
     float* slot_state = state + (size_t)slots[e] * slot_stride;
     float* chunk_state = scratch ? scratch + ((size_t)e * max_chunks + ch) * HS : nullptr;
-    const float* init = pass == 0 ? slot_state : (pass == 3 ? chunk_state : nullptr);
+    const float* init = PASS == 0 ? slot_state : (PASS == 3 ? chunk_state : nullptr);
     float2 S[NPT / 2];
 #pragma unroll
     for (int i = 0; i < NPT; ++i) {
@@ -210,18 +218,18 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
         if (i & 1) S[i / 2].y = s0; else S[i / 2].x = s0;
     }
     float dt_sum = 0.f;
-    for (int tb = t0; tb < t1; tb += REC_TT) {
-        const int nt = min(REC_TT, t1 - tb);
+    for (int tb = t0; tb < t1; tb += SEL_TT) {
+        const int nt = min(SEL_TT, t1 - tb);
         // this thread's channel of the tile's tokens, straight into registers: every load is on its way before the
         // first is used (the R threads of a channel read the same addresses)
-        T ur[REC_TT], zr[REC_TT];
-        float dr[REC_TT];
+        T ur[SEL_TT], zr[SEL_TT];
+        float dr[SEL_TT];
 #pragma unroll
-        for (int tt = 0; tt < REC_TT; ++tt) {
+        for (int tt = 0; tt < SEL_TT; ++tt) {
             const bool in = real && tt < nt;
             const size_t t = (size_t)(tb + tt);
             ur[tt] = in ? u[t * u_stride + c] : from_float<T>(0.f);
-            dr[tt] = in ? dt_raw[t * inner + c] : 0.f;
+            dr[tt] = in ? (PASS == 3 ? steps : dt_raw)[t * inner + c] : 0.f;
             if (WRITE_Y) zr[tt] = in ? zg[t * z_stride + c] : from_float<T>(0.f);
         }
         __syncthreads();
@@ -233,9 +241,10 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
         }
         __syncthreads();
 #pragma unroll
-        for (int tt = 0; tt < REC_TT; ++tt) {
+        for (int tt = 0; tt < SEL_TT; ++tt) {
             if (tt >= nt) break;
-            const float uv = to_float(ur[tt]), step = real ? softplus_f(dr[tt] + dtb) : 0.f;
+            const float uv = to_float(ur[tt]), step = PASS == 3 ? dr[tt] : (real ? softplus_f(dr[tt] + dtb) : 0.f);
+            if (PASS == 1 && real && r == 0) steps[(size_t)(tb + tt) * inner + c] = step;
             const float dx = step * uv;
             const float* Bt = Bs + tt * NP + r * SL;
             const float* Ct = Cs + tt * NP + r * SL;
@@ -260,13 +269,14 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
                 for (int s = R >> 1; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
                 if (real && r == 0) {
                     const float y = fmaf(dskip, uv, acc);
-                    out[(size_t)(tb + tt) * inner + c] = from_float<T>(y * silu_f(to_float(zr[tt])));
+                    out[(size_t)(tb + tt) * inner + c] = from_float<T>(y * silu_as<T>(to_float(zr[tt])));
                 }
             }
             dt_sum += step;
         }
     }
-    float* fin = pass == 1 ? chunk_state + HS : ((pass == 0 || ch == nchunks - 1) ? slot_state : nullptr);
+    // (pass 1 runs an entry's last chunk for its step sizes alone)
+    float* fin = PASS == 1 ? (ch < nchunks - 1 ? chunk_state + HS : nullptr) : ((PASS == 0 || ch == nchunks - 1) ? slot_state : nullptr);
     if (fin && real) {
 #pragma unroll
         for (int i = 0; i < NPT; ++i) {
@@ -274,7 +284,7 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
             if (n < N) fin[(size_t)c * N + n] = (i & 1) ? S[i / 2].y : S[i / 2].x;
         }
     }
-    if (pass == 1 && real && r == 0) dt_sums[((size_t)e * max_chunks + ch) * inner + c] = dt_sum;
+    if (PASS == 1 && real && r == 0) dt_sums[((size_t)e * max_chunks + ch) * inner + c] = dt_sum;
 }
 
 // scratch[e, 0] = the slot's state; scratch[e, c] = exp(A * (sum of the steps of chunk c - 1)) * scratch[e, c - 1] + scratch[e, c].
@@ -301,8 +311,8 @@ selective_chunk_states_kernel(const float* __restrict__ state, long long slot_st
     }
 }
 
-extern "C" size_t selective_scan_scratch_floats(int S, int inner, int N, int max_chunks) {
-    return (size_t)S * max_chunks * ((size_t)inner * N + inner);
+extern "C" size_t selective_scan_scratch_floats(int T, int S, int inner, int N, int max_chunks) {
+    return (size_t)S * max_chunks * ((size_t)inner * N + inner) + (size_t)T * inner;
 }
 
 extern "C" int selective_scan(const void* u, long long u_stride, const float* dt_raw, const float* dt_bias, const void* bc,
@@ -315,38 +325,39 @@ extern "C" int selective_scan(const void* u, long long u_stride, const float* dt
     if (!rec_geometry(N, inner, &NPT, &R, &CPB)) return (int)cudaErrorInvalidValue;
     if (CPB * R > 128) CPB = 128 / R > 0 ? 128 / R : 1;  // 128 threads a block: more blocks for few requests
     const int blocks = (inner + CPB - 1) / CPB, threads = ((CPB * R + 31) / 32) * 32;
-    const size_t smem = (size_t)(2 * REC_TT * R * (R > 1 ? NPT + 4 : NPT)) * sizeof(float);
+    const size_t smem = (size_t)(2 * SEL_TT * R * (R > 1 ? NPT + 4 : NPT)) * sizeof(float);
     if (smem > 96 * 1024) return (int)cudaErrorInvalidValue;
     float* dt_sums = scratch ? scratch + (size_t)S * max_chunks * (size_t)inner * N : nullptr;
-#define SEL_CASE(TT, K, W, pass, chunks)                                                                                    \
+    float* steps = dt_sums ? dt_sums + (size_t)S * max_chunks * inner : nullptr;  // [T, inner]
+#define SEL_CASE(TT, K, pass, chunks)                                                                                    \
     case K: {                                                                                                              \
         static size_t configured = 0;                                                                                      \
         if (smem > 48 * 1024 && smem > configured) {                                                                       \
-            cudaError_t ce = cudaFuncSetAttribute(selective_scan_kernel<TT, K, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+            cudaError_t ce = cudaFuncSetAttribute(selective_scan_kernel<TT, K, pass>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
             if (ce != cudaSuccess) return (int)ce;                                                                         \
             configured = smem;                                                                                             \
         }                                                                                                                  \
-        err = (int)launch_kernel(selective_scan_kernel<TT, K, W>, dim3(blocks, S, chunks), threads, smem, stream, (const TT*)u, u_stride, \
+        err = (int)launch_kernel(selective_scan_kernel<TT, K, pass>, dim3(blocks, S, chunks), threads, smem, stream, (const TT*)u, u_stride, \
                                  dt_raw, dt_bias, (const TT*)bc, bc_stride, (const TT*)zg, z_stride, a_log, d_skip, state,       \
-                                 slot_stride, (TT*)out, meta, cu_tokens, slots, inner, N, R, CPB, pass, chunk_len, max_chunks,   \
-                                 scratch, dt_sums);                                                                        \
+                                 slot_stride, (TT*)out, meta, cu_tokens, slots, inner, N, R, CPB, chunk_len, max_chunks,   \
+                                 scratch, dt_sums, steps);                                                                        \
         break;                                                                                                             \
     }
-#define SEL_PASS(TT, W, pass, chunks)                                                                                       \
-    switch (NPT) { SEL_CASE(TT, 8, W, pass, chunks) SEL_CASE(TT, 16, W, pass, chunks) SEL_CASE(TT, 32, W, pass, chunks) SEL_CASE(TT, 64, W, pass, chunks) }
+#define SEL_PASS(TT, pass, chunks)                                                                                       \
+    switch (NPT) { SEL_CASE(TT, 8, pass, chunks) SEL_CASE(TT, 16, pass, chunks) SEL_CASE(TT, 32, pass, chunks) SEL_CASE(TT, 64, pass, chunks) }
     int err = 0;
     if (chunk_len <= 0 || max_chunks <= 1 || !scratch) {
-        if (dtype == DT_F32) { SEL_PASS(float, true, 0, 1) } else { SEL_PASS(__nv_bfloat16, true, 0, 1) }
+        if (dtype == DT_F32) { SEL_PASS(float, 0, 1) } else { SEL_PASS(__nv_bfloat16, 0, 1) }
         return err;
     }
-    if (dtype == DT_F32) { SEL_PASS(float, false, 1, max_chunks) } else { SEL_PASS(__nv_bfloat16, false, 1, max_chunks) }
+    if (dtype == DT_F32) { SEL_PASS(float, 1, max_chunks) } else { SEL_PASS(__nv_bfloat16, 1, max_chunks) }
     if (err) return err;
     const long long HS = (long long)inner * N;
     err = (int)launch_kernel(selective_chunk_states_kernel, dim3((unsigned)((HS + 255) / 256), S), 256, 0, stream,
                              (const float*)state, slot_stride, scratch, (const float*)dt_sums, a_log, meta, cu_tokens, slots,
                              inner, N, chunk_len, max_chunks);
     if (err) return err;
-    if (dtype == DT_F32) { SEL_PASS(float, true, 3, max_chunks) } else { SEL_PASS(__nv_bfloat16, true, 3, max_chunks) }
+    if (dtype == DT_F32) { SEL_PASS(float, 3, max_chunks) } else { SEL_PASS(__nv_bfloat16, 3, max_chunks) }
     return err;
 #undef SEL_PASS
 #undef SEL_CASE

@@ -992,7 +992,7 @@ class CudaOps:
             raise KernelError("selective_scan: step sizes are contiguous float32, the output has the inputs' type")
         (up, us), (bp, bs), (zp, zs) = (self._rows(t, "selective_scan") for t in (u, bc, zg))
         chunk, chunks = self._scan_chunks(ctx)
-        scratch = (torch.empty(lib.selective_scan_scratch_floats(ctx.S, inner, nstate, chunks), dtype=torch.float32, device=out.device)
+        scratch = (torch.empty(lib.selective_scan_scratch_floats(ctx.T, ctx.S, inner, nstate, chunks), dtype=torch.float32, device=out.device)
                    if chunk else None)
         self._check(lib.selective_scan(up, us, _p(dt_raw), _p(dt_bias), bp, bs, zp, zs, _code(u), _p(a_log), _p(d_skip), _p(state),
                                        slot_stride, _p(out), _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, inner,
