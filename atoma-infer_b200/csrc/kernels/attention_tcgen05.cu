@@ -6,7 +6,7 @@
 //   * two copy warps, one for K and one for V: pages travel by TMA (one box per page, 128-byte swizzle)
 //     straight from the paged cache into two-stage shared-memory rings; the page ids come from the
 //     block table in shared memory;
-//   * an MMA warp (one elected thread): S = Q K^T is one tcgen05.mma chain (M = 128, N = 128,
+//   * two MMA warps (one elected thread each, one a product): S = Q K^T is one tcgen05.mma chain (M = 128, N = 128,
 //     K = head size) into tensor memory; O += P V is a second chain whose A operand P is read from
 //     tensor memory and whose B operand V is read MN-major from shared memory (no transpose copy); O
 //     stays in tensor memory from the first tile to the last;
@@ -20,15 +20,20 @@
 // and the copies run two tiles ahead.  (A K stage is free long before a V stage: one warp that waited for both in turn
 // started K so late that every tile's scores waited some 2,000 clocks for it.  A box a page and 64-column half
 // instead of one a page kept the copy engine, which starts a box in about a hundred clocks, busy for longer than a
-// tile takes.  32 heads of 128 over 8, 4,096 tokens: 247 -> 217 us; over 4, 16,384 tokens: 3,111 -> 2,579 us.)  Two blocks fit a multiprocessor for
+// tile takes.  32 heads of 128 over 8, 4,096 tokens: 247 -> 217 us; over 4, 16,384 tokens: 3,111 -> 2,579 us.
+// A warp each for the two products, so that neither waits behind the other's operands: 198 and 2,276 us.  What a block does
+// before its first scores was a chain of four round trips to memory, some 4 us of a block: the request is found from one
+// round of loads, and K sets out beside the loads of Q and of the block table; with a mask of two comparisons a score
+// 188 and 2,215 us, prompts of 1,391, 402 and 255 tokens 63 -> 53 us, at heads of 64 44 -> 38.)  Two blocks fit a multiprocessor for
 // head size 64; the softmax warps then take registers that the other two warps give up.
 // A portion of a prompt that starts inside a cached context attends to all of it.
 //
 // Head size 256 serves attention whose cache holds the same vector on the key and the value plane (latent attention): a tile of
 // 128 such vectors is 64 KB, so Q and two stages of ONE plane fill a multiprocessor's shared memory, and separate values
 // would not fit.  A stage is both products' B operand, K-major for the scores and MN-major for P V, and is free when P V is
-// done.  Measured, 16 heads of 256 over one, window 1,024, learned sinks, a prompt of 4,096 tokens: 119 us; the
-// mma.sync kernel over both planes 596.  The tensor pipe is 27 % busy: one block a multiprocessor, and its softmax is a chain.
+// done.  Measured, 16 heads of 256 over one, window 1,024, learned sinks, a prompt of 4,096 tokens: 101 us; the
+// mma.sync kernel over both planes 596.  One block a multiprocessor, and its softmax is a chain that leaves the tensor pipe idle
+// for two thirds of the time.
 //
 // The reference's prefill kernel is FlashAttention-2 for sm80 (csrc/kernels/flash_fwd_kernel.h:56-500,
 // mma.sync m16n8k16, cp.async), which also cannot see a cached prefix (models/src/flash_attention.rs:384-410).
@@ -66,7 +71,7 @@ template <bool CS, bool STATS = false>
 __global__ void __launch_bounds__(TC_THREADS, HEAD_DIM == 64 ? 2 : 1)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* __restrict__ q, int q_stride,
                        CacheLayout L, const int* __restrict__ meta, int group, const int* __restrict__ cu_tokens,
-                       const int* __restrict__ ctx_lens, bf16* __restrict__ out, int nq, int window, int chunk_arg, int sink_arg,
+                       const int* __restrict__ ctx_lens, int S, bf16* __restrict__ out, int nq, int window, int chunk_arg, int sink_arg,
                        const float* __restrict__ sink_values, float scale_log2, int num_pages, int bt_cap,
                        float softcap_arg, const float* __restrict__ slopes_arg, int* __restrict__ status, float* __restrict__ lse) {
     const int chunk = CS ? chunk_arg : 0, sink = CS ? sink_arg : 0;
@@ -92,17 +97,48 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
     float* row_max = reinterpret_cast<float*>(tmem_slot + 2);  // [2 sets][2 halves][128 rows]
     int* bt_s = reinterpret_cast<int*>(row_max + 4 * BQ);
 
-    // Late query tiles see the most keys: they go first, for all heads before any earlier tile (blocks start in
-    // the order of their linear index, x fastest), so the longest blocks are not the last to start.
-    const int qt = gridDim.y - 1 - blockIdx.y, kvh = blockIdx.x, e = blockIdx.z;
-    if (e >= meta[META_NUM_ENTRIES]) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int G = nq / L.num_kv_heads, TPT = BQ / G, ps = L.page_size;
-    const int row0 = cu_tokens[e], q_len = cu_tokens[e + 1] - row0, ctx = ctx_lens[e];
+    if (warp == COPY_WARP && lane == 0) {
+        asm volatile("prefetch.tensormap [%0];" ::"l"(&map_kv) : "memory");
+        for (int i = 0; i < 8; ++i) mbar_init(&bars[i], 1);
+        for (int i = 8; i < 10; ++i) mbar_init(&bars[i], SOFTMAX_WARPS);  // one arrival per softmax warp
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // blockIdx.y counts the query tiles of all requests, a request's late ones first: they see the most keys, and blocks
+    // start in the order of their linear index (x fastest), so that a request's longest blocks are not the last to start.
+    // Every warp finds the tile's request for itself; what it needs of all of them is one round of loads.
+    const int kvh = blockIdx.x, entries = meta[META_NUM_ENTRIES];
+    const int bt_offset = meta[META_BT_OFFSET + group], bt_stride = meta[META_BT_STRIDE + group];
+    int e = -1, qt = 0, row0 = 0, q_len = 0, ctx = 0;
+    for (int base = 0, before = 0; base < S; base += 32) {
+        const int i = base + lane, lo = i < S ? cu_tokens[i] : 0, hi = i < S ? cu_tokens[i + 1] : 0, cx = i < S ? ctx_lens[i] : 0;
+        int upto = i < entries ? (hi - lo + TPT - 1) / TPT : 0;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, d);
+            if (lane >= d) upto += v;
+        }
+        upto += before;
+        const uint32_t past = __ballot_sync(0xffffffffu, upto > (int)blockIdx.y);
+        if (past) {
+            // (a reduction's result is one value for the warp to the compiler as well, a shuffle's is not: with shuffles the key
+            // loop carried its bounds in every thread's registers, 4,096 tokens of 32 heads of 128 over 8 206 us instead of 202)
+            const bool mine = lane == __ffs(past) - 1;
+            e = __reduce_add_sync(0xffffffffu, mine ? i : 0);
+            row0 = __reduce_add_sync(0xffffffffu, mine ? lo : 0);
+            q_len = __reduce_add_sync(0xffffffffu, mine ? hi - lo : 0);
+            ctx = __reduce_add_sync(0xffffffffu, mine ? cx : 0);
+            qt = __reduce_add_sync(0xffffffffu, mine ? upto - 1 - (int)blockIdx.y : 0);
+            break;
+        }
+        before = __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (e < 0) return;  // before anything is allocated
     const int t0 = qt * TPT;
-    if (t0 >= q_len) return;  // before anything is allocated
     const int nt = min(TPT, q_len - t0);
-    const int* bt = meta + meta[META_BT_OFFSET + group] + (size_t)e * meta[META_BT_STRIDE + group];
+    const int* bt = meta + bt_offset + (size_t)e * bt_stride;
     const int p_first = ctx + t0, p_last = p_first + nt - 1;
     // chunk > 0: a row sees only the keys of its own chunk of positions; the first row's chunk starts earliest
     int kbeg = window > 0 ? max(0, p_first - window + 1) : 0;
@@ -117,6 +153,36 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
         if (tid == 0) atomicExch(&status[STATUS_BAD_PAGE], 1 + kend);
         page_cnt = bt_cap;
     }
+    // A copy warp's part of tile t, the K (kv = 0) or V (kv = 1) rows of `page`, lane i's page being the tile's i-th: one box
+    // per page.  Lane 0 announces the bytes, then every lane starts its page's box (starting a copy costs about a hundred
+    // cycles; eight pages started by one thread would take eight times as long).
+    const int kv = warp == COPY_V_WARP;
+    unsigned char* ring = kv ? v_s : k_s;
+    uint64_t* full = kv ? v_full : k_full;
+    auto start = [&](int t, int page) {
+        const bool mine = page > 0 && page < num_pages;
+        const uint32_t pages = __popc(__ballot_sync(0xffffffffu, mine));
+        uint64_t* bar = &full[t & 1];
+        if (lane == 0) mbar_expect_tx(bar, pages * (uint32_t)ps * 128u * HALVES);
+        __syncwarp();
+        if (mine) {
+            int r = ((page * 2 + kv) * L.num_kv_heads + kvh) * ps;  // row of the page's first slot in the cache as a matrix
+            tma_load_4d(ring + (t & 1) * STAGE + lane * ps * 128 * HALVES, &map_kv, 0, 0, 0, r / 8, bar);
+        }
+    };
+    auto lane_page = [&](int t) {  // place of lane's page of tile t in the block's slice of the table, or -1
+        const int i = (k_first + t * BKV) / ps + lane - page_lo;
+        return lane < BKV / ps && i < page_cnt ? i : -1;
+    };
+    if (warp == COPY_WARP) {
+        // K of the first two tiles sets out beside the loads of Q and of the table, its pages straight from the table
+        __syncwarp();
+        fence_async_smem();
+        for (int t = 0; t < 2 && t < ntiles; ++t) {
+            const int i = lane_page(t);
+            start(t, i >= 0 ? bt[page_lo + i] : 0);
+        }
+    }
     int bad = 0;
     for (int i = tid; i < page_cnt; i += TC_THREADS) {
         int page = bt[page_lo + i];
@@ -127,12 +193,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
             bad = 1;
         }
         bt_s[i] = page;
-    }
-    if (tid == 0) {
-        for (int i = 0; i < 8; ++i) mbar_init(&bars[i], 1);
-        for (int i = 8; i < 10; ++i) mbar_init(&bars[i], SOFTMAX_WARPS);  // one arrival per softmax warp
-        *abort_flag = 0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == MMA_WARP) {
         tmem_alloc(tmem_slot, TMEM_COLS);
@@ -162,33 +222,21 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
         if (D == 64) regs_release<32>();
         if (warp == COPY_WARP || (warp == COPY_V_WARP && !STATS && !ONE_PLANE)) {
             // ------------------------------------------------------------------ copies, two tiles ahead
-            // The K (kv = 0) or V (kv = 1) rows of tile t: one box per page.
-            // Lane 0 announces the bytes, then lane i starts the box of page i (starting a copy costs
-            // about a hundred cycles; eight pages started by one thread would take eight times as long).
-            const int kv = warp == COPY_V_WARP;
-            unsigned char* ring = kv ? v_s : k_s;
-            uint64_t* full = kv ? v_full : k_full;
             // a K stage is free when the scores of its tile are done (with one plane: when its P V is), a V stage when its P V is
             uint64_t* empty = !STATS && (ONE_PLANE || kv) ? pv_done : s_done;
-            auto start = [&](int t) {
-                const int k0 = k_first + t * BKV;
-                const int pg = lane, pidx = k0 / ps + pg - page_lo;
-                const bool mine = pg < BKV / ps && pidx < page_cnt && bt_s[pidx] > 0;
-                const uint32_t pages = __popc(__ballot_sync(0xffffffffu, mine));
-                uint64_t* bar = &full[t & 1];
-                if (lane == 0) mbar_expect_tx(bar, pages * (uint32_t)ps * 128u * HALVES);
-                __syncwarp();
-                if (mine) {
-                    int r = ((bt_s[pidx] * 2 + kv) * L.num_kv_heads + kvh) * ps;  // row of the page's first slot in the cache as a matrix
-                    tma_load_4d(ring + (t & 1) * STAGE + pg * ps * 128 * HALVES, &map_kv, 0, 0, 0, r / 8, bar);
-                }
+            auto kept_page = [&](int t) {
+                const int i = lane_page(t);
+                return i >= 0 ? bt_s[i] : 0;
             };
             int last[2] = {-1, -1};  // the last tile whose copy was started into a stage
-            for (int t = 0; t < 2 && t < ntiles; ++t) { start(t); last[t] = t; }
+            for (int t = 0; t < 2 && t < ntiles; ++t) {
+                if (kv) start(t, kept_page(t));
+                last[t] = t;
+            }
             for (int t = 0; t + 2 < ntiles; ++t) {
                 const int b = t & 1;
                 if (!mbar_wait(&empty[b], (uint32_t)(t >> 1) & 1u, status, abort_flag)) break;
-                start(t + 2);
+                start(t + 2, kept_page(t + 2));
                 last[b] = t + 2;
             }
             if (*abort_flag && lane == 0) {
@@ -271,12 +319,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
             if (lane == 0) mbar_arrive(s_free);
             const bool need_mask = (window > 0 && k0 <= p_last - window) || k0 + BKV - 1 > p_first || k0 < kbeg || nt < TPT || k0 < chunk_last;  // same for the whole block
             if (need_mask) {
+                const int first = my_lo - k0 - half * 64, last = my_pos - k0 - half * 64;  // the keys of my half that my row sees
 #pragma unroll
-                for (int i = 0; i < 64; ++i) {
-                    int key = k0 + half * 64 + i;
-                    bool vis = CS ? (key <= my_pos && key >= my_lo) : (key <= my_pos && (window <= 0 || my_pos - key < window));
-                    v[i] = vis ? v[i] : -INFINITY;
-                }
+                for (int i = 0; i < 64; ++i) v[i] = i <= last && i >= first ? v[i] : -INFINITY;
+                asm volatile("");  // (nothing of it outside of the branch: most tiles of a long prompt need no mask)
             }
             if (CS && scored) {
                 // - slope (my_pos - key) = c0 + slope i for key = k0 + 64 half + i: two multiply-adds a score, no conversion
@@ -408,6 +454,10 @@ int table_slice(int max_context, int page_size, int tpt, int window, int chunk) 
     if (chunk > 0) span = min(span, chunk + tpt + 2 * BKV);
     return span / page_size + 2 + BKV / page_size;
 }
+// Blocks enough for S requests of T tokens together: n tokens are at most (n + tpt - 1) / tpt tiles.  (A grid of the longest
+// request's tiles for every request: 31,000 blocks that left at once for one prompt of 1,988 tokens beside 60 single tokens,
+// 32 heads of 64 over 8 256 us, of 128 280 us; so 60 and 86 us.)
+dim3 query_tiles(int T, int S, int nkv, int tpt) { return dim3(nkv, (T + (long long)S * (tpt - 1)) / tpt); }
 }  // namespace
 
 extern "C" int attn_tc_head_dim() { return D; }
@@ -423,25 +473,11 @@ extern "C" int attn_prefill_tc_fits(int page_size, int nq, int nkv, int window, 
     return TC_SMEM_FIXED + (size_t)table_slice(max_context, page_size, BQ / (nq / nkv), window, chunk) * sizeof(int) <= 227 * 1024;
 }
 
-// sink_values (one float per query head, or null): the sink's score per head instead of 0.
-extern "C" int attn_prefill_tc_scores(const void* q, int q_stride, const void* cache, const int* meta, int group,
-                                      const int* cu_tokens, const int* ctx_lens, void* out, int S, int max_q_len, int nq,
-                                      int nkv, int page_size, int num_pages, int window, int chunk, int sink,
-                                      const float* sink_values, float scale, int max_context, float softcap, const float* slopes,
-                                      int* status, cudaStream_t stream);
-
-extern "C" int attn_prefill_tc_sinks(const void* q, int q_stride, const void* cache, const int* meta, int group,
-                                     const int* cu_tokens, const int* ctx_lens, void* out, int S, int max_q_len, int nq,
-                                     int nkv, int page_size, int num_pages, int window, int chunk, int sink,
-                                     const float* sink_values, float scale, int max_context, int* status, cudaStream_t stream) {
-    return attn_prefill_tc_scores(q, q_stride, cache, meta, group, cu_tokens, ctx_lens, out, S, max_q_len, nq, nkv, page_size,
-                                  num_pages, window, chunk, sink, sink_values, scale, max_context, 0.f, nullptr, status, stream);
-}
-
-// softcap > 0: a score s becomes softcap * tanh(s / softcap); slopes (one float per query head, or null): slopes[h] * (query
+// T: rows of q (at least the requests' tokens together).  sink_values (one float per query head, or null): the sink's score
+// per head instead of 0.  softcap > 0: a score s becomes softcap * tanh(s / softcap); slopes (one float per query head, or null): slopes[h] * (query
 // position - key position) is taken off the score.  (A window that keeps first keys is the mma.sync kernel's.)
 extern "C" int attn_prefill_tc_scores(const void* q, int q_stride, const void* cache, const int* meta, int group,
-                                      const int* cu_tokens, const int* ctx_lens, void* out, int S, int max_q_len, int nq,
+                                      const int* cu_tokens, const int* ctx_lens, void* out, int T, int S, int max_q_len, int nq,
                                       int nkv, int page_size, int num_pages, int window, int chunk, int sink,
                                       const float* sink_values, float scale, int max_context, float softcap, const float* slopes,
                                       int* status, cudaStream_t stream) {
@@ -462,14 +498,14 @@ extern "C" int attn_prefill_tc_scores(const void* q, int q_stride, const void* c
         if (err != cudaSuccess) return (int)err;
         configured[cs] = smem;
     }
-    dim3 grid(nkv, (max_q_len + tpt - 1) / tpt, S);
+    const dim3 grid = query_tiles(T, S, nkv, tpt);
     if (cs)
         attn_prefill_tc_kernel<true><<<grid, TC_THREADS, smem, stream>>>(map, (const bf16*)q, q_stride, L, meta, group, cu_tokens,
-                                                                  ctx_lens, (bf16*)out, nq, window, chunk, sink, sink_values,
+                                                                  ctx_lens, S, (bf16*)out, nq, window, chunk, sink, sink_values,
                                                                   scale * LOG2E, num_pages, bt_cap, softcap, slopes, status, nullptr);
     else
         attn_prefill_tc_kernel<false><<<grid, TC_THREADS, smem, stream>>>(map, (const bf16*)q, q_stride, L, meta, group, cu_tokens,
-                                                                   ctx_lens, (bf16*)out, nq, window, 0, 0, nullptr, scale * LOG2E,
+                                                                   ctx_lens, S, (bf16*)out, nq, window, 0, 0, nullptr, scale * LOG2E,
                                                                    num_pages, bt_cap, 0.f, nullptr, status, nullptr);
     LAUNCH_RETURN();
 }
@@ -477,7 +513,7 @@ extern "C" int attn_prefill_tc_scores(const void* q, int q_stride, const void* c
 // lse[row, h] (float32, base 2) = log2 of the sum over the keys that query head h of the row sees of exp(score); chunk as above.
 // For kernels that need the finished softmax of every head before they weigh values.
 extern "C" int attn_prefill_tc_stats(const void* q, int q_stride, const void* cache, const int* meta, int group, const int* cu_tokens,
-                                     const int* ctx_lens, float* lse, int S, int max_q_len, int nq, int nkv, int page_size, int num_pages,
+                                     const int* ctx_lens, float* lse, int T, int S, int max_q_len, int nq, int nkv, int page_size, int num_pages,
                                      int chunk, float scale, int max_context, int* status, cudaStream_t stream) {
     if (S <= 0 || max_q_len <= 0) return 0;
     if (!attn_prefill_tc_supports(page_size, nq, nkv) || scale <= 0.f) return (int)cudaErrorInvalidValue;
@@ -494,24 +530,8 @@ extern "C" int attn_prefill_tc_stats(const void* q, int q_stride, const void* ca
         if (err != cudaSuccess) return (int)err;
         configured = smem;
     }
-    attn_prefill_tc_kernel<true, true><<<dim3(nkv, (max_q_len + tpt - 1) / tpt, S), TC_THREADS, smem, stream>>>(
-        map, (const bf16*)q, q_stride, L, meta, group, cu_tokens, ctx_lens, nullptr, nq, 0, chunk, 0, nullptr, scale * LOG2E, num_pages,
+    attn_prefill_tc_kernel<true, true><<<query_tiles(T, S, nkv, tpt), TC_THREADS, smem, stream>>>(
+        map, (const bf16*)q, q_stride, L, meta, group, cu_tokens, ctx_lens, S, nullptr, nq, 0, chunk, 0, nullptr, scale * LOG2E, num_pages,
         bt_cap, 0.f, nullptr, status, lse);
     LAUNCH_RETURN();
-}
-
-extern "C" int attn_prefill_tc_masked(const void* q, int q_stride, const void* cache, const int* meta, int group,
-                                      const int* cu_tokens, const int* ctx_lens, void* out, int S, int max_q_len, int nq,
-                                      int nkv, int page_size, int num_pages, int window, int chunk, int sink, float scale,
-                                      int max_context, int* status, cudaStream_t stream) {
-    return attn_prefill_tc_sinks(q, q_stride, cache, meta, group, cu_tokens, ctx_lens, out, S, max_q_len, nq, nkv, page_size,
-                                 num_pages, window, chunk, sink, nullptr, scale, max_context, status, stream);
-}
-
-extern "C" int attn_prefill_tc(const void* q, int q_stride, const void* cache, const int* meta, int group,
-                               const int* cu_tokens, const int* ctx_lens, void* out, int S, int max_q_len, int nq, int nkv,
-                               int page_size, int num_pages, int window, float scale, int max_context, int* status,
-                               cudaStream_t stream) {
-    return attn_prefill_tc_masked(q, q_stride, cache, meta, group, cu_tokens, ctx_lens, out, S, max_q_len, nq, nkv, page_size,
-                                  num_pages, window, 0, 0, scale, max_context, status, stream);
 }

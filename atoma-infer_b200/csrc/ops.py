@@ -543,7 +543,7 @@ class CudaOps:
                 # (a window that keeps first keys is the mma.sync kernel's: its kept keys are tiles of their own)
                 tc = self._prefill_tc(d, page_size, nq, nkv, one_plane, (window, int(chunk), ctx.max_context))
                 self._check(tc.attn_prefill_tc_scores(_p(q), q_stride, _p(cache_layer), _p(ctx.meta), group, _p(ctx.cu_tokens),
-                                                      _p(ctx.context_lens), _p(out), S, ctx.max_tokens_per_entry, nq, nkv,
+                                                      _p(ctx.context_lens), _p(out), T, S, ctx.max_tokens_per_entry, nq, nkv,
                                                       page_size, num_pages, window, int(chunk), int(bool(sink)), _p(sinks),
                                                       ctypes.c_float(scale), ctx.max_context, ctypes.c_float(float(softcap)),
                                                       _p(slopes), _p(self.status), self._stream()),
@@ -1184,7 +1184,7 @@ class CudaOps:
             return False
         lse = torch.empty((ctx.T, nq), dtype=torch.float32, device=q.device)
         self._check(stats.attn_prefill_tc_stats(_p(q), q_stride, _p(cache_layer), _p(ctx.meta), group, _p(ctx.cu_tokens),
-                                                _p(ctx.context_lens), _p(lse), ctx.S, ctx.max_tokens_per_entry, nq, nkv, page_size,
+                                                _p(ctx.context_lens), _p(lse), ctx.T, ctx.S, ctx.max_tokens_per_entry, nq, nkv, page_size,
                                                 num_pages, chunk, ctypes.c_float(scale), ctx.max_context, _p(self.status), self._stream()),
                     "attn_prefill_tc_stats")
         self._check(lib.attn_talk_prefill_tc(_p(q), q_stride, _p(cache_layer), _p(ctx.meta), group, _p(ctx.cu_tokens), _p(ctx.context_lens),

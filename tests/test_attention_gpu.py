@@ -352,3 +352,15 @@ def test_prefill_over_one_plane_of_wide_heads(rts, nq, page, window, sink):
         assert (outs[0][row:row + n] - want).abs().max() < 2e-2  # values are O(1); bfloat16 P and outputs
         assert (outs[1][row:row + n] - want).abs().max() < 2e-2
         row += n
+
+
+@pytest.mark.parametrize("d,nq,nkv", [(64, 8, 2), (128, 3, 1)])
+@pytest.mark.parametrize("requests", [1, 31, 32, 33, 97])
+def test_prefill_tiles_of_many_requests(rts, d, nq, nkv, requests):
+    """The tcgen05 kernel numbers the query tiles of all requests through: single tokens behind long contexts between portions of a
+    tile, one more and several tiles, around the 32 requests that one round of the search for a tile's request covers."""
+    rows = 128 // (nq // nkv)  # tokens of a tile
+    sizes = [1, rows + 1, 1, rows, 2 * rows + 7, 1, 1]
+    entries = [((i * 37) % 150, sizes[i % 7]) for i in range(requests - 1)] + [(40, 3 * rows + 5)]
+    got, want = run_attention(rts["bfloat16"], entries, nq, nkv, d, 16, seed=requests)
+    assert worst(got, want) < 2e-2  # values are O(1); bfloat16 P and outputs
