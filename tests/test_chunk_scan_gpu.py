@@ -42,22 +42,33 @@ def err(got, want):
     return ((got.double().cpu() - want).abs().max() / want.abs().max()).item()
 
 
-def both(rt, run):
-    """``run()`` on the chunked kernels (three launches) and on the one that goes token by token."""
-    got = []
+ENTRY = {"space": ("_mixers", "ssm_chunk_scan"), "memory": ("_matrix_recurrent", "memory_chunk_scan"),
+         "decay": ("_recurrent", "gla_row_scan"), "bonus": ("_matrix_recurrent", "bonus_row_scan")}
+
+
+def both(rt, kind, run, monkeypatch, one_head=0):
+    """``run()`` on the chunked kernels and on the one that goes token by token, and that it was so.  ``one_head``: the chunked one
+    gets scratch for one head of that many floats."""
+    lib, name = getattr(rt.ops, ENTRY[kind][0])(), ENTRY[kind][1]
+    entry, calls, got = getattr(lib, name), [], []
+    monkeypatch.setattr(lib, name, lambda *args: (calls.append(args), entry(*args))[1])
     for flag in (True, False):
-        rt.ops.matrix_scan = flag
-        try:
+        with monkeypatch.context() as m:
+            m.setattr(rt.ops, "matrix_scan", flag)
+            if flag and one_head:
+                m.setattr(rt.ops, "ROW_SCAN_SCRATCH", one_head + 100)
+                m.setattr(lib, name.replace("_row_scan", "_scan_scratch_floats"), lambda *args: 0)
             got.append(run())
-        finally:
-            rt.ops.matrix_scan = type(rt.ops).matrix_scan
+        assert len(calls) == 1
+    if one_head:
+        assert calls[0][-2].value // one_head == 1
     rt.ops.check_status()
     return got
 
 
 @pytest.mark.parametrize("lengths", LENGTHS)
 @pytest.mark.parametrize("heads,P,N,G", [(2, 64, 128, 1), (4, 8, 8, 2), (2, 72, 40, 2), (3, 136, 64, 3), (2, 128, 120, 1)])
-def test_state_space_in_matrix_chunks(rt, lengths, heads, P, N, G):
+def test_state_space_in_matrix_chunks(rt, monkeypatch, lengths, heads, P, N, G):
     g = torch.Generator().manual_seed(heads * P + N + len(lengths))
     T, inner = sum(lengths), heads * P
     xbc = (torch.randn(T, inner + 2 * G * N, generator=g) * 0.7).bfloat16()
@@ -85,13 +96,13 @@ def test_state_space_in_matrix_chunks(rt, lengths, heads, P, N, G):
         assert torch.equal(state[:, :3].cpu(), S0[:, :3]) and torch.equal(state[:, -2:].cpu(), S0[:, -2:])
         return err(y, want_y), err(mats, want_s)
 
-    new, old = both(rt, run)
+    new, old = both(rt, "space", run, monkeypatch)
     assert max(new) < TOL, (new, old)
 
 
 @pytest.mark.parametrize("lengths", LENGTHS)
 @pytest.mark.parametrize("heads,dim,vdim", [(2, 128, 256), (3, 8, 72), (2, 64, 64), (1, 104, 8)])
-def test_matrix_memory_in_matrix_chunks(rt, lengths, heads, dim, vdim):
+def test_matrix_memory_in_matrix_chunks(rt, monkeypatch, lengths, heads, dim, vdim):
     g = torch.Generator().manual_seed(heads * dim + vdim + len(lengths))
     T, cap, nk, nv = sum(lengths), 9.0, heads * dim, heads * vdim
     rows = torch.randn(T, 2 * nk + nv + 8, generator=g).bfloat16()
@@ -135,7 +146,7 @@ def test_matrix_memory_in_matrix_chunks(rt, lengths, heads, dim, vdim):
                            ctx, o, nq, floor, heads=heads, dim=dim, vdim=vdim)
         return err(o, wo), err(nq, wn), err(state, ws[0]), err(n_state, ws[1]), err(m_state, ws[2])
 
-    new, old = both(rt, run)
+    new, old = both(rt, "memory", run, monkeypatch)
     assert max(new) < TOL, (new, old)
 
 
@@ -143,7 +154,7 @@ def test_matrix_memory_in_matrix_chunks(rt, lengths, heads, dim, vdim):
 @pytest.mark.parametrize("heads,dim,vdim", [(3, 128, 256), (2, 8, 72), (2, 64, 64), (1, 104, 8), (2, 40, 16)])
 @pytest.mark.parametrize("kind", ["decay", "bonus"])
 @pytest.mark.parametrize("rounds", [False, True])
-def test_a_decay_per_row_in_matrix_chunks(rt, lengths, heads, dim, vdim, kind, rounds):
+def test_a_decay_per_row_in_matrix_chunks(rt, monkeypatch, lengths, heads, dim, vdim, kind, rounds):
     """Sub-blocks of 16 tokens and triangles of 8 inside chunks of 64; strong decays (rows that forget within a token, whose logs sum
     to thousands within a chunk) beside weak ones; all heads at once, and in rounds of one where scratch is short."""
     g = torch.Generator().manual_seed(heads * dim + vdim + len(lengths))
@@ -185,15 +196,12 @@ def test_a_decay_per_row_in_matrix_chunks(rt, lengths, heads, dim, vdim, kind, r
         assert torch.equal(st[:, :3].cpu(), S0[:, :3]) and torch.equal(st[:, -2:].cpu(), S0[:, -2:])
         return err(o, wo), err(state, ws)
 
+    head = 0
     if rounds:
         lib = rt.ops._recurrent() if kind == "decay" else rt.ops._matrix_recurrent()
         x = torch.empty(16, device=rt.device, dtype=torch.bfloat16)
         p, stride = ctypes.c_void_p(x.data_ptr()), ctypes.c_longlong(8)
         head = getattr(lib, ("gla" if kind == "decay" else "bonus") + "_row_scan_head_floats")(p, stride, p, stride, p, stride, p, dim, vdim,
                                                                                                ctx.T // 64 + ctx.S)
-        rt.ops.ROW_SCAN_SCRATCH = head + 100  # at least one head's; the other kernel's scratch may make it more
-    try:
-        new, old = both(rt, run)
-    finally:
-        rt.ops.ROW_SCAN_SCRATCH = type(rt.ops).ROW_SCAN_SCRATCH
+    new, old = both(rt, kind, run, monkeypatch, head)
     assert max(new) < TOL, (new, old)
