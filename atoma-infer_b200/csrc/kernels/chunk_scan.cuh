@@ -14,6 +14,10 @@
 // (relative, 2-norm; one prompt of 2,048 tokens, 64 heads of 128 x 64): outputs 1.4e-7, last state 6.4e-8; token by token in
 // float32 1.5e-7 and 7.0e-8, and with slow decays 1.4e-7 and 2.4e-7 against 5.2e-7 and 9.2e-7.
 //
+// Values that are not finite, and columns whose results are not, are taken token by token (chunk_in_order).
+//
+// Values that are not finite, and columns whose results are not, are taken token by token (chunk_in_order).
+//
 // What bounds it: the phases of a block (loads, logs, conversion, products) follow one another and two blocks share a
 // multiprocessor; the tensor pipe is 33 to 37 % busy, issue slots 40 %.  The state shares (N * P floats a chunk and head,
 // written, chained and read) stay in L2.  CHUNK = 128: 64 would double the shares' traffic for a tenth fewer products, 256
@@ -171,11 +175,89 @@ __device__ __forceinline__ bool chunk_of(const int* __restrict__ meta, const int
     return false;
 }
 
+// ----------------------------------------------------------------------------- token by token
+// A block's columns of its chunk in order and in float32, for what the products cannot carry: a weight of 0 times a later token's
+// infinity is no number, and an infinity is no sum of three bfloat16 numbers.  A kernel whose results are not all finite ends with
+// it, so that only the tokens behind such a value see it, as a scan in order gives it.  `outputs`: o (and n . q) from the chunk's S_in;
+// else the chunk's share of S_out, or for an entry's only chunk the slot, what it held staying as S_in.  All 256 threads: a
+// column of the block each, the rows dealt out over four of them.  (It finds its chunk by itself: nothing has to be kept for it.)
+template <int NB, int KIND>
+__device__ __noinline__ void chunk_in_order(const ChunkArgs& A, int col_blocks, bool outputs) {
+    const int h = blockIdx.x / col_blocks, p0 = blockIdx.x % col_blocks * CHUNK_PB;
+    ChunkPlace at;
+    if (!chunk_of<CHUNK>(A.meta, A.cu_tokens, blockIdx.y, at)) return;
+    const size_t HS = (size_t)A.N * A.P, CS = HS + (KIND == CHUNK_MEMORY ? A.N : 0);
+    float* kept = A.scratch + ((size_t)blockIdx.y * A.heads + h) * CS;
+    float* slot = A.state + (size_t)A.slots[at.e] * A.slot_stride + (size_t)h * HS;
+    const float* from = outputs ? kept : (at.only ? slot : nullptr);
+    float *first = !outputs && at.only ? kept : nullptr, *last = outputs ? nullptr : (at.only ? slot : kept);
+    constexpr int ROWS = NB / 4;
+    __shared__ float part[4][CHUNK_PB];
+    const int col = threadIdx.x % CHUNK_PB, p = p0 + col, n0 = threadIdx.x / CHUNK_PB * ROWS;
+    const bool real = p < A.P;
+    float S[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        S[i] = from && real && n0 + i < A.N ? from[(size_t)(n0 + i) * A.P + p] : 0.f;
+        if (first && real && n0 + i < A.N) first[(size_t)(n0 + i) * A.P + p] = S[i];
+    }
+    for (int t = at.t0; t < at.t0 + at.nt; ++t) {
+        const __nv_bfloat16 *q = A.q + (size_t)t * A.q_stride + (size_t)(h / A.share) * A.N, *k = A.k + (size_t)t * A.k_stride + (size_t)(h / A.share) * A.N;
+        const float v = real ? __bfloat162float(A.v[(size_t)t * A.v_stride + (size_t)h * A.P + p]) : 0.f;
+        float a, b;
+        if (KIND == CHUNK_SSM) {
+            const float raw = __bfloat162float(A.dt[(size_t)t * A.dt_stride + h]) + A.dt_bias[h];
+            b = raw > 20.f ? raw : log1pf(expf(raw));
+            a = expf(-expf(A.a_log[h]) * b);
+        } else {
+            a = A.gates[((size_t)t * A.heads + h) * 2], b = A.gates[((size_t)t * A.heads + h) * 2 + 1];
+        }
+        float sum = 0.f;
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            if (n0 + i >= A.N) break;
+            const float kv = __bfloat162float(k[n0 + i]);
+            S[i] = fmaf(a, S[i], KIND == CHUNK_SSM ? kv * (b * v) : kv * b * v);
+            sum = fmaf(S[i], __bfloat162float(q[n0 + i]) * A.q_scale, sum);
+        }
+        if (!outputs) continue;
+        __syncthreads();
+        part[threadIdx.x / CHUNK_PB][col] = sum;
+        __syncthreads();
+        if (threadIdx.x < CHUNK_PB && real) {
+            const float y = (part[0][col] + part[1][col]) + (part[2][col] + part[3][col]);
+            A.o[((size_t)t * A.heads + h) * A.P + p] = KIND == CHUNK_SSM ? fmaf(A.d_skip[h], v, y) : y;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+        if (last && real && n0 + i < A.N) last[(size_t)(n0 + i) * A.P + p] = S[i];
+    if (KIND == CHUNK_MEMORY && outputs && p0 == 0 && threadIdx.x < 32) {  // n . q
+        float n[NB / 32];
+#pragma unroll
+        for (int i = 0; i < NB / 32; ++i) n[i] = threadIdx.x + i * 32 < A.N ? kept[HS + threadIdx.x + i * 32] : 0.f;
+        for (int t = at.t0; t < at.t0 + at.nt; ++t) {
+            const __nv_bfloat16 *q = A.q + (size_t)t * A.q_stride + (size_t)h * A.N, *k = A.k + (size_t)t * A.k_stride + (size_t)h * A.N;
+            const float a = A.gates[((size_t)t * A.heads + h) * 2], b = A.gates[((size_t)t * A.heads + h) * 2 + 1];
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < NB / 32; ++i) {
+                const int row = threadIdx.x + i * 32;
+                if (row >= A.N) break;
+                n[i] = fmaf(a, n[i], __bfloat162float(k[row]) * b);
+                sum = fmaf(n[i], __bfloat162float(q[row]) * A.q_scale, sum);
+            }
+            sum = warp_sum(sum);
+            if (threadIdx.x == 0) A.nq[(size_t)t * A.heads + h] = sum;
+        }
+    }
+}
+
 // ----------------------------------------------------------------------------- every chunk's share of the state
 // One block per (head x column block, chunk): NB (N rounded up) rows x CHUNK_PB columns, the eight warps a grid of WM x WN.
 // The k values are the A operand, read transposed; the weighted v the B operand, as three pairs.
 template <int NB, int KIND>
-__global__ void __launch_bounds__(256, 2) chunk_states_kernel(const ChunkArgs A, int col_blocks) {
+__global__ void __launch_bounds__(256, 2) chunk_states_kernel(const __grid_constant__ ChunkArgs A, int col_blocks) {
     constexpr int WM = NB >= 64 ? 4 : 2, WN = 8 / WM, MT = NB / 16 / WM, NT = CHUNK_PB / 8 / WN, KROW = NB * 2, VROW = CHUNK_PB * 2;
     extern __shared__ __align__(128) char chunk_smem[];
     char *ks = chunk_smem, *vs = chunk_smem + CHUNK * KROW;  // [CHUNK][NB]; three tiles [CHUNK][CHUNK_PB]
@@ -243,25 +325,36 @@ __global__ void __launch_bounds__(256, 2) chunk_states_kernel(const ChunkArgs A,
     const float decay = expf(L.hi[CHUNK - 1] + L.lo[CHUNK - 1]);
     // an entry's only chunk needs no chain: what the slot holds is its S_in, and the slot is updated here
     float* slot = A.state + (size_t)A.slots[at.e] * A.slot_stride + (size_t)h * HS;
+    float odd = 0.f;  // no number as soon as one result is not finite
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int z = 0; z < 2; ++z) {
-                const int row = m0 + i * 16 + (lane >> 2) + z * 8, p = p0 + n0 + n * 8 + (lane & 3) * 2;
-                if (p >= A.P || row >= A.N) continue;
-                float2 x = make_float2(acc[i][n][2 * z], acc[i][n][2 * z + 1]);
-                if (at.only) {
-                    float* s = slot + (size_t)row * A.P + p;
-                    const float2 in = A.slot_pairs ? *reinterpret_cast<const float2*>(s) : make_float2(s[0], s[1]);
-                    const float2 out = make_float2(fmaf(decay, in.x, x.x), fmaf(decay, in.y, x.y));
-                    if (A.slot_pairs) *reinterpret_cast<float2*>(s) = out;
-                    else s[0] = out.x, s[1] = out.y;
-                    x = in;
+            for (int j = 0; j < 4; ++j) odd = fmaf(acc[i][n][j], 0.f, odd);
+    if (__syncthreads_or(odd != 0.f)) {
+        chunk_in_order<NB, KIND>(A, col_blocks, false);
+    } else {
+#pragma unroll
+        for (int i = 0; i < MT; ++i)
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int z = 0; z < 2; ++z) {
+                    const int row = m0 + i * 16 + (lane >> 2) + z * 8, p = p0 + n0 + n * 8 + (lane & 3) * 2;
+                    if (p >= A.P || row >= A.N) continue;
+                    float2 x = make_float2(acc[i][n][2 * z], acc[i][n][2 * z + 1]);
+                    if (at.only) {
+                        float* s = slot + (size_t)row * A.P + p;
+                        const float2 in = A.slot_pairs ? *reinterpret_cast<const float2*>(s) : make_float2(s[0], s[1]);
+                        const float2 out = make_float2(fmaf(decay, in.x, x.x), fmaf(decay, in.y, x.y));
+                        if (A.slot_pairs) *reinterpret_cast<float2*>(s) = out;
+                        else s[0] = out.x, s[1] = out.y;
+                        x = in;
+                    }
+                    *reinterpret_cast<float2*>(dst + (size_t)row * A.P + p) = x;
                 }
-                *reinterpret_cast<float2*>(dst + (size_t)row * A.P + p) = x;
-            }
+    }
     if (p0 == 0) {
         if (KIND == CHUNK_MEMORY && tid < A.N) {
             float s = 0.f;
@@ -333,7 +426,7 @@ __global__ void __launch_bounds__(256) chunk_chain_kernel(const ChunkArgs A) {
 // One block per (head x column block, chunk); a warp has 16 tokens (warps of one scheduler get rows whose causal work adds up
 // to the same).  q waits in registers; its tile's place then holds S_in as three pairs.
 template <int NB, int KIND>
-__global__ void __launch_bounds__(256, 2) chunk_outputs_kernel(const ChunkArgs A, int col_blocks) {
+__global__ void __launch_bounds__(256, 2) chunk_outputs_kernel(const __grid_constant__ ChunkArgs A, int col_blocks) {
     constexpr int KROW = NB * 2, VROW = CHUNK_PB * 2, KT = NB / 16, NT = CHUNK_PB / 8;
     constexpr int SHARED0 = CHUNK * KROW > 3 * NB * VROW ? CHUNK * KROW : 3 * NB * VROW;
     extern __shared__ __align__(128) char chunk_smem[];
@@ -380,109 +473,113 @@ __global__ void __launch_bounds__(256, 2) chunk_outputs_kernel(const ChunkArgs A
         for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(ss + j * NB * VROW + piece<VROW>(n, pc)) = make_uint4(s[j][0], s[j][1], s[j][2], s[j][3]);
     }
     __syncthreads();
-    if (!busy) return;
-
-    float acc[NT][4] = {};
+    float odd = 0.f;  // no number as soon as one result is not finite
+    if (busy) {
+        float acc[NT][4] = {};
 #pragma unroll
-    for (int k2 = 0; k2 < KT; k2 += 2) {  // q^T S_in: two steps of k a run
+        for (int k2 = 0; k2 < KT; k2 += 2) {  // q^T S_in: two steps of k a run
 #pragma unroll
-        for (int n = 0; n < NT; n += 2) {
-            float run[2][4] = {};
+            for (int n = 0; n < NT; n += 2) {
+                float run[2][4] = {};
 #pragma unroll
-            for (int k = k2; k < k2 + 2; ++k)
+                for (int k = k2; k < k2 + 2; ++k)
 #pragma unroll
-                for (int j = 2; j >= 0; --j) {
-                    uint32_t b[4];
-                    ldmatrix4_t(b, smem_address(ss) + j * NB * VROW + piece<VROW>(k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n + (lane >> 4)));
-                    mma16816(run[0], qa[k], b[0], b[1]);
-                    mma16816(run[1], qa[k], b[2], b[3]);
+                    for (int j = 2; j >= 0; --j) {
+                        uint32_t b[4];
+                        ldmatrix4_t(b, smem_address(ss) + j * NB * VROW + piece<VROW>(k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n + (lane >> 4)));
+                        mma16816(run[0], qa[k], b[0], b[1]);
+                        mma16816(run[1], qa[k], b[2], b[3]);
+                    }
+#pragma unroll
+                for (int z = 0; z < 2; ++z)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[n + z][j] += run[z][j];
+            }
+        }
+        const int ta = rb * 16 + g, tb = ta + 8;
+        const float hi_a = L.hi[ta], lo_a = L.lo[ta], hi_b = L.hi[tb], lo_b = L.lo[tb], ea = expf(hi_a + lo_a), eb = expf(hi_b + lo_b);
+        float na = 0.f, nb = 0.f;  // CHUNK_MEMORY: n . q
+        if (KIND == CHUNK_MEMORY) {
+#pragma unroll
+            for (int k = 0; k < KT; ++k)
+#pragma unroll
+                for (int z = 0; z < 4; ++z) {  // registers 0 and 2: row g, 1 and 3: row g + 8; 0 and 1: k, 2 and 3: k + 8
+                    const int n = k * 16 + q2 + (z >> 1) * 8;
+                    float& s = z & 1 ? nb : na;
+                    s = fmaf(__uint_as_float(qa[k][z] << 16), n_in[n], s);
+                    s = fmaf(__uint_as_float(qa[k][z] & 0xffff0000u), n_in[n + 1], s);
                 }
-#pragma unroll
-            for (int z = 0; z < 2; ++z)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[n + z][j] += run[z][j];
+            na *= ea, nb *= eb;
         }
-    }
-    const int ta = rb * 16 + g, tb = ta + 8;
-    const float hi_a = L.hi[ta], lo_a = L.lo[ta], hi_b = L.hi[tb], lo_b = L.lo[tb], ea = expf(hi_a + lo_a), eb = expf(hi_b + lo_b);
-    float na = 0.f, nb = 0.f;  // CHUNK_MEMORY: n . q
-    if (KIND == CHUNK_MEMORY) {
 #pragma unroll
-        for (int k = 0; k < KT; ++k)
-#pragma unroll
-            for (int z = 0; z < 4; ++z) {  // registers 0 and 2: row g, 1 and 3: row g + 8; 0 and 1: k, 2 and 3: k + 8
-                const int n = k * 16 + q2 + (z >> 1) * 8;
-                float& s = z & 1 ? nb : na;
-                s = fmaf(__uint_as_float(qa[k][z] << 16), n_in[n], s);
-                s = fmaf(__uint_as_float(qa[k][z] & 0xffff0000u), n_in[n + 1], s);
-            }
-        na *= ea, nb *= eb;
-    }
-#pragma unroll
-    for (int n = 0; n < NT; ++n) acc[n][0] *= ea, acc[n][1] *= ea, acc[n][2] *= eb, acc[n][3] *= eb;
+        for (int n = 0; n < NT; ++n) acc[n][0] *= ea, acc[n][1] *= ea, acc[n][2] *= eb, acc[n][3] *= eb;
 #pragma unroll 1
-    for (int sb = 0; sb <= rb; ++sb) {
-        float sc[2][4] = {};
+        for (int sb = 0; sb <= rb; ++sb) {
+            float sc[2][4] = {};
 #pragma unroll
-        for (int k = 0; k < KT; ++k) {
-            uint32_t b[4];
-            ldmatrix4(b, smem_address(ks) + piece<KROW>(sb * 16 + (lane & 7) + (lane >> 4) * 8, k * 2 + ((lane >> 3) & 1)));
-            mma16816(sc[0], qa[k], b[0], b[1]);
-            mma16816(sc[1], qa[k], b[2], b[3]);
-        }
-        uint32_t w[3][4];
-#pragma unroll
-        for (int z = 0; z < 2; ++z) {
-            const int s0 = sb * 16 + z * 8 + q2;
-            float v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int s = s0 + (j & 1), t = j < 2 ? ta : tb;
-                const float f = decay_between(j < 2 ? hi_a : hi_b, j < 2 ? lo_a : lo_b, L.hi[s], L.lo[s]) * L.b[s];
-                v[j] = s <= t ? sc[z][j] * f : 0.f;
+            for (int k = 0; k < KT; ++k) {
+                uint32_t b[4];
+                ldmatrix4(b, smem_address(ks) + piece<KROW>(sb * 16 + (lane & 7) + (lane >> 4) * 8, k * 2 + ((lane >> 3) & 1)));
+                mma16816(sc[0], qa[k], b[0], b[1]);
+                mma16816(sc[1], qa[k], b[2], b[3]);
             }
-            if (KIND == CHUNK_MEMORY) na += v[0] + v[1], nb += v[2] + v[3];
-            split_pair(v[0], v[1], w[0][z * 2], w[1][z * 2], w[2][z * 2]);
-            split_pair(v[2], v[3], w[0][z * 2 + 1], w[1][z * 2 + 1], w[2][z * 2 + 1]);
+            uint32_t w[3][4];
+#pragma unroll
+            for (int z = 0; z < 2; ++z) {
+                const int s0 = sb * 16 + z * 8 + q2;
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int s = s0 + (j & 1), t = j < 2 ? ta : tb;
+                    const float f = decay_between(j < 2 ? hi_a : hi_b, j < 2 ? lo_a : lo_b, L.hi[s], L.lo[s]) * L.b[s];
+                    v[j] = s <= t ? sc[z][j] * f : 0.f;
+                }
+                if (KIND == CHUNK_MEMORY) na += v[0] + v[1], nb += v[2] + v[3];
+                split_pair(v[0], v[1], w[0][z * 2], w[1][z * 2], w[2][z * 2]);
+                split_pair(v[2], v[3], w[0][z * 2 + 1], w[1][z * 2 + 1], w[2][z * 2 + 1]);
+            }
+#pragma unroll
+            for (int n = 0; n < NT; n += 2) {
+                uint32_t b[4];
+                ldmatrix4_t(b, smem_address(vs) + piece<VROW>(sb * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n + (lane >> 4)));
+                float run[2][4] = {};
+#pragma unroll
+                for (int j = 2; j >= 0; --j) mma16816(run[0], w[j], b[0], b[1]), mma16816(run[1], w[j], b[2], b[3]);
+#pragma unroll
+                for (int z = 0; z < 2; ++z)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[n + z][j] += run[z][j];
+            }
         }
+        const size_t out_stride = (size_t)A.heads * A.P;
+        float* oa = A.o + (size_t)(t0 + ta) * out_stride + (size_t)h * A.P + p0 + q2;
+        const float dskip = KIND == CHUNK_SSM ? A.d_skip[h] : 0.f;
 #pragma unroll
-        for (int n = 0; n < NT; n += 2) {
-            uint32_t b[4];
-            ldmatrix4_t(b, smem_address(vs) + piece<VROW>(sb * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n + (lane >> 4)));
-            float run[2][4] = {};
+        for (int n = 0; n < NT; ++n) {
+            if (p0 + n * 8 >= A.P) break;
+            float* x = acc[n];
+            if (KIND == CHUNK_SSM) {
+                const uint32_t va = *reinterpret_cast<const uint32_t*>(vs + piece<VROW>(ta, n) + q2 * 2), vb = *reinterpret_cast<const uint32_t*>(vs + piece<VROW>(tb, n) + q2 * 2);
+                x[0] = fmaf(dskip, __uint_as_float(va << 16), x[0]), x[1] = fmaf(dskip, __uint_as_float(va & 0xffff0000u), x[1]);
+                x[2] = fmaf(dskip, __uint_as_float(vb << 16), x[2]), x[3] = fmaf(dskip, __uint_as_float(vb & 0xffff0000u), x[3]);
+            } else {
+                x[0] *= A.q_scale, x[1] *= A.q_scale, x[2] *= A.q_scale, x[3] *= A.q_scale;
+            }
+            odd = fmaf(x[0], 0.f, fmaf(x[1], 0.f, fmaf(x[2], 0.f, fmaf(x[3], 0.f, odd))));
+            if (ta < nt) *reinterpret_cast<float2*>(oa + n * 8) = make_float2(x[0], x[1]);
+            if (tb < nt) *reinterpret_cast<float2*>(oa + 8 * out_stride + n * 8) = make_float2(x[2], x[3]);
+        }
+        if (KIND == CHUNK_MEMORY && p0 == 0) {
 #pragma unroll
-            for (int j = 2; j >= 0; --j) mma16816(run[0], w[j], b[0], b[1]), mma16816(run[1], w[j], b[2], b[3]);
-#pragma unroll
-            for (int z = 0; z < 2; ++z)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[n + z][j] += run[z][j];
+            for (int d = 1; d < 4; d <<= 1) na += __shfl_xor_sync(0xffffffffu, na, d), nb += __shfl_xor_sync(0xffffffffu, nb, d);
+            odd = fmaf(na, 0.f, fmaf(nb, 0.f, odd));
+            if ((lane & 3) == 0) {
+                if (ta < nt) A.nq[(size_t)(t0 + ta) * A.heads + h] = na * A.q_scale;
+                if (tb < nt) A.nq[(size_t)(t0 + tb) * A.heads + h] = nb * A.q_scale;
+            }
         }
     }
-    const size_t out_stride = (size_t)A.heads * A.P;
-    float* oa = A.o + (size_t)(t0 + ta) * out_stride + (size_t)h * A.P + p0 + q2;
-    const float dskip = KIND == CHUNK_SSM ? A.d_skip[h] : 0.f;
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        if (p0 + n * 8 >= A.P) break;
-        float* x = acc[n];
-        if (KIND == CHUNK_SSM) {
-            const uint32_t va = *reinterpret_cast<const uint32_t*>(vs + piece<VROW>(ta, n) + q2 * 2), vb = *reinterpret_cast<const uint32_t*>(vs + piece<VROW>(tb, n) + q2 * 2);
-            x[0] = fmaf(dskip, __uint_as_float(va << 16), x[0]), x[1] = fmaf(dskip, __uint_as_float(va & 0xffff0000u), x[1]);
-            x[2] = fmaf(dskip, __uint_as_float(vb << 16), x[2]), x[3] = fmaf(dskip, __uint_as_float(vb & 0xffff0000u), x[3]);
-        } else {
-            x[0] *= A.q_scale, x[1] *= A.q_scale, x[2] *= A.q_scale, x[3] *= A.q_scale;
-        }
-        if (ta < nt) *reinterpret_cast<float2*>(oa + n * 8) = make_float2(x[0], x[1]);
-        if (tb < nt) *reinterpret_cast<float2*>(oa + 8 * out_stride + n * 8) = make_float2(x[2], x[3]);
-    }
-    if (KIND == CHUNK_MEMORY && p0 == 0) {
-#pragma unroll
-        for (int d = 1; d < 4; d <<= 1) na += __shfl_xor_sync(0xffffffffu, na, d), nb += __shfl_xor_sync(0xffffffffu, nb, d);
-        if ((lane & 3) == 0) {
-            if (ta < nt) A.nq[(size_t)(t0 + ta) * A.heads + h] = na * A.q_scale;
-            if (tb < nt) A.nq[(size_t)(t0 + tb) * A.heads + h] = nb * A.q_scale;
-        }
-    }
+    if (__syncthreads_or(odd != 0.f)) chunk_in_order<NB, KIND>(A, col_blocks, true);
 }
 
 // ----------------------------------------------------------------------------- launches

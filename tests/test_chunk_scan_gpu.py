@@ -205,3 +205,53 @@ def test_a_decay_per_row_in_matrix_chunks(rt, monkeypatch, lengths, heads, dim, 
                                                                                                ctx.T // 64 + ctx.S)
     new, old = both(rt, kind, run, monkeypatch, head)
     assert max(new) < TOL, (new, old)
+
+
+# what is written where before the scan: tensor, token of the step, index in its row (or slot and index), value
+ODD = [("v", 150, 3, float("inf")), ("v", 167, 67, float("nan")), ("v", 5, 71, float("-inf")), ("k", 160, 9, float("inf")), ("q", 140, 2, float("-inf")),
+       ("state", 0, 77, float("inf")), ("v", 137, 3, float("inf")), ("v", 130, 1, 1e36)]
+
+
+@pytest.mark.parametrize("odd", ODD, ids=lambda o: f"{o[0]}-{o[1]}-{o[3]}")
+@pytest.mark.parametrize("kind,dim", [("space", 64), ("space", 128), ("memory", 128), ("memory", 24)])
+def test_what_is_no_finite_number_reaches_later_tokens_only(rt, monkeypatch, kind, dim, odd):
+    """An infinity or no number in a row or a state: the same tokens, columns and states as on the kernel that goes token by token
+    (where it stands in the middle of a run of 16, tokens of its run come before and behind it)."""
+    what, token, place, value = odd
+    heads, vdim, lengths, tau = 2, 72, (129, 1, 16, 200), 2.0
+    g = torch.Generator().manual_seed(dim)
+    T, nk, nv = sum(lengths), heads * dim, heads * vdim
+    ctx, dev = context(rt, lengths), lambda t: t.to(rt.device)
+    q, k, v = ((torch.randn(T, n, generator=g) * 0.5).bfloat16() for n in (nk, nk, nv))
+    S0 = torch.randn(len(lengths), nk * vdim + 2 * nk + 2 * heads, generator=g) * 0.5
+    {"q": q, "k": k, "v": v, "state": S0}[what][token, place] = value
+    z, bias, u = torch.randn(T, nk, generator=g), torch.randn(nk, generator=g), torch.randn(nk, generator=g)
+    z += -5 if kind == "bonus" else 3  # memories of some tens of tokens: no decay over a chunk is zero
+    dt = (torch.randn(T, heads, generator=g) * 0.5 - 4).bfloat16()
+    logits = torch.randn(T, 2 * heads, generator=g) + torch.tensor([0.0] * heads + [4.0] * heads)
+    zeros, ones = torch.zeros(2 * heads, device=rt.device), torch.ones(heads, device=rt.device)
+
+    def run():
+        st, o = dev(S0.clone()), torch.full((T, nv), 7.0, device=rt.device)
+        state, more = st[:, :nk * vdim].view(len(lengths), heads, dim, vdim), ()
+        if kind == "space":
+            rt.ops.ssm_scan(dev(torch.cat([v, k, q], 1)), dev(dt), zeros[:heads], zeros[:heads], ones, state, ctx, o, heads=heads, head_dim=vdim, nstate=dim, groups=heads)
+        elif kind == "memory":
+            n_state, m_state = st[:, nk * vdim:nk * vdim + nk].view(-1, heads, dim), st[:, nk * vdim + nk:nk * vdim + nk + heads]
+            nq, floor = torch.empty(T, heads, device=rt.device), torch.empty(T, heads, device=rt.device)
+            rt.ops.memory_scan(dev(q), dev(k), dev(v), dev(logits), zeros, 9.0, dim ** -0.5, state, n_state, m_state, ctx, o, nq, floor,
+                               heads=heads, dim=dim, vdim=vdim)
+            more = (nq, n_state)
+        elif kind == "decay":
+            rt.ops.gla_scan(dev(q), dev(k), dev(v), dev(z), dev(bias), tau, dim ** -0.5, state, ctx, o, heads=heads, dim=dim, vdim=vdim)
+        else:
+            rt.ops.bonus_scan(dev(q), dev(k), dev(v), dev(z), dev(bias), dev(u), state, ctx, o, heads=heads, dim=dim, vdim=vdim)
+        return tuple(t.double().cpu() for t in (o, state) + more)
+
+    for new, old in zip(*both(rt, kind, run, monkeypatch)):
+        assert torch.equal(new.isnan(), old.isnan())
+        assert torch.equal(new.isinf(), old.isinf()) and torch.equal(new[new.isinf()], old[old.isinf()])
+        ok = old.isfinite()
+        small = ok & (old.abs() < 1e30)  # (beside the largest numbers there are)
+        assert bool(((new - old)[small].abs() <= TOL * max(1.0, old[small].abs().max().item())).all())
+        assert bool(((new - old)[ok].abs() <= TOL * old[ok].abs().max().item()).all())
