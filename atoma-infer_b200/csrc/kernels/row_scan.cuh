@@ -269,9 +269,62 @@ __device__ __forceinline__ void load_split(uint32_t (&f)[3][4], const uint4* src
     }
 }
 
+// ----------------------------------------------------------------------------- token by token
+// As chunk_in_order (chunk_scan.cuh), for the same reasons; the decays from the logits again.
+template <int NB, int KIND>
+__device__ __noinline__ void row_in_order(const RowScanArgs& A, int col_blocks, bool outputs) {
+    const int hl = blockIdx.x / col_blocks, h = A.h0 + hl, p0 = blockIdx.x % col_blocks * CHUNK_PB;
+    ChunkPlace at;
+    if (!chunk_of<RCHUNK>(A.meta, A.cu_tokens, blockIdx.y, at)) return;
+    const size_t HS = (size_t)A.N * A.P;
+    float* kept = A.share + ((size_t)blockIdx.y * A.hn + hl) * HS;
+    float* slot = A.state + (size_t)A.slots[at.e] * A.slot_stride + (size_t)h * HS;
+    const float* from = outputs ? kept : (at.only ? slot : nullptr);
+    float *first = !outputs && at.only ? kept : nullptr, *last = outputs ? nullptr : (at.only ? slot : kept);
+    constexpr int ROWS = NB / 4;
+    __shared__ float part[2][4][CHUNK_PB];
+    const int col = threadIdx.x % CHUNK_PB, p = p0 + col, g = threadIdx.x / CHUNK_PB, n0 = g * ROWS;
+    const bool real = p < A.P;
+    float S[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+        S[i] = from && real && n0 + i < A.N ? from[(size_t)(n0 + i) * A.P + p] : 0.f;
+        if (first && real && n0 + i < A.N) first[(size_t)(n0 + i) * A.P + p] = S[i];
+    }
+    for (int t = at.t0; t < at.t0 + at.nt; ++t) {
+        const __nv_bfloat16 *q = A.q + (size_t)t * A.q_stride + (size_t)h * A.N, *k = A.k + (size_t)t * A.k_stride + (size_t)h * A.N;
+        const float* z = A.z + (size_t)t * A.z_stride + (size_t)h * A.N;
+        const float v = real ? __bfloat162float(A.v[(size_t)t * A.v_stride + (size_t)h * A.P + p]) : 0.f;
+        float sum = 0.f, own = 0.f;  // ROW_BONUS: `own`, the current token's weight on its own v
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i) {
+            const int n = n0 + i;
+            if (n >= A.N) break;
+            const float x = z[n] + (A.z_bias ? A.z_bias[(size_t)h * A.N + n] : 0.f), kv = __bfloat162float(k[n]);
+            const float a = KIND == ROW_BONUS ? expf(-expf(x)) : expf(-(-x > 20.f ? -x : log1pf(expf(-x))) * A.inv_tau);
+            const float qv = __bfloat162float(q[n]) * A.q_scale, before = S[i];
+            S[i] = fmaf(a, before, kv * v);
+            sum = fmaf(KIND == ROW_BONUS ? before : S[i], qv, sum);
+            if (KIND == ROW_BONUS) own = fmaf(qv * A.bonus[(size_t)h * A.N + n], kv, own);
+        }
+        if (!outputs) continue;
+        __syncthreads();
+        part[0][g][col] = sum, part[1][g][col] = own;
+        __syncthreads();
+        if (g == 0 && real) {
+            float y = (part[0][0][col] + part[0][1][col]) + (part[0][2][col] + part[0][3][col]);
+            if (KIND == ROW_BONUS) y = fmaf((part[1][0][col] + part[1][1][col]) + (part[1][2][col] + part[1][3][col]), v, y);
+            A.o[((size_t)t * A.heads + h) * A.P + p] = y;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+        if (last && real && n0 + i < A.N) last[(size_t)(n0 + i) * A.P + p] = S[i];
+}
+
 // ----------------------------------------------------------------------------- every chunk's share of the state
-template <int NB>
-__global__ void __launch_bounds__(256, 2) row_states_kernel(const RowScanArgs A, int col_blocks) {
+template <int NB, int KIND>
+__global__ void __launch_bounds__(256, 2) row_states_kernel(const __grid_constant__ RowScanArgs A, int col_blocks) {
     constexpr int MT = NB / 16, WN = 8 / MT, NT = CHUNK_PB / 8 / WN, VROW = CHUNK_PB * 2;
     __shared__ __align__(128) char vs[RCHUNK * VROW];
     const int hl = blockIdx.x / col_blocks, h = A.h0 + hl, p0 = blockIdx.x % col_blocks * CHUNK_PB, c = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -311,6 +364,15 @@ __global__ void __launch_bounds__(256, 2) row_states_kernel(const RowScanArgs A,
     const size_t HS = (size_t)A.N * A.P;
     float* dst = A.share + ch * HS;
     float* slot = A.state + (size_t)A.slots[at.e] * A.slot_stride + (size_t)h * HS;
+    float odd = 0.f;  // no number as soon as one result is not finite
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) odd = fmaf(acc[n][j], 0.f, odd);
+    if (__syncthreads_or(odd != 0.f)) {
+        row_in_order<NB, KIND>(A, col_blocks, false);
+        return;
+    }
 #pragma unroll
     for (int z = 0; z < 2; ++z) {
         const int row = mt * 16 + (lane >> 2) + z * 8;
@@ -384,8 +446,8 @@ static __global__ void __launch_bounds__(256) row_chain_kernel(const RowScanArgs
 
 // ----------------------------------------------------------------------------- the outputs
 // One block per (head x column block, chunk): four rows of 16 tokens x two halves of the columns, a warp each.
-template <int NB>
-__global__ void __launch_bounds__(256, 2) row_outputs_kernel(const RowScanArgs A, int col_blocks) {
+template <int NB, int KIND>
+__global__ void __launch_bounds__(256, 2) row_outputs_kernel(const __grid_constant__ RowScanArgs A, int col_blocks) {
     constexpr int KT = NB / 16, NT = CHUNK_PB / 16, VROW = CHUNK_PB * 2;
     extern __shared__ __align__(128) char row_out_smem[];
     char *ss = row_out_smem, *vs = row_out_smem + 3 * NB * VROW;  // S_in as three tiles [NB][CHUNK_PB]; v
@@ -419,59 +481,63 @@ __global__ void __launch_bounds__(256, 2) row_outputs_kernel(const RowScanArgs A
     if (rb * 16 < nt) load_split(a, qsrc);
     copies_done();
     __syncthreads();
-    if (rb * 16 >= nt) return;
-    float acc[NT][4] = {};
+    float odd = 0.f;  // no number as soon as one result is not finite
+    if (rb * 16 < nt) {
+        float acc[NT][4] = {};
 #pragma unroll 2
-    for (int kt = 0; kt < KT; ++kt) {
-        uint32_t next[3][4];
-        load_split(next, qsrc + min(kt + 1, KT - 1) * 96);
-        float run[NT][4] = {};
+        for (int kt = 0; kt < KT; ++kt) {
+            uint32_t next[3][4];
+            load_split(next, qsrc + min(kt + 1, KT - 1) * 96);
+            float run[NT][4] = {};
 #pragma unroll
-        for (int n = 0; n < NT; n += 2) {
-            uint32_t b0[3][2], b1[3][2];
+            for (int n = 0; n < NT; n += 2) {
+                uint32_t b0[3][2], b1[3][2];
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                uint32_t b[4];
-                ldmatrix4_t(b, smem_address(ss) + j * NB * VROW + piece<VROW>(kt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n0 + n + (lane >> 4)));
-                b0[j][0] = b[0], b0[j][1] = b[1], b1[j][0] = b[2], b1[j][1] = b[3];
+                for (int j = 0; j < 3; ++j) {
+                    uint32_t b[4];
+                    ldmatrix4_t(b, smem_address(ss) + j * NB * VROW + piece<VROW>(kt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n0 + n + (lane >> 4)));
+                    b0[j][0] = b[0], b0[j][1] = b[1], b1[j][0] = b[2], b1[j][1] = b[3];
+                }
+                mma_split6(run[n], a, b0);
+                mma_split6(run[n + 1], a, b1);
             }
-            mma_split6(run[n], a, b0);
-            mma_split6(run[n + 1], a, b1);
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[n][j] += run[n][j];
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+#pragma unroll
+                for (int z = 0; z < 4; ++z) a[j][z] = next[j][z];
         }
+        const uint4* wsrc = A.wf + (ch * 4 + rb) * 4 * 96 + lane;
+        for (int sb = 0; sb <= rb; ++sb) {
+            load_split(a, wsrc + sb * 96);
+            float run[NT][4] = {};
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+            for (int n = 0; n < NT; n += 2) {
+                uint32_t b[4];
+                ldmatrix4_t(b, smem_address(vs) + piece<VROW>(sb * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n0 + n + (lane >> 4)));
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[n][j] += run[n][j];
+                for (int j = 2; j >= 0; --j) mma16816(run[n], a[j], b[0], b[1]), mma16816(run[n + 1], a[j], b[2], b[3]);
+            }
 #pragma unroll
-        for (int j = 0; j < 3; ++j)
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int z = 0; z < 4; ++z) a[j][z] = next[j][z];
-    }
-    const uint4* wsrc = A.wf + (ch * 4 + rb) * 4 * 96 + lane;
-    for (int sb = 0; sb <= rb; ++sb) {
-        load_split(a, wsrc + sb * 96);
-        float run[NT][4] = {};
-#pragma unroll
-        for (int n = 0; n < NT; n += 2) {
-            uint32_t b[4];
-            ldmatrix4_t(b, smem_address(vs) + piece<VROW>(sb * 16 + (lane & 7) + ((lane >> 3) & 1) * 8, n0 + n + (lane >> 4)));
-#pragma unroll
-            for (int j = 2; j >= 0; --j) mma16816(run[n], a[j], b[0], b[1]), mma16816(run[n + 1], a[j], b[2], b[3]);
+                for (int j = 0; j < 4; ++j) acc[n][j] += run[n][j];
         }
+        const int ta = rb * 16 + g;
+        const size_t stride = (size_t)A.heads * A.P;
+        float* oa = A.o + (size_t)(t0 + ta) * stride + (size_t)h * A.P + p0 + q2;
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[n][j] += run[n][j];
+        for (int n = 0; n < NT; ++n) {
+            if (p0 + (n0 + n) * 8 >= A.P) break;
+            odd = fmaf(acc[n][0], 0.f, fmaf(acc[n][1], 0.f, fmaf(acc[n][2], 0.f, fmaf(acc[n][3], 0.f, odd))));
+            if (ta < nt) *reinterpret_cast<float2*>(oa + (n0 + n) * 8) = make_float2(acc[n][0] * A.q_scale, acc[n][1] * A.q_scale);
+            if (ta + 8 < nt) *reinterpret_cast<float2*>(oa + 8 * stride + (n0 + n) * 8) = make_float2(acc[n][2] * A.q_scale, acc[n][3] * A.q_scale);
+        }
     }
-    const int ta = rb * 16 + g;
-    const size_t stride = (size_t)A.heads * A.P;
-    float* oa = A.o + (size_t)(t0 + ta) * stride + (size_t)h * A.P + p0 + q2;
-#pragma unroll
-    for (int n = 0; n < NT; ++n) {
-        if (p0 + (n0 + n) * 8 >= A.P) break;
-        if (ta < nt) *reinterpret_cast<float2*>(oa + (n0 + n) * 8) = make_float2(acc[n][0] * A.q_scale, acc[n][1] * A.q_scale);
-        if (ta + 8 < nt) *reinterpret_cast<float2*>(oa + 8 * stride + (n0 + n) * 8) = make_float2(acc[n][2] * A.q_scale, acc[n][3] * A.q_scale);
-    }
+    if (__syncthreads_or(odd != 0.f)) row_in_order<NB, KIND>(A, col_blocks, true);
 }
 
 // ----------------------------------------------------------------------------- launches
@@ -490,7 +556,7 @@ static int row_scan_run(RowScanArgs a, float* scratch, size_t scratch_floats, cu
     cudaError_t err = cudaSuccess;
     if (!configured) {
         err = cudaFuncSetAttribute(row_prepare_kernel<NB, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p);
-        if (err == cudaSuccess) err = cudaFuncSetAttribute(row_outputs_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_o);
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(row_outputs_kernel<NB, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_o);
         if (err != cudaSuccess) return (int)err;
         configured = true;
     }
@@ -507,10 +573,10 @@ static int row_scan_run(RowScanArgs a, float* scratch, size_t scratch_floats, cu
         a.share = reinterpret_cast<float*>(a.wf + units * 16 * 96);
         a.decay = a.share + units * a.N * a.P;
         err = launch_kernel(row_prepare_kernel<NB, KIND>, dim3(a.hn, a.max_chunks), PREPARE_THREADS, smem_p, stream, a);
-        if (err == cudaSuccess) err = launch_kernel(row_states_kernel<NB>, dim3(a.hn * col_blocks, a.max_chunks), 256, 0, stream, a, col_blocks);
+        if (err == cudaSuccess) err = launch_kernel(row_states_kernel<NB, KIND>, dim3(a.hn * col_blocks, a.max_chunks), 256, 0, stream, a, col_blocks);
         if (err == cudaSuccess)
             err = launch_kernel(row_chain_kernel, dim3(a.hn, a.S, (unsigned)(((size_t)a.N * a.P + 1023) / 1024)), 256, 0, stream, a);
-        if (err == cudaSuccess) err = launch_kernel(row_outputs_kernel<NB>, dim3(a.hn * col_blocks, a.max_chunks), 256, smem_o, stream, a, col_blocks);
+        if (err == cudaSuccess) err = launch_kernel(row_outputs_kernel<NB, KIND>, dim3(a.hn * col_blocks, a.max_chunks), 256, smem_o, stream, a, col_blocks);
         if (err != cudaSuccess) return (int)err;
     }
     return 0;

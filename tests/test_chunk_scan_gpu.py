@@ -213,7 +213,7 @@ ODD = [("v", 150, 3, float("inf")), ("v", 167, 67, float("nan")), ("v", 5, 71, f
 
 
 @pytest.mark.parametrize("odd", ODD, ids=lambda o: f"{o[0]}-{o[1]}-{o[3]}")
-@pytest.mark.parametrize("kind,dim", [("space", 64), ("space", 128), ("memory", 128), ("memory", 24)])
+@pytest.mark.parametrize("kind,dim", [("space", 64), ("space", 128), ("memory", 128), ("memory", 24), ("decay", 128), ("decay", 64), ("bonus", 40), ("bonus", 128)])
 def test_what_is_no_finite_number_reaches_later_tokens_only(rt, monkeypatch, kind, dim, odd):
     """An infinity or no number in a row or a state: the same tokens, columns and states as on the kernel that goes token by token
     (where it stands in the middle of a run of 16, tokens of its run come before and behind it)."""
