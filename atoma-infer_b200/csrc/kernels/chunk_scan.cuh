@@ -106,6 +106,7 @@ __device__ __forceinline__ void chunk_logs(ChunkLogs& L, const ChunkArgs& A, int
                 b = A.gates[(t * A.heads + h) * 2 + 1];
                 la = A.log_a[t * A.heads + h];
             }
+            la = la < -1e4f ? -1e4f : la;  // (a factor of zero either way, and no difference of infinities)
         }
         L.b[tid] = b;
         s = (double)la;

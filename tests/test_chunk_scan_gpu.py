@@ -255,3 +255,23 @@ def test_what_is_no_finite_number_reaches_later_tokens_only(rt, monkeypatch, kin
         small = ok & (old.abs() < 1e30)  # (beside the largest numbers there are)
         assert bool(((new - old)[small].abs() <= TOL * max(1.0, old[small].abs().max().item())).all())
         assert bool(((new - old)[ok].abs() <= TOL * old[ok].abs().max().item()).all())
+
+
+@pytest.mark.parametrize("a_log", [30.0, 87.0, 89.0, 120.0])
+def test_a_head_that_forgets_everything(rt, monkeypatch, a_log):
+    """Rates up to infinity: a state that keeps nothing of the tokens before, beside a head that keeps."""
+    heads, P, N, lengths = 2, 64, 64, (200, 16)
+    g = torch.Generator().manual_seed(3)
+    T = sum(lengths)
+    ctx, dev = context(rt, lengths), lambda t: t.to(rt.device)
+    xbc = torch.randn(T, heads * (P + 2 * N), generator=g).bfloat16()
+    dt = torch.randn(T, heads, generator=g).bfloat16()
+    rate, S0 = torch.tensor([a_log, 0.0]), torch.randn(len(lengths), heads, N, P, generator=g)
+
+    def run():
+        state, y = dev(S0.clone()), torch.full((T, heads * P), float("nan"), device=rt.device)
+        rt.ops.ssm_scan(dev(xbc), dev(dt), dev(torch.zeros(heads)), dev(rate), dev(torch.ones(heads)), state, ctx, y, heads=heads, head_dim=P, nstate=N, groups=heads)
+        return y.double().cpu(), state.double().cpu()
+
+    for new, old in zip(*both(rt, "space", run, monkeypatch)):
+        assert bool(old.isfinite().all()) and err(new, old) < TOL
