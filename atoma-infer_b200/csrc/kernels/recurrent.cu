@@ -156,7 +156,7 @@ extern "C" int head_norm_gate(const float* o, const void* g, int dtype, long lon
 // neighbouring states that one two-wide instruction updates.  y is the even states' sum plus the odd states', each in
 // ascending order, then the R threads' sums by halving.  B and C of SEL_TT tokens are staged in shared memory; the channel's
 // own u, step size and gate input of those tokens go straight into the thread's registers.  Pass 1 leaves the
-// step sizes for pass 3, so an entry's last chunk runs it too.
+// step sizes of its chunks for pass 3, which computes those of an entry's last chunk itself.
 // Bound by the special-function pipe (an ex2 per state, token and pass: 60 of the us below) and the issue slots beside it:
 // tiles of 8 tokens (128 registers, four blocks a multiprocessor; tiles of 16 took 236, two blocks) and then the softplus
 // once instead of in both passes and bfloat16 gates by the reciprocal instruction took the scan of 2,048 tokens of 4,096
@@ -204,7 +204,8 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
     if (e >= meta[META_NUM_ENTRIES]) return;
     const int first = cu_tokens[e], count = cu_tokens[e + 1] - first;
     const int nchunks = PASS == 0 ? 1 : (count + chunk_len - 1) / chunk_len;
-    if (ch >= nchunks) return;
+    if (ch >= nchunks || (PASS == 1 && ch == nchunks - 1)) return;
+    const bool kept = PASS == 3 && ch < nchunks - 1;  // whether pass 1 has left this chunk's step sizes
     const int t0 = first + (PASS == 0 ? 0 : ch * chunk_len), t1 = PASS == 0 ? first + count : min(first + count, t0 + chunk_len);
     const size_t HS = (size_t)inner * N;
     float* slot_state = state + (size_t)slots[e] * slot_stride;
@@ -229,7 +230,7 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
             const bool in = real && tt < nt;
             const size_t t = (size_t)(tb + tt);
             ur[tt] = in ? u[t * u_stride + c] : from_float<T>(0.f);
-            dr[tt] = in ? (PASS == 3 ? steps : dt_raw)[t * inner + c] : 0.f;
+            dr[tt] = in ? (kept ? steps : dt_raw)[t * inner + c] : 0.f;
             if (WRITE_Y) zr[tt] = in ? zg[t * z_stride + c] : from_float<T>(0.f);
         }
         __syncthreads();
@@ -243,7 +244,7 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
 #pragma unroll
         for (int tt = 0; tt < SEL_TT; ++tt) {
             if (tt >= nt) break;
-            const float uv = to_float(ur[tt]), step = PASS == 3 ? dr[tt] : (real ? softplus_f(dr[tt] + dtb) : 0.f);
+            const float uv = to_float(ur[tt]), step = kept ? dr[tt] : (real ? softplus_f(dr[tt] + dtb) : 0.f);
             if (PASS == 1 && real && r == 0) steps[(size_t)(tb + tt) * inner + c] = step;
             const float dx = step * uv;
             const float* Bt = Bs + tt * NP + r * SL;
@@ -275,8 +276,7 @@ selective_scan_kernel(const T* __restrict__ u, long long u_stride, const float* 
             dt_sum += step;
         }
     }
-    // (pass 1 runs an entry's last chunk for its step sizes alone)
-    float* fin = PASS == 1 ? (ch < nchunks - 1 ? chunk_state + HS : nullptr) : ((PASS == 0 || ch == nchunks - 1) ? slot_state : nullptr);
+    float* fin = PASS == 1 ? chunk_state + HS : ((PASS == 0 || ch == nchunks - 1) ? slot_state : nullptr);
     if (fin && real) {
 #pragma unroll
         for (int i = 0; i < NPT; ++i) {
