@@ -177,12 +177,7 @@ extern "C" int gemm_f32(const float* x, const float* w, float* y, int M, int N, 
     // x 8192 422 / 1,036, 8 x 2048 x 8192 275 / 1,023, 1 x 16384 x 2048 74 / 302, 8 x 128256 x 2048 275 / 1,513.
     static const struct { int bm, bn; float alone, more; } tiles[] = {
         {128, 128, 113.f, 91.f}, {64, 128, 77.f, 51.5f}, {64, 64, 47.f, 25.4f}, {32, 64, 36.f, 16.1f}, {16, 128, 34.f, 18.3f}};
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
-        sms = n;
-    }
+    const int sms = multiprocessors();
     int best = 0;
     float least = 0.f;
     for (int i = 0; i < 5; ++i) {

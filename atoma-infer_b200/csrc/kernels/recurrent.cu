@@ -135,11 +135,10 @@ static int launch_head_norm_vec(const float* o, const T* g, long long g_stride, 
 extern "C" int head_norm_gate(const float* o, const void* g, int dtype, long long g_stride, const float* w, float eps, void* out,
                               const int* meta, int T, int heads, int P, cudaStream_t stream) {
     if (T <= 0) return 0;
-    const int esz = dtype == DT_F32 ? 4 : 2;
-    if ((long)T * heads >= 8 * 148 && P % 4 == 0 && P <= 512 && g_stride % 4 == 0 && (((uintptr_t)o | (uintptr_t)w) & 15) == 0 && ((uintptr_t)g | (uintptr_t)out) % (4 * esz) == 0) {
-        if (dtype == DT_F32) return launch_head_norm_vec(o, (const float*)g, g_stride, w, eps, (float*)out, meta, T, heads, P, stream);
+    // (float32 keeps one order of a row's sum, however many rows there are)
+    if (dtype != DT_F32 && (long)T * heads >= 8 * multiprocessors() && P % 4 == 0 && P <= 512 && g_stride % 4 == 0 &&
+        (((uintptr_t)o | (uintptr_t)w) & 15) == 0 && (((uintptr_t)g | (uintptr_t)out) & 7) == 0)
         return launch_head_norm_vec(o, (const __nv_bfloat16*)g, g_stride, w, eps, (__nv_bfloat16*)out, meta, T, heads, P, stream);
-    }
     const dim3 grid(T, (heads + 3) / 4);
     if (dtype == DT_F32)
         return (int)launch_kernel(head_norm_gate_kernel<float>, grid, 128, 0, stream, o, (const float*)g, g_stride, w, eps,

@@ -699,11 +699,9 @@ extern "C" int gated_group_norm(const float* y, const void* z, int dtype, long l
     // four values per access: parts and rows start on multiples of four elements and the buffers on 16 bytes
     const int vec4 = len % 4 == 0 && z_stride % 4 == 0 && (((uintptr_t)y | (uintptr_t)z | (uintptr_t)w | (uintptr_t)out) & 15) == 0;
     // enough parts for a block of eight a multiprocessor; with fewer a block a part is the faster one (4 rows: 28.7 against 29.7 us
-    // for a whole state-space layer)
-    if (vec4 && len <= 1024 && (long)T * parts >= 8 * 148) {
-        if (dtype == DT_F32) return launch_group_norm_warp(y, (const float*)z, z_stride, w, eps, (float*)out, meta, T, n, parts, stream);
+    // for a whole state-space layer).  float32 stays with a block a part: a row's sum must not depend on how many rows there are
+    if (dtype != DT_F32 && vec4 && len <= 1024 && (long)T * parts >= 8 * multiprocessors())
         return launch_group_norm_warp(y, (const __nv_bfloat16*)z, z_stride, w, eps, (__nv_bfloat16*)out, meta, T, n, parts, stream);
-    }
     if (dtype == DT_F32)
         return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, gated_group_norm_kernel<float>, dim3(T, parts), threads, 0, stream, y,
                                       (const float*)z, z_stride, w, eps, (float*)out, meta, n, parts, vec4);

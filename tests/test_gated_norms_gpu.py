@@ -102,3 +102,25 @@ def test_activation_behind_the_convolution(rts, dtype):
     out = torch.empty(T, C, dtype=rt.dtype, device=rt.device)
     rt.ops.causal_conv_act(u.to(rt.device), w.to(rt.device), None, torch.zeros(1, 1, C, device=rt.device), ctx, out)
     same(out, silu(u), REL[dtype])
+
+
+@pytest.mark.parametrize("which", ["parts", "heads", "weights"])
+def test_a_float32_row_has_one_order_of_summation(rts, which):
+    """Rows alone and among many more (bfloat16 takes other kernels from about a thousand rows on): the same bits."""
+    rt, T, parts, P = rts["float32"], 700, 4, 256
+    g = torch.Generator().manual_seed(7)
+    y, z, w = (torch.randn(*shape, generator=g).to(rt.device) for shape in ((T, parts * P), (T, parts * P + 8), (parts * P,)))
+
+    def run(n):
+        out, meta, gate = torch.empty(n, parts * P, device=rt.device), rows(rt, n).meta, z[:n, 8:]
+        if which == "parts":
+            rt.ops.gated_group_norm(y[:n], gate, w, parts, 1e-5, out, meta)
+        elif which == "heads":
+            rt.ops.head_norm_gate(y[:n], gate, w[:P].contiguous(), 1e-5, out, meta, parts)
+        else:
+            rt.ops.head_weight_norm_gate(y[:n], gate, w, 1e-5, out, meta, parts, kind="sigmoid")
+        return out
+
+    many = run(T)
+    for n in (1, 5, 250):
+        assert torch.equal(run(n), many[:n])
