@@ -5,13 +5,15 @@
 #include "common.cuh"
 
 // ----------------------------------------------------------------------------- router
-// Logits of TOK tokens: z[q * stride + e] = w[e] . x_q (float32; a warp takes EXP experts at a time, its lanes run over k, summed in
-// the fixed order of warp_sum, so a logit's sum depends on H alone).  Bound by the shared reads of x and w through the
-// first-level cache: a row of w is read once for TOK tokens, a row of x once for EXP experts.
+// Logits of the TOK tokens from t0 on: z[q * stride + e] = w[e] . h_(t0 + q) (float32; a warp takes EXP experts at a time, its lanes
+// run over k, summed in the fixed order of warp_sum; four columns a lane where h and w start on four elements and H is a
+// multiple of four, which is the same for every token of every step).  Bound by the shared reads of h and w through the
+// first-level cache: a row of w is read once for TOK tokens, a row of h once for EXP experts.
 template <typename T, int TOK, int EXP>
-__device__ __forceinline__ void route_logits(const T* __restrict__ x, const float* __restrict__ w, int H, int E, int tokens, float* z, int stride) {
+__device__ __forceinline__ void route_logits(const T* __restrict__ h, const float* __restrict__ w, int H, int E, int t0, int tokens, float* z, int stride) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    const bool vec = H % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
+    const bool vec = H % 4 == 0 && (uintptr_t)h % (4 * sizeof(T)) == 0 && (uintptr_t)w % 16 == 0;
+    const T* x = h + (size_t)t0 * H;
     for (int e0 = warp * EXP; e0 < E; e0 += nwarps * EXP) {
         float acc[TOK][EXP];
         if (vec) {  // four columns a lane and step
@@ -89,7 +91,7 @@ moe_route_kernel(const T* __restrict__ h, const float* __restrict__ w, int* __re
     pdl_launch_dependents();
     const int t0 = blockIdx.x * TOK, tokens = min(TOK, meta[META_NUM_TOKENS] - t0);
     if (tokens <= 0) return;
-    route_logits<T, TOK, EXP>(h + (size_t)t0 * H, w, H, E, tokens, sh, E);
+    route_logits<T, TOK, EXP>(h, w, H, E, t0, tokens, sh, E);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp >= tokens) return;
@@ -172,7 +174,7 @@ moe_route_sigmoid_kernel(const T* __restrict__ h, const float* __restrict__ w, c
     if (tokens <= 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int stride = 2 * E + (groups > 1 ? 2 * groups : 0);
-    route_logits<T, TOK, TOK == 1 ? 1 : 2>(h + (size_t)t0 * H, w, H, E, tokens, sh, stride);
+    route_logits<T, TOK, TOK == 1 ? 1 : 2>(h, w, H, E, t0, tokens, sh, stride);
     __syncthreads();
     if (warp >= tokens) return;
     const int t = t0 + warp;
