@@ -106,10 +106,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // blockIdx.y counts the query tiles of all requests, a request's late ones first: they see the most keys, and blocks
-    // start in the order of their linear index (x fastest), so that a request's longest blocks are not the last to start.
+    // blockIdx.y (and z behind it) counts the query tiles of all requests, a request's late ones first: they see the most keys, and
+    // blocks start in the order of their linear index (x fastest), so that a request's longest blocks are not the last to start.
     // Every warp finds the tile's request for itself; what it needs of all of them is one round of loads.
-    const int kvh = blockIdx.x, entries = meta[META_NUM_ENTRIES];
+    const int kvh = blockIdx.x, tile = blockIdx.z * gridDim.y + blockIdx.y, entries = meta[META_NUM_ENTRIES];
     const int bt_offset = meta[META_BT_OFFSET + group], bt_stride = meta[META_BT_STRIDE + group];
     int e = -1, qt = 0, row0 = 0, q_len = 0, ctx = 0;
     for (int base = 0, before = 0; base < S; base += 32) {
@@ -121,7 +121,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
             if (lane >= d) upto += v;
         }
         upto += before;
-        const uint32_t past = __ballot_sync(0xffffffffu, upto > (int)blockIdx.y);
+        const uint32_t past = __ballot_sync(0xffffffffu, upto > tile);
         if (past) {
             // (a reduction's result is one value for the warp to the compiler as well, a shuffle's is not: with shuffles the key
             // loop carried its bounds in every thread's registers, 4,096 tokens of 32 heads of 128 over 8 206 us instead of 202)
@@ -130,7 +130,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_kv, const bf16* _
             row0 = __reduce_add_sync(0xffffffffu, mine ? lo : 0);
             q_len = __reduce_add_sync(0xffffffffu, mine ? hi - lo : 0);
             ctx = __reduce_add_sync(0xffffffffu, mine ? cx : 0);
-            qt = __reduce_add_sync(0xffffffffu, mine ? upto - 1 - (int)blockIdx.y : 0);
+            qt = __reduce_add_sync(0xffffffffu, mine ? upto - 1 - tile : 0);
             break;
         }
         before = __shfl_sync(0xffffffffu, upto, 31);
@@ -457,7 +457,10 @@ int table_slice(int max_context, int page_size, int tpt, int window, int chunk) 
 // Blocks enough for S requests of T tokens together: n tokens are at most (n + tpt - 1) / tpt tiles.  (A grid of the longest
 // request's tiles for every request: 31,000 blocks that left at once for one prompt of 1,988 tokens beside 60 single tokens,
 // 32 heads of 64 over 8 256 us, of 128 280 us; so 60 and 86 us.)
-dim3 query_tiles(int T, int S, int nkv, int tpt) { return dim3(nkv, (T + (long long)S * (tpt - 1)) / tpt); }
+dim3 query_tiles(int T, int S, int nkv, int tpt) {
+    const long long tiles = (T + (long long)S * (tpt - 1)) / tpt, rows = tiles < 65535 ? tiles : 65535;  // (65,535: a grid's most in y)
+    return dim3(nkv, (unsigned)rows, (unsigned)((tiles + rows - 1) / rows));
+}
 }  // namespace
 
 extern "C" int attn_tc_head_dim() { return D; }
@@ -481,7 +484,7 @@ extern "C" int attn_prefill_tc_scores(const void* q, int q_stride, const void* c
                                       int nkv, int page_size, int num_pages, int window, int chunk, int sink,
                                       const float* sink_values, float scale, int max_context, float softcap, const float* slopes,
                                       int* status, cudaStream_t stream) {
-    if (S <= 0 || max_q_len <= 0) return 0;
+    if (T <= 0 || S <= 0 || max_q_len <= 0) return 0;
     if (!attn_prefill_tc_supports(page_size, nq, nkv)) return (int)cudaErrorInvalidValue;
     CUtensorMap map;
     if (!cache_map_groups(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;
@@ -515,7 +518,7 @@ extern "C" int attn_prefill_tc_scores(const void* q, int q_stride, const void* c
 extern "C" int attn_prefill_tc_stats(const void* q, int q_stride, const void* cache, const int* meta, int group, const int* cu_tokens,
                                      const int* ctx_lens, float* lse, int T, int S, int max_q_len, int nq, int nkv, int page_size, int num_pages,
                                      int chunk, float scale, int max_context, int* status, cudaStream_t stream) {
-    if (S <= 0 || max_q_len <= 0) return 0;
+    if (T <= 0 || S <= 0 || max_q_len <= 0) return 0;
     if (!attn_prefill_tc_supports(page_size, nq, nkv) || scale <= 0.f) return (int)cudaErrorInvalidValue;
     CUtensorMap map;
     if (!cache_map_groups(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;

@@ -364,3 +364,25 @@ def test_prefill_tiles_of_many_requests(rts, d, nq, nkv, requests):
     entries = [((i * 37) % 150, sizes[i % 7]) for i in range(requests - 1)] + [(40, 3 * rows + 5)]
     got, want = run_attention(rts["bfloat16"], entries, nq, nkv, d, 16, seed=requests)
     assert worst(got, want) < 2e-2  # values are O(1); bfloat16 P and outputs
+
+
+def test_prefill_of_more_query_tiles_than_a_grid_counts_in_one_dimension(rts):
+    """66,560 tiles of eight tokens (16 query heads over one): requests at both ends of the step as they are by themselves."""
+    rt, nq, d, page, n, requests = rts["bfloat16"], 16, 64, 128, 1024, 520
+    per = n // page
+    g = torch.Generator(device=rt.device).manual_seed(0)
+    cache = torch.randn(1 + requests * per, 2, 1, page, d, generator=g, device=rt.device, dtype=torch.float32).to(rt.dtype)
+    qkv = torch.randn(requests * n, (nq + 2) * d, generator=g, device=rt.device, dtype=rt.dtype)
+    tables = [list(range(1 + r * per, 1 + (r + 1) * per)) for r in range(requests)]
+
+    def run(which):
+        ctx, _ = K.make_context(rt, [(0, n)] * len(which), page, [tables[r] for r in which])
+        rows = torch.cat([qkv[r * n:(r + 1) * n] for r in which]) if len(which) < requests else qkv
+        out = torch.full((ctx.T, nq * d), float("nan"), dtype=rt.dtype, device=rt.device)
+        rt.ops.attention(rows, rows.shape[1], cache, ctx, 0, out, nq, 1, d, page, cache.shape[0], 0, d ** -0.5)
+        rt.ops.check_status()
+        return out
+
+    out = run(list(range(requests)))
+    for r in (0, 1, 511, 512, requests - 1):
+        assert torch.equal(run([r]), out[r * n:(r + 1) * n])
