@@ -241,9 +241,9 @@ causal_conv_save_kernel(const T* __restrict__ u, long long u_stride, float* __re
                         const int* __restrict__ slots, int C, int R) {
     pdl_launch_dependents();
     pdl_wait();
-    const int e = blockIdx.y, c = blockIdx.z * blockDim.x + threadIdx.x;
+    const int e = blockIdx.x, c = blockIdx.z * blockDim.x + threadIdx.x;
     if (e >= meta[META_NUM_ENTRIES] || c >= C) return;
-    const int t = cu_tokens[e + 1] - 1 - (int)blockIdx.x;
+    const int t = cu_tokens[e + 1] - 1 - (int)blockIdx.y;
     if (t < cu_tokens[e]) return;
     state[(size_t)slots[e] * slot_stride + (size_t)(positions[t] % R) * C + c] = to_float(u[(size_t)t * u_stride + c]);
 }
@@ -252,7 +252,7 @@ extern "C" int causal_conv_save(const void* u, int dtype, long long u_stride, fl
                                 const int* meta, const int* positions, const int* cu_tokens, const int* slots, int T, int S, int C,
                                 int taps, cudaStream_t stream) {
     if (T <= 0 || S <= 0 || taps <= 1) return 0;
-    const dim3 grid(taps - 1, S, (C + 255) / 256);
+    const dim3 grid(S, taps - 1, (C + 255) / 256);
     if (dtype == DT_F32)
         return (int)launch_kernel(causal_conv_save_kernel<float>, grid, 256, 0, stream, (const float*)u, u_stride, state,
                                   slot_stride, meta, positions, cu_tokens, slots, C, taps - 1);

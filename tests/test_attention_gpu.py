@@ -386,3 +386,13 @@ def test_prefill_of_more_query_tiles_than_a_grid_counts_in_one_dimension(rts):
     out = run(list(range(requests)))
     for r in (0, 1, 511, 512, requests - 1):
         assert torch.equal(run([r]), out[r * n:(r + 1) * n])
+
+
+def test_convolution_state_of_more_requests_than_a_grid_counts_in_one_dimension(rts):
+    rt, S, C, taps = rts["bfloat16"], 65540, 8, 3
+    ctx, _ = K.make_context(rt, [(3, 2)] * S, 16, [[1]] * S)
+    u = torch.randn(2 * S, C, device=rt.device).to(rt.dtype)
+    state = torch.zeros(S, taps - 1, C, device=rt.device)
+    rt.ops.causal_conv_save(u, state, ctx, taps)
+    want = u.float().view(S, 2, C)
+    assert torch.equal(state[:, 1], want[:, 0]) and torch.equal(state[:, 0], want[:, 1])  # positions 3 and 4, place = position mod 2
