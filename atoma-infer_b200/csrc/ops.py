@@ -724,11 +724,13 @@ class CudaOps:
         SCAN_CHUNK_FROM tokens of the step's longest entry on.  Measured there, one prompt, 64 heads of 128 x 64: 200 tokens 25
         against 90 us, 2,048 tokens 108 against 471.  Shorter ones stay in order: they need no scratch memory, which a
         step of many short entries would otherwise ask for (40 tokens: 19 against 28 us).  Above 256 chunks the other kernel's
-        scratch stops growing and this one's would not.  Returns at least as many chunks as all entries have together, or 0."""
+        scratch stops growing and this one's would not; above 65,535 chunks in all (many short entries beside a long one) a grid
+        does not count them.  Returns at least as many chunks as all entries have together, or 0."""
         longest = ctx.max_tokens_per_entry
         if not self.matrix_scan or not self.SCAN_CHUNK_FROM <= longest <= 256 * self.MATRIX_SCAN_CHUNK:
             return 0
-        return ctx.T // self.MATRIX_SCAN_CHUNK + ctx.S
+        chunks = ctx.T // self.MATRIX_SCAN_CHUNK + ctx.S
+        return chunks if chunks <= 65535 else 0
 
     def ssm_scan(self, xbc, dt, dt_bias, a_log, d_skip, state, ctx, y, *, heads: int, head_dim: int, nstate: int, groups: int):
         """The state-space recurrence of every entry's tokens: rows of ``xbc`` are [x | B | C], ``dt`` a slice of wider

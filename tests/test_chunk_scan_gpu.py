@@ -275,3 +275,26 @@ def test_a_head_that_forgets_everything(rt, monkeypatch, a_log):
 
     for new, old in zip(*both(rt, "space", run, monkeypatch)):
         assert bool(old.isfinite().all()) and err(new, old) < TOL
+
+
+def test_more_chunks_than_a_grid_counts(rt):
+    """One entry of 130 tokens beside 65,499 single ones: the kernel that goes token by token takes them."""
+    P = N = 8
+    entries = [(3, 130)] + [(3, 1)] * 65499
+    T = sum(n for _, n in entries)
+    g = torch.Generator(device=rt.device).manual_seed(5)
+    xbc, dt = (torch.randn(T, n, generator=g, device=rt.device).bfloat16() for n in (P + 2 * N, 1))
+    S0 = torch.randn(len(entries), 1, N, P, generator=g, device=rt.device)
+    one = torch.ones(1, device=rt.device)
+
+    def run(first, rows, count):
+        ctx, _ = K.make_context(rt, entries[first:first + count], 16, [[1] * 9] * count)
+        state, y = S0[first:first + count].clone(), torch.full((ctx.T, P), float("nan"), device=rt.device)
+        rt.ops.ssm_scan(xbc[rows:rows + ctx.T], dt[rows:rows + ctx.T], one - 3, one, one, state, ctx, y, heads=1, head_dim=P, nstate=N, groups=1)
+        return y, state
+
+    y, state = run(0, 0, len(entries))
+    for first, rows, count in ((0, 0, 1), (1, 130, 200), (len(entries) - 70, T - 70, 70)):
+        some_y, some_state = run(first, rows, count)
+        n = some_y.shape[0]
+        assert err(some_y, y[rows:rows + n].double().cpu()) < TOL and err(some_state, state[first:first + count].double().cpu()) < TOL
