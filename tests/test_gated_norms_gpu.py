@@ -124,3 +124,30 @@ def test_a_float32_row_has_one_order_of_summation(rts, which):
     many = run(T)
     for n in (1, 5, 250):
         assert torch.equal(run(n), many[:n])
+
+
+@pytest.mark.parametrize("pad", [8, 3])  # gates on and off the boundaries of vector accesses
+@pytest.mark.parametrize("length", [4, 124, 128, 132, 256, 260, 512, 516, 1020, 1024, 1028])
+@pytest.mark.parametrize("which", ["parts", "heads", "weights"])
+def test_norms_of_many_rows(rts, which, length, pad):
+    """Rows enough for the kernels in which a warp takes a part or a head, lengths that fill its lanes' loads or leave lanes empty."""
+    rt, n = rts["bfloat16"], 3
+    T = 8 * torch.cuda.get_device_properties(0).multi_processor_count // n + 17
+    g = torch.Generator().manual_seed(length)
+    y, w = torch.randn(T, n * length, generator=g), torch.rand(n * length, generator=g) + 0.5
+    z = torch.randn(T, n * length + pad, generator=g).to(rt.dtype)[:, pad:]
+    out, meta, dev = torch.full((T, n * length), float("nan"), dtype=rt.dtype, device=rt.device), rows(rt, T).meta, lambda t: t.to(rt.device)
+    v, gate = y.double().view(T, n, length), silu(z).view(T, n, length)
+    if which == "parts":
+        rt.ops.gated_group_norm(dev(y), dev(z), dev(w), n, 1e-5, out, meta)
+        v = v * gate
+        want = v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5) * w.double().view(n, length)
+    else:
+        v = v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-5) * gate
+        if which == "heads":
+            rt.ops.head_norm_gate(dev(y), dev(z), dev(w[:length].contiguous()), 1e-5, out, meta, n)
+            want = v * w[:length].double()
+        else:
+            rt.ops.head_weight_norm_gate(dev(y), dev(z), dev(w), 1e-5, out, meta, n, kind="silu")
+            want = v * w.double().view(n, length)
+    same(out, want.reshape(T, -1), REL["bfloat16"])
