@@ -258,7 +258,10 @@ moe_sort_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __r
         for (int i0 = from; i0 < to; i0 += 128) {
             int id[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) id[u] = i0 + u * 32 + lane < to ? ids[i0 + u * 32 + lane] : -1;
+            for (int u = 0; u < 4; ++u) {
+                const int x = i0 + u * 32 + lane < to ? ids[i0 + u * 32 + lane] : -1;
+                id[u] = x < E ? x : -1;  // (what names no expert stands in no stretch)
+            }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const unsigned same = __match_any_sync(0xffffffffu, id[u]);

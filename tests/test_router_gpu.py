@@ -74,19 +74,34 @@ def test_a_token_is_routed_alike_wherever_it_stands(rts, dtype, kind, H):
         assert torch.equal(some[0], ids[first:first + n]) and torch.equal(some[1], wts[first:first + n])
 
 
+def sort(rt, ids, T, top, E):
+    dev = ids.to(rt.device)
+    offsets = torch.full((E + 1,), -1, dtype=torch.int32, device=rt.device)
+    order, place = (torch.full((T * top,), -1, dtype=torch.int32, device=rt.device) for _ in range(2))
+    rt.ops._check(rt.ops._mixers().moe_sort(O._p(dev), O._p(offsets), O._p(order), O._p(place), O._p(meta(rt, T)), top, E, rt.ops._stream()), "moe_sort")
+    return offsets.cpu().long(), order.cpu().long(), place.cpu().long()
+
+
 @pytest.mark.parametrize("top", [1, 3])
 @pytest.mark.parametrize("T", [1, 31, 1025, 3001, 4097, 9001])
 @pytest.mark.parametrize("E", [1, 16, 37, 400, 1000])
 @pytest.mark.parametrize("skewed", [False, True])
 def test_sort_by_expert(rts, top, T, E, skewed):
-    rt, n = rts["bfloat16"], T * top
+    n = T * top
     x = torch.rand(n, generator=torch.Generator().manual_seed(T + E))
     ids = ((x ** 6 if skewed else x) * E).int().clamp_(max=E - 1)
-    dev = ids.to(rt.device)
-    offsets = torch.full((E + 1,), -1, dtype=torch.int32, device=rt.device)
-    order, place = (torch.full((n,), -1, dtype=torch.int32, device=rt.device) for _ in range(2))
-    rt.ops._check(rt.ops._mixers().moe_sort(O._p(dev), O._p(offsets), O._p(order), O._p(place), O._p(meta(rt, T)), top, E, rt.ops._stream()), "moe_sort")
+    offsets, order, place = sort(rts["bfloat16"], ids, T, top, E)
     want = torch.argsort(ids.long(), stable=True)
-    assert torch.equal(order.cpu().long(), want)
-    assert torch.equal(offsets.cpu().long(), torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(ids.long(), minlength=E).cumsum(0)]))
-    assert torch.equal(place.cpu().long()[want], torch.arange(n))
+    assert torch.equal(order, want) and torch.equal(place[want], torch.arange(n))
+    assert torch.equal(offsets, torch.cat([torch.zeros(1, dtype=torch.int64), torch.bincount(ids.long(), minlength=E).cumsum(0)]))
+
+
+def test_sort_leaves_out_what_names_no_expert(rts):
+    T, E = 3001, 37
+    ids = torch.randint(-2, E + 4, (T,), generator=torch.Generator().manual_seed(0), dtype=torch.int32)
+    ids[::500] = 1 << 30
+    offsets, order, place = sort(rts["bfloat16"], ids, T, 1, E)
+    real = ((ids >= 0) & (ids < E)).nonzero()[:, 0]
+    want = real[torch.argsort(ids[real].long(), stable=True)]
+    assert torch.equal(order[:len(real)], want) and bool((order[len(real):] == -1).all()) and int(offsets[-1]) == len(real)
+    assert torch.equal(place[want], torch.arange(len(real))) and int((place >= 0).sum()) == len(real)
