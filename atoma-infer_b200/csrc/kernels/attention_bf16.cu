@@ -461,8 +461,8 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_kv, int use_tma, bf16
 }
 
 // ----------------------------------------------------------------------------- decode, large batches
-// Decode attention for batches with many (request, head group) pairs: all key tiles dealt out evenly over as many
-// blocks as the GPU holds (flat_attention in attention_tiles.cuh says how).
+// Decode attention for batches with many (request, head group) pairs: all key tiles, and a pair's fixed cost as
+// tiles of its own, dealt out over as many blocks as the GPU holds (flat_attention in attention_tiles.cuh says how).
 namespace {
 constexpr size_t FLAT_SMEM_FIXED = DEC_MAIN_BYTES;  // then (requests + 1) ints: tiles before each request
 }

@@ -25,7 +25,7 @@
 // before its first scores was a chain of four round trips to memory, some 4 us of a block: the request is found from one
 // round of loads, and K sets out beside the loads of Q and of the block table; with a mask of two comparisons a score
 // 188 and 2,215 us, prompts of 1,391, 402 and 255 tokens 63 -> 53 us, at heads of 64 44 -> 38.)  Two blocks fit a multiprocessor for
-// head size 64; the softmax warps then take registers that the other two warps give up.
+// head size 64; the softmax warps then take registers that the copy and MMA warps give up.
 // A portion of a prompt that starts inside a cached context attends to all of it.
 //
 // Head size 256 serves attention whose cache holds the same vector on the key and the value plane (latent attention): a tile of
@@ -520,6 +520,9 @@ extern "C" int attn_prefill_tc_stats(const void* q, int q_stride, const void* ca
                                      int chunk, float scale, int max_context, int* status, cudaStream_t stream) {
     if (T <= 0 || S <= 0 || max_q_len <= 0) return 0;
     if (!attn_prefill_tc_supports(page_size, nq, nkv) || scale <= 0.f) return (int)cudaErrorInvalidValue;
+    if constexpr (ONE_PLANE) {
+        return (int)cudaErrorInvalidValue;  // (nothing that mixes heads has one plane: no kernel is built for it)
+    } else {
     CUtensorMap map;
     if (!cache_map_groups(&map, cache, num_pages, nkv, page_size)) return (int)cudaErrorNotSupported;
     CacheLayout L{nkv, page_size, D};
@@ -537,4 +540,5 @@ extern "C" int attn_prefill_tc_stats(const void* q, int q_stride, const void* ca
         map, (const bf16*)q, q_stride, L, meta, group, cu_tokens, ctx_lens, S, nullptr, nq, 0, chunk, 0, nullptr, scale * LOG2E, num_pages,
         bt_cap, 0.f, nullptr, status, lse);
     LAUNCH_RETURN();
+    }
 }

@@ -333,11 +333,12 @@ __device__ __forceinline__ void decode_segment_finish(float* mbuf, int tid, cons
 
 }  // namespace
 
-// ----------------------------------------------------------------------------- decode, key tiles dealt out evenly
+// ----------------------------------------------------------------------------- decode, key tiles dealt out over the chip
 // The same attention for batches with more (request, head group) pairs than about half the blocks the GPU
 // holds: there, one block per pair (or per fixed split of a pair) leaves a last partial wave of blocks that
 // run almost alone.  Here the grid is as many blocks as the GPU holds at once and the 32-key tiles of all
-// pairs, in (request, head group, key) order, are dealt out evenly: a block takes a contiguous run of
+// pairs, in (request, head group, key) order, every pair with FLAT_PAIR_COST tiles ahead of its own that stand for
+// its fixed cost, are dealt out evenly: a block takes a contiguous run of
 // tiles, which may end one pair and begin the next (a run is cut into segments at pair boundaries).  A
 // pair that one block covers alone is written directly; otherwise every segment's partial result goes to
 // scratch slot (block index + pair index), a pair's slots being consecutive, and the last block to arrive

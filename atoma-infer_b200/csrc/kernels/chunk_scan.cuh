@@ -2,7 +2,7 @@
 // S_t = a_t S_(t-1) + b_t k_t v_t^T and o_t = S_t^T q_t, with bfloat16 q, k and v.  Over a chunk of CHUNK tokens this is
 //     o_t = exp(c_t) q_t^T S_in + sum over s <= t of (q_t . k_s) exp(c_t - c_s) b_s v_s,     c_t = log a_1 + .. + log a_t,
 //     S_out = exp(c_end) S_in + sum over s of k_s (exp(c_end - c_s) b_s v_s)^T,
-// matrix products instead of a chain over the tokens.  Three launches: chunk_states_kernel leaves every chunk's own share of
+// matrix products instead of a chain over the tokens (the chunked form of state-space duality, Dao and Gu 2024).  Three launches: chunk_states_kernel leaves every chunk's own share of
 // S_out (from S_in = 0), chunk_chain_kernel turns the shares into the chunks' S_in in order and updates the slot, and
 // chunk_outputs_kernel writes o.
 //

@@ -524,8 +524,7 @@ __device__ __forceinline__ void pv_streamed(float (&o)[DTILES][4], const float (
     }
 }
 
-// The key tiles of all requests and head groups are dealt out evenly over the blocks as in flat_attention; a block's
-// run is cut into segments at (request, head group) boundaries, a segment's tiles are packed two to a stage, and an
+// A block walks segments, runs of key tiles of one (request, head group); a segment's tiles are packed two to a stage, and an
 // arithmetic warp takes whole stages (stage i of the segment goes to warp i mod ST_WARPS).
 // Which keys a block walks.  With at most as many (request, head group) pairs as blocks, every pair is cut into
 // `split` = blocks / pairs parts of equal tile counts and block c takes part c % split of pair c / split: one segment a

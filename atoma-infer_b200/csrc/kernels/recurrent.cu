@@ -7,7 +7,8 @@
 // request's tokens run in order from its state slot (pass 0), or, for long portions, cut into chunks of time that run
 // side by side: pass 1 runs every chunk but the last from a zero state and leaves its end state and what its decays
 // amount to, a small kernel chains the chunks' start states in order, pass 3 runs every chunk again from its start
-// state and writes the outputs, the last chunk the slot.  Every sum runs in an order that depends on the sizes only.
+// state and writes the outputs, the last chunk the slot.  Every sum runs in an order that depends on the sizes only; the norm of
+// bfloat16 rows takes one of two orders by the number of rows.
 #include "matrix_scan.cuh"
 #include "row_scan.cuh"
 

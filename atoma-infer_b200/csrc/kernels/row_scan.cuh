@@ -10,7 +10,8 @@
 // row_states_kernel every chunk's own share of S_out; row_chain_kernel the chunks' S_in in order, and the slot;
 // row_outputs_kernel o.
 //
-// W: between two sub-blocks of 16 tokens both factors are taken relative to the earlier one's last token, q exp(c_t - c_e) and
+// W (the two-level chunking of gated linear attention, Yang et al. 2023, with a third level below): between two sub-blocks of 16
+// tokens both factors are taken relative to the earlier one's last token, q exp(c_t - c_e) and
 // k exp(c_e - c_s), so no exponent is above zero; the half of a diagonal sub-block below its corner likewise with 8 tokens;
 // the triangles of 8 that remain are summed over the channels directly.
 //

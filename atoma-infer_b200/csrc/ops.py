@@ -79,7 +79,7 @@ class CudaOps:
         self.tc_attention = True    # tcgen05 prefill attention where the geometry allows
         self.decode_cluster = True  # split merge of the decode attention inside a cluster
         self.tc_gemm = True         # gate/up + SwiGLU of long prompts on tcgen05
-        # large decode batches: key tiles dealt out evenly over as many blocks as the GPU holds ("0": never;
+        # large decode batches: key tiles dealt out over as many blocks as the GPU holds ("0": never;
         # a number above 1: always, with that many blocks, for experiments and tests)
         flat = os.environ.get("ATOMA_INFER_DECODE_FLAT", "1")
         self.decode_flat = flat != "0"
