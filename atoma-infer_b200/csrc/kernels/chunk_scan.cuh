@@ -16,8 +16,6 @@
 //
 // Values that are not finite, and columns whose results are not, are taken token by token (chunk_in_order).
 //
-// Values that are not finite, and columns whose results are not, are taken token by token (chunk_in_order).
-//
 // What bounds it: the phases of a block (loads, logs, conversion, products) follow one another and two blocks share a
 // multiprocessor; the tensor pipe is 33 to 37 % busy, issue slots 40 %.  The state shares (N * P floats a chunk and head,
 // written, chained and read) stay in L2.  CHUNK = 128: 64 would double the shares' traffic for a tenth fewer products, 256
