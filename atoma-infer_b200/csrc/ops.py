@@ -716,6 +716,7 @@ class CudaOps:
     SCAN_CHUNK_FROM = 128  # ... which happens from this many tokens of the step's longest entry on
 
     MATRIX_SCAN_CHUNK = 128
+    MATRIX_SCAN_TOKENS = 8  # tokens an entry of the step, on average, from which its prompts run as matrix products
     matrix_scan = True  # (a test lever)
 
     def _matrix_scan_chunks(self, ctx) -> int:
@@ -725,9 +726,15 @@ class CudaOps:
         against 90 us, 2,048 tokens 108 against 471.  Shorter ones stay in order: they need no scratch memory, which a
         step of many short entries would otherwise ask for (40 tokens: 19 against 28 us).  Above 256 chunks the other kernel's
         scratch stops growing and this one's would not; above 65,535 chunks in all (many short entries beside a long one) a grid
-        does not count them.  Returns at least as many chunks as all entries have together, or 0."""
+        does not count them.  An entry of one token costs these kernels a whole chunk, some 4.5 us in a crowd against 2.5 in order, so a
+        step needs MATRIX_SCAN_TOKENS tokens an entry: beside 60 single tokens a prompt of 128 takes 286 against 239 us, of 300
+        292 against 280, of 512 299 against 333, of 1,988 366 against 791; beside 250 one of 128 takes 1,222 against 669, beside 16
+        80 against 118; 60 portions of 20 tokens beside one of 200 take 312 against 386.
+        Returns at least as many chunks as all entries have together, or 0."""
         longest = ctx.max_tokens_per_entry
         if not self.matrix_scan or not self.SCAN_CHUNK_FROM <= longest <= 256 * self.MATRIX_SCAN_CHUNK:
+            return 0
+        if ctx.T < self.MATRIX_SCAN_TOKENS * ctx.S:
             return 0
         chunks = ctx.T // self.MATRIX_SCAN_CHUNK + ctx.S
         return chunks if chunks <= 65535 else 0
