@@ -716,10 +716,12 @@ class CudaOps:
     SCAN_CHUNK_FROM = 128  # ... which happens from this many tokens of the step's longest entry on
 
     MATRIX_SCAN_CHUNK = 128
-    MATRIX_SCAN_TOKENS = 8  # tokens an entry of the step, on average, from which its prompts run as matrix products
+    # tokens an entry of the step, on average, from which its prompts run as matrix products: state space, and the other scans
+    MATRIX_SCAN_TOKENS = 8
+    MATRIX_SCAN_TOKENS_OTHER = 2
     matrix_scan = True  # (a test lever)
 
-    def _matrix_scan_chunks(self, ctx) -> int:
+    def _matrix_scan_chunks(self, ctx, tokens: int) -> int:
         """bfloat16 prompts whose state decays by one number per head and token run the recurrence as matrix products over
         chunks of 128 tokens (kernels/chunk_scan.cuh) where the other kernel would cut it into chunks of time too: from
         SCAN_CHUNK_FROM tokens of the step's longest entry on.  Measured there, one prompt, 64 heads of 128 x 64: 200 tokens 25
@@ -727,14 +729,15 @@ class CudaOps:
         step of many short entries would otherwise ask for (40 tokens: 19 against 28 us).  Above 256 chunks the other kernel's
         scratch stops growing and this one's would not; above 65,535 chunks in all (many short entries beside a long one) a grid
         does not count them.  An entry of one token costs these kernels a whole chunk, some 4.5 us in a crowd against 2.5 in order, so a
-        step needs MATRIX_SCAN_TOKENS tokens an entry: beside 60 single tokens a prompt of 128 takes 286 against 239 us, of 300
+        step needs ``tokens`` tokens an entry, eight for the state space: beside 60 single tokens a prompt of 128 takes 286 against 239 us, of 300
         292 against 280, of 512 299 against 333, of 1,988 366 against 791; beside 250 one of 128 takes 1,222 against 669, beside 16
-        80 against 118; 60 portions of 20 tokens beside one of 200 take 312 against 386.
+        80 against 118; 60 portions of 20 tokens beside one of 200 take 312 against 386.  Two for the matrix memory, whose scan in order is slower
+        (12 heads of 128 x 256): 300 tokens beside 60 single ones 254 against 356, 128 beside 250 1,043 against 884.
         Returns at least as many chunks as all entries have together, or 0."""
         longest = ctx.max_tokens_per_entry
         if not self.matrix_scan or not self.SCAN_CHUNK_FROM <= longest <= 256 * self.MATRIX_SCAN_CHUNK:
             return 0
-        if ctx.T < self.MATRIX_SCAN_TOKENS * ctx.S:
+        if ctx.T < tokens * ctx.S:
             return 0
         chunks = ctx.T // self.MATRIX_SCAN_CHUNK + ctx.S
         return chunks if chunks <= 65535 else 0
@@ -747,7 +750,7 @@ class CudaOps:
             raise KernelError("a recurrence state is float32 [slots, heads, rows, columns] with contiguous slots")
         dp, ds = self._rows(dt, "ssm_scan")
         lib = self._mixers()
-        chunks = self._matrix_scan_chunks(ctx) if xbc.dtype == torch.bfloat16 else 0
+        chunks = self._matrix_scan_chunks(ctx, self.MATRIX_SCAN_TOKENS) if xbc.dtype == torch.bfloat16 else 0
         if chunks and lib.ssm_chunk_scan_takes(_p(xbc), xbc.stride(0), _p(y), heads, head_dim, nstate, groups):
             scratch = torch.empty(lib.ssm_chunk_scan_scratch_floats(heads, head_dim, nstate, chunks), dtype=torch.float32, device=y.device)
             self._check(lib.ssm_chunk_scan(_p(xbc), xbc.stride(0), dp, ds, _p(dt_bias), _p(a_log), _p(d_skip), _p(state),
@@ -927,9 +930,11 @@ class CudaOps:
         """bfloat16 prompts whose state decays by a number per row run as matrix products over chunks of 64 tokens
         (kernels/row_scan.cuh) where the other kernel would cut them into chunks of time.  Its scratch holds the chunks' operands
         beside their states, about twice the other's; where that is more than the other kernel would take and more than
-        ROW_SCAN_SCRATCH, the heads run in rounds, and where not one head fits, the other kernel runs.  Returns (at least the
+        ROW_SCAN_SCRATCH, the heads run in rounds, and where not one head fits, the other kernel runs.  So it does for fewer than two
+        tokens an entry: every entry takes a chunk of its own, and 128 tokens beside 250 single ones took 662 us here against 603 (8
+        heads of 128 x 256; a bonus, 32 of 64 x 64: 553 against 356), beside 60 169 against 232 (130 against 165).  Returns (at least the
         chunks of all entries together, scratch), or None."""
-        if not chunk or not self.matrix_scan or q.dtype != torch.bfloat16:
+        if not chunk or not self.matrix_scan or q.dtype != torch.bfloat16 or ctx.T < self.MATRIX_SCAN_TOKENS_OTHER * ctx.S:
             return None
         most = ctx.T // self.ROW_SCAN_CHUNK + ctx.S
         head = getattr(lib, name + "_row_scan_head_floats")(*rows, _p(o), dim, vdim, most)
@@ -1273,14 +1278,14 @@ class CudaOps:
             raise KernelError("memory_scan: two gates per head")
         (qp, qs), (kp, ks), (vp, vs) = (self._rows(t, "memory_scan") for t in (q, k, v))
         gates = torch.empty((ctx.T, heads, 2), dtype=torch.float32, device=o.device)
-        chunked = bool(q.dtype == torch.bfloat16 and self._matrix_scan_chunks(ctx)
+        chunked = bool(q.dtype == torch.bfloat16 and self._matrix_scan_chunks(ctx, self.MATRIX_SCAN_TOKENS_OTHER)
                        and lib.memory_chunk_scan_takes(qp, qs, kp, ks, vp, vs, _p(o), dim, vdim))
         log_a = torch.empty((ctx.T, heads), dtype=torch.float32, device=o.device) if chunked else None
         self._check(lib.memory_gates(_p(logits), _p(bias), ctypes.c_float(cap), _p(m_state), slot_stride, _p(gates), _p(floor), _p(log_a),
                                      _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, heads, ctx.max_tokens_per_entry,
                                      self._stream()), "memory_gates")
         if chunked:
-            chunks = self._matrix_scan_chunks(ctx)
+            chunks = self._matrix_scan_chunks(ctx, self.MATRIX_SCAN_TOKENS_OTHER)
             scratch = torch.empty(lib.memory_chunk_scan_scratch_floats(heads, dim, vdim, chunks), dtype=torch.float32, device=o.device)
             self._check(lib.memory_chunk_scan(qp, qs, kp, ks, vp, vs, _p(gates), _p(log_a), ctypes.c_float(q_scale), _p(state), _p(n_state),
                                               slot_stride, _p(o), _p(nq), _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, heads,
