@@ -26,7 +26,7 @@ SKINNY_MAX_ROWS = 16  # bfloat16 linears with at most this many rows stream the 
 
 CORE_SOURCES = ["kernels/core.cu", "kernels/gemm_f32.cu", "kernels/layer_ops.cu", "kernels/linear_bf16.cu", "kernels/linear_stream.cu", "kernels/sampling.cu"]
 ATTENTION_SOURCES = ["kernels/attention_bf16.cu"]
-GEMM_SOURCES = ["kernels/gemm_tcgen05.cu"]
+GEMM_SOURCES = ["kernels/gemm_tcgen05.cu", "kernels/gemm_f32_tcgen05.cu"]
 ATTENTION_TC_SOURCES = ["kernels/attention_tcgen05.cu"]
 DECODE_STACK_SOURCES = ["kernels/decode_stack.cu"]
 ATTENTION_TALK_SOURCES = ["kernels/attention_talk.cu"]  # weights mixed across heads; one library per head size
@@ -78,6 +78,7 @@ class CudaOps:
         # levers for the kernel tests (each kernel is compared with the one it stands in for)
         self.tc_attention = True    # tcgen05 prefill attention where the geometry allows
         self.decode_cluster = True  # split merge of the decode attention inside a cluster
+        self.tc_f32 = True          # float32 products of large weights on tcgen05
         self.tc_gemm = True         # gate/up + SwiGLU of long prompts on tcgen05
         # large decode batches: key tiles dealt out over as many blocks as the GPU holds ("0": never;
         # a number above 1: always, with that many blocks, for experiments and tests)
@@ -253,7 +254,13 @@ class CudaOps:
         n_out = N // 2 if silu_mul else N
         if x.dtype == torch.float32:
             y = torch.empty((M, N), dtype=torch.float32, device=x.device)
-            self._check(self.lib.gemm_f32(_p(x), _p(w), _p(y), M, N, K, self._stream()), "gemm_f32")
+            if self._f32_on_tcgen05(x, w, y):
+                split = torch.empty((2, M, K), dtype=torch.float32, device=x.device)
+                self._check(self._gemm_library().gemm_f32_tcgen05(_p(x), _p(w), _p(y), _p(split), M, N, K, _p(self.status), self._stream()),
+                            "gemm_f32_tcgen05")
+                self.launches += 1  # (the split of x)
+            else:
+                self._check(self.lib.gemm_f32(_p(x), _p(w), _p(y), M, N, K, self._stream()), "gemm_f32")
             if silu_mul:
                 out = torch.empty((M, n_out), dtype=torch.float32, device=x.device)
                 self.silu_mul(y, out, meta, M, n_out)
@@ -346,18 +353,31 @@ class CudaOps:
         stacked and the result has RB/2 columns.  ``ksplit``: blocks of a cluster that share a tile's K.
         ``persistent`` (untransposed, unsplit): one block per multiprocessor walks the tiles and stores a tile
         while the tensor core computes the next."""
-        if self._gemm_lib is None:
-            self._gemm_lib = build.load_library("gemm_tcgen05", GEMM_SOURCES, cuda=True)
         out_dtype = out_dtype or a.dtype
         ra, K = a.shape
         rb = b.shape[0] // 2 if silu_mul else b.shape[0]
         shape = (rb, ra) if transpose else (ra, rb)
         c = out if out is not None else torch.empty(shape, dtype=out_dtype, device=a.device)
-        self._check(self._gemm_lib.gemm_tcgen05(_p(a), _p(b), _p(c), ra, rb, K, shape[1], _code(c), int(silu_mul),
+        self._check(self._gemm_library().gemm_tcgen05(_p(a), _p(b), _p(c), ra, rb, K, shape[1], _code(c), int(silu_mul),
                                                 int(transpose), bn, ksplit, int(persistent and not transpose and ksplit == 1),
                                                 _p(self.status), self._stream()),
                     "gemm_tcgen05")
         return c
+
+    def _gemm_library(self):
+        if self._gemm_lib is None:
+            self._gemm_lib = build.load_library("gemm_tcgen05", GEMM_SOURCES, cuda=True)
+        return self._gemm_lib
+
+    def _f32_on_tcgen05(self, x, w, y) -> bool:
+        """Whether a float32 product runs on the tensor cores as three TF32 products with short sums (kernels/gemm_f32_tcgen05.cu;
+        closer to float64 than one float32 accumulator).  By the weight alone, so that a row's bits do not depend on the rows
+        beside it.  Measured against the plain kernel, us for 1 / 8 / 333 rows: 1024 x 1024 34 / 34 / 36 for 40 / 40 / 52, 2048 x 2048
+        34 / 34 / 40 for 75 / 75 / 113, 512 x 2048 30 / 30 / 36 for 75 / 75 / 73; 2048 x 512 - / 26 / 28 for - / 24 / 34, hence K from
+        1,024 on; 8 rows of 128256 x 2048 (an output head, which has few rows) 292 for 281, hence N up to 65,536."""
+        N, K = w.shape
+        return (self.tc_f32 and K % 4 == 0 and K >= 1024 and N * K >= 1 << 20 and N <= 65536 and x.is_contiguous() and w.is_contiguous()
+                and (x.data_ptr() | w.data_ptr() | y.data_ptr()) % 16 == 0)
 
     def silu_mul(self, gu, out, meta, T: int, inter: int):
         self._check(self.lib.silu_mul(_p(gu), _p(out), _code(gu), _p(meta), T, inter, self._stream()), "silu_mul")
