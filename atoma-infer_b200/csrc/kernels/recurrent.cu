@@ -11,6 +11,7 @@
 // bfloat16 rows takes one of two orders by the number of rows.
 #include "matrix_scan.cuh"
 #include "row_scan.cuh"
+#include "selective_prompt.cuh"
 
 int g_use_pdl = 1;
 extern "C" void kernels_set_pdl(int mode) { g_use_pdl = mode; }
@@ -162,16 +163,7 @@ extern "C" int head_norm_gate(const float* o, const void* g, int dtype, long lon
 // once instead of in both passes and bfloat16 gates by the reciprocal instruction took the scan of 2,048 tokens of 4,096
 // channels x 16 states from 175 over 156 to 147 us, of 8,192 channels from 324 over 292 to 272, and 200 tokens of 4,096
 // from 53 over 49 to 44.  Loading the next tile ahead (4 to 8 tokens, B and C of 64 at a time) gave 147 to 163 us.
-#define LOG2E_F 1.4426950408889634f
 #define SEL_TT 8
-
-// 2^x for x <= 0 by one approximate PTX instruction (a result below the smallest normal number is zero, which a decay of
-// that size is for every state that float32 holds).
-__device__ __forceinline__ float ex2_nonpositive(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 
 template <typename T, int NPT, int PASS>
 __global__ void __launch_bounds__(128, NPT <= 16 ? 4 : 1)
@@ -313,6 +305,24 @@ selective_chunk_states_kernel(const float* __restrict__ state, long long slot_st
 
 extern "C" size_t selective_scan_scratch_floats(int T, int S, int inner, int N, int max_chunks) {
     return (size_t)S * max_chunks * ((size_t)inner * N + inner) + (size_t)T * inner;
+}
+
+// The same in one pass, in order, for prompts (selective_prompt.cuh), and whether it takes these inputs.
+extern "C" int selective_scan_prompt_takes(const void* u, long long u_stride, const float* dt_raw, const void* bc, long long bc_stride,
+                                           const void* zg, long long z_stride, int dtype, const void* out, int inner, int N) {
+    return selective_prompt_takes(u, u_stride, dt_raw, bc, bc_stride, zg, z_stride, dtype, out, inner, N);
+}
+extern "C" int selective_scan_prompt(const void* u, long long u_stride, const float* dt_raw, const float* dt_bias, const void* bc,
+                                     long long bc_stride, const void* zg, long long z_stride, int dtype, const float* a_log,
+                                     const float* d_skip, float* state, long long slot_stride, void* out, const int* meta,
+                                     const int* cu_tokens, const int* slots, int S, int inner, int N, cudaStream_t stream) {
+    if (S <= 0) return 0;
+    if (!selective_prompt_takes(u, u_stride, dt_raw, bc, bc_stride, zg, z_stride, dtype, out, inner, N)) return (int)cudaErrorInvalidValue;
+    if (dtype == DT_F32)
+        return selective_prompt<float>(u, u_stride, dt_raw, dt_bias, bc, bc_stride, zg, z_stride, a_log, d_skip, state, slot_stride, out, meta,
+                                       cu_tokens, slots, S, inner, N, stream);
+    return selective_prompt<__nv_bfloat16>(u, u_stride, dt_raw, dt_bias, bc, bc_stride, zg, z_stride, a_log, d_skip, state, slot_stride, out,
+                                           meta, cu_tokens, slots, S, inner, N, stream);
 }
 
 extern "C" int selective_scan(const void* u, long long u_stride, const float* dt_raw, const float* dt_bias, const void* bc,

@@ -78,6 +78,7 @@ class CudaOps:
         # levers for the kernel tests (each kernel is compared with the one it stands in for)
         self.tc_attention = True    # tcgen05 prefill attention where the geometry allows
         self.decode_cluster = True  # split merge of the decode attention inside a cluster
+        self.selective_prompt = None  # the selective scan of prompts in one pass: None: by the rule, else always or never
         self.tc_f32 = True          # float32 products of large weights on tcgen05
         self.tc_gemm = True         # gate/up + SwiGLU of long prompts on tcgen05
         # large decode batches: key tiles dealt out over as many blocks as the GPU holds ("0": never;
@@ -1025,6 +1026,12 @@ class CudaOps:
         if dt_raw.dtype != torch.float32 or not dt_raw.is_contiguous() or not out.is_contiguous() or out.dtype != u.dtype:
             raise KernelError("selective_scan: step sizes are contiguous float32, the output has the inputs' type")
         (up, us), (bp, bs), (zp, zs) = (self._rows(t, "selective_scan") for t in (u, bc, zg))
+        rows = (up, us, _p(dt_raw))
+        if self._selective_in_order(ctx, inner) and lib.selective_scan_prompt_takes(*rows, bp, bs, zp, zs, _code(u), _p(out), inner, nstate):
+            self._check(lib.selective_scan_prompt(*rows, _p(dt_bias), bp, bs, zp, zs, _code(u), _p(a_log), _p(d_skip), _p(state), slot_stride,
+                                                  _p(out), _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, inner, nstate,
+                                                  self._stream()), "selective_scan")
+            return
         chunk, chunks = self._scan_chunks(ctx)
         scratch = (torch.empty(lib.selective_scan_scratch_floats(ctx.T, ctx.S, inner, nstate, chunks), dtype=torch.float32, device=out.device)
                    if chunk else None)
@@ -1033,6 +1040,23 @@ class CudaOps:
                                        nstate, chunk, chunks, _p(scratch), self._stream()), "selective_scan")
         if chunk:
             self.launches += 2
+
+    def _selective_in_order(self, ctx, inner: int) -> bool:
+        """Whether a step's selective scan runs in one pass (kernels/selective_prompt.cuh): where its estimated time is the shorter
+        one.  It takes 0.04 us a token of the longest entry, or, with more blocks of 32 channels than multiprocessors, their share
+        of all tokens and 2.2 us an entry; the scan cut in chunks of time 48 us and two passes over everything, the one in order
+        (steps of short entries) 0.4 us a token of the longest.  Measured, us, one pass / the other, 16 states, channels x tokens:
+        4096 x 2048 86 / 163, 8192 x 2048 165 / 296, 2048 x 2048 85 / 103, 1024 x 3000 121 / 91, 1024 x 1000 45 / 58, 4096 x 64 10 / 32,
+        4096 x 16 8 / 15; 4096 channels, 128 tokens beside 20 single ones 49 / 81, 8 x 16 29 / 16, 8 x 64 35 / 37, 64 x 1 126 / 39."""
+        longest = ctx.max_tokens_per_entry
+        if self.selective_prompt is not None:
+            return self.selective_prompt
+        if longest < 16:
+            return False
+        share, work = -(-inner // 32) / self.num_sms, ctx.T * inner
+        one_pass = 4.0 + max(0.0405 * longest, share * (2.2 * ctx.S + 0.0405 * ctx.T))
+        other = 48.0 + 1.35e-5 * work if longest >= self.SCAN_CHUNK_FROM else 6.0 + max(0.4 * longest, 1.1e-5 * work)
+        return one_pass < other
 
     def moe_route(self, h, w_router, ids, wts, meta, bias=None, over_chosen: bool = False):
         """Per token: float32 logits w_router h (+ ``bias``, float32 [experts]), softmax over all experts, the ids.shape[1]
