@@ -81,7 +81,7 @@ __device__ __forceinline__ int take_best(float* v, int n, float* value = nullptr
 // Logits (+ bias); scores softmax(z); the `top` largest scores, ties to the lower index; weights = those scores divided by their
 // sum (+ 1e-20).  over_chosen: the largest logits choose and the weights are the softmax over the chosen logits alone.
 // A block takes TOK tokens and a warp a token chooses.  Measured, 2,048 tokens of 2,048, 16 experts: a block a token with one
-// choosing thread 40 us, four tokens a block 27 (waiting for x and w; they are 8 MB and 128 KB).
+// choosing thread 40 us, four tokens a block 20 (two rounds of blocks that wait for x and w, 8 MB and 128 KB); eight 27.
 template <typename T, int TOK, int EXP>
 __global__ void __launch_bounds__(256, 2)
 moe_route_kernel(const T* __restrict__ h, const float* __restrict__ w, int* __restrict__ ids, float* __restrict__ wts,

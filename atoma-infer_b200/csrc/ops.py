@@ -26,7 +26,7 @@ SKINNY_MAX_ROWS = 16  # bfloat16 linears with at most this many rows stream the 
 
 CORE_SOURCES = ["kernels/core.cu", "kernels/gemm_f32.cu", "kernels/layer_ops.cu", "kernels/linear_bf16.cu", "kernels/linear_stream.cu", "kernels/sampling.cu"]
 ATTENTION_SOURCES = ["kernels/attention_bf16.cu"]
-GEMM_SOURCES = ["kernels/gemm_tcgen05.cu", "kernels/gemm_f32_tcgen05.cu"]
+GEMM_SOURCES = ["kernels/gemm_tcgen05.cu", "kernels/gemm_f32_tcgen05.cu", "kernels/moe_tcgen05.cu"]
 ATTENTION_TC_SOURCES = ["kernels/attention_tcgen05.cu"]
 DECODE_STACK_SOURCES = ["kernels/decode_stack.cu"]
 ATTENTION_TALK_SOURCES = ["kernels/attention_talk.cu"]  # weights mixed across heads; one library per head size
@@ -1067,20 +1067,33 @@ class CudaOps:
                                                     _p(meta), h.shape[0], H, E, ids.shape[1], self._stream()), "moe_route")
 
     MOE_PAIR_ROWS = 64       # up to this many (token, choice) pairs, bfloat16: a pair at a time
-    MOE_LIBRARY_ROWS = 256   # from this many pairs on, bfloat16: the library's grouped products
-    moe_library = hasattr(torch, "_grouped_mm")  # (a test lever too)
+    MOE_TC_ROWS = 65         # from this many pairs on, bfloat16: grouped products on tcgen05
 
-    def moe_experts(self, h, ids, wts, w_gate_up, w_down, shared, out, meta):
+    def _moe_on_tcgen05(self, h, pairs: int, E: int, F: int) -> bool:
+        H = h.shape[1]
+        return (h.dtype == torch.bfloat16 and pairs >= self.MOE_TC_ROWS and H % 8 == 0 and F % 8 == 0 and h.is_contiguous()
+                and h.data_ptr() % 16 == 0 and E <= self._gemm_library().moe_tc_most_experts())
+
+    def moe_takes_shared(self, h, top: int, w_gate_up, ws_gate_up) -> bool:
+        """Whether ``moe_experts`` makes the shared expert's product beside the others' (``shared_weights``)."""
+        return (self._moe_on_tcgen05(h, h.shape[0] * top, w_gate_up.shape[0], w_gate_up.shape[1] // 2)
+                and ws_gate_up.shape[0] % 16 == 0)
+
+    def moe_experts(self, h, ids, wts, w_gate_up, w_down, shared, out, meta, shared_weights=None):
         """out[t] = sum_k wts[t, k] * expert ids[t, k] of h[t] (+ shared[t]); an expert is down(silu(gate x) * up x) with
         ``w_gate_up`` [E, 2F, H] (gate rows first) and ``w_down`` [E, H, F].  The (token, choice) pairs are sorted by expert
         on the device and the two linears run as grouped products over that order: on the engine's own tile kernel
         (float32 always: every output's order of summation is then the same for any batch), or, in bfloat16, a pair at a
-        time for a handful of pairs and through the library's grouped product for many."""
+        time for a handful of pairs and on tcgen05 for many.  ``shared_weights`` (where ``moe_takes_shared``): the shared
+        expert's [2Fs, H] and [H, Fs], instead of its result ``shared``."""
         T, top = ids.shape
         E, F2, H = w_gate_up.shape
         F = F2 // 2
         lib, dev = self._mixers(), h.device
         pairs, bf = T * top, h.dtype == torch.bfloat16
+        on_tc = self._moe_on_tcgen05(h, pairs, E, F)
+        if shared_weights is not None and not on_tc:
+            raise KernelError("moe_experts: this call does not take the shared expert's weights")
         act = torch.empty((pairs, F), dtype=h.dtype, device=dev)
         if bf and pairs <= self.MOE_PAIR_ROWS and H % 8 == 0 and F % 8 == 0 and max(H, F) * 2 <= 96 * 1024:
             # a handful of pairs (decode steps): every pair streams its expert's rows itself, no sorting
@@ -1095,23 +1108,25 @@ class CudaOps:
         order = torch.empty(pairs, dtype=torch.int32, device=dev)
         place = torch.empty(pairs, dtype=torch.int32, device=dev)
         self._check(lib.moe_sort(_p(ids), _p(offsets), _p(order), _p(place), _p(meta), top, E, self._stream()), "moe_sort")
-        if bf and pairs >= self.MOE_LIBRARY_ROWS and self.moe_library and H % 8 == 0 and F % 8 == 0:
-            # many pairs: rows gathered in sorted order, the two products as the library's grouped products over the
-            # experts' stretches (offsets on the device: no host round trip), like the many-row linears
+        if on_tc:
+            # many pairs: rows gathered in sorted order, then both linears over the experts' stretches (offsets on the device: no
+            # host round trip), the shared expert's rows as one more stretch
             xs = torch.empty((pairs, H), dtype=h.dtype, device=dev)
+            y = torch.empty((pairs, H), dtype=h.dtype, device=dev)
             self._check(lib.moe_gather_rows(_p(h), _p(xs), _p(order), _p(meta), T, top, H * 2, self._stream()), "moe_gather_rows")
-            ends = offsets[1:]
-            try:
-                gu = torch._grouped_mm(xs, w_gate_up.transpose(1, 2), offs=ends)
-                self.silu_mul(gu, act, None, pairs, F)
-                y = torch._grouped_mm(act, w_down.transpose(1, 2), offs=ends)
-            except (RuntimeError, TypeError, NotImplementedError):
-                y = None  # the library refuses these sizes or strides: the engine's own grouped kernel from now on
-                self.moe_library = False
-            if y is not None:
-                self._check(lib.moe_combine(_p(y), DT_BF16, _p(place), _p(wts), _p(shared), _p(out), _code(out), _p(meta), T, top,
-                                            H, self._stream()), "moe_combine")
-                return
+            ws_gate_up, ws_down = shared_weights or (None, None)
+            act_s = None
+            if ws_down is not None:
+                act_s = torch.empty((T, ws_down.shape[1]), dtype=h.dtype, device=dev)
+                shared = torch.empty((T, H), dtype=h.dtype, device=dev)
+            self._check(self._gemm_library().moe_tc_ff(_p(xs), _p(w_gate_up), _p(act), _p(w_down), _p(y), _p(offsets), pairs, E, H, F, _p(h),
+                                                       _p(ws_gate_up), _p(act_s), _p(ws_down), _p(shared) if act_s is not None else None,
+                                                       T if act_s is not None else 0, ws_down.shape[1] if act_s is not None else 0, _p(meta),
+                                                       _p(self.status), self._stream()), "moe_tc_ff")
+            self.launches += 1
+            self._check(lib.moe_combine(_p(y), DT_BF16, _p(place), _p(wts), _p(shared), _p(out), _code(out), _p(meta), T, top, H,
+                                        self._stream()), "moe_combine")
+            return
         y = torch.empty((pairs, H), dtype=torch.float32, device=dev)
         self._check(lib.moe_grouped_ff(_p(h), _p(w_gate_up), _p(act), _p(w_down), _p(y), _p(offsets), _p(order), _code(h), T, top,
                                        E, H, F, self._stream()), "moe_grouped_ff")

@@ -102,11 +102,15 @@ class RoutedExperts(FeedForward):
             ops.moe_route(x, self.w_router, ids, wts, ctx.meta, bias=self.b_router, over_chosen=self.over_chosen)
         else:
             ops.moe_route(x, self.w_router, ids, wts, ctx.meta)
-        shared = None
+        shared, inside = None, {}
         if self.shared:
-            shared = ops.linear(ops.linear(x, self.ws_gate_up, silu_mul=True, meta=ctx.meta), self.ws_down, meta=ctx.meta)
+            takes = getattr(ops, "moe_takes_shared", None)
+            if takes and takes(x, self.top, self.w_gate_up, self.ws_gate_up):
+                inside = {"shared_weights": (self.ws_gate_up, self.ws_down)}
+            else:
+                shared = ops.linear(ops.linear(x, self.ws_gate_up, silu_mul=True, meta=ctx.meta), self.ws_down, meta=ctx.meta)
         out = torch.empty((T, self.hidden), dtype=x.dtype, device=x.device)
-        ops.moe_experts(x, ids, wts, self.w_gate_up, self.w_down, shared, out, ctx.meta)
+        ops.moe_experts(x, ids, wts, self.w_gate_up, self.w_down, shared, out, ctx.meta, **inside)
         return out
 
 

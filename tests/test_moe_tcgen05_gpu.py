@@ -1,0 +1,51 @@
+"""Routed experts' linears on tcgen05: stretches of no, one, 15 to 17, 255 to 257 and 600 rows, results that are no multiple of a tile's 64 or
+128 rows, depths that are no multiple of 64, with the shared expert in the same launches and without it."""
+import pytest
+import torch
+
+import kernel_utils as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def rt():
+    from atoma_infer_b200.engine.runtime import make_runtime
+
+    return make_runtime("bfloat16", "cuda:0")
+
+
+@pytest.mark.parametrize("H,F,Fs", [(136, 72, 40), (256, 128, 0), (520, 200, 264), (64, 8, 8)])
+@pytest.mark.parametrize("counts,top", [([0, 1, 15, 16, 17, 0, 255, 256, 257, 600, 3], 2), ([128], 1), ([0, 0, 130, 0], 1), ([300] * 40, 3)])
+def test_experts(rt, H, F, Fs, counts, top):
+    E, pairs = len(counts), sum(counts)
+    T, g = pairs // top, torch.Generator().manual_seed(H + E)
+    ids = torch.repeat_interleave(torch.arange(E), torch.tensor(counts))[torch.randperm(pairs, generator=g)][: T * top].view(T, top).int()
+
+    def draw(*shape, std=1.0):
+        return (torch.randn(*shape, generator=g) * std).bfloat16().to(rt.device)
+
+    h, gu, down = draw(T, H), draw(E, 2 * F, H, std=H ** -0.5), draw(E, H, F, std=F ** -0.5)
+    wts = torch.rand(T, top, generator=g).to(rt.device)
+    ids, weights, want = ids.to(rt.device), None, torch.zeros(T, H, dtype=torch.float64, device=rt.device)
+
+    def expert(x, gu, down):
+        a, b = (x.double() @ gu.double().T).chunk(2, -1)
+        return (a * torch.sigmoid(a) * b) @ down.double().T
+
+    for e in range(E):
+        t, k = (ids == e).nonzero(as_tuple=True)
+        want.index_add_(0, t, wts[t, k].double()[:, None] * expert(h[t], gu[e], down[e]))
+    if Fs:
+        weights = (draw(2 * Fs, H, std=H ** -0.5), draw(H, Fs, std=Fs ** -0.5))
+        want += expert(h, *weights)
+        assert rt.ops.moe_takes_shared(h, top, gu, weights[0])
+    meta = K.make_context(rt, [(0, T)], 16, [[1] * (-(-T // 16))])[0].meta
+    out = torch.full((T, H), float("nan"), dtype=rt.dtype, device=rt.device)
+    rt.ops.moe_experts(h, ids, wts, gu, down, None, out, meta, **({"shared_weights": weights} if Fs else {}))
+    rt.ops.check_status()
+    # three roundings to bfloat16 (the activation, a pair's result, the sum): 2^-9 of a value each at most
+    assert float((out.double() - want).norm() / want.norm()) < 3 * 2.0 ** -9
+    again = torch.empty_like(out)
+    rt.ops.moe_experts(h, ids, wts, gu, down, None, again, meta, **({"shared_weights": weights} if Fs else {}))
+    assert torch.equal(out, again)
