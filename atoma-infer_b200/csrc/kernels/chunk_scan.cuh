@@ -20,7 +20,8 @@
 // multiprocessor; the tensor pipe is 33 to 37 % busy, issue slots 40 %.  The state shares (N * P floats a chunk and head,
 // written, chained and read) stay in L2.  CHUNK = 128: 64 would double the shares' traffic for a tenth fewer products, 256
 // would not fit its operands into half of a multiprocessor's shared memory.  Measured, one prompt of 2,048 tokens, 64 heads of
-// 128 x 64: 471 us token by token in chunks of time, 108 us here (states 33, chain 13, outputs 65).
+// 128 x 64: 471 us token by token in chunks of time, 101 us here (states 33, chain 9, outputs 60; 67 while a block asked for S_in
+// only after its logs and rows).
 #pragma once
 #include "common.cuh"
 
@@ -445,6 +446,22 @@ __global__ void __launch_bounds__(256, 2) chunk_outputs_kernel(const __grid_cons
     const size_t HS = (size_t)A.N * A.P, CS = HS + (KIND == CHUNK_MEMORY ? A.N : 0);
     const float* s_in = A.scratch + ((size_t)c * A.heads + h) * CS;
     if (KIND == CHUNK_MEMORY && tid < NB) n_in[tid] = tid < A.N ? s_in[HS + tid] : 0.f;
+    constexpr int S_ITEMS = NB * (CHUNK_PB / 8) / 256;
+    float4 sx[S_ITEMS][2];
+    auto fetch_s = [&]() {
+#pragma unroll
+        for (int u = 0; u < S_ITEMS; ++u) {
+            const int i = tid + u * 256, n = i / (CHUNK_PB / 8), p = p0 + i % (CHUNK_PB / 8) * 8;
+            sx[u][0] = sx[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (n < A.N && p < A.P) {
+                sx[u][0] = *reinterpret_cast<const float4*>(s_in + (size_t)n * A.P + p);
+                sx[u][1] = *reinterpret_cast<const float4*>(s_in + (size_t)n * A.P + p + 4);
+            }
+        }
+    };
+    // S_in sets out with the rows and waits in registers until q's tile is read (67 -> 60 us; the memory's logs are loads, not
+    // arithmetic, and there it cost 1 of 51)
+    if (KIND == CHUNK_SSM) fetch_s();
     chunk_logs<KIND>(L, A, h, t0, nt);
     copies_done();
     __syncthreads();
@@ -455,14 +472,12 @@ __global__ void __launch_bounds__(256, 2) chunk_outputs_kernel(const __grid_cons
 #pragma unroll
         for (int k = 0; k < KT; ++k) ldmatrix4(qa[k], smem_address(qs) + piece<KROW>(rb * 16 + (lane & 15), k * 2 + (lane >> 4)));
     }
+    if (KIND != CHUNK_SSM) fetch_s();
     __syncthreads();  // q's tile is read: S_in takes its place
-    for (int i = tid; i < NB * (CHUNK_PB / 8); i += 256) {
-        const int n = i / (CHUNK_PB / 8), pc = i % (CHUNK_PB / 8), p = p0 + pc * 8;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
-        if (n < A.N && p < A.P) {
-            x = *reinterpret_cast<const float4*>(s_in + (size_t)n * A.P + p);
-            y = *reinterpret_cast<const float4*>(s_in + (size_t)n * A.P + p + 4);
-        }
+#pragma unroll
+    for (int u = 0; u < S_ITEMS; ++u) {
+        const int i = tid + u * 256, n = i / (CHUNK_PB / 8), pc = i % (CHUNK_PB / 8);
+        const float4 x = sx[u][0], y = sx[u][1];
         uint32_t s[3][4];
         split_pair(x.x, x.y, s[0][0], s[1][0], s[2][0]);
         split_pair(x.z, x.w, s[0][1], s[1][1], s[2][1]);

@@ -21,7 +21,8 @@
 // together, 8 heads of 128 x 256): outputs 1.3e-7, last states 7.9e-8; token by token in float32 2.5e-7 and 2.6e-7.
 //
 // What bounds it: the chain of phases of a block that prepares (40 us; a block a head and chunk is few blocks, hence 16 warps), then
-// mma.sync (shares of the state 21 us, outputs 37) and the chunks' states through L2 (11).  107 us for the prompts above; token by
+// mma.sync (shares of the state 21 us, outputs 35, 37 before all of S_in
+// was on its way at once) and the chunks' states through L2 (11).  105 us for the prompts above; token by
 // token in chunks of time 283.  Heads of 64 x 64 (32 of them, 2,048 tokens): 131 against 184.
 #pragma once
 #include "chunk_scan.cuh"
@@ -461,13 +462,25 @@ __global__ void __launch_bounds__(256, 2) row_outputs_kernel(const __grid_consta
     stage_rows<VROW>(vs, A.v + (size_t)h * A.P + p0, A.v_stride, t0, nt, rows, A.P - p0);
     const size_t ch = (size_t)c * A.hn + hl, HS = (size_t)A.N * A.P;
     const float* s_in = A.share + ch * HS;
-    for (int i = tid; i < NB * (CHUNK_PB / 8); i += 256) {
-        const int n = i / (CHUNK_PB / 8), pc = i % (CHUNK_PB / 8), p = p0 + pc * 8;
-        float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+    const int lane = tid & 31, warp = tid >> 5, rb = warp >> 1, n0 = (warp & 1) * NT, g = lane >> 2, q2 = (lane & 3) * 2;
+    const uint4* qsrc = A.qf + (ch * 4 + rb) * KT * 96 + lane;
+    constexpr int S_ITEMS = NB * (CHUNK_PB / 8) / 256;
+    float4 sx[S_ITEMS][2];  // all of S_in on its way before the first of it is split
+#pragma unroll
+    for (int u = 0; u < S_ITEMS; ++u) {
+        const int i = tid + u * 256, n = i / (CHUNK_PB / 8), p = p0 + i % (CHUNK_PB / 8) * 8;
+        sx[u][0] = sx[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (n < A.N && p < A.P) {
-            x = *reinterpret_cast<const float4*>(s_in + (size_t)n * A.P + p);
-            y = *reinterpret_cast<const float4*>(s_in + (size_t)n * A.P + p + 4);
+            sx[u][0] = *reinterpret_cast<const float4*>(s_in + (size_t)n * A.P + p);
+            sx[u][1] = *reinterpret_cast<const float4*>(s_in + (size_t)n * A.P + p + 4);
         }
+    }
+    uint32_t a[3][4];
+    if (rb * 16 < nt) load_split(a, qsrc);
+#pragma unroll
+    for (int u = 0; u < S_ITEMS; ++u) {
+        const int i = tid + u * 256, n = i / (CHUNK_PB / 8), pc = i % (CHUNK_PB / 8);
+        const float4 x = sx[u][0], y = sx[u][1];
         uint32_t s[3][4];
         split_pair(x.x, x.y, s[0][0], s[1][0], s[2][0]);
         split_pair(x.z, x.w, s[0][1], s[1][1], s[2][1]);
@@ -476,10 +489,6 @@ __global__ void __launch_bounds__(256, 2) row_outputs_kernel(const __grid_consta
 #pragma unroll
         for (int j = 0; j < 3; ++j) *reinterpret_cast<uint4*>(ss + j * NB * VROW + piece<VROW>(n, pc)) = make_uint4(s[j][0], s[j][1], s[j][2], s[j][3]);
     }
-    const int lane = tid & 31, warp = tid >> 5, rb = warp >> 1, n0 = (warp & 1) * NT, g = lane >> 2, q2 = (lane & 3) * 2;
-    const uint4* qsrc = A.qf + (ch * 4 + rb) * KT * 96 + lane;
-    uint32_t a[3][4];
-    if (rb * 16 < nt) load_split(a, qsrc);
     copies_done();
     __syncthreads();
     float odd = 0.f;  // no number as soon as one result is not finite
