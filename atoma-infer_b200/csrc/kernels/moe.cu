@@ -572,7 +572,7 @@ extern "C" int moe_pair_ff(const void* x, const void* w_gate_up, void* act, cons
                                   (__nv_bfloat16*)nullptr, y, ids, meta, top, F, H);
 }
 
-// ----------------------------------------------------------------------------- many pairs: rows gathered for a library's grouped product
+// ----------------------------------------------------------------------------- many pairs: rows gathered for the grouped products on tcgen05
 // xs[i] = x[order[i] / top] for the pairs in sorted order (16 bytes a thread; H * element size a multiple of 16).
 __global__ void __launch_bounds__(256)
 moe_gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, const int* __restrict__ order,

@@ -3,6 +3,7 @@
 // run side by side), and the gated norm in equal parts behind it.  Storage is float32 or bfloat16; the recurrence,
 // its step sizes and decays, the gate and the norm are float32 always.
 #include "chunk_scan.cuh"
+#include "ssm_token.cuh"
 
 // ----------------------------------------------------------------------------- causal convolution, bias, activation
 // y[t, c] = act(bias[c] + sum_j w[j, c] * u[t - taps + 1 + j, c]) over the rows of each request, zeros before its
@@ -580,11 +581,13 @@ extern "C" int ssm_chunk_scan(const void* xbc, int xbc_stride, const void* dt, l
 template <typename T>
 __global__ void __launch_bounds__(256)
 gated_group_norm_kernel(const float* __restrict__ y, const T* __restrict__ z, long long z_stride, const float* __restrict__ w,
-                        float eps, T* __restrict__ out, const int* __restrict__ meta, int n, int parts, int vec4) {
+                        float eps, T* __restrict__ out, const int* __restrict__ meta, int n, int parts, int vec4,
+                        const __grid_constant__ RingRow<T> ring) {
     __shared__ float red[33];
     pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x, part = blockIdx.y, len = n / parts, at = part * len;
+    if (part >= parts) return ring_row(ring, t, part - parts, meta);  // (blocks of a decode step that write the convolution's ring)
     if (t >= meta[META_NUM_TOKENS]) return;
     const float* yr = y + (size_t)t * n + at;
     const T* zr = z + (size_t)t * z_stride + at;
@@ -712,6 +715,14 @@ static int launch_group_norm_warp(const float* y, const T* z, long long z_stride
 #undef NORM_CASE
 }
 
+template <typename T>
+static int launch_group_norm(const float* y, const T* z, long long z_stride, const float* w, float eps, T* out, const int* meta, int rows, int n,
+                             int parts, int threads, int vec4, const RingRow<T>& ring, cudaStream_t stream) {
+    const int more = ring.ring ? (ring.channels + threads - 1) / threads : 0;
+    return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, gated_group_norm_kernel<T>, dim3(rows, parts + more), threads, 0, stream, y, z, z_stride, w,
+                                  eps, out, meta, n, parts, vec4, ring);
+}
+
 extern "C" int gated_group_norm(const float* y, const void* z, int dtype, long long z_stride, const float* w, float eps,
                                 void* out, const int* meta, int T, int n, int parts, cudaStream_t stream) {
     if (T <= 0) return 0;
@@ -724,8 +735,46 @@ extern "C" int gated_group_norm(const float* y, const void* z, int dtype, long l
     if (dtype != DT_F32 && vec4 && len <= 1024 && (long)T * parts >= 8 * multiprocessors())
         return launch_group_norm_warp(y, (const __nv_bfloat16*)z, z_stride, w, eps, (__nv_bfloat16*)out, meta, T, n, parts, stream);
     if (dtype == DT_F32)
-        return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, gated_group_norm_kernel<float>, dim3(T, parts), threads, 0, stream, y,
-                                      (const float*)z, z_stride, w, eps, (float*)out, meta, n, parts, vec4);
-    return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, gated_group_norm_kernel<__nv_bfloat16>, dim3(T, parts), threads, 0, stream,
-                                  y, (const __nv_bfloat16*)z, z_stride, w, eps, (__nv_bfloat16*)out, meta, n, parts, vec4);
+        return launch_group_norm(y, (const float*)z, z_stride, w, eps, (float*)out, meta, T, n, parts, threads, vec4, RingRow<float>{}, stream);
+    return launch_group_norm(y, (const __nv_bfloat16*)z, z_stride, w, eps, (__nv_bfloat16*)out, meta, T, n, parts, threads, vec4,
+                             RingRow<__nv_bfloat16>{}, stream);
+}
+
+// Convolution, recurrence and gated norm of a step whose entries bring a token each, in two launches (ssm_token.cuh); y: S rows of
+// scratch.  ssm_token_step_takes: whether these sizes and addresses are served (and steps small enough to gain by it, with a norm that takes
+// a block a part).
+extern "C" int ssm_token_step_takes(const float* ring, const float* state, long long slot_stride, int S, int heads, int P, int N, int groups, int parts,
+                                    int taps) {
+    return ssm_token_takes(heads, P, N, groups, taps) && (taps == 1 || ring) && slot_stride % 4 == 0 && ((uintptr_t)state & 15) == 0 && parts > 0 &&
+           heads * P % parts == 0 && (long)S * heads <= TOKEN_BLOCKS * multiprocessors() && (long)S * parts < 8 * multiprocessors();
+}
+
+template <typename T>
+static int ssm_token_run(const SsmToken<T>& a, int S, int P, const T* z, long long z_stride, const float* norm_w, int parts, float eps, float* ring,
+                         T* out, cudaStream_t stream) {
+    const dim3 grid(a.heads, S);
+    const cudaError_t err = P == 32   ? launch_kernel(ssm_token_kernel<T, 8>, grid, 256, 0, stream, a)
+                            : P == 64 ? launch_kernel(ssm_token_kernel<T, 16>, grid, 256, 0, stream, a)
+                                      : launch_kernel(ssm_token_kernel<T, 32>, grid, 256, 0, stream, a);
+    if (err != cudaSuccess) return (int)err;
+    const int n = a.heads * P, len = n / parts;
+    const int vec4 = len % 4 == 0 && z_stride % 4 == 0 && (((uintptr_t)a.y | (uintptr_t)z | (uintptr_t)norm_w | (uintptr_t)out) & 15) == 0;
+    const RingRow<T> row{a.u, a.u_stride, a.taps > 1 ? ring : nullptr, a.ring_stride, a.positions, a.cu_tokens, a.slots, n + 2 * a.groups * a.N, a.taps - 1};
+    return launch_group_norm(a.y, z, z_stride, norm_w, eps, out, a.meta, S, n, parts, len >= 1024 ? 256 : 128, vec4, row, stream);
+}
+
+extern "C" int ssm_token_step(const void* u, long long u_stride, const void* z, long long z_stride, const void* dt, long long dt_stride, int dtype,
+                              const float* conv_w, const float* conv_b, float* ring, long long ring_stride, const float* dt_bias, const float* a_log,
+                              const float* d_skip, float* state, long long slot_stride, float* y, const float* norm_w, int parts, float eps, void* out,
+                              const int* meta, const int* positions, const int* cu_tokens, const int* slots, int S, int heads, int P, int N, int groups,
+                              int taps, cudaStream_t stream) {
+    if (S <= 0) return 0;
+    if (!ssm_token_step_takes(ring, state, slot_stride, S, heads, P, N, groups, parts, taps)) return (int)cudaErrorInvalidValue;
+#define TOKEN_CASE(T)                                                                                                      \
+    return ssm_token_run<T>({(const T*)u, (const T*)dt, u_stride, dt_stride, conv_w, conv_b, ring, ring_stride, dt_bias, a_log, d_skip, state, \
+                             slot_stride, y, meta, positions, cu_tokens, slots, heads, N, groups, taps}, S, P, (const T*)z, z_stride, norm_w, parts, \
+                            eps, ring, (T*)out, stream)
+    if (dtype == DT_F32) TOKEN_CASE(float);
+    TOKEN_CASE(__nv_bfloat16);
+#undef TOKEN_CASE
 }

@@ -799,6 +799,25 @@ class CudaOps:
         self._check(self._mixers().gated_group_norm(_p(y), zp, _code(z), zs, _p(w), ctypes.c_float(eps), _p(out), _p(meta),
                                                     y.shape[0], y.shape[1], groups, self._stream()), "gated_group_norm")
 
+    def ssm_token_step(self, u, z, dt, conv_w, conv_b, ring, dt_bias, a_log, d_skip, state, norm_w, groups: int, norm_groups: int, eps: float,
+                       ctx, out) -> bool:
+        """Convolution, recurrence and gated norm (``causal_conv_act``, ``ssm_scan``, ``gated_group_norm``) of a step whose entries
+        bring one token each, in two launches; ``u``, ``z``, ``dt`` slices of wider rows.  False (and nothing done) for other steps and sizes."""
+        if not ctx.decode_only or ctx.T != ctx.S or state.dtype != torch.float32 or not state[0].is_contiguous():
+            return False
+        (up, us), (zp, zs), (dp, ds) = (self._rows(t, "ssm_token_step") for t in (u, z, dt))
+        lib, taps, (heads, N, P) = self._mixers(), conv_w.shape[0], state.shape[1:]
+        ss = ctypes.c_longlong(state.stride(0))
+        if not lib.ssm_token_step_takes(_p(ring), _p(state), ss, ctx.S, heads, P, N, groups, norm_groups, taps):
+            return False
+        y = torch.empty((ctx.T, heads * P), dtype=torch.float32, device=out.device)
+        self._check(lib.ssm_token_step(up, us, zp, zs, dp, ds, _code(u), _p(conv_w), _p(conv_b), _p(ring), self._slot_stride(ring), _p(dt_bias),
+                                       _p(a_log), _p(d_skip), _p(state), ss, _p(y), _p(norm_w), norm_groups, ctypes.c_float(eps), _p(out), _p(ctx.meta),
+                                       _p(ctx.positions), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, heads, P, N, groups, taps, self._stream()),
+                    "ssm_token_step")
+        self.launches += 1
+        return True
+
     def rms_rows(self, x, w, eps: float, out, meta):
         """out = x * rsqrt(mean(x^2) + eps) * w row by row; ``x`` a slice of wider rows, ``w`` float32."""
         xp, xs = self._rows(x, "rms_rows")

@@ -95,13 +95,17 @@ class Mamba2Mixer(Mixer):
         proj = ops.linear(x, self.w_in, meta=ctx.meta)
         z, u, dt = proj[:, :inner], proj[:, inner:inner + self.channels], proj[:, inner + self.channels:]
         ring = self.ring(cache.state)
+        g = torch.empty((T, inner), dtype=x.dtype, device=x.device)
+        token_step = getattr(ops, "ssm_token_step", None)
+        if token_step and token_step(u, z, dt, self.conv_w, self.conv_b, ring, self.dt_bias, self.a_log, self.d_skip, self.matrices(cache.state),
+                                     self.norm_w, self.groups, self.norm_groups, self.eps, ctx, g):
+            return ops.linear(g, self.w_out, meta=ctx.meta)
         xbc = torch.empty((T, self.channels), dtype=x.dtype, device=x.device)
         if not ops.causal_conv_act(u, self.conv_w, self.conv_b, ring, ctx, xbc, act="silu"):
             ops.causal_conv_save(u, ring, ctx, self.taps)  # after the convolution has read the ring
         y = torch.empty((T, inner), dtype=torch.float32, device=x.device)
         ops.ssm_scan(xbc, dt, self.dt_bias, self.a_log, self.d_skip, self.matrices(cache.state), ctx, y,
                      heads=self.heads, head_dim=self.head_dim, nstate=self.nstate, groups=self.groups)
-        g = torch.empty((T, inner), dtype=x.dtype, device=x.device)
         ops.gated_group_norm(y, z, self.norm_w, self.norm_groups, self.eps, g, ctx.meta)
         return ops.linear(g, self.w_out, meta=ctx.meta)
 

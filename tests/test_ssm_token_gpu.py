@@ -1,0 +1,70 @@
+"""The state-space mixer's decode step in two launches, beside the convolution, the scan in order and the gated norm as kernels of their
+own: every column count, the most rows and odd numbers of them, one to four taps, first tokens, slots out of order."""
+import pytest
+import torch
+
+import kernel_utils as K
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,P,N,G,taps", [(16, 64, 128, 2, 4), (8, 64, 72, 1, 3), (6, 32, 250, 2, 4), (3, 32, 40, 3, 2), (4, 128, 64, 2, 4),
+                                              (2, 128, 33, 2, 1), (5, 64, 8, 1, 4), (14, 64, 127, 2, 4)])
+def test_against_three_kernels(dtype, heads, P, N, G, taps):
+    from atoma_infer_b200.engine.runtime import make_runtime
+
+    rt = make_runtime(dtype, "cuda:0")
+    ops, dev = rt.ops, rt.device
+    g = torch.Generator().manual_seed(heads * N)
+    past = [0, 1, 2, 57, 400]
+    S, inner, ch = len(past), heads * P, heads * P + 2 * G * N
+    rows = -(-(ch + inner + heads) // 8) * 8  # (wide rows; some slices start on odd elements)
+    ctx, _ = K.make_context(rt, [(c, 1) for c in past], 16, [[1 + i] * 32 for i in range(S)])
+    assert ctx.decode_only and ctx.T == ctx.S
+    ctx.state_slots.copy_(torch.tensor([3, 0, 4, 1, 2], dtype=torch.int32))
+
+    def f(*shape, std=1.0, mean=0.0):
+        return (torch.randn(*shape, generator=g) * std + mean).to(dev)
+
+    proj = f(S, rows).to(rt.dtype)
+    z, u, dt = proj[:, :inner], proj[:, inner:inner + ch], proj[:, inner + ch:inner + ch + heads]
+    conv_w, conv_b, dt_bias, a_log, d, w = f(taps, ch, std=0.3), f(ch, std=0.1), f(heads, mean=-3), f(heads, std=0.5), f(heads), f(inner, std=0.1, mean=1)
+    ring_floats = -(-(taps - 1) * ch // 4) * 4
+    state = f(S, ring_floats + heads * N * P, std=0.5)
+
+    def parts(s):
+        ring = s[:, :(taps - 1) * ch].view(S, taps - 1, ch) if taps > 1 else None
+        return ring, s[:, ring_floats:].view(S, heads, N, P)
+
+    ours, theirs = state.clone(), state.clone()
+    got, want = (torch.full((S, inner), float("nan"), dtype=rt.dtype, device=dev) for _ in range(2))
+    assert ops.ssm_token_step(u, z, dt, conv_w, conv_b, parts(ours)[0], dt_bias, a_log, d, parts(ours)[1], w, G, G, 1e-5, ctx, got)
+    xbc, y = torch.empty(S, ch, dtype=rt.dtype, device=dev), torch.empty(S, inner, device=dev)
+    if not ops.causal_conv_act(u, conv_w, conv_b, parts(theirs)[0], ctx, xbc):
+        ops.causal_conv_save(u, parts(theirs)[0], ctx, taps)
+    ops.ssm_scan(xbc, dt, dt_bias, a_log, d, parts(theirs)[1], ctx, y, heads=heads, head_dim=P, nstate=N, groups=G)
+    ops.gated_group_norm(y, z, w, G, 1e-5, want, ctx.meta)
+    ops.check_status()
+    # the same products and roundings; sums over N rows in another order: sqrt(N) 2^-24 of the terms and, in bfloat16, now and then the
+    # neighbouring number (2^-8 of a value, of which the 2-norm sees few)
+    assert torch.equal(ours[:, :ring_floats], theirs[:, :ring_floats])
+    assert float((ours - theirs).norm() / theirs.norm()) < 1e-6
+    assert float((got.double() - want.double()).norm() / want.double().norm()) < (2e-6 if dtype == "float32" else 1e-3)
+
+
+def test_other_steps_are_left_alone():
+    from atoma_infer_b200.engine.runtime import make_runtime
+
+    rt = make_runtime("bfloat16", "cuda:0")
+    t = torch.zeros(4, 512, dtype=rt.dtype, device=rt.device)
+    state = torch.zeros(4, 2, 16, 64, device=rt.device)
+    one = torch.zeros(512, device=rt.device)
+
+    def takes(entries, norm_groups=1):
+        ctx, _ = K.make_context(rt, entries, 16, [[1 + i] for i in range(len(entries))])
+        return rt.ops.ssm_token_step(t[:ctx.T, :160], t[:ctx.T, :128], t[:ctx.T, :2], one[:160].view(1, 160), None, None, one[:2], one[:2], one[:2], state,
+                                     one[:128], 1, norm_groups, 1e-5, ctx, torch.zeros_like(t[:ctx.T, :128]))
+
+    assert takes([(3, 1), (4, 1)])
+    assert not takes([(0, 2), (4, 1)]) and not takes([(3, 1)], norm_groups=3)
