@@ -1088,15 +1088,16 @@ class CudaOps:
     MOE_PAIR_ROWS = 64       # up to this many (token, choice) pairs, bfloat16: a pair at a time
     MOE_TC_ROWS = 65         # from this many pairs on, bfloat16: grouped products on tcgen05
 
-    def _moe_on_tcgen05(self, h, pairs: int, E: int, F: int) -> bool:
-        H = h.shape[1]
-        return (h.dtype == torch.bfloat16 and pairs >= self.MOE_TC_ROWS and H % 8 == 0 and F % 8 == 0 and h.is_contiguous()
-                and h.data_ptr() % 16 == 0 and E <= self._gemm_library().moe_tc_most_experts())
+    def _moe_on_tcgen05(self, pairs: int, E: int, F: int, *tensors) -> bool:
+        """``tensors``: the rows first, then the weights that take part."""
+        h = tensors[0]
+        return (h.dtype == torch.bfloat16 and pairs >= self.MOE_TC_ROWS and h.shape[1] % 8 == 0 and F % 8 == 0
+                and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in tensors) and E <= self._gemm_library().moe_tc_most_experts())
 
-    def moe_takes_shared(self, h, top: int, w_gate_up, ws_gate_up) -> bool:
+    def moe_takes_shared(self, h, top: int, w_gate_up, w_down, ws_gate_up, ws_down) -> bool:
         """Whether ``moe_experts`` makes the shared expert's product beside the others' (``shared_weights``)."""
-        return (self._moe_on_tcgen05(h, h.shape[0] * top, w_gate_up.shape[0], w_gate_up.shape[1] // 2)
-                and ws_gate_up.shape[0] % 16 == 0)
+        return ws_down.shape[1] % 8 == 0 and self._moe_on_tcgen05(h.shape[0] * top, w_down.shape[0], w_down.shape[2], h, w_gate_up, w_down,
+                                                                  ws_gate_up, ws_down)
 
     def moe_experts(self, h, ids, wts, w_gate_up, w_down, shared, out, meta, shared_weights=None):
         """out[t] = sum_k wts[t, k] * expert ids[t, k] of h[t] (+ shared[t]); an expert is down(silu(gate x) * up x) with
@@ -1110,7 +1111,7 @@ class CudaOps:
         F = F2 // 2
         lib, dev = self._mixers(), h.device
         pairs, bf = T * top, h.dtype == torch.bfloat16
-        on_tc = self._moe_on_tcgen05(h, pairs, E, F)
+        on_tc = self._moe_on_tcgen05(pairs, E, F, h, w_gate_up, w_down, *(shared_weights or ()))
         if shared_weights is not None and not on_tc:
             raise KernelError("moe_experts: this call does not take the shared expert's weights")
         act = torch.empty((pairs, F), dtype=h.dtype, device=dev)

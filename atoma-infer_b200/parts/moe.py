@@ -105,7 +105,7 @@ class RoutedExperts(FeedForward):
         shared, inside = None, {}
         if self.shared:
             takes = getattr(ops, "moe_takes_shared", None)
-            if takes and takes(x, self.top, self.w_gate_up, self.ws_gate_up):
+            if takes and takes(x, self.top, self.w_gate_up, self.w_down, self.ws_gate_up, self.ws_down):
                 inside = {"shared_weights": (self.ws_gate_up, self.ws_down)}
             else:
                 shared = ops.linear(ops.linear(x, self.ws_gate_up, silu_mul=True, meta=ctx.meta), self.ws_down, meta=ctx.meta)

@@ -39,7 +39,7 @@ def test_experts(rt, H, F, Fs, counts, top):
     if Fs:
         weights = (draw(2 * Fs, H, std=H ** -0.5), draw(H, Fs, std=Fs ** -0.5))
         want += expert(h, *weights)
-        assert rt.ops.moe_takes_shared(h, top, gu, weights[0])
+        assert rt.ops.moe_takes_shared(h, top, gu, down, *weights)
     meta = K.make_context(rt, [(0, T)], 16, [[1] * (-(-T // 16))])[0].meta
     out = torch.full((T, H), float("nan"), dtype=rt.dtype, device=rt.device)
     rt.ops.moe_experts(h, ids, wts, gu, down, None, out, meta, **({"shared_weights": weights} if Fs else {}))
