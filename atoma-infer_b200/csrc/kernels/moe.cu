@@ -240,7 +240,7 @@ extern "C" int moe_route_sigmoid(const void* h, int dtype, const float* w, const
 // One block.  offsets[e] .. offsets[e + 1] is expert e's stretch of `order`, which lists its pairs (token * top + choice)
 // in ascending order.  Every warp takes a stretch of the pairs, 32 at a time: pairs of one expert find one another by a match
 // across the warp, once to count (base[warp][expert]) and, after the counts have become places, once to write.
-// `place` (optional): place[pair] = where the pair stands in `order`.
+// `place` (optional): place[pair] = where the pair stands in `order`, -1 for a choice that names no expert (it stands nowhere).
 // Bound by the chain of loads and matches of one block: 4,096 pairs of 16 experts 7.5 us (each expert's warp walking all pairs
 // twice: 38 us).
 __global__ void __launch_bounds__(1024)
@@ -265,7 +265,7 @@ moe_sort_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __r
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const unsigned same = __match_any_sync(0xffffffffu, id[u]);
-                if (id[u] >= 0) visit(i0 + u * 32 + lane, id[u], __popc(same & ((1u << lane) - 1u)));
+                if (i0 + u * 32 + lane < to) visit(i0 + u * 32 + lane, id[u], __popc(same & ((1u << lane) - 1u)));
                 __syncwarp();
                 if (id[u] >= 0 && lane == __ffs(same) - 1) own[id[u]] += __popc(same);
                 __syncwarp();
@@ -302,8 +302,8 @@ moe_sort_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __r
     }
     __syncthreads();
     walk([&](int i, int e, int rank) {
-        const int at = own[e] + rank;
-        order[at] = i;
+        const int at = e >= 0 ? own[e] + rank : -1;
+        if (e >= 0) order[at] = i;
         if (place) place[i] = at;
     });
 }
@@ -428,7 +428,7 @@ extern "C" int moe_grouped_ff(const void* x, const void* w_gate_up, void* act, c
 
 // ----------------------------------------------------------------------------- weighted sum
 // out[t] = sum_k wts[t, k] * y[row of pair t * top + k] (+ shared[t]), choices in order, float32; a pair's row is the
-// pair itself, or place[pair] when the rows are in sorted order.
+// pair itself, or place[pair] when the rows are in sorted order (a pair of place -1 adds nothing).
 template <typename TY, typename T>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, const float* __restrict__ wts,
@@ -441,8 +441,9 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, cons
         for (int i = threadIdx.x * 4; i < H; i += blockDim.x * 4) {
             float acc[4] = {0.f, 0.f, 0.f, 0.f}, v[4];
             for (int k = 0; k < top; ++k) {
-                const size_t row = place ? (size_t)place[(size_t)t * top + k] : (size_t)t * top + k;
+                const long long row = place ? (long long)place[(size_t)t * top + k] : (long long)t * top + k;
                 const float weight = wts[(size_t)t * top + k];
+                if (row < 0) continue;
                 load4(y + row * H + i, v);
 #pragma unroll
                 for (int j = 0; j < 4; ++j) acc[j] = fmaf(weight, v[j], acc[j]);
@@ -459,8 +460,8 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, cons
     for (int i = threadIdx.x; i < H; i += blockDim.x) {
         float acc = 0.f;
         for (int k = 0; k < top; ++k) {
-            const size_t row = place ? (size_t)place[(size_t)t * top + k] : (size_t)t * top + k;
-            acc = fmaf(wts[(size_t)t * top + k], to_float(y[row * H + i]), acc);
+            const long long row = place ? (long long)place[(size_t)t * top + k] : (long long)t * top + k;
+            if (row >= 0) acc = fmaf(wts[(size_t)t * top + k], to_float(y[row * H + i]), acc);
         }
         if (shared) acc += to_float(shared[(size_t)t * H + i]);
         out[(size_t)t * H + i] = from_float<T>(acc);
@@ -573,22 +574,23 @@ extern "C" int moe_pair_ff(const void* x, const void* w_gate_up, void* act, cons
 }
 
 // ----------------------------------------------------------------------------- many pairs: rows gathered for the grouped products on tcgen05
-// xs[i] = x[order[i] / top] for the pairs in sorted order (16 bytes a thread; H * element size a multiple of 16).
+// xs[i] = x[order[i] / top] for the `sorted` pairs that stand in an expert's stretch (offsets[E]: behind them `order` holds
+// nothing); 16 bytes a thread, H * element size a multiple of 16.
 __global__ void __launch_bounds__(256)
 moe_gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, const int* __restrict__ order,
-                       const int* __restrict__ meta, int top, int chunks) {
+                       const int* __restrict__ sorted, int top, int chunks) {
     pdl_launch_dependents();
     pdl_wait();
     const int i = blockIdx.x;
-    if (i >= meta[META_NUM_TOKENS] * top) return;
+    if (i >= *sorted) return;
     const uint4* src = x + (size_t)(order[i] / top) * chunks;
     for (int c = threadIdx.x; c < chunks; c += blockDim.x) xs[(size_t)i * chunks + c] = src[c];
 }
 
-extern "C" int moe_gather_rows(const void* x, void* xs, const int* order, const int* meta, int T, int top, int row_bytes,
+extern "C" int moe_gather_rows(const void* x, void* xs, const int* order, const int* sorted, int T, int top, int row_bytes,
                                cudaStream_t stream) {
     if (T <= 0) return 0;
     if (row_bytes % 16) return (int)cudaErrorInvalidValue;
-    return (int)launch_kernel(moe_gather_rows_kernel, T * top, 256, 0, stream, (const uint4*)x, (uint4*)xs, order, meta, top,
+    return (int)launch_kernel(moe_gather_rows_kernel, T * top, 256, 0, stream, (const uint4*)x, (uint4*)xs, order, sorted, top,
                               row_bytes / 16);
 }

@@ -1133,7 +1133,7 @@ class CudaOps:
             # host round trip), the shared expert's rows as one more stretch
             xs = torch.empty((pairs, H), dtype=h.dtype, device=dev)
             y = torch.empty((pairs, H), dtype=h.dtype, device=dev)
-            self._check(lib.moe_gather_rows(_p(h), _p(xs), _p(order), _p(meta), T, top, H * 2, self._stream()), "moe_gather_rows")
+            self._check(lib.moe_gather_rows(_p(h), _p(xs), _p(order), _p(offsets[E:]), T, top, H * 2, self._stream()), "moe_gather_rows")
             ws_gate_up, ws_down = shared_weights or (None, None)
             act_s = None
             if ws_down is not None:

@@ -49,3 +49,23 @@ def test_experts(rt, H, F, Fs, counts, top):
     again = torch.empty_like(out)
     rt.ops.moe_experts(h, ids, wts, gu, down, None, again, meta, **({"shared_weights": weights} if Fs else {}))
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("T", [40, 300])  # 80 and 600 pairs
+def test_a_choice_that_names_no_expert_adds_nothing(rt, T):
+    """Such a pair stands nowhere in the sorted order: no row is gathered for it and none is added."""
+    E, H, F, g = 5, 72, 40, torch.Generator().manual_seed(T)
+    ids = torch.randint(0, E, (T, 2), generator=g, dtype=torch.int32)
+    ids[::3, 0], ids[1::7, 1], ids[5] = E, -1, 1 << 30
+    h, gu, down = (torch.randn(*s, generator=g).bfloat16().to(rt.device) for s in ((T, H), (E, 2 * F, H), (E, H, F)))
+    wts = torch.rand(T, 2, generator=g).to(rt.device)
+    meta = K.make_context(rt, [(0, T)], 16, [[1] * (-(-T // 16))])[0].meta
+
+    def run(ids, wts):
+        out = torch.full((T, H), float("nan"), dtype=rt.dtype, device=rt.device)
+        rt.ops.moe_experts(h, ids.to(rt.device), wts, gu, down, None, out, meta)
+        rt.ops.check_status()
+        return out
+
+    bad = (ids < 0) | (ids >= E)
+    assert torch.equal(run(ids, wts), run(ids.masked_fill(bad, 0), wts.masked_fill(bad.to(rt.device), 0.0)))
