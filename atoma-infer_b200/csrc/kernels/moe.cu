@@ -468,7 +468,7 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, cons
     }
 }
 
-// y_dtype: float32 rows in pair order (place null), or rows of the compute type in sorted order with `place`.
+// y: rows in pair order (place null) or in sorted order with `place`; float32, or of the compute type.
 extern "C" int moe_combine(const void* y, int y_dtype, const int* place, const float* wts, const void* shared, void* out,
                            int dtype, const int* meta, int T, int top, int H, cudaStream_t stream) {
     if (T <= 0) return 0;

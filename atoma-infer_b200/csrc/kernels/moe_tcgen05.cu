@@ -73,6 +73,9 @@ __device__ __forceinline__ void pair_commit(uint64_t* bar) {
                  ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
 
+__device__ __forceinline__ void store_two(bf16* p, float2 v) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(v.x, v.y); }
+__device__ __forceinline__ void store_two(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
+
 // A meeting of the two warps that hold the halves of a result.
 __device__ __forceinline__ void pair_barrier(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 
@@ -81,7 +84,9 @@ struct GroupedArgs {
     const int* meta;     // the step's tokens: the shared expert's rows
     int experts, rows, depth;                              // an expert's results a row (mode 1: F) and its K
     int shared_tokens, shared_rows, shared_depth;          // (0 tokens: no shared expert)
-    bf16 *out, *shared_out;                                // [sorted rows, rows], [tokens, shared_rows]
+    void* out;                                             // [sorted rows, rows]: bfloat16, or (mode 0) float32 with `wide`
+    bf16* shared_out;                                      // [tokens, shared_rows]
+    int wide;
 };
 
 // A tile: `count` rows of x from `first` on, results from `w0` on, of expert `e` (or the shared one: -1).
@@ -249,13 +254,13 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         bool ok = true;
         // Two neighbouring lanes swap half of their results, so that each stores two neighbouring results of every other row of x
         // (half the stores, 64 bytes a row of x).
-        auto store16 = [&](bf16* dst, int ld, int row, int rows, int first_col, int cols, const float (&v)[16]) {
+        auto store16 = [&](auto* dst, int ld, int row, int rows, int first_col, int cols, const float (&v)[16]) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const float got = __shfl_xor_sync(0xffffffffu, lane & 1 ? v[2 * i] : v[2 * i + 1], 1);
                 const int col = first_col + 2 * i + (lane & 1);
-                const __nv_bfloat162 two = lane & 1 ? __floats2bfloat162_rn(got, v[2 * i + 1]) : __floats2bfloat162_rn(v[2 * i], got);
-                if (ok && col < cols && row < rows) *reinterpret_cast<__nv_bfloat162*>(dst + (size_t)col * ld + (row & ~1)) = two;
+                const float2 two = lane & 1 ? make_float2(got, v[2 * i + 1]) : make_float2(v[2 * i], got);
+                if (ok && col < cols && row < rows) store_two(dst + (size_t)col * ld + (row & ~1), two);
             }
         };
         // (after a timeout every wait returns at once and nothing is stored, but the pairs of warps still meet at their barriers)
@@ -263,7 +268,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             const Tile at = T.find(tile, seg);
             const bool own = at.e < 0;
             const int rows = own ? a.shared_rows : a.rows;
-            bf16* dst = (own ? a.shared_out : a.out) + (size_t)at.first * rows;
+            bf16* dst = (own ? a.shared_out : (bf16*)a.out) + (size_t)at.first * rows;
             const int buf = n & 1;
             if (!mbar_wait(&acc_full[buf], ((uint32_t)n >> 1) & 1u, status, abort_flag)) ok = false;
             tc_fence_after();
@@ -273,7 +278,9 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
                 for (int c0 = part * 16; c0 < at.count; c0 += 32) {
                     float v[16];
                     tmem_ld16(acc + c0, v);
-                    store16(dst, rows, at.w0 + rank * SPAN + quarter * 32 + lane, rows, c0, at.count, v);
+                    const int row = at.w0 + rank * SPAN + quarter * 32 + lane;
+                    if (a.wide && !own) store16((float*)a.out + (size_t)at.first * rows, rows, row, rows, c0, at.count, v);
+                    else store16(dst, rows, row, rows, c0, at.count, v);
                 }
             } else {
                 const int up = quarter >> 1;  // quarters 0 and 1 hold the gate, 2 and 3 up; each finishes every other 16 columns
@@ -361,19 +368,20 @@ int launch_grouped(const void* x, const void* w, int pairs, const void* sx, cons
 
 }  // namespace
 
-// act [pairs, F] = SwiGLU of the sorted rows xs [pairs, H] under w_gate_up [E, 2F, H], y [pairs, H] = act times w_down [E, H, F]; with
+// act [pairs, F] = SwiGLU of the sorted rows xs [pairs, H] under w_gate_up [E, 2F, H], y [pairs, H] (float32 if `wide`) = act times
+// w_down [E, H, F]; with
 // T > 0 rows h also act_s [T, Fs] and y_s [T, H] of the shared expert (ws_gate_up [2 Fs, H], ws_down [H, Fs]).  H, F and Fs multiples
 // of 8, matrices on 16 bytes, E <= moe_tc_most_experts().  Rows beyond the experts' stretches stay as they are.
 extern "C" int moe_tc_most_experts() { return MAX_EXPERTS; }
 extern "C" int moe_tc_ff(const void* xs, const void* w_gate_up, void* act, const void* w_down, void* y, const int* offsets, int pairs, int E, int H,
-                         int F, const void* h, const void* ws_gate_up, void* act_s, const void* ws_down, void* y_s, int T, int Fs, const int* meta,
-                         int* status, cudaStream_t stream) {
+                         int F, const void* h, const void* ws_gate_up, void* act_s, const void* ws_down, void* y_s, int T, int Fs, int wide,
+                         const int* meta, int* status, cudaStream_t stream) {
     if (pairs <= 0) return 0;
     if (E < 1 || E > MAX_EXPERTS || H <= 0 || F <= 0 || (H | F | Fs) % 8 || (T > 0 && Fs <= 0)) return (int)cudaErrorInvalidValue;
     if (((uintptr_t)xs | (uintptr_t)w_gate_up | (uintptr_t)act | (uintptr_t)w_down | (uintptr_t)y | (uintptr_t)h | (uintptr_t)ws_gate_up |
          (uintptr_t)act_s | (uintptr_t)ws_down | (uintptr_t)y_s) & 15)
         return (int)cudaErrorInvalidValue;
-    const int rc = launch_grouped<1>(xs, w_gate_up, pairs, h, ws_gate_up, {offsets, meta, E, F, H, T, Fs, H, (bf16*)act, (bf16*)act_s}, status, stream);
+    const int rc = launch_grouped<1>(xs, w_gate_up, pairs, h, ws_gate_up, {offsets, meta, E, F, H, T, Fs, H, act, (bf16*)act_s, 0}, status, stream);
     if (rc) return rc;
-    return launch_grouped<0>(act, w_down, pairs, act_s, ws_down, {offsets, meta, E, H, F, T, H, Fs, (bf16*)y, (bf16*)y_s}, status, stream);
+    return launch_grouped<0>(act, w_down, pairs, act_s, ws_down, {offsets, meta, E, H, F, T, H, Fs, y, (bf16*)y_s, wide}, status, stream);
 }

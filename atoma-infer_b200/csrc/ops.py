@@ -1087,6 +1087,7 @@ class CudaOps:
 
     MOE_PAIR_ROWS = 64       # up to this many (token, choice) pairs, bfloat16: a pair at a time
     MOE_TC_ROWS = 65         # from this many pairs on, bfloat16: grouped products on tcgen05
+    MOE_ROUNDED_ROWS = 256   # ... whose results wait for the weighted sum in bfloat16 from this many on, in float32 below
 
     def _moe_on_tcgen05(self, pairs: int, E: int, F: int, *tensors) -> bool:
         """``tensors``: the rows first, then the weights that take part."""
@@ -1132,7 +1133,8 @@ class CudaOps:
             # many pairs: rows gathered in sorted order, then both linears over the experts' stretches (offsets on the device: no
             # host round trip), the shared expert's rows as one more stretch
             xs = torch.empty((pairs, H), dtype=h.dtype, device=dev)
-            y = torch.empty((pairs, H), dtype=h.dtype, device=dev)
+            wide = pairs < self.MOE_ROUNDED_ROWS
+            y = torch.empty((pairs, H), dtype=torch.float32 if wide else h.dtype, device=dev)
             self._check(lib.moe_gather_rows(_p(h), _p(xs), _p(order), _p(offsets[E:]), T, top, H * 2, self._stream()), "moe_gather_rows")
             ws_gate_up, ws_down = shared_weights or (None, None)
             act_s = None
@@ -1141,10 +1143,10 @@ class CudaOps:
                 shared = torch.empty((T, H), dtype=h.dtype, device=dev)
             self._check(self._gemm_library().moe_tc_ff(_p(xs), _p(w_gate_up), _p(act), _p(w_down), _p(y), _p(offsets), pairs, E, H, F, _p(h),
                                                        _p(ws_gate_up), _p(act_s), _p(ws_down), _p(shared) if act_s is not None else None,
-                                                       T if act_s is not None else 0, ws_down.shape[1] if act_s is not None else 0, _p(meta),
-                                                       _p(self.status), self._stream()), "moe_tc_ff")
+                                                       T if act_s is not None else 0, ws_down.shape[1] if act_s is not None else 0, int(wide),
+                                                       _p(meta), _p(self.status), self._stream()), "moe_tc_ff")
             self.launches += 1
-            self._check(lib.moe_combine(_p(y), DT_BF16, _p(place), _p(wts), _p(shared), _p(out), _code(out), _p(meta), T, top, H,
+            self._check(lib.moe_combine(_p(y), _code(y), _p(place), _p(wts), _p(shared), _p(out), _code(out), _p(meta), T, top, H,
                                         self._stream()), "moe_combine")
             return
         y = torch.empty((pairs, H), dtype=torch.float32, device=dev)

@@ -69,3 +69,25 @@ def test_a_choice_that_names_no_expert_adds_nothing(rt, T):
 
     bad = (ids < 0) | (ids >= E)
     assert torch.equal(run(ids, wts), run(ids.masked_fill(bad, 0), wts.masked_fill(bad.to(rt.device), 0.0)))
+
+
+@pytest.mark.parametrize("T,shared", [(33, False), (127, True)])
+def test_results_of_up_to_255_pairs_are_summed_in_float32(rt, T, shared):
+    """The second expert takes back all but a 64th of what the first one adds: a result rounded to bfloat16 before the weighted sum would
+    put 2^-9 of the whole into the rest."""
+    H, F, g = 136, 72, torch.Generator().manual_seed(T)
+
+    def draw(*shape, std=1.0):
+        return (torch.randn(*shape, generator=g) * std).bfloat16().to(rt.device)
+
+    h, gu, down = draw(T, H), draw(1, 2 * F, H, std=H ** -0.5).repeat(2, 1, 1), draw(2, H, F, std=F ** -0.5)
+    down[1] = (-down[0].float() * (1 + torch.randn(H, F, generator=g).to(rt.device) / 64)).bfloat16()
+    weights = (torch.zeros_like(gu[0]), torch.zeros_like(down[0])) if shared else None
+    ids = torch.tensor([[0, 1]]).repeat(T, 1).int().to(rt.device)
+    out, meta = torch.empty_like(h), K.make_context(rt, [(0, T)], 16, [[1] * (-(-T // 16))])[0].meta
+    rt.ops.moe_experts(h, ids, torch.ones(T, 2, device=rt.device), gu, down, None, out, meta, **({"shared_weights": weights} if shared else {}))
+    rt.ops.check_status()
+    a, b = (h.double() @ gu[0].double().T).chunk(2, -1)
+    want = (a * torch.sigmoid(a) * b) @ (down[0].double() + down[1].double()).T
+    # the activation and the sum are rounded to bfloat16 (2^-9 each at most); float32 sums of results 64 times as large: 64 * 1e-6
+    assert float((out.double() - want).norm() / want.norm()) < 2 * 2.0 ** -9 + 1e-4
