@@ -31,10 +31,12 @@
 namespace {
 
 constexpr int MAX_CHUNK = 256;  // rows of x in a tile at most
-constexpr int W_BYTES = BM * BK * 2, X_BYTES = MAX_CHUNK / 2 * BK * 2, STAGE_BYTES = W_BYTES + X_BYTES, STAGES = 6;
+constexpr int W_BYTES = BM * BK * 2, X_BYTES = MAX_CHUNK / 2 * BK * 2, STAGE_BYTES = W_BYTES + X_BYTES;
 constexpr int STORE_WARPS = 8, THREADS = 64 + 32 * STORE_WARPS;  // (four: the last tiles' stores took 3 us more of a launch)
 constexpr int SWAP_FLOATS = STORE_WARPS * 16 * 32;  // 16 columns of a warp's lanes
-constexpr int MAX_EXPERTS = 1024;
+// Six stages, or four where a count for every expert would not fit beside them (three cost 8 % of a launch's time); MAX_EXPERTS is what
+// the sort by expert takes, too.
+constexpr int STAGES_FEW = 6, STAGES_MANY = 4, FEW_EXPERTS = 1024, MAX_EXPERTS = 12287;
 
 // ---- pairs of blocks
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -130,7 +132,7 @@ struct Tiles {
 
 struct RowMaps { CUtensorMap box[4]; };  // 16, 32, 64 and 128 rows in a copy
 
-template <int MODE>
+template <int MODE, int STAGES>
 __global__ void __launch_bounds__(THREADS, 1)
 moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ RowMaps map_x, const __grid_constant__ CUtensorMap map_sw,
                       const __grid_constant__ RowMaps map_sx, const GroupedArgs a, int* __restrict__ status) {
@@ -333,7 +335,7 @@ bool make_row_maps(RowMaps* maps, const void* x, int rows, int K) {
     return true;
 }
 
-template <int MODE>
+template <int MODE, int STAGES>
 int launch_grouped(const void* x, const void* w, int pairs, const void* sx, const void* sw, const GroupedArgs& a, int* status, cudaStream_t stream) {
     CUtensorMap mw, msw;
     RowMaps mx, msx;
@@ -347,7 +349,7 @@ int launch_grouped(const void* x, const void* w, int pairs, const void* sx, cons
     const size_t smem = STAGES * STAGE_BYTES + SWAP_FLOATS * 4 + (2 * STAGES + 4) * 8 + 8 + (a.experts + 2) * 4 + 1024;
     static size_t configured = 0;
     if (smem > configured) {
-        const cudaError_t e = cudaFuncSetAttribute(moe_grouped_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = cudaFuncSetAttribute(moe_grouped_tc_kernel<MODE, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         configured = smem;
     }
@@ -363,7 +365,7 @@ int launch_grouped(const void* x, const void* w, int pairs, const void* sx, cons
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = (g_use_pdl & 1) ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, moe_grouped_tc_kernel<MODE>, mw, mx, msw, msx, a, status);
+    return (int)cudaLaunchKernelEx(&cfg, moe_grouped_tc_kernel<MODE, STAGES>, mw, mx, msw, msx, a, status);
 }
 
 }  // namespace
@@ -381,7 +383,11 @@ extern "C" int moe_tc_ff(const void* xs, const void* w_gate_up, void* act, const
     if (((uintptr_t)xs | (uintptr_t)w_gate_up | (uintptr_t)act | (uintptr_t)w_down | (uintptr_t)y | (uintptr_t)h | (uintptr_t)ws_gate_up |
          (uintptr_t)act_s | (uintptr_t)ws_down | (uintptr_t)y_s) & 15)
         return (int)cudaErrorInvalidValue;
-    const int rc = launch_grouped<1>(xs, w_gate_up, pairs, h, ws_gate_up, {offsets, meta, E, F, H, T, Fs, H, act, (bf16*)act_s, 0}, status, stream);
+    const GroupedArgs first{offsets, meta, E, F, H, T, Fs, H, act, (bf16*)act_s, 0}, second{offsets, meta, E, H, F, T, H, Fs, y, (bf16*)y_s, wide};
+    const bool few = E <= FEW_EXPERTS;
+    const int rc = few ? launch_grouped<1, STAGES_FEW>(xs, w_gate_up, pairs, h, ws_gate_up, first, status, stream)
+                       : launch_grouped<1, STAGES_MANY>(xs, w_gate_up, pairs, h, ws_gate_up, first, status, stream);
     if (rc) return rc;
-    return launch_grouped<0>(act, w_down, pairs, act_s, ws_down, {offsets, meta, E, H, F, T, H, Fs, y, (bf16*)y_s, wide}, status, stream);
+    return few ? launch_grouped<0, STAGES_FEW>(act, w_down, pairs, act_s, ws_down, second, status, stream)
+               : launch_grouped<0, STAGES_MANY>(act, w_down, pairs, act_s, ws_down, second, status, stream);
 }

@@ -91,3 +91,20 @@ def test_results_of_up_to_255_pairs_are_summed_in_float32(rt, T, shared):
     want = (a * torch.sigmoid(a) * b) @ (down[0].double() + down[1].double()).T
     # the activation and the sum are rounded to bfloat16 (2^-9 each at most); float32 sums of results 64 times as large: 64 * 1e-6
     assert float((out.double() - want).norm() / want.norm()) < 2 * 2.0 ** -9 + 1e-4
+
+
+@pytest.mark.parametrize("E", [1024, 1025, 12287])
+def test_very_many_experts(rt, E):
+    """The counts of all experts wait in shared memory beside the stages, of which there are fewer then."""
+    T, top, H, F, g = 150, 2, 64, 8, torch.Generator().manual_seed(E)
+    ids = torch.randint(0, E, (T, top), generator=g, dtype=torch.int32)
+    ids[:70, 0], ids[70:, 1], ids[:70, 1] = 0, E - 1, 1
+    h, gu, down = (torch.randn(*s, generator=g).bfloat16().to(rt.device) for s in ((T, H), (E, 2 * F, H), (E, H, F)))
+    ids, wts = ids.to(rt.device), torch.rand(T, top, generator=g).to(rt.device)
+    assert rt.ops._moe_on_tcgen05(T * top, E, F, h, gu, down)
+    out, meta = torch.full_like(h, float("nan")), K.make_context(rt, [(0, T)], 16, [[1] * (-(-T // 16))])[0].meta
+    rt.ops.moe_experts(h, ids, wts, gu, down, None, out, meta)
+    rt.ops.check_status()
+    a, b = torch.einsum("td,tkfd->tkf", h.double(), gu[ids.long()].double()).chunk(2, -1)
+    want = torch.einsum("tk,tkf,tkdf->td", wts.double(), a * torch.sigmoid(a) * b, down[ids.long()].double())
+    assert float((out.double() - want).norm() / want.norm()) < 3 * 2.0 ** -9
