@@ -163,8 +163,7 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
     }
-    pdl_launch_dependents();
-    pdl_wait();
+    pdl_launch_dependents();  // (these launches start when the one ahead has drained; the weighted sum behind them starts early: 1 us)
     if (warp == 2) {
         int upto = 0;
         for (int s0 = 0; s0 < T.segments(); s0 += 32) {
@@ -358,13 +357,11 @@ int launch_grouped(const void* x, const void* w, int pairs, const void* sx, cons
     cfg.blockDim = dim3(THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = (g_use_pdl & 1) ? 2 : 1;
+    cfg.numAttrs = 1;
     return (int)cudaLaunchKernelEx(&cfg, moe_grouped_tc_kernel<MODE, STAGES>, mw, mx, msw, msx, a, status);
 }
 

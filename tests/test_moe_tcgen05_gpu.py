@@ -41,6 +41,7 @@ def test_experts(rt, H, F, Fs, counts, top):
         want += expert(h, *weights)
         assert rt.ops.moe_takes_shared(h, top, gu, down, *weights)
     meta = K.make_context(rt, [(0, T)], 16, [[1] * (-(-T // 16))])[0].meta
+    assert rt.ops._moe_on_tcgen05(pairs, E, F, h, gu, down)  # (not the tile kernel for few rows)
     out = torch.full((T, H), float("nan"), dtype=rt.dtype, device=rt.device)
     rt.ops.moe_experts(h, ids, wts, gu, down, None, out, meta, **({"shared_weights": weights} if Fs else {}))
     rt.ops.check_status()
@@ -108,3 +109,31 @@ def test_very_many_experts(rt, E):
     a, b = torch.einsum("td,tkfd->tkf", h.double(), gu[ids.long()].double()).chunk(2, -1)
     want = torch.einsum("tk,tkf,tkdf->td", wts.double(), a * torch.sigmoid(a) * b, down[ids.long()].double())
     assert float((out.double() - want).norm() / want.norm()) < 3 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("T", [90, 300])
+def test_rows_that_are_no_numbers_and_rows_beyond_the_step(rt, T):
+    """Rows that hold an infinity or a NaN beside other experts' and their own expert's rows, in a step whose last ten rows are
+    padding (the launch is sized for them, the step's metadata is not): every other row comes out to the bit as without them."""
+    E, top, H, F, g = 4, 2, 72, 40, torch.Generator().manual_seed(T)
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).int().to(rt.device)
+    h, gu, down = (torch.randn(*s, generator=g).bfloat16().to(rt.device) for s in ((T, H), (E, 2 * F, H), (E, H, F)))
+    weights, wts = (gu[0] * 0.5, down[0] * 0.5), torch.rand(T, top, generator=g).to(rt.device)
+    real = T - 10
+    meta = K.make_context(rt, [(0, real)], 16, [[1] * (-(-T // 16))])[0].meta
+
+    def run(h, ids):
+        out = torch.full((T, H), 7.0, dtype=rt.dtype, device=rt.device)
+        rt.ops.moe_experts(h, ids, wts, gu, down, None, out, meta, shared_weights=weights)
+        rt.ops.check_status()
+        return out
+
+    want = run(h, ids)
+    odd, odd_ids = h.clone(), ids.clone()
+    odd[3, 5], odd[17], odd[40, 1], odd[real:] = float("inf"), float("nan"), float("-inf"), float("nan")
+    odd_ids[real:] = 1 << 30  # what stands behind the step's rows is never looked at
+    got = run(odd, odd_ids)
+    rest = [t for t in range(real) if t not in (3, 17, 40)]
+    assert torch.equal(got[rest], want[rest]) and bool(torch.isfinite(got[rest]).all())
+    assert bool(got[17].isnan().all()) and not bool(torch.isfinite(got[[3, 40]]).all(1).any())
+    assert bool((got[real:] == 7.0).all())
