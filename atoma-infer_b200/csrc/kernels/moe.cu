@@ -443,10 +443,9 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, cons
             for (int k = 0; k < top; ++k) {
                 const long long row = place ? (long long)place[(size_t)t * top + k] : (long long)t * top + k;
                 const float weight = wts[(size_t)t * top + k];
-                if (row < 0) continue;
-                load4(y + row * H + i, v);
+                load4(y + max(row, 0ll) * H + i, v);  // (a load for every choice: a branch here would put them one behind the other)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[j] = fmaf(weight, v[j], acc[j]);
+                for (int j = 0; j < 4; ++j) acc[j] = row < 0 ? acc[j] : fmaf(weight, v[j], acc[j]);
             }
             if (shared) {
                 load4(shared + (size_t)t * H + i, v);
@@ -581,9 +580,9 @@ moe_gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, cons
                        const int* __restrict__ sorted, int top, int chunks) {
     pdl_launch_dependents();
     pdl_wait();
-    const int i = blockIdx.x;
+    const int i = blockIdx.x, pair = order[i];  // (both loads at once; what `order` holds behind the last stretch is not used)
     if (i >= *sorted) return;
-    const uint4* src = x + (size_t)(order[i] / top) * chunks;
+    const uint4* src = x + (size_t)(pair / top) * chunks;
     for (int c = threadIdx.x; c < chunks; c += blockDim.x) xs[(size_t)i * chunks + c] = src[c];
 }
 
