@@ -769,11 +769,13 @@ extern "C" int ssm_token_step(const void* u, long long u_stride, const void* z, 
                               const int* meta, const int* positions, const int* cu_tokens, const int* slots, int S, int heads, int P, int N, int groups,
                               int taps, cudaStream_t stream) {
     if (S <= 0) return 0;
-    if (!ssm_token_step_takes(ring, state, slot_stride, S, heads, P, N, groups, parts, taps)) return (int)cudaErrorInvalidValue;
+    int R = 0, NPT = 0;
+    if (!ssm_token_step_takes(ring, state, slot_stride, S, heads, P, N, groups, parts, taps) || !scan_geometry(N, P, &R, &NPT))
+        return (int)cudaErrorInvalidValue;
 #define TOKEN_CASE(T)                                                                                                      \
     return ssm_token_run<T>({(const T*)u, (const T*)dt, u_stride, dt_stride, conv_w, conv_b, ring, ring_stride, dt_bias, a_log, d_skip, state, \
-                             slot_stride, y, meta, positions, cu_tokens, slots, heads, N, groups, taps}, S, P, (const T*)z, z_stride, norm_w, parts, \
-                            eps, ring, (T*)out, stream)
+                             slot_stride, y, meta, positions, cu_tokens, slots, heads, N, groups, taps, R, NPT}, S, P, (const T*)z, z_stride, norm_w, \
+                            parts, eps, ring, (T*)out, stream)
     if (dtype == DT_F32) TOKEN_CASE(float);
     TOKEN_CASE(__nv_bfloat16);
 #undef TOKEN_CASE

@@ -3,6 +3,9 @@
 // the head's matrix in registers, four neighbouring columns of every RG-th row a thread, and takes the head's columns of x and the group's B
 // and C through the convolution itself.  The heads of a group share B and C, so nobody may change the ring while another block may still
 // read it: the gated norm's launch, the next one, writes the new row (ring_row).
+// In float32 the sum over a column's rows is taken in the scan's own order (ssm_scan_kernel: R shares of NPT rows, each in order, then by
+// halving) from a copy of the new matrix in shared memory: a request's bits do not depend on how many others bring a token, which is
+// what chooses this kernel.  In bfloat16 a thread sums the rows that it keeps.
 // Bound by fixed cost for few entries and by the state's bytes for many.  The state is asked into the L2 before the wait for the
 // linear ahead: a hint, so it may run before that state's last writer has finished.
 // Measured, a whole layer (both linears too) of width 2,048 (64 heads of 128 x 64), us, in brackets the three kernels: 1 request 22.7 (26.8), 4
@@ -27,13 +30,15 @@ struct SsmToken {
     float* y;                                    // [T, heads * P]
     const int *meta, *positions, *cu_tokens, *slots;
     int heads, N, groups, taps;
+    int R, NPT;                                  // float32: the scan's shares of a column (R * P at most 512)
 };
 
 template <typename T, int PQ>
 __global__ void __launch_bounds__(256)
 ssm_token_kernel(const __grid_constant__ SsmToken<T> A) {
     constexpr int P = PQ * 4, RG = 256 / PQ, MAX_N = RG * TOKEN_ROWS, ITEMS = (P + 2 * MAX_N + 255) / 256;
-    __shared__ __align__(16) float xs[P], part[8][P], bc[2 * MAX_N];
+    constexpr bool IN_ORDER = sizeof(T) == 4;
+    __shared__ __align__(16) float xs[P], part[IN_ORDER ? 512 / P : 8][P], bc[2 * MAX_N], mat[IN_ORDER ? MAX_N * P : 4];
     const int h = blockIdx.x, e = blockIdx.y, g = h / (A.heads / A.groups), tid = threadIdx.x, N = A.N;
     const int inner = A.heads * P, channels = inner + 2 * A.groups * N, R = A.taps - 1;
     if (e >= A.meta[META_NUM_ENTRIES]) return;
@@ -97,7 +102,31 @@ ssm_token_kernel(const __grid_constant__ SsmToken<T> A) {
         s[i].x = fmaf(dec, s[i].x, bn * dx.x), s[i].y = fmaf(dec, s[i].y, bn * dx.y);
         s[i].z = fmaf(dec, s[i].z, bn * dx.z), s[i].w = fmaf(dec, s[i].w, bn * dx.w);
         *reinterpret_cast<float4*>(S + (size_t)n * P + q * 4) = s[i];
+        if (IN_ORDER) {
+            *reinterpret_cast<float4*>(mat + n * P + q * 4) = s[i];
+            continue;
+        }
         y.x = fmaf(s[i].x, cn, y.x), y.y = fmaf(s[i].y, cn, y.y), y.z = fmaf(s[i].z, cn, y.z), y.w = fmaf(s[i].w, cn, y.w);
+    }
+    if (IN_ORDER) {
+        __syncthreads();
+        for (int i = tid; i < A.R * P; i += 256) {
+            const int col = i % P, r = i / P;
+            float v = 0.f;
+#pragma unroll 8
+            for (int j = 0; j < A.NPT; ++j) {
+                const int n = r * A.NPT + j;
+                if (n < N) v = fmaf(mat[n * P + col], bc[N + n], v);
+            }
+            part[r][col] = v;
+        }
+        __syncthreads();
+        if (tid < P) {
+            for (int o = A.R >> 1; o > 0; o >>= 1)
+                for (int r = 0; r < o; ++r) part[r][tid] += part[r + o][tid];
+            A.y[(size_t)t * inner + h * P + tid] = fmaf(dskip, xs[tid], part[0][tid]);
+        }
+        return;
     }
 #pragma unroll
     for (int o = PQ; o < 32; o <<= 1) {

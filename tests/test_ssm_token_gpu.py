@@ -68,3 +68,41 @@ def test_other_steps_are_left_alone():
 
     assert takes([(3, 1), (4, 1)])
     assert not takes([(0, 2), (4, 1)]) and not takes([(3, 1)], norm_groups=3)
+
+
+@pytest.mark.parametrize("heads,P,N,G", [(64, 64, 128, 8), (64, 32, 100, 4), (48, 128, 64, 3), (64, 64, 20, 1)])
+def test_float32_bits_do_not_depend_on_the_other_requests(heads, P, N, G):
+    """A request's token alone, among others at the two sides of where the step stops being taken, and beside a prompt: the layer's
+    output and state are the same to the bit."""
+    from atoma_infer_b200.engine.runtime import make_runtime
+    from atoma_infer_b200.parts.ssm import Mamba2Mixer
+    from atoma_infer_b200.cache.spec import LayerCache
+
+    rt = make_runtime("float32", "cuda:0")
+    g, dev, H, taps = torch.Generator().manual_seed(P + N), rt.device, 192, 4
+    inner, ch = heads * P, heads * P + 2 * G * N
+
+    def f(*shape, std=1.0, mean=0.0):
+        return (torch.randn(*shape, generator=g) * std + mean).to(dev)
+
+    part = Mamba2Mixer({"hidden": H, "heads": heads, "head_dim": P, "state": N, "groups": G, "taps": taps, "norm_groups": G, "eps": 1e-5}, "p")
+    part.bind({"p.in": f(inner + ch + heads, H, std=H ** -0.5), "p.conv": f(ch, taps, std=0.3), "p.conv.b": f(ch, std=0.1),
+               "p.dt_bias": f(heads, mean=-3), "p.A_log": f(heads, std=0.5), "p.D": f(heads), "p.norm": f(inner, std=0.1, mean=1),
+               "p.o": f(H, inner, std=inner ** -0.5)}, rt)
+    most = 14 * rt.ops.num_sms // heads  # (more than any limit of the rule)
+    x, kept = f(most + 3, H), f(most + 3, part.state_bytes() // 4, std=0.5)
+
+    def run(lens):
+        """Requests of one token each (row i of x for request i), the last one of lens[-1] tokens."""
+        ctx, _ = K.make_context(rt, [(50 + i, n) for i, n in enumerate(lens)], 16, [[1 + i] * 32 for i in range(len(lens))])
+        state = kept[:len(lens)].clone()
+        rows = torch.cat([x[:len(lens) - 1], x[len(lens) - 1:len(lens)].repeat(lens[-1], 1)])
+        cache = LayerCache(group=-1, pages=None, num_pages=0, page_size=16, writes=False, state=state.view(torch.uint8))
+        y = part.forward(rows, ctx, cache)
+        rt.ops.check_status()
+        return y, state
+
+    want_y, want_state = run([1])
+    for lens in ([1] * 2, [1] * 9, [1] * most, [1] * (most + 1), [1] * (most + 3), [1, 1, 40]):
+        y, state = run(lens)
+        assert torch.equal(y[0], want_y[0]) and torch.equal(state[0], want_state[0]), len(lens)
