@@ -741,12 +741,11 @@ extern "C" int gated_group_norm(const float* y, const void* z, int dtype, long l
 }
 
 // Convolution, recurrence and gated norm of a step whose entries bring a token each, in two launches (ssm_token.cuh); y: S rows of
-// scratch.  ssm_token_step_takes: whether these sizes and addresses are served (and steps small enough to gain by it, with a norm that takes
-// a block a part).
+// scratch.  ssm_token_step_takes: whether these sizes and addresses are served (and the norm is one that takes a block a part).
 extern "C" int ssm_token_step_takes(const float* ring, const float* state, long long slot_stride, int S, int heads, int P, int N, int groups, int parts,
                                     int taps) {
     return ssm_token_takes(heads, P, N, groups, taps) && (taps == 1 || ring) && slot_stride % 4 == 0 && ((uintptr_t)state & 15) == 0 && parts > 0 &&
-           heads * P % parts == 0 && (long)S * heads <= TOKEN_BLOCKS * multiprocessors() && (long)S * parts < 8 * multiprocessors();
+           heads * P % parts == 0 && (long)S * parts < 8 * multiprocessors();
 }
 
 template <typename T>

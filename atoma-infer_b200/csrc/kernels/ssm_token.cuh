@@ -10,12 +10,11 @@
 // linear ahead: a hint, so it may run before that state's last writer has finished.
 // Measured, a whole layer (both linears too) of width 2,048 (64 heads of 128 x 64), us, in brackets the three kernels: 1 request 22.7 (26.8), 4
 // 24.6 (27.0), 16 34.9 (39.0), 40 67.6 (68.5), 64 89.5 (85.9); width 4,096 (128 heads) 1 47.5 (53.1), 16 73.7 (77.9), 40 136 (130).  With many
-// blocks the convolution of B and C, which every head repeats, costs more than the launch: TOKEN_BLOCKS a multiprocessor are the most.
+// blocks the convolution of B and C, which every head repeats, costs more than the launch; how many are worth it is the caller's rule.
 #pragma once
 #include "common.cuh"
 
 #define TOKEN_ROWS 8     // rows of the state a thread keeps
-#define TOKEN_BLOCKS 14
 
 template <typename T>
 struct SsmToken {

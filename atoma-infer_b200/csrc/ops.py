@@ -807,6 +807,8 @@ class CudaOps:
             return False
         (up, us), (zp, zs), (dp, ds) = (self._rows(t, "ssm_token_step") for t in (u, z, dt))
         lib, taps, (heads, N, P) = self._mixers(), conv_w.shape[0], state.shape[1:]
+        if ctx.S * heads > self._token_step_blocks(u.dtype, N, P) * self.num_sms:
+            return False
         ss = ctypes.c_longlong(state.stride(0))
         if not lib.ssm_token_step_takes(_p(ring), _p(state), ss, ctx.S, heads, P, N, groups, norm_groups, taps):
             return False
@@ -817,6 +819,23 @@ class CudaOps:
                     "ssm_token_step")
         self.launches += 1
         return True
+
+    @staticmethod
+    def _token_step_blocks(dtype, N: int, P: int) -> int:
+        """How many (request, head) blocks a multiprocessor ``ssm_token_step`` is worth: every block takes B and C through the convolution
+        again, which a large state hides and a small one does not, more so with few columns (more items a thread); float32 sums
+        once more from shared memory.  Measured, us, two launches / three, N x P at blocks a multiprocessor: bfloat16 128 x 64 13.8
+        28.4 / 31.4, 96 x 64 13.8 23.5 / 26.0, 64 x 64 5.2 11.2 / 12.3, 10.4 17.6 / 17.8, 13.8 21.4 / 19.0, 32 x 64 3.5 9.3 / 9.6, 5.2
+        10.6 / 10.2, 64 x 128 13.8 25.5 / 31.0, 32 x 128 13.8 20.2 / 22.8, 16 x 128 5.2 10.6 / 11.1, 7.8 13.5 / 12.2, 128 x 32 1.7 7.8 /
+        11.0, 3.5 11.9 / 11.4, 16 x 32 3.5 9.8 / 8.9; float32 128 x 64 2.6 9.7 / 12.2, 3.9 14.5 / 13.4, 64 x 64 2.6 7.9 / 10.6, 3.5 11.0
+        / 10.9, 64 x 128 13.8 29.2 / 30.7, 16 x 128 2.6 7.6 / 9.7, 7.8 13.9 / 13.5, 256 x 32 1.7 9.1 / 11.4, 2.6 14.5 / 12.3."""
+        if P < 64:
+            return 2
+        if dtype == torch.float32 and P < 128:
+            return 3
+        if N * P >= (6144 if P < 128 else 4096):
+            return 14
+        return 6 if N * P >= 4096 else 3
 
     def rms_rows(self, x, w, eps: float, out, meta):
         """out = x * rsqrt(mean(x^2) + eps) * w row by row; ``x`` a slice of wider rows, ``w`` float32."""

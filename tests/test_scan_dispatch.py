@@ -39,3 +39,21 @@ def test_prompts_with_a_decay_per_row_beside_many_single_tokens_go_in_order(sing
     lib = SimpleNamespace(gla_row_scan_head_floats=lambda *args: 64, gla_scan_scratch_floats=lambda *args: 0)
     rows = CudaOps._row_scan(ops, lib, "gla", (), torch.empty(0, dtype=torch.bfloat16), ctx, torch.empty(1), 4, 64, 64, 64, 2)
     assert (rows is None) == (singles > 126)
+
+
+@pytest.mark.parametrize("dtype,N,P,blocks", [("bfloat16", 128, 64, 14), ("bfloat16", 96, 64, 14), ("bfloat16", 64, 64, 6), ("bfloat16", 16, 64, 3),
+                                              ("bfloat16", 32, 128, 14), ("bfloat16", 16, 128, 3), ("bfloat16", 256, 32, 2),
+                                              ("float32", 128, 64, 3), ("float32", 64, 128, 14), ("float32", 31, 128, 3), ("float32", 16, 32, 2)])
+def test_decode_steps_of_the_state_space_mixer_in_two_launches(dtype, N, P, blocks):
+    """Up to so many heads of all requests a multiprocessor; beyond, the call is refused before anything is launched."""
+    sms, heads = 148, 4
+    taken = []
+    ops = SimpleNamespace(num_sms=sms, _token_step_blocks=CudaOps._token_step_blocks, _rows=lambda t, what: (None, 0), launches=0,
+                          _mixers=lambda: SimpleNamespace(ssm_token_step_takes=lambda *args: taken.append(args) or 0))
+    for S, takes in ((1, True), (blocks * sms // heads, True), (blocks * sms // heads + 1, False)):
+        taken.clear()
+        state = torch.empty(1, heads, N, P).expand(S, heads, N, P)
+        u = torch.empty(S, 8, dtype=getattr(torch, dtype))
+        ctx = SimpleNamespace(decode_only=True, T=S, S=S)
+        CudaOps.ssm_token_step(ops, u, u, u, torch.empty(4, 8), None, None, None, None, None, state, None, 1, 1, 1e-5, ctx, u)
+        assert bool(taken) == takes
