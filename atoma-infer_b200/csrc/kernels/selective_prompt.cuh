@@ -97,7 +97,7 @@ selective_prompt_kernel(const T* __restrict__ u, long long u_stride, const float
     if (count <= 0) return;
     float* slot_state = state + (size_t)slots[e] * slot_stride;
 
-    // ---- what warps 4..7 do (ht: thread of them)
+    // ---- what the other sixteen warps do (ht: thread of them)
     const int ht = scans ? 0 : tid - SP_SCAN;
     // This thread's 16-byte copies of a tile: what from, to where in the first tile's place, how far on the next tile and place are.
     constexpr int DT = SP_TT * SP_CH / 4, ROWS = SP_TT * SP_CH / PER16, COPIES = (DT + 2 * ROWS + SP_TT * 2 * SP_N / PER16 + SP_HELP - 1) / SP_HELP;
@@ -175,7 +175,7 @@ selective_prompt_kernel(const T* __restrict__ u, long long u_stride, const float
         T* dst = out + (size_t)(first + t) * inner + c0 + pc;
         sp_store(dst, y);
     };
-    auto copies_done = [&]() {  // this thread's copies but the last two groups, then the other threads' of warps 4..7
+    auto copies_done = [&]() {  // this thread's copies but the last two groups, then those of the other threads that copy
         asm volatile("cp.async.wait_group 2;" ::: "memory");
         asm volatile("bar.sync 1, %0;" ::"n"(SP_HELP) : "memory");
     };
@@ -194,6 +194,9 @@ selective_prompt_kernel(const T* __restrict__ u, long long u_stride, const float
         }
         A2[0] = make_float2(a[0], a[1]), A2[1] = make_float2(a[2], a[3]);
         S[0] = make_float2(s[0], s[1]), S[1] = make_float2(s[2], s[3]);
+        // states beyond N take no part (an infinite input would make a NaN of their zeros): their share of the sum is 0
+        if (n0 >= N)
+            for (int i = cl; i < 2 * SP_TT * SP_CH; i += 32) sm.y[i / (SP_TT * SP_CH)][r][i / SP_CH % SP_TT][i % SP_CH] = 0.f;
     } else {
 #pragma unroll
         for (int i = 0; i < SP_W; ++i) {
@@ -209,7 +212,7 @@ selective_prompt_kernel(const T* __restrict__ u, long long u_stride, const float
 
     for (int tile = 0; tile < tiles; ++tile) {
         const int buf = tile & 1;
-        if (scans) {
+        if (scans && n0 < N) {
             const int nt = min(SP_TT, count - tile * SP_TT);
             const float2* steps = &sm.step[buf][0][cl];
             const float* bs = &sm.b[buf][0][n0];
@@ -252,7 +255,7 @@ selective_prompt_kernel(const T* __restrict__ u, long long u_stride, const float
                     take(k, t);
                 }
             }
-        } else {
+        } else if (!scans) {
             finish(tile - 1);
             copy(tile + 3);
             copies_done();
