@@ -1065,7 +1065,7 @@ class CudaOps:
             raise KernelError("selective_scan: step sizes are contiguous float32, the output has the inputs' type")
         (up, us), (bp, bs), (zp, zs) = (self._rows(t, "selective_scan") for t in (u, bc, zg))
         rows = (up, us, _p(dt_raw))
-        if self._selective_in_order(ctx, inner) and lib.selective_scan_prompt_takes(*rows, bp, bs, zp, zs, _code(u), _p(out), inner, nstate):
+        if self._selective_in_order(ctx, inner, u.dtype) and lib.selective_scan_prompt_takes(*rows, bp, bs, zp, zs, _code(u), _p(out), inner, nstate):
             self._check(lib.selective_scan_prompt(*rows, _p(dt_bias), bp, bs, zp, zs, _code(u), _p(a_log), _p(d_skip), _p(state), slot_stride,
                                                   _p(out), _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, inner, nstate,
                                                   self._stream()), "selective_scan")
@@ -1079,7 +1079,7 @@ class CudaOps:
         if chunk:
             self.launches += 2
 
-    def _selective_in_order(self, ctx, inner: int) -> bool:
+    def _selective_in_order(self, ctx, inner: int, dtype) -> bool:
         """Whether a step's selective scan runs in one pass (kernels/selective_prompt.cuh): where its estimated time is the shorter
         one.  It takes 0.04 us a token of the longest entry, or, with more blocks of 32 channels than multiprocessors, their share
         of all tokens and 2.2 us an entry; the scan cut in chunks of time 48 us and two passes over everything, the one in order
@@ -1089,8 +1089,8 @@ class CudaOps:
         longest = ctx.max_tokens_per_entry
         if self.selective_prompt is not None:
             return self.selective_prompt
-        if longest < 16:
-            return False
+        if longest < 16 or (dtype == torch.float32 and longest < self.SCAN_CHUNK_FROM):
+            return False  # (float32 below the chunks of time: a token's sum has one order, whatever else the step brings)
         share, work = -(-inner // 32) / self.num_sms, ctx.T * inner
         one_pass = 4.0 + max(0.0405 * longest, share * (2.2 * ctx.S + 0.0405 * ctx.T))
         other = 48.0 + 1.35e-5 * work if longest >= self.SCAN_CHUNK_FROM else 6.0 + max(0.4 * longest, 1.1e-5 * work)

@@ -57,3 +57,13 @@ def test_decode_steps_of_the_state_space_mixer_in_two_launches(dtype, N, P, bloc
         ctx = SimpleNamespace(decode_only=True, T=S, S=S)
         CudaOps.ssm_token_step(ops, u, u, u, torch.empty(4, 8), None, None, None, None, None, state, None, 1, 1, 1e-5, ctx, u)
         assert bool(taken) == takes
+
+
+@pytest.mark.parametrize("dtype,longest,one_pass", [("bfloat16", 15, False), ("bfloat16", 16, True), ("bfloat16", 127, True),
+                                                    ("float32", 16, False), ("float32", 127, False), ("float32", 128, True), ("float32", 2048, True)])
+def test_selective_scans_of_float32_go_in_order_below_the_chunks_of_time(dtype, longest, one_pass):
+    """The one pass sums a token's states in another order, and it is chosen by the whole step: where chunks of time are not, a float32
+    request must not see what else the step brings."""
+    ops = SimpleNamespace(selective_prompt=None, num_sms=148, SCAN_CHUNK_FROM=CudaOps.SCAN_CHUNK_FROM)
+    ctx = SimpleNamespace(T=longest, S=1, max_tokens_per_entry=longest)
+    assert CudaOps._selective_in_order(ops, ctx, 4096, getattr(torch, dtype)) == one_pass

@@ -86,3 +86,24 @@ def test_what_is_not_finite_reaches_what_it_reaches_in_order(dtype, N, one_sign)
     for new, old in zip(*results):
         assert torch.equal(new.isnan(), old.isnan())
         assert torch.equal(new.isinf(), old.isinf()) and torch.equal(new[new.isinf()], old[old.isinf()])
+
+
+def test_float32_bits_do_not_depend_on_the_other_requests():
+    """A request's 40 tokens alone and beside so many others that another kernel would be the shorter way."""
+    rt = make_runtime("float32", "cuda:0")
+    g = torch.Generator().manual_seed(3)
+    C, N, n = 4096, 16, 40
+    a_log, d_skip, dt_bias = (torch.randn(*s, generator=g).to(rt.device) for s in ((C, N), (C,), (C,)))
+    lens = [n] + [1, 30, 64, 2] * 10
+    T = sum(lens)
+    row, dt = torch.randn(T, 2 * C + 2 * N, generator=g).to(rt.device), torch.randn(T, C, generator=g).to(rt.device)
+
+    def run(lens):
+        t = sum(lens)
+        state, out = torch.zeros((len(lens), C, N), device=rt.device), torch.empty((t, C), device=rt.device)
+        ctx = _context(rt, [(i, 0, m) for i, m in enumerate(lens)], list(range(len(lens))))
+        rt.ops.selective_scan(row[:t, :C], dt[:t], dt_bias, row[:t, 2 * C:], row[:t, C:2 * C], a_log, d_skip, state, ctx, out, inner=C, nstate=N)
+        return out[:n], state[0]
+
+    for alone, beside in zip(run([n]), run(lens)):
+        assert torch.equal(alone, beside)
