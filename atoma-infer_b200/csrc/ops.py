@@ -1065,7 +1065,7 @@ class CudaOps:
             raise KernelError("selective_scan: step sizes are contiguous float32, the output has the inputs' type")
         (up, us), (bp, bs), (zp, zs) = (self._rows(t, "selective_scan") for t in (u, bc, zg))
         rows = (up, us, _p(dt_raw))
-        if self._selective_in_order(ctx, inner, u.dtype) and lib.selective_scan_prompt_takes(*rows, bp, bs, zp, zs, _code(u), _p(out), inner, nstate):
+        if self._selective_in_order(ctx, inner, nstate, u.dtype) and lib.selective_scan_prompt_takes(*rows, bp, bs, zp, zs, _code(u), _p(out), inner, nstate):
             self._check(lib.selective_scan_prompt(*rows, _p(dt_bias), bp, bs, zp, zs, _code(u), _p(a_log), _p(d_skip), _p(state), slot_stride,
                                                   _p(out), _p(ctx.meta), _p(ctx.cu_tokens), _p(ctx.state_slots), ctx.S, inner, nstate,
                                                   self._stream()), "selective_scan")
@@ -1079,22 +1079,26 @@ class CudaOps:
         if chunk:
             self.launches += 2
 
-    def _selective_in_order(self, ctx, inner: int, dtype) -> bool:
+    def _selective_in_order(self, ctx, inner: int, nstate: int, dtype) -> bool:
         """Whether a step's selective scan runs in one pass (kernels/selective_prompt.cuh): where its estimated time is the shorter
-        one.  It takes 0.04 us a token of the longest entry, or, with more blocks of 32 channels than multiprocessors, their share
-        of all tokens and 2.2 us an entry; the scan cut in chunks of time 48 us and two passes over everything, the one in order
-        (steps of short entries) 0.4 us a token of the longest.  Measured, us, one pass / the other, 16 states, channels x tokens:
-        4096 x 2048 86 / 163, 8192 x 2048 165 / 296, 2048 x 2048 85 / 103, 1024 x 3000 121 / 91, 1024 x 1000 45 / 58, 4096 x 64 10 / 32,
-        4096 x 16 8 / 15; 4096 channels, 128 tokens beside 20 single ones 49 / 81, 8 x 16 29 / 16, 8 x 64 35 / 37, 64 x 1 126 / 39."""
+        one.  It takes 0.0375 us a token of the longest entry, or, with more blocks of 32 channels than multiprocessors, their share
+        of all tokens and 2.2 us an entry, with 8 states as with 16; the scan cut in chunks of time 36 us, 1.2 an entry and two passes
+        over everything, whose work follows the states; the one in order (steps of short entries) 0.4 us a token of the longest (0.35 with 8
+        states).  Measured, us, one pass / the other, bfloat16 (float32 within 5 %), channels x tokens, 16 states: 4096 x 2048 80 / 156,
+        8192 x 2048 160 / 285, 2048 x 2048 79 / 96, 1024 x 3000 115 / 82, 1024 x 1000 41 / 50, 4096 x 64 6 / 27, 4096 x 16 5 / 10; 8 states:
+        4096 x 2048 79 / 119, 2048 x 2048 78 / 72, 1024 x 3000 114 / 64, 1024 x 1000 40 / 43, 4096 x 64 6 / 24; 4096 channels and 16 (8)
+        states, 128 tokens beside 20 single ones 47 / 72 (48 / 52), 1,000 beside 40 114 / 267 (116 / 140), 8 x 16 25 / 13 (24 / 10), 8 x 64
+        32 / 33 (31 / 28)."""
         longest = ctx.max_tokens_per_entry
         if self.selective_prompt is not None:
             return self.selective_prompt
         if longest < 16 or (dtype == torch.float32 and longest < self.SCAN_CHUNK_FROM):
             return False  # (float32 below the chunks of time: a token's sum has one order, whatever else the step brings)
         share, work = -(-inner // 32) / self.num_sms, ctx.T * inner
-        one_pass = 4.0 + max(0.0405 * longest, share * (2.2 * ctx.S + 0.0405 * ctx.T))
-        other = 48.0 + 1.35e-5 * work if longest >= self.SCAN_CHUNK_FROM else 6.0 + max(0.4 * longest, 1.1e-5 * work)
-        return one_pass < other
+        one_pass = 3.0 + max(0.0375 * longest, share * (2.2 * ctx.S + 0.0375 * ctx.T))
+        if longest >= self.SCAN_CHUNK_FROM:
+            return one_pass < 36.0 + 1.2 * ctx.S + (0.5 + 0.058 * nstate) * 1e-5 * work
+        return one_pass < 6.0 + max((0.3 + 0.00625 * nstate) * longest, 1.1e-5 * work)
 
     def moe_route(self, h, w_router, ids, wts, meta, bias=None, over_chosen: bool = False):
         """Per token: float32 logits w_router h (+ ``bias``, float32 [experts]), softmax over all experts, the ids.shape[1]
