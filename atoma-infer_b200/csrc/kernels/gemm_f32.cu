@@ -29,11 +29,19 @@ struct Stage {
     static __device__ __forceinline__ int at(int row, int k) { return k * LD + (row ^ ((k >> 3) * RW)); }
 };
 
+__device__ __forceinline__ bool finite(float v) { return fabsf(v) <= 3.402823466e38f; }
+
+// What a launch that takes again what is not finite looks at: a flag without which there is nothing to do, and where the number of
+// rows that count stands (null: all M do).
+struct Repair {
+    const int *odd, *limit;
+};
+
 // BM x BN outputs a block, TM x TN (in groups of four rows and four columns) a thread.  VEC: rows of x and w start on 16
-// bytes and K is a multiple of 4.
-template <int BM, int BN, int TM, int TN, int GK, bool VEC>
+// bytes and K is a multiple of 4.  REPAIR: only the elements of y that are not finite, in the tiles that have one.
+template <int BM, int BN, int TM, int TN, int GK, bool VEC, bool REPAIR>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
-gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K, int vec_out) {
+gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K, int vec_out, Repair repair) {
     constexpr int NT = (BM / TM) * (BN / TN), C4 = GK / 4, QA = BM * C4, QB = BN * C4;
     constexpr int LA = (QA + NT - 1) / NT, LB = (QB + NT - 1) / NT;
     using SA = Stage<BM, GK>;
@@ -41,6 +49,18 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
     __shared__ __align__(16) float xs[2][GK * SA::LD], ws[2][GK * SB::LD];
     const int tid = threadIdx.x, m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
     const int tx = tid % (BN / TN), ty = tid / (BN / TN);
+    int rows = M;  // that are stored
+    if (REPAIR) {
+        pdl_wait();
+        if (!*repair.odd) return;
+        if (repair.limit) rows = min(M, *repair.limit);
+        int any = 0;
+        for (int i = tid; i < BM * BN && !any; i += NT) {
+            const int m = m0 + i / BN, n = n0 + i % BN;
+            any = m < rows && n < N && !finite(y[(size_t)m * N + n]);
+        }
+        if (!__syncthreads_or(any)) return;
+    }
     float4 ra[LA], rb[LB];
 
     auto quad = [&](const float* __restrict__ src, int row, int rows, int k) {
@@ -133,7 +153,7 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
         const int m = m0 + i / 4 * (BM / TM * 4) + ty * 4 + i % 4;
-        if (m >= M) continue;
+        if (m >= rows) continue;
 #pragma unroll
         for (int j = 0; j < TN; j += 4) {
             const int n = n0 + j / 4 * (BN / TN * 4) + tx * 4;
@@ -141,7 +161,11 @@ gemm_f32_kernel(const float* __restrict__ x, const float* __restrict__ w, float*
             float v[4];
             asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[i][j / 2]));
             asm("mov.b64 {%0, %1}, %2;" : "=f"(v[2]), "=f"(v[3]) : "l"(acc[i][j / 2 + 1]));
-            if (vec_out && n + 3 < N) {
+            if (REPAIR) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (n + c < N && !finite(dst[c])) dst[c] = v[c];
+            } else if (vec_out && n + 3 < N) {
                 store4(dst, v);
             } else {
 #pragma unroll
@@ -157,8 +181,8 @@ int launch(const float* x, const float* w, float* y, int M, int N, int K, cudaSt
     const dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
     const int vec = K % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0, vec_out = N % 4 == 0 && ((uintptr_t)y & 15) == 0;
     constexpr int threads = (BM / TM) * (BN / TN);
-    if (vec) return (int)launch_kernel(gemm_f32_kernel<BM, BN, TM, TN, GK, true>, grid, threads, 0, stream, x, w, y, M, N, K, vec_out);
-    return (int)launch_kernel(gemm_f32_kernel<BM, BN, TM, TN, GK, false>, grid, threads, 0, stream, x, w, y, M, N, K, vec_out);
+    if (vec) return (int)launch_kernel(gemm_f32_kernel<BM, BN, TM, TN, GK, true, false>, grid, threads, 0, stream, x, w, y, M, N, K, vec_out, Repair{});
+    return (int)launch_kernel(gemm_f32_kernel<BM, BN, TM, TN, GK, false, false>, grid, threads, 0, stream, x, w, y, M, N, K, vec_out, Repair{});
 }
 
 }  // namespace
@@ -193,4 +217,17 @@ extern "C" int gemm_f32(const float* x, const float* w, float* y, int M, int N, 
         case 3: return launch<32, 64, 4, 4, 32>(x, w, y, M, N, K, stream);
         default: return launch<16, 128, 4, 4, 32>(x, w, y, M, N, K, stream);
     }
+}
+
+// The elements of y that are not finite again, by the product above (with its bits); the others stay.  odd: a device word without which nothing
+// is done (the launch then ends at once); limit: a device word that says how many rows count (or null).  x and w on 16 bytes, K a
+// multiple of 4.
+extern "C" int gemm_f32_repair(const float* x, const float* w, float* y, const int* odd, const int* limit, int M, int N, int K, cudaStream_t stream) {
+    if (M <= 0 || N <= 0) return 0;
+    if (K % 4 || (((uintptr_t)x | (uintptr_t)w) & 15)) return (int)cudaErrorInvalidValue;
+    if (M <= 32)
+        return (int)launch_kernel(gemm_f32_kernel<32, 64, 4, 4, 32, true, true>, dim3((N + 63) / 64, 1), 128, 0, stream, x, w, y, M, N, K, 0,
+                                  Repair{odd, limit});
+    return (int)launch_kernel(gemm_f32_kernel<128, 128, 8, 8, 16, true, true>, dim3((N + 127) / 128, (M + 127) / 128), 256, 0, stream, x, w, y, M, N, K,
+                              0, Repair{odd, limit});
 }

@@ -256,9 +256,13 @@ class CudaOps:
         if x.dtype == torch.float32:
             y = torch.empty((M, N), dtype=torch.float32, device=x.device)
             if self._f32_on_tcgen05(x, w, y):
-                split = torch.empty((2, M, K), dtype=torch.float32, device=x.device)
-                self._check(self._gemm_library().gemm_f32_tcgen05(_p(x), _p(w), _p(y), _p(split), M, N, K, _p(self.status), self._stream()),
+                lib = self._gemm_library()
+                scratch = torch.empty(lib.gemm_f32_tcgen05_scratch(M, K), dtype=torch.uint8, device=x.device)
+                # rows behind the step's own (a captured step's padding) hold anything: they raise no flag
+                limit = None if meta is None else ctypes.c_void_p(meta.data_ptr() + 4 * (META_NUM_ROWS if use_rows else META_NUM_TOKENS))
+                self._check(lib.gemm_f32_tcgen05(_p(x), _p(w), _p(y), _p(scratch), limit, M, N, K, _p(self.status), self._stream()),
                             "gemm_f32_tcgen05")
+                self._check(self.lib.gemm_f32_repair(_p(x), _p(w), _p(y), _p(scratch[-16:]), limit, M, N, K, self._stream()), "gemm_f32_repair")
                 self.launches += 1  # (the split of x)
             else:
                 self._check(self.lib.gemm_f32(_p(x), _p(w), _p(y), M, N, K, self._stream()), "gemm_f32")
@@ -368,14 +372,17 @@ class CudaOps:
     def _gemm_library(self):
         if self._gemm_lib is None:
             self._gemm_lib = build.load_library("gemm_tcgen05", GEMM_SOURCES, cuda=True)
+            self._gemm_lib.gemm_f32_tcgen05_scratch.restype = ctypes.c_size_t
         return self._gemm_lib
 
     def _f32_on_tcgen05(self, x, w, y) -> bool:
-        """Whether a float32 product runs on the tensor cores as three TF32 products with short sums (kernels/gemm_f32_tcgen05.cu;
-        closer to float64 than one float32 accumulator).  By the weight alone, so that a row's bits do not depend on the rows
-        beside it.  Measured against the plain kernel, us for 1 / 8 / 333 rows: 1024 x 1024 34 / 34 / 36 for 40 / 40 / 52, 2048 x 2048
-        34 / 34 / 40 for 75 / 75 / 113, 512 x 2048 30 / 30 / 36 for 75 / 75 / 73; 2048 x 512 - / 26 / 28 for - / 24 / 34, hence K from
-        1,024 on; 8 rows of 128256 x 2048 (an output head, which has few rows) 292 for 281, hence N up to 65,536."""
+        """Whether a float32 product runs on the tensor cores (kernels/gemm_f32_tcgen05.cu: three bfloat16 numbers an operand, eight
+        products with short sums; never further from float64 than one float32 accumulator).  By the weight alone, so that a row's bits
+        do not depend on the rows beside it.  Measured against the plain kernel, us for 1 / 8 / 333 rows: 1024 x 1024 25 / 26 / 30 for
+        34 / 34 / 44, 2048 x 2048 30 / 30 / 39 for 70 / 70 / 107, 512 x 2048 26 / 27 / 31 for 67 / 67 / 68, 16384 x 1024 30 / 31 / - for 37
+        / 38 / -; for 8 / 128 rows: 32768 x 1024 54 / 84 for 49 / 204, 32768 x 2048 91 / 129 for 92 / 403, 49152 x 2048 133 / 182 for 121 /
+        604, 65536 x 1024 99 / - for 80 / -.  2048 x 512 is too few
+        runs along K to pay for the start, hence K from 1,024 on."""
         N, K = w.shape
         return (self.tc_f32 and K % 4 == 0 and K >= 1024 and N * K >= 1 << 20 and N <= 65536 and x.is_contiguous() and w.is_contiguous()
                 and (x.data_ptr() | w.data_ptr() | y.data_ptr()) % 16 == 0)
