@@ -70,6 +70,99 @@ def test_other_steps_are_left_alone():
     assert not takes([(0, 2), (4, 1)]) and not takes([(3, 1)], norm_groups=3)
 
 
+class Step:
+    """Five requests' tokens, in slots out of order, with rows of their own and a state that both ways start from."""
+
+    def __init__(self, rt, heads, P, N, G, taps, seed):
+        g, dev = torch.Generator().manual_seed(seed), rt.device
+        self.rt, self.sizes, self.past = rt, (heads, P, N, G, taps), [0, 1, 2, 57, 400]
+        S, inner, ch = len(self.past), heads * P, heads * P + 2 * G * N
+        self.ctx, _ = K.make_context(rt, [(c, 1) for c in self.past], 16, [[1 + i] * 32 for i in range(S)])
+        self.slots = [3, 0, 4, 1, 2]
+        self.ctx.state_slots.copy_(torch.tensor(self.slots, dtype=torch.int32))
+
+        def f(*shape, std=1.0, mean=0.0):
+            return (torch.randn(*shape, generator=g) * std + mean).to(dev)
+
+        self.proj = f(S, -(-(2 * inner + 2 * G * N + heads) // 8) * 8).to(rt.dtype)
+        self.z, self.u, self.dt = self.proj[:, :inner], self.proj[:, inner:inner + ch], self.proj[:, inner + ch:inner + ch + heads]
+        self.conv_w, self.conv_b, self.dt_bias = f(taps, ch, std=0.3), f(ch, std=0.1), f(heads, mean=-3)
+        self.a_log, self.d, self.w = f(heads, std=0.5), f(heads), f(inner, std=0.1, mean=1)
+        self.ring, self.state = f(S, taps - 1, ch), f(S, heads, N, P, std=0.5)
+
+    def two_launches(self):
+        heads, P, N, G, taps = self.sizes
+        ring, state, out = self.ring.clone(), self.state.clone(), torch.empty(len(self.past), heads * P, dtype=self.rt.dtype, device=self.rt.device)
+        assert self.rt.ops.ssm_token_step(self.u, self.z, self.dt, self.conv_w, self.conv_b, ring, self.dt_bias, self.a_log, self.d, state, self.w, G, G,
+                                          1e-5, self.ctx, out)
+        self.rt.ops.check_status()
+        return out, state, ring
+
+    def three_kernels(self):
+        heads, P, N, G, taps = self.sizes
+        ops, ring, state = self.rt.ops, self.ring.clone(), self.state.clone()
+        xbc, y = torch.empty_like(self.u, memory_format=torch.contiguous_format), torch.empty(len(self.past), heads * P, device=self.rt.device)
+        out = torch.empty(len(self.past), heads * P, dtype=self.rt.dtype, device=self.rt.device)
+        if not ops.causal_conv_act(self.u, self.conv_w, self.conv_b, ring, self.ctx, xbc):
+            ops.causal_conv_save(self.u, ring, self.ctx, taps)
+        ops.ssm_scan(xbc, self.dt, self.dt_bias, self.a_log, self.d, state, self.ctx, y, heads=heads, head_dim=P, nstate=N, groups=G)
+        ops.gated_group_norm(y, self.z, self.w, G, 1e-5, out, self.ctx.meta)
+        return out, state, ring
+
+    def exact(self):
+        """The same in 64 bits, without a rounding on the way."""
+        heads, P, N, G, taps = self.sizes
+        outs, state, ring, R = [], self.state.double(), self.ring.double(), taps - 1
+        for e, p in enumerate(self.past):
+            s, u = self.slots[e], self.u[e].double()
+            acc = self.conv_b.double() + self.conv_w[R].double() * u
+            for back in range(1, R + 1):
+                if p - back >= 0:
+                    acc = acc + self.conv_w[R - back].double() * ring[s, (p - back) % R]
+            ring[s, p % R] = u
+            x, B, C = (acc * torch.sigmoid(acc)).split([heads * P, G * N, G * N])
+            x, B, C = x.view(heads, P), *(t.view(G, N).repeat_interleave(heads // G, 0) for t in (B, C))
+            step = torch.nn.functional.softplus(self.dt[e].double() + self.dt_bias.double())
+            decay = torch.exp(-torch.exp(self.a_log.double()) * step)
+            state[s] = decay[:, None, None] * state[s] + torch.einsum("hn,hp->hnp", B, step[:, None] * x)
+            y = (torch.einsum("hnp,hn->hp", state[s], C) + self.d.double()[:, None] * x).reshape(-1)
+            z = self.z[e].double()
+            v = (y * z * torch.sigmoid(z)).view(G, -1)
+            outs.append((v / (v.square().mean(1, keepdim=True) + 1e-5).sqrt()).reshape(-1) * self.w.double())
+        return torch.stack(outs), state, ring
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,P,N,G,taps", [(16, 64, 128, 2, 4), (6, 32, 250, 2, 4), (4, 128, 64, 2, 2), (14, 64, 37, 7, 3)])
+def test_against_64_bits(dtype, heads, P, N, G, taps):
+    from atoma_infer_b200.engine.runtime import make_runtime
+
+    step = Step(make_runtime(dtype, "cuda:0"), heads, P, N, G, taps, seed=heads + N)
+    got, want = step.two_launches(), step.exact()
+    assert torch.equal(got[2].double(), want[2])
+    # float32: sums of up to 250 terms, 250^0.5 2^-24 and exponentials of a few 2^-24; bfloat16: x, B and C are rounded behind the
+    # convolution and the result once more, 2^-9 of a value each at most
+    for a, b in zip(got[:2], want[:2]):
+        assert float((a.double() - b).norm() / b.norm()) < (2e-6 if dtype == "float32" else 4 * 2.0 ** -9)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_what_is_not_finite(dtype):
+    """Infinities and NaN in a row, a step size and a state: where the three kernels have them, and nowhere else."""
+    from atoma_infer_b200.engine.runtime import make_runtime
+
+    heads, P, N, G = 4, 64, 128, 2
+    step = Step(make_runtime(dtype, "cuda:0"), heads, P, N, G, 4, seed=1)
+    inner = heads * P
+    step.u[0, 5], step.u[1, inner + 3], step.dt[2, 1] = float("inf"), float("nan"), float("inf")  # x of a head, B of a group, a step size
+    step.state[step.slots[3], 2, 7, 9], step.state[step.slots[4], 0, 0, 0], step.ring[step.slots[4], 1, 70] = float("-inf"), float("nan"), float("inf")
+    for a, b in zip(step.two_launches(), step.three_kernels()):
+        assert torch.equal(a.isnan(), b.isnan()) and torch.equal(a.isinf(), b.isinf()) and not bool(torch.isfinite(a).all())
+        assert bool(torch.isfinite(a).any())
+        if dtype == "float32":
+            assert torch.equal(a.nan_to_num(), b.nan_to_num())
+
+
 @pytest.mark.parametrize("heads,P,N,G", [(64, 64, 128, 8), (64, 32, 100, 4), (48, 128, 64, 3), (64, 64, 20, 1)])
 def test_float32_bits_do_not_depend_on_the_other_requests(heads, P, N, G):
     """A request's token alone, among others at the two sides of where the step stops being taken, and beside a prompt: the layer's
