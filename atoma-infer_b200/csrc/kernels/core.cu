@@ -1,7 +1,8 @@
 // Core kernels, for float32 and bfloat16 storage alike; all arithmetic is float32.
 //
-// These are the plain kernels of the engine: the whole float32 path runs on them,
-// and the bfloat16 path uses them wherever no faster kernel exists for a size.
+// These are the plain kernels of the engine: the float32 path runs on them (its products
+// of large weights on gemm_f32_tcgen05.cu), and the bfloat16 path uses them wherever no
+// faster kernel exists for a size.
 // Every reduction runs in an order that depends only on the element it belongs to
 // (never on the batch, the portioning of a prompt, or the pages used), so float32
 // logits are bit-identical however the work is cut.

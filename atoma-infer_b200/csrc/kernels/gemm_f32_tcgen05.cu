@@ -23,7 +23,8 @@
 // operand lost up to 2^-23 and a product up to 2^-21, more where a rest fell below 2^-126.)
 //
 // Measured (B200, us, cold weights; in brackets gemm_f32.cu): 333 x 16384 x 2048 162 (608), 333 x 2048 x 8192 96 (420), 2048 x 16384 x 2048 785
-// (2,600; 1.40 PFLOP/s of bfloat16, the library's sustained rate), 8 x 16384 x 2048 52 (72), 8 x 2048 x 8192 51 (274), 1 x 1024 x 1024 25 (34).
+// (2,600; 1.40 PFLOP/s of bfloat16, the library's sustained rate), 8 x 16384 x 2048 52 (72), 8 x 2048 x 8192 51 (274), 1 x 1024 x 1024 25 (34);
+// of that the repair, when there is nothing to do, 1.0 to 2.8.  A whole batch of NaN, 333 x 4096 x 2048: 268 (176).
 #include <cuda.h>
 
 #include "common.cuh"
