@@ -106,14 +106,16 @@ causal_conv_act_vec_kernel(const T* __restrict__ u, long long u_stride, const fl
     }
 }
 
-// The same for steps with prompt tokens: a thread takes V channels of TOKENS tokens, so weights, bias and all rows but the
+// The same for steps with prompt tokens: a thread takes V channels of CONV_TOKENS tokens, so weights, bias and all rows but the
 // first TAPS - 1 are loaded once (each token for itself read every row TAPS times and TAPS rows of float32 weights for one row of
 // results).  All of a thread's rows are in flight before the first is used.  Most of its time goes into the activation's
 // instructions and, before, into looking up every token's place: tiles within one entry do not.  Measured, us, 4 taps, bfloat16 (first
 // the form of 8 tokens by 4 channels with a look-up a token, then 8 x 4, 8 x 8 and 4 x 8 without; in brackets the copy bandwidth's
 // time): 2,048 tokens of 6,144 channels 27.2, 23.0, 20.6, 19.3 (7.7); of 4,096 18.7, 16.2, 16.1, 13.5; 3,000 of 12,288 76.5, 68.4, 56.8,
-// 53.3; 301 of 6,144 6.1, 6.5, 7.8, 6.0.
-template <typename T, int V, int TOKENS, int TAPS>
+// 53.3; 301 of 6,144 6.1, 6.5, 7.8, 6.0.  float32, 4 channels: 8 tokens with a look-up a token, 8 and 4 tokens without: 2,048 of 6,144
+// 27.7, 23.2, 20.0; 301 of 6,144 6.3, 6.7, 5.0; 64 of 1,024 4.8, 5.3, 3.2.
+#define CONV_TOKENS 4
+template <typename T, int V, int TAPS>
 __global__ void __launch_bounds__(128)
 causal_conv_tile_kernel(const T* __restrict__ u, long long u_stride, const float* __restrict__ w, const float* __restrict__ bias,
                         const float* __restrict__ state, long long slot_stride, T* __restrict__ y, const int* __restrict__ meta,
@@ -121,8 +123,8 @@ causal_conv_tile_kernel(const T* __restrict__ u, long long u_stride, const float
                         const int* __restrict__ slots, int C, int act) {
     constexpr int R = TAPS - 1;
     struct alignas(V * sizeof(T)) Row { T x[V]; };
-    const int t0 = blockIdx.x * TOKENS, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
-    const int n = min(TOKENS, meta[META_NUM_TOKENS] - t0);
+    const int t0 = blockIdx.x * CONV_TOKENS, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
+    const int n = min(CONV_TOKENS, meta[META_NUM_TOKENS] - t0);
     const bool live = n > 0 && c < C;
     float wv[TAPS][V], bv[V];
     if (live) {  // weights and bias depend on no earlier kernel: fetched before the wait
@@ -141,9 +143,9 @@ causal_conv_tile_kernel(const T* __restrict__ u, long long u_stride, const float
     pdl_wait();
     pdl_launch_dependents();
     if (!live) return;
-    Row rows[TOKENS + R];  // tokens t0 - R ..: those ahead of t0 may belong to another entry, and are then not used
+    Row rows[CONV_TOKENS + R];  // tokens t0 - R ..: those ahead of t0 may belong to another entry, and are then not used
 #pragma unroll
-    for (int i = 0; i < TOKENS + R; ++i) {
+    for (int i = 0; i < CONV_TOKENS + R; ++i) {
         const int t = t0 - R + i;
         if (t >= 0 && t < t0 + n) rows[i] = *reinterpret_cast<const Row*>(u + (size_t)t * u_stride + c);
     }
@@ -155,9 +157,9 @@ causal_conv_tile_kernel(const T* __restrict__ u, long long u_stride, const float
     };
     // most tiles lie within one entry, taps and all: no look at a token's place
     const int e0 = token_entry[t0];
-    if (n == TOKENS && e0 == token_entry[t0 + TOKENS - 1] && t0 - R >= cu_tokens[e0]) {
+    if (n == CONV_TOKENS && e0 == token_entry[t0 + CONV_TOKENS - 1] && t0 - R >= cu_tokens[e0]) {
 #pragma unroll
-        for (int tt = 0; tt < TOKENS; ++tt) {
+        for (int tt = 0; tt < CONV_TOKENS; ++tt) {
             float acc[V];
 #pragma unroll
             for (int i = 0; i < V; ++i) acc[i] = bv[i];
@@ -170,7 +172,7 @@ causal_conv_tile_kernel(const T* __restrict__ u, long long u_stride, const float
         return;
     }
 #pragma unroll
-    for (int tt = 0; tt < TOKENS; ++tt) {
+    for (int tt = 0; tt < CONV_TOKENS; ++tt) {
         if (tt >= n) break;
         const int t = t0 + tt, e = token_entry[t], p = positions[t], first = cu_tokens[e];
         float acc[V];
@@ -197,13 +199,13 @@ causal_conv_tile_kernel(const T* __restrict__ u, long long u_stride, const float
     }
 }
 
-template <typename T, int V, int TOKENS>
+template <typename T, int V>
 static int launch_conv_tile(const T* u, long long u_stride, const float* w, const float* bias, const float* state, long long slot_stride, T* y,
                             const int* meta, const int* positions, const int* token_entry, const int* cu_tokens, const int* slots, int rows,
                             int C, int taps, int act, cudaStream_t stream) {
-    const dim3 grid((rows + TOKENS - 1) / TOKENS, (C / V + 127) / 128);
+    const dim3 grid((rows + CONV_TOKENS - 1) / CONV_TOKENS, (C / V + 127) / 128);
 #define CONV_CASE(K)                                                                                                       \
-    case K: return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, causal_conv_tile_kernel<T, V, TOKENS, K>, grid, 128, 0, stream, u, u_stride, w, bias, \
+    case K: return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, causal_conv_tile_kernel<T, V, K>, grid, 128, 0, stream, u, u_stride, w, bias, \
                                           state, slot_stride, y, meta, positions, token_entry, cu_tokens, slots, C, act);
     switch (taps) { CONV_CASE(2) CONV_CASE(3) CONV_CASE(4) }
 #undef CONV_CASE
@@ -222,9 +224,9 @@ extern "C" int causal_conv_act(const void* u, int dtype, long long u_stride, con
         // two to four taps, unless the ring is updated on the way (one token an entry)
         if (!save_own && taps >= 2 && taps <= 4) {
             if (dtype == DT_F32)
-                return launch_conv_tile<float, 4, 8>((const float*)u, u_stride, w, bias, state, slot_stride, (float*)y, meta, positions, token_entry,
-                                                  cu_tokens, slots, T, C, taps, act, stream);
-            return launch_conv_tile<__nv_bfloat16, 8, 4>((const __nv_bfloat16*)u, u_stride, w, bias, state, slot_stride, (__nv_bfloat16*)y, meta,
+                return launch_conv_tile<float, 4>((const float*)u, u_stride, w, bias, state, slot_stride, (float*)y, meta, positions, token_entry,
+                                                     cu_tokens, slots, T, C, taps, act, stream);
+            return launch_conv_tile<__nv_bfloat16, 8>((const __nv_bfloat16*)u, u_stride, w, bias, state, slot_stride, (__nv_bfloat16*)y, meta,
                                                       positions, token_entry, cu_tokens, slots, T, C, taps, act, stream);
         }
         dim3 grid(T, (C / V + 127) / 128);
