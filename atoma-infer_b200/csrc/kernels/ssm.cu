@@ -580,7 +580,8 @@ extern "C" int ssm_chunk_scan(const void* xbc, int xbc_stride, const void* dt, l
 // ----------------------------------------------------------------------------- gate, then the norm in equal parts
 // v = y * silu(z); out = v / sqrt(mean(v^2) + eps) * w, the mean taken over each of `parts` equal parts of the row.
 // y is float32 [T, n]; z a slice of a wider row.  One block per (token, part).
-template <typename T>
+// RING: further blocks of a decode step write the convolution's ring (ssm_token.cuh).
+template <typename T, bool RING>
 __global__ void __launch_bounds__(256)
 gated_group_norm_kernel(const float* __restrict__ y, const T* __restrict__ z, long long z_stride, const float* __restrict__ w,
                         float eps, T* __restrict__ out, const int* __restrict__ meta, int n, int parts, int vec4,
@@ -589,7 +590,7 @@ gated_group_norm_kernel(const float* __restrict__ y, const T* __restrict__ z, lo
     pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x, part = blockIdx.y, len = n / parts, at = part * len;
-    if (part >= parts) return ring_row(ring, t, part - parts, meta);  // (blocks of a decode step that write the convolution's ring)
+    if (RING && part >= parts) return ring_row(ring, t, part - parts, meta);
     if (t >= meta[META_NUM_TOKENS]) return;
     const float* yr = y + (size_t)t * n + at;
     const T* zr = z + (size_t)t * z_stride + at;
@@ -721,8 +722,8 @@ template <typename T>
 static int launch_group_norm(const float* y, const T* z, long long z_stride, const float* w, float eps, T* out, const int* meta, int rows, int n,
                              int parts, int threads, int vec4, const RingRow<T>& ring, cudaStream_t stream) {
     const int more = ring.ring ? (ring.channels + threads - 1) / threads : 0;
-    return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, gated_group_norm_kernel<T>, dim3(rows, parts + more), threads, 0, stream, y, z, z_stride, w,
-                                  eps, out, meta, n, parts, vec4, ring);
+    return (int)launch_kernel_pdl((g_use_pdl & 5) != 0, more ? gated_group_norm_kernel<T, true> : gated_group_norm_kernel<T, false>,
+                                  dim3(rows, parts + more), threads, 0, stream, y, z, z_stride, w, eps, out, meta, n, parts, vec4, ring);
 }
 
 extern "C" int gated_group_norm(const float* y, const void* z, int dtype, long long z_stride, const float* w, float eps,
