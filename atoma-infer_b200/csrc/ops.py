@@ -380,11 +380,13 @@ class CudaOps:
         products with short sums; never further from float64 than one float32 accumulator).  By the weight alone, so that a row's bits
         do not depend on the rows beside it.  Measured against the plain kernel, us for 1 / 8 / 333 rows: 1024 x 1024 25 / 26 / 30 for
         34 / 34 / 44, 2048 x 2048 30 / 30 / 39 for 70 / 70 / 107, 512 x 2048 26 / 27 / 31 for 67 / 67 / 68, 16384 x 1024 30 / 31 / - for 37
-        / 38 / -; for 8 / 128 rows: 32768 x 1024 54 / 84 for 49 / 204, 32768 x 2048 91 / 129 for 92 / 403, 49152 x 2048 133 / 182 for 121 /
-        604, 65536 x 1024 99 / - for 80 / -: beyond 32,768 columns stand output heads, which have few rows.  2048 x 512 is too few
+        / 38 / -; for 8 / 128 rows, with more columns than one round of blocks takes: 24576 x 1024 52 / 86 for 48 / 182, 32768 x 1024
+        54 / 84 for 49 / 204, 32768 x 1536 72 / 106 for 69 / 304, 32768 x 2048 91 / 129 for 92 / 403, 49152 x 2048 133 / 182 for 121 /
+        604: narrow weights of so many columns, and all beyond 32,768, are output heads, which have few rows.  2048 x 512 is too few
         runs along K to pay for the start, hence K from 1,024 on."""
         N, K = w.shape
-        return (self.tc_f32 and K % 4 == 0 and K >= 1024 and N * K >= 1 << 20 and N <= 32768 and x.is_contiguous() and w.is_contiguous()
+        most = 32768 if K >= 2048 else 128 * self.num_sms
+        return (self.tc_f32 and K % 4 == 0 and K >= 1024 and N * K >= 1 << 20 and N <= most and x.is_contiguous() and w.is_contiguous()
                 and (x.data_ptr() | w.data_ptr() | y.data_ptr()) % 16 == 0)
 
     def silu_mul(self, gu, out, meta, T: int, inter: int):

@@ -1,4 +1,4 @@
-"""Which steps run the scans of recurrent layers as matrix products over chunks: by sizes alone, so without a GPU."""
+"""Which steps run the scans of recurrent layers as matrix products over chunks, and other rules by sizes alone: without a GPU."""
 from types import SimpleNamespace
 
 import pytest
@@ -76,3 +76,12 @@ def test_selective_scans_in_one_pass_where_that_was_measured_to_be_shorter(nstat
     ops = SimpleNamespace(selective_prompt=None, num_sms=148, SCAN_CHUNK_FROM=CudaOps.SCAN_CHUNK_FROM)
     ctx = SimpleNamespace(T=sum(lengths), S=len(lengths), max_tokens_per_entry=max(lengths))
     assert CudaOps._selective_in_order(ops, ctx, inner, nstate, torch.bfloat16) == one_pass
+
+
+@pytest.mark.parametrize("N,K,takes", [(1024, 1024, True), (1023, 1024, False), (512, 2048, True), (4096, 1020, False), (1024, 1026, False),
+                                       (18944, 1024, True), (18945, 1024, False), (32768, 2048, True), (32769, 2048, False), (32768, 2044, False)])
+def test_float32_products_on_the_tensor_cores_by_the_weight_alone(N, K, takes):
+    w, ops = torch.empty(N, K, device="meta"), SimpleNamespace(tc_f32=True, num_sms=148)
+    for M in (1, 17, 4096):
+        x, y = torch.empty(M, K, device="meta"), torch.empty(M, N, device="meta")
+        assert CudaOps._f32_on_tcgen05(ops, x, w, y) == takes
