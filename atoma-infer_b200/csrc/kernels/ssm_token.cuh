@@ -40,7 +40,10 @@ ssm_token_kernel(const __grid_constant__ SsmToken<T> A) {
     __shared__ __align__(16) float xs[P], part[IN_ORDER ? 512 / P : 8][P], bc[2 * MAX_N], mat[IN_ORDER ? MAX_N * P : 4];
     const int h = blockIdx.x, e = blockIdx.y, g = h / (A.heads / A.groups), tid = threadIdx.x, N = A.N;
     const int inner = A.heads * P, channels = inner + 2 * A.groups * N, R = A.taps - 1;
-    if (e >= A.meta[META_NUM_ENTRIES]) return;
+    if (e >= A.meta[META_NUM_ENTRIES]) {  // (padding; it waits all the same, so that no block is done before the linear ahead)
+        pdl_wait();
+        return;
+    }
     const int t = A.cu_tokens[e], p = A.positions[t], slot = A.slots[e];
     float* S = A.state + (size_t)slot * A.slot_stride + (size_t)h * N * P;
     for (int i = tid * 32; i < N * P; i += 256 * 32) asm volatile("prefetch.global.L2 [%0];" ::"l"(S + i));
