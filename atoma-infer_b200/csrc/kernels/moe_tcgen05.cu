@@ -2,7 +2,7 @@
 // stretch of them times that expert's weights, and the shared expert's product in the same launch.
 //
 //   mode 1: a[i, f] = silu(w[e, f] . x[i]) * (w[e, F + f] . x[i])   (w [E, 2F, K], f < F)
-//   mode 0: y[i, n] = w[e, n] . a[i]                                (w [E, N, K])
+//   mode 0: y[i, n] = w[e, n] . a[i]                                (w [E, N, K]); mode 2: the same, stored as float32
 //
 // The weights are the MMA's row side and the tokens its columns: a stretch of n rows is cut into equal chunks of at most 256,
 // rounded up to 32, so that an expert of 260 rows does the work of 320 and not of 384, as it does where 128 rows are the tile's least; and
@@ -86,9 +86,8 @@ struct GroupedArgs {
     const int* meta;     // the step's tokens: the shared expert's rows
     int experts, rows, depth;                              // an expert's results a row (mode 1: F) and its K
     int shared_tokens, shared_rows, shared_depth;          // (0 tokens: no shared expert)
-    void* out;                                             // [sorted rows, rows]: bfloat16, or (mode 0) float32 with `wide`
+    void* out;                                             // [sorted rows, rows], bfloat16 (mode 2: float32)
     bf16* shared_out;                                      // [tokens, shared_rows]
-    int wide;
 };
 
 // A tile: `count` rows of x from `first` on, results from `w0` on, of expert `e` (or the shared one: -1).
@@ -274,13 +273,13 @@ moe_grouped_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
             if (!mbar_wait(&acc_full[buf], ((uint32_t)n >> 1) & 1u, status, abort_flag)) ok = false;
             tc_fence_after();
             const uint32_t acc = tmem_base + buf * MAX_CHUNK + ((uint32_t)(quarter * 32) << 16);
-            if (MODE == 0) {
+            if (MODE != 1) {
 #pragma unroll 1
                 for (int c0 = part * 16; c0 < at.count; c0 += 32) {
                     float v[16];
                     tmem_ld16(acc + c0, v);
                     const int row = at.w0 + rank * SPAN + quarter * 32 + lane;
-                    if (a.wide && !own) store16((float*)a.out + (size_t)at.first * rows, rows, row, rows, c0, at.count, v);
+                    if (MODE == 2 && !own) store16((float*)a.out + (size_t)at.first * rows, rows, row, rows, c0, at.count, v);
                     else store16(dst, rows, row, rows, c0, at.count, v);
                 }
             } else {
@@ -380,11 +379,14 @@ extern "C" int moe_tc_ff(const void* xs, const void* w_gate_up, void* act, const
     if (((uintptr_t)xs | (uintptr_t)w_gate_up | (uintptr_t)act | (uintptr_t)w_down | (uintptr_t)y | (uintptr_t)h | (uintptr_t)ws_gate_up |
          (uintptr_t)act_s | (uintptr_t)ws_down | (uintptr_t)y_s) & 15)
         return (int)cudaErrorInvalidValue;
-    const GroupedArgs first{offsets, meta, E, F, H, T, Fs, H, act, (bf16*)act_s, 0}, second{offsets, meta, E, H, F, T, H, Fs, y, (bf16*)y_s, wide};
+    const GroupedArgs first{offsets, meta, E, F, H, T, Fs, H, act, (bf16*)act_s}, second{offsets, meta, E, H, F, T, H, Fs, y, (bf16*)y_s};
     const bool few = E <= FEW_EXPERTS;
     const int rc = few ? launch_grouped<1, STAGES_FEW>(xs, w_gate_up, pairs, h, ws_gate_up, first, status, stream)
                        : launch_grouped<1, STAGES_MANY>(xs, w_gate_up, pairs, h, ws_gate_up, first, status, stream);
     if (rc) return rc;
+    if (wide)
+        return few ? launch_grouped<2, STAGES_FEW>(act, w_down, pairs, act_s, ws_down, second, status, stream)
+                   : launch_grouped<2, STAGES_MANY>(act, w_down, pairs, act_s, ws_down, second, status, stream);
     return few ? launch_grouped<0, STAGES_FEW>(act, w_down, pairs, act_s, ws_down, second, status, stream)
                : launch_grouped<0, STAGES_MANY>(act, w_down, pairs, act_s, ws_down, second, status, stream);
 }
