@@ -254,7 +254,7 @@ moe_sort_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __r
     for (int i = threadIdx.x; i < nwarps * E; i += blockDim.x) base[i] = 0;
     __syncthreads();
     int* own = base + warp * E;
-    auto walk = [&](auto&& visit) {
+    auto walk = [&](auto&& visit, auto&& left_out) {
         for (int i0 = from; i0 < to; i0 += 128) {
             int id[4];
 #pragma unroll
@@ -265,14 +265,15 @@ moe_sort_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __r
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
                 const unsigned same = __match_any_sync(0xffffffffu, id[u]);
-                if (i0 + u * 32 + lane < to) visit(i0 + u * 32 + lane, id[u], __popc(same & ((1u << lane) - 1u)));
+                if (id[u] >= 0) visit(i0 + u * 32 + lane, id[u], __popc(same & ((1u << lane) - 1u)));
+                else if (i0 + u * 32 + lane < to) left_out(i0 + u * 32 + lane);
                 __syncwarp();
                 if (id[u] >= 0 && lane == __ffs(same) - 1) own[id[u]] += __popc(same);
                 __syncwarp();
             }
         }
     };
-    walk([](int, int, int) {});
+    walk([](int, int, int) {}, [](int) {});
     __syncthreads();
     if (warp == 0) {
         int before = 0;
@@ -301,11 +302,15 @@ moe_sort_kernel(const int* __restrict__ ids, int* __restrict__ offsets, int* __r
         if (lane == 0) offsets[E] = before;
     }
     __syncthreads();
-    walk([&](int i, int e, int rank) {
-        const int at = e >= 0 ? own[e] + rank : -1;
-        if (e >= 0) order[at] = i;
-        if (place) place[i] = at;
-    });
+    walk(
+        [&](int i, int e, int rank) {
+            const int at = own[e] + rank;
+            order[at] = i;
+            if (place) place[i] = at;
+        },
+        [&](int i) {
+            if (place) place[i] = -1;
+        });
 }
 
 extern "C" int moe_sort(const int* ids, int* offsets, int* order, int* place, const int* meta, int top, int E,
@@ -428,7 +433,7 @@ extern "C" int moe_grouped_ff(const void* x, const void* w_gate_up, void* act, c
 
 // ----------------------------------------------------------------------------- weighted sum
 // out[t] = sum_k wts[t, k] * y[row of pair t * top + k] (+ shared[t]), choices in order, float32; a pair's row is the
-// pair itself, or place[pair] when the rows are in sorted order (a pair of place -1 adds nothing).
+// pair itself, or place[pair] when the rows are in sorted order (a pair of place -1 adds row -1, which holds zeros: no question here).
 template <typename TY, typename T>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, const float* __restrict__ wts,
@@ -443,9 +448,9 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, cons
             for (int k = 0; k < top; ++k) {
                 const long long row = place ? (long long)place[(size_t)t * top + k] : (long long)t * top + k;
                 const float weight = wts[(size_t)t * top + k];
-                load4(y + max(row, 0ll) * H + i, v);  // (a load for every choice: a branch here would put them one behind the other)
+                load4(y + row * H + i, v);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[j] = row < 0 ? acc[j] : fmaf(weight, v[j], acc[j]);
+                for (int j = 0; j < 4; ++j) acc[j] = fmaf(weight, v[j], acc[j]);
             }
             if (shared) {
                 load4(shared + (size_t)t * H + i, v);
@@ -460,7 +465,7 @@ moe_combine_kernel(const TY* __restrict__ y, const int* __restrict__ place, cons
         float acc = 0.f;
         for (int k = 0; k < top; ++k) {
             const long long row = place ? (long long)place[(size_t)t * top + k] : (long long)t * top + k;
-            if (row >= 0) acc = fmaf(wts[(size_t)t * top + k], to_float(y[row * H + i]), acc);
+            acc = fmaf(wts[(size_t)t * top + k], to_float(y[row * H + i]), acc);
         }
         if (shared) acc += to_float(shared[(size_t)t * H + i]);
         out[(size_t)t * H + i] = from_float<T>(acc);
@@ -574,12 +579,14 @@ extern "C" int moe_pair_ff(const void* x, const void* w_gate_up, void* act, cons
 
 // ----------------------------------------------------------------------------- many pairs: rows gathered for the grouped products on tcgen05
 // xs[i] = x[order[i] / top] for the `sorted` pairs that stand in an expert's stretch (offsets[E]: behind them `order` holds
-// nothing); 16 bytes a thread, H * element size a multiple of 16.
+// nothing); 16 bytes a thread, H * element size a multiple of 16.  `zeros`: a row that is cleared on the way.
 __global__ void __launch_bounds__(256)
 moe_gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, const int* __restrict__ order,
-                       const int* __restrict__ sorted, int top, int chunks) {
+                       const int* __restrict__ sorted, int top, int chunks, uint4* __restrict__ zeros, int zero_chunks) {
     pdl_launch_dependents();
     pdl_wait();
+    if (blockIdx.x == 0)
+        for (int c = threadIdx.x; c < zero_chunks; c += blockDim.x) zeros[c] = make_uint4(0, 0, 0, 0);
     const int i = blockIdx.x, pair = order[i];  // (both loads at once; what `order` holds behind the last stretch is not used)
     if (i >= *sorted) return;
     const uint4* src = x + (size_t)(pair / top) * chunks;
@@ -587,9 +594,9 @@ moe_gather_rows_kernel(const uint4* __restrict__ x, uint4* __restrict__ xs, cons
 }
 
 extern "C" int moe_gather_rows(const void* x, void* xs, const int* order, const int* sorted, int T, int top, int row_bytes,
-                               cudaStream_t stream) {
+                               void* zeros, int zero_bytes, cudaStream_t stream) {
     if (T <= 0) return 0;
-    if (row_bytes % 16) return (int)cudaErrorInvalidValue;
+    if (row_bytes % 16 || zero_bytes % 16) return (int)cudaErrorInvalidValue;
     return (int)launch_kernel(moe_gather_rows_kernel, T * top, 256, 0, stream, (const uint4*)x, (uint4*)xs, order, sorted, top,
-                              row_bytes / 16);
+                              row_bytes / 16, (uint4*)zeros, zero_bytes / 16);
 }

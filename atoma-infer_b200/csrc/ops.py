@@ -1166,8 +1166,10 @@ class CudaOps:
             # host round trip), the shared expert's rows as one more stretch
             xs = torch.empty((pairs, H), dtype=h.dtype, device=dev)
             wide = pairs < self.MOE_ROUNDED_ROWS
-            y = torch.empty((pairs, H), dtype=torch.float32 if wide else h.dtype, device=dev)
-            self._check(lib.moe_gather_rows(_p(h), _p(xs), _p(order), _p(offsets[E:]), T, top, H * 2, self._stream()), "moe_gather_rows")
+            rows = torch.empty((pairs + 1, H), dtype=torch.float32 if wide else h.dtype, device=dev)
+            y = rows[1:]  # (a choice that names no expert stands at -1: the row of zeros ahead)
+            self._check(lib.moe_gather_rows(_p(h), _p(xs), _p(order), _p(offsets[E:]), T, top, H * 2, _p(rows), H * rows.element_size(),
+                                            self._stream()), "moe_gather_rows")
             ws_gate_up, ws_down = shared_weights or (None, None)
             act_s = None
             if ws_down is not None:
