@@ -1092,12 +1092,12 @@ class CudaOps:
         """Whether a step's selective scan runs in one pass (kernels/selective_prompt.cuh): where its estimated time is the shorter
         one.  It takes 0.0375 us a token of the longest entry, or, with more blocks of 32 channels than multiprocessors, their share
         of all tokens and 2.2 us an entry, with 8 states as with 16; the scan cut in chunks of time 36 us, 1.2 an entry and two passes
-        over everything, whose work follows the states; the one in order (steps of short entries) 0.4 us a token of the longest (0.35 with 8
-        states).  Measured, us, one pass / the other, bfloat16 (float32 within 5 %), channels x tokens, 16 states: 4096 x 2048 80 / 156,
+        over everything, whose work follows the states; the one in order (steps of short entries) 4 us and 0.37 a token of the longest (3 and 0.33
+        with 8 states), a third more for every further 20,000 channels of all entries.  Measured, us, one pass / the other, bfloat16 (float32 within 5 %), channels x tokens, 16 states: 4096 x 2048 80 / 156,
         8192 x 2048 160 / 285, 2048 x 2048 79 / 96, 1024 x 3000 115 / 82, 1024 x 1000 41 / 50, 4096 x 64 6 / 27, 4096 x 16 5 / 10; 8 states:
         4096 x 2048 79 / 119, 2048 x 2048 78 / 72, 1024 x 3000 114 / 64, 1024 x 1000 40 / 43, 4096 x 64 6 / 24; 4096 channels and 16 (8)
         states, 128 tokens beside 20 single ones 47 / 72 (48 / 52), 1,000 beside 40 114 / 267 (116 / 140), 8 x 16 25 / 13 (24 / 10), 8 x 64
-        32 / 33 (31 / 28)."""
+        32 / 33 (31 / 28), 3 x 20 12.0 / 12.0 (12.1 / 10.3); 6144 channels, 2 x 16 11.4 / 10.2 (11.2 / 8.6), 67, 75 and 46 21 / 33 (21 / 28)."""
         longest = ctx.max_tokens_per_entry
         if self.selective_prompt is not None:
             return self.selective_prompt
@@ -1107,7 +1107,8 @@ class CudaOps:
         one_pass = 3.0 + max(0.0375 * longest, share * (2.2 * ctx.S + 0.0375 * ctx.T))
         if longest >= self.SCAN_CHUNK_FROM:
             return one_pass < 36.0 + 1.2 * ctx.S + (0.5 + 0.058 * nstate) * 1e-5 * work
-        return one_pass < 6.0 + max((0.3 + 0.00625 * nstate) * longest, 1.1e-5 * work)
+        waves = 1.0 + 0.35 * max(0.0, ctx.S * inner / 20000 - 1.0)
+        return one_pass < 2.0 + nstate / 8 + max((0.296 + 0.0046 * nstate) * longest * waves, 1.1e-5 * work)
 
     def moe_route(self, h, w_router, ids, wts, meta, bias=None, over_chosen: bool = False):
         """Per token: float32 logits w_router h (+ ``bias``, float32 [experts]), softmax over all experts, the ids.shape[1]

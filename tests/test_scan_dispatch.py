@@ -71,7 +71,8 @@ def test_selective_scans_of_float32_go_in_order_below_the_chunks_of_time(dtype, 
 
 @pytest.mark.parametrize("nstate,inner,lengths,one_pass", [
     (16, 2048, [2048], True), (8, 2048, [2048], False), (8, 4096, [2048], True), (16, 1024, [3000], False), (8, 1024, [1000], True),
-    (16, 4096, [128] + [1] * 20, True), (8, 4096, [1000] + [1] * 40, True), (16, 4096, [16] * 8, False), (8, 4096, [64] * 8, False)])
+    (16, 4096, [128] + [1] * 20, True), (8, 4096, [1000] + [1] * 40, True), (16, 4096, [16] * 8, False), (8, 4096, [64] * 8, False),
+    (16, 6144, [16] * 2, False), (8, 4096, [20] * 3, False), (8, 6144, [67, 75, 46], True), (16, 4096, [16], True)])
 def test_selective_scans_in_one_pass_where_that_was_measured_to_be_shorter(nstate, inner, lengths, one_pass):
     ops = SimpleNamespace(selective_prompt=None, num_sms=148, SCAN_CHUNK_FROM=CudaOps.SCAN_CHUNK_FROM)
     ctx = SimpleNamespace(T=sum(lengths), S=len(lengths), max_tokens_per_entry=max(lengths))
